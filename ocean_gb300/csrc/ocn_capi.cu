@@ -282,6 +282,7 @@ int ocn_ctx_create(const ocn_dims* d, ocn_ctx** out) {
   c->red_blocks = (int)std::min<size_t>(2 * (size_t)c->sm_count, std::max<size_t>(1, (c->npsi + 511) / 512));
   c->lr_xsplit = std::max(1, std::min((2 * c->sm_count + nk - 1) / nk, std::max(1, nx / 64)));
   int rc = OCN_OK;
+  if (d->precision == OCN_PREC_FP64 && (rc = slice_init(c))) return fail(rc);
   if ((rc = dev_alloc(c, &c->d_er, c->npsi)) || (rc = dev_alloc(c, &c->d_ei, c->npsi)) ||
       (rc = dev_alloc(c, &c->d_allow, c->npsi)) ||
       (rc = dev_alloc(c, &c->d_u, (size_t)c->nb * nk * nx * c->nspn)) ||
@@ -312,6 +313,7 @@ int ocn_ctx_destroy(ocn_ctx* c) {
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
   if (c->mixed) mixed_free(c);
+  slice_free(c);
   void* bufs[] = {c->d_er, c->d_ei, c->d_allow, c->d_u, c->d_W, c->d_tw, c->d_so, c->d_phi, c->d_acc,
                   c->d_accpart, c->d_vec, c->d_red, c->d_scal, c->mult.mpc, c->mult.mpm, c->mult.mh,
                   c->mult.p_l, c->mult.p_m, c->mult.p_nu, c->mult.d_pfirst, c->mult.d_nproj,
@@ -430,7 +432,7 @@ int ocn_lr_init(ocn_ctx* c, const ocn_lr_params* p) {
   c->have_bloch = true;
   c->have_W = true;
   if (c->dims.precision == OCN_PREC_MIXED) return mixed_set_bloch(c);
-  return OCN_OK;
+  return slice_set_bloch(c);
 }
 
 int ocn_set_W(ocn_ctx* c, const double* W) {
@@ -637,7 +639,7 @@ int ocn_apply_H(ocn_ctx* c, const double* ir, const double* ii, double* orr, dou
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   cudaFree(buf);
   if (e != cudaSuccess) return cuda_fail(c, e, "ocn_apply_H");
-  if (rc == OCN_OK && c->mixed) rc = mixed_check(c);
+  if (rc == OCN_OK) rc = tc_check(c);
   return rc;
 }
 
@@ -879,7 +881,7 @@ int haydock_finish(ocn_ctx* c, const HayRun& R, int done, bool graph_timing, dou
     (void)cudaGetLastError();  // a failed timing query must not poison later calls
   }
   int rc;
-  if (c->mixed && (rc = mixed_check(c))) return rc;
+  if ((rc = tc_check(c))) return rc;
   const size_t out1 = (size_t)R.niter + 1;
   for (int v = 0; v < R.nv; ++v)
     for (int i = 0; i <= R.niter; ++i) {
@@ -1208,7 +1210,7 @@ int ocn_apply_H_block(ocn_ctx* c, int nv, const double* ir, const double* ii, do
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   cudaFree(buf);
   if (e != cudaSuccess) return cuda_fail(c, e, "ocn_apply_H_block");
-  if (rc == OCN_OK && c->mixed) rc = mixed_check(c);
+  if (rc == OCN_OK) rc = tc_check(c);
   return rc;
 }
 
@@ -1324,7 +1326,7 @@ int ocn_haydock_nonherm(ocn_ctx* c, const double* psi0_r, const double* psi0_i, 
   cudaFree(pool);
   if (niter_done) *niter_done = done;
   if (rc == OCN_OK && e != cudaSuccess) rc = cuda_fail(c, e, "ocn_haydock_nonherm");
-  if (rc == OCN_OK && c->mixed) rc = mixed_check(c);
+  if (rc == OCN_OK) rc = tc_check(c);
   return rc;
 }
 

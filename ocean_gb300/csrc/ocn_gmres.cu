@@ -991,7 +991,7 @@ int gmres_solve(ocn_ctx* c, const double* d_rhs, double kpref, const double* eli
   op.H = [c, n](const double* in, double* out) { return apply_H_impl(c, in, in + n, out, out + n, nullptr, 0); };
   op.Hblock = [c](int nv, const double* in, double* out) { return apply_H_block_impl(c, nv, in, out, nullptr, 0); };
   op.err = [c](int code, const std::string& msg) { return set_err(c, code, msg); };
-  if (c->mixed) op.finish = [c]() { return mixed_check(c); };
+  op.finish = [c]() { return tc_check(c); };
   return gmres_solve_op(op, d_rhs, kpref, elist, nomega, p, nlanes, out_re, out_im, rel_err, iters, on_x, adjoint);
 }
 

@@ -19,6 +19,7 @@
 namespace ocn {
 
 struct MixedLR;  // split-BF16 / tcgen05 state (ocn_mixed.cu)
+struct SliceLR;  // digit-sliced FP64 contractions (ocn_slice.cu)
 
 // Strides between the vectors of a block of psi (chain v = blockIdx.y).
 struct BlockStrides {
@@ -135,6 +136,7 @@ struct ocn_ctx {
 
   ocn::MultDev mult;
   ocn::MixedLR* mixed = nullptr;
+  ocn::SliceLR* slice = nullptr;  // FP64 contexts
 
   ocn::Timing timing;
 
@@ -352,6 +354,15 @@ int conv_check_launch(ocn_ctx* c, const double* ra, const double* ia, const doub
 int cf_eval_noalloc(const double* ra, const double* ia, const double* rb, int iter, double kpref,
                     const ocn_cf_params* p, double* out, std::string* err);
 
+// ---- FP64 contractions on the tensor cores (ocn_slice.cu)
+int slice_init(ocn_ctx* c);        // geometry and vector-side buffers; sets lr_xsplit
+void slice_free(ocn_ctx* c);
+int slice_set_bloch(ocn_ctx* c);   // digit operands from d_u (not ready when they do not fit)
+bool slice_ready(const ocn_ctx* c);
+int slice_band_to_x(ocn_ctx* c, const double* d_pr, const double* d_pi, double2* phi);  // phi[k][x][a]
+int slice_x_to_band(ocn_ctx* c, const double2* phi);  // d_accpart slices from phi'[k][x][a]
+int slice_check(ocn_ctx* c);       // reads and clears the device timeout flag
+
 // ---- mixed precision (ocn_mixed.cu)
 int mixed_init(ocn_ctx* c);
 int mixed_free(ocn_ctx* c);
@@ -372,6 +383,7 @@ int haydock_to_df(ocn_ctx* c, double* buf, int nv);
 int mixed_norm_prep(ocn_ctx* c, int nv, const double* psi, double* h, double* ra, double* ia, double* rb,
                     size_t cstride, const int* itp);
 int mixed_check(ocn_ctx* c);       // reads and clears the device timeout flag
+inline int tc_check(ocn_ctx* c) { return c->mixed ? mixed_check(c) : (slice_ready(c) ? slice_check(c) : OCN_OK); }
 int mixed_set_starve(ocn_ctx* c, int on);  // test hook of ocn_test_starve_tc
 // multiplet on the tensor cores: operands from c->mult (after ocn_set_mult), and
 // the action's multiplet term of nv vectors into its d_accpart slices

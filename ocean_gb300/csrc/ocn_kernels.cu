@@ -1024,7 +1024,10 @@ int zero_acc(ocn_ctx* c, int nv) {
 
 int lr_apply_fp64(ocn_ctx* c, const double* d_pr, const double* d_pi) {
   const int nb = c->nb, nk = c->nk, nx = c->nx, na = c->na;
-  {
+  const bool sliced = slice_ready(c);
+  if (sliced) {
+    if (int rc = slice_band_to_x(c, d_pr, d_pi, c->d_phi)) return rc;
+  } else {
     const size_t sm = sizeof(double2) * ((size_t)c->nspn * G1_N * (G1_X + 1) + (size_t)na * G1_N);
     dim3 grid((nx + G1_X - 1) / G1_X, nk);
     TimedScope ts(c, T_LR_GEMM1);
@@ -1046,6 +1049,7 @@ int lr_apply_fp64(ocn_ctx* c, const double* d_pr, const double* d_pi) {
     ++c->launches;
     OCN_CUDA(c, cudaGetLastError());
   }
+  if (sliced) return slice_x_to_band(c, c->d_phi);
   {
     const int xs = c->lr_xsplit;
     const int xper = (nx + xs - 1) / xs;
@@ -1071,12 +1075,17 @@ int lr_wgrad_fp64(ocn_ctx* c, const double* x, const double* y, double2* phi, do
   const size_t n = c->npsi;
   double2* phx = phi;
   double2* phy = phi + (size_t)nk * nx * na;
-  const size_t sm = sizeof(double2) * ((size_t)c->nspn * G1_N * (G1_X + 1) + (size_t)na * G1_N);
-  const dim3 grid((nx + G1_X - 1) / G1_X, nk);
-  k_lr_gemm1_fp64<<<grid, G1_X, sm, c->stream>>>(c->d_u, x, x + n, c->d_allow, phx, nb, nk, nx, na, c->nspn);
-  k_lr_gemm1_fp64<<<grid, G1_X, sm, c->stream>>>(c->d_u, y, y + n, c->d_allow, phy, nb, nk, nx, na, c->nspn);
-  c->launches += 2;
-  OCN_CUDA(c, cudaGetLastError());
+  if (slice_ready(c)) {
+    int rc;
+    if ((rc = slice_band_to_x(c, x, x + n, phx)) || (rc = slice_band_to_x(c, y, y + n, phy))) return rc;
+  } else {
+    const size_t sm = sizeof(double2) * ((size_t)c->nspn * G1_N * (G1_X + 1) + (size_t)na * G1_N);
+    const dim3 grid((nx + G1_X - 1) / G1_X, nk);
+    k_lr_gemm1_fp64<<<grid, G1_X, sm, c->stream>>>(c->d_u, x, x + n, c->d_allow, phx, nb, nk, nx, na, c->nspn);
+    k_lr_gemm1_fp64<<<grid, G1_X, sm, c->stream>>>(c->d_u, y, y + n, c->d_allow, phy, nb, nk, nx, na, c->nspn);
+    c->launches += 2;
+    OCN_CUDA(c, cudaGetLastError());
+  }
   WgradFnD f = wgrad_fn(c->dims.kmesh[0]);
   const size_t wsm = kmesh_cube_smem<double>(c->dims.kmesh[0], 2 * na);
   if (int rc_ = allow_max_smem(c, f)) return rc_;

@@ -44,6 +44,7 @@
 #include "ocn_df.cuh"
 #include "ocn_internal.h"
 #include "ocn_kmesh_dft.cuh"
+#include "ocn_tc.cuh"
 
 namespace ocn {
 
@@ -54,7 +55,6 @@ constexpr int TC_BM = 128;
 constexpr int TC_BK = 64;  // bf16 elements per 128-byte swizzle row
 constexpr int TC_THREADS = 192;
 constexpr int TC_MAX_NCOL = 256;  // MMA N limit for M = 128
-constexpr long long TC_WAIT_CYCLES = 2000000000LL;  // ~1 s at 2 GHz
 constexpr size_t TC_SMEM_BUDGET = 220 * 1024;
 
 
@@ -92,42 +92,6 @@ struct TcGroupMaps {
   CUtensorMap m[TC_GROUP_MAX][3];  // A hi, A lo, B
 };
 
-__device__ __forceinline__ uint32_t su32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Bounded wait: false when the time limit passed or another role aborted.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          long long limit) {
-  const long long t0 = clock64();
-  while (!mbar_test(bar, parity)) {
-    if (*abort_flag) return false;
-    if (clock64() - t0 > limit) return false;
-  }
-  return true;
-}
-
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0,
                                             int c1, int c2) {
   asm volatile(
@@ -144,13 +108,6 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
       " [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(dst),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
       : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() {
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
 // K-major operand tile with 128-byte swizzling: rows of 128 bytes, 8-row core
@@ -177,11 +134,6 @@ __device__ __forceinline__ void umma_bf16(uint32_t dtmem, uint64_t adesc, uint64
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-               : "memory");
-}
-
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   uint32_t r[16];
   asm volatile(
@@ -194,8 +146,6 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
 struct TileInfo {
   int k, row0, c0, c1, mt, sp;
 };

@@ -1,0 +1,898 @@
+// ocn_slice.cu -- the FP64 contractions of the BSE action on the FP8 tensor cores.
+//
+//   phi(k,x,t)    = sum_n u(n,k,x) q(n,k,t)              (band -> x)
+//   part(n,k,t)   = - sum_x conj(u(n,k,x)) phi'(k,x,t)   (x -> band)
+//
+// GB300 issues FP64 at 2 fused multiply-adds per clock and SM, so on the FP64
+// pipe these two sums cost 4.3 and 5.9 ms on the 8^3 k / 100-band / 12^3 x case
+// while their operands could be read in 0.2 ms.  Here every operand row (a row of
+// u over the summed index, a column of q or phi') is written as a binary fixed
+// point number of 60 bits against the largest exponent of the row, cut into
+// S = 12 signed base-32 digits (|d| <= 16, exact in E4M3), and
+//   sum a b = 2^(ea + eb - 118) sum_(i,j) 32^(22-i-j) sum_K d_i(a) d_j(b)
+// is formed on the tensor cores.  |d_i d_j| <= 256, so the FP32 accumulator of a
+// group i + j is an exact integer while K * pairs * 256 <= 2^24 (checked where
+// the K splits are chosen); the groups i + j <= 11 are added in 64-bit integers
+// and rounded to binary64 once.  What is left out (digits below 2^-60 of a row's
+// largest element, pairs with i + j > 11) is below the rounding error of an FP64
+// sum: 2-norm error 5e-17 against 3e-16 (100 bands) and 1.4e-15 (1728 x-points)
+// for binary64 multiply-adds on Gaussian rows, and still below it for rows that
+// spread over six decades (with S = 11 it is not).  The sums are exact, so results
+// do not depend on tiling, splits or the number of vectors sharing a launch.
+//
+// Layout.  The digits of u are stored in the order in which the kernel consumes
+// them, as no-swizzle K-major core matrices ([granule of 16 K][row][16 bytes]), so
+// every pipeline stage is one contiguous bulk copy:
+//   A[spin][k][row tile of 128][K chunk][box][granule][row][16]
+// box = slice (band -> x: K runs over re n then im n) or plane * 12 + slice (x ->
+// band: re and im planes of u, K over x).  12 bytes per real against 8 for FP64.
+// The vector side is small and rebuilt per action:
+//   B[k][granule][part][slice][column][16]
+// In shared memory each granule's digit rows follow 11 empty slices, so the
+// operand of slice i of A is the same buffer read from row (11 - i) C: its digit j
+// meets output column group i + j, and one MMA of N = 12 C columns per (slice, 32
+// K) adds every pair of that slice.  part: re/im columns; both in one MMA when
+// 24 C' <= 256 (band -> x of up to two 1s vectors), else one MMA per part (x ->
+// band swaps the parts between the planes and negates A for the last of the four).
+// The kernel is persistent and warp-specialised like k_lr_tc; CTAs take
+// contiguous tile ranges so that the B operand of a k-point is read once.
+//
+// Measured, 8^3 k / 100 bands / 12^3 x, 1s: band -> x 4.3 ms on the FP64 pipe ->
+// 0.331 ms (2.2 GB, 6.7 TB/s), x -> band 5.9 ms -> 0.355 ms (6.2 TB/s): bound by
+// the read of A.  2p, 6^3 k / 64 bands / 10^3 x (12 columns): 0.093 and 0.123 ms
+// (3.6 and 2.5 TB/s): there the 144-column MMAs (72 cycles) and the epilogue's
+// 288 integer columns per row weigh as much as the 0.3 GB read.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
+#include <new>
+#include <string>
+
+#include "ocn_internal.h"
+#include "ocn_tc.cuh"
+
+namespace ocn {
+
+namespace {
+
+constexpr int SL_S = 12;           // digits per value
+constexpr int SL_FRAC = 59;        // fixed point: t = v 2^(59 - e), |v| < 2^e
+constexpr int SL_ROWS = 128;       // rows per tile (MMA M)
+constexpr int SL_THREADS = 192;
+constexpr int SL_MAX_STAGES = 8;
+constexpr size_t SL_SMEM = 222 * 1024;
+constexpr int SL_NAN = 0x40000000;  // exponent of a row that holds an Inf or NaN
+constexpr int SL_MAX_K = 2730;      // K per plane and accumulation: 2 * 2730 * 12 * 256 < 2^24
+constexpr unsigned long long SL_BIAS = 0x0842108421084210ull;  // sum of 16 * 32^i, i < 12
+
+struct SliceParams {
+  const uint8_t *A, *B;
+  const int *eA, *eB;
+  int nk, rows, nt, rl, R;   // rows of A per k; row tiles; rows of the last tile and of a k-point (multiples of 8)
+  int G, Ge, KC, nch;        // 16-wide K granules (A; B padded to even), granules per chunk, chunks
+  int ks, cps;               // K splits, chunks per split
+  int ntiles, stages;
+  int bshared, koff, spin;   // B one k slice for all k; added to k for A; -1 or the spin whose columns are written
+  int na, nvw;               // channels per vector; vectors written
+  double2* phi;              // band -> x: [k][row][t]
+  double* part;              // x -> band: [split][vector][re|im][npsi]
+  size_t part_stride, npsi;
+  int nb;
+  int* err;
+};
+
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+// K-major operand without swizzling: 8-row core matrices of 128 bytes (stride
+// byte offset 128), consecutive 16-byte K granules lbo bytes apart.
+// Low word of the descriptor; addresses stay below 2^18, so adding (bytes >> 4)
+// moves the start address.  The high word is the same for every operand.
+__device__ __forceinline__ uint32_t plain_desc(uint32_t saddr, uint32_t lbo) {
+  return ((saddr >> 4) & 0x3FFFu) | ((lbo >> 4) << 16);
+}
+constexpr uint32_t PLAIN_DESC_HI = (128 >> 4) | (1u << 14);
+__device__ __forceinline__ void umma_fp8(uint32_t dtmem, uint32_t adesc, uint32_t bdesc, uint32_t idesc,
+                                         uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
+      "mov.b64 a, {%1, %5};\n\t"
+      "mov.b64 b, {%2, %5};\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, p;\n\t}" ::"r"(dtmem),
+      "r"(adesc), "r"(bdesc), "r"(idesc), "r"(accumulate), "r"(PLAIN_DESC_HI)
+      : "memory");
+}
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+  return ok != 0;
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
+  uint32_t r[8];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// r 2^e for a finite r (r = 0 allowed)
+__device__ __forceinline__ double scale_pow2(double r, int e) {
+  const int hw = __double2hiint(r);
+  const int ne = ((hw >> 20) & 0x7ff) + e;
+  if (ne > 0 && ne < 2047 && (hw & 0x7ff00000)) return __hiloint2double(hw + (e << 20), __double2loint(r));
+  return ldexp(r, e);
+}
+
+// Six accumulator groups (most significant first) of C columns as integers.
+template <int C>
+__device__ __forceinline__ void add_groups(uint32_t ta, long long (&acc)[C]) {
+  float v[6 * C];
+#pragma unroll
+  for (int c = 0; c < 6 * C; c += 8) tmem_ld8(ta + c, v + c);
+  tmem_ld_wait();
+#pragma unroll
+  for (int c = 0; c < C; ++c) acc[c] = 0;
+#pragma unroll
+  for (int g = 0; g < 6; ++g)
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+      acc[c] += (long long)__float2int_rn(v[g * C + c]) * (long long)(1 << (5 * (5 - g)));
+}
+
+struct SliceTile {
+  int k, mt, sp, c0, c1, rt;
+};
+template <int MODE>
+__device__ __forceinline__ SliceTile slice_decode(const SliceParams& p, int t) {
+  SliceTile ti;
+  const int per_k = p.nt * p.ks;
+  ti.k = t / per_k;
+  const int r = t - ti.k * per_k;
+  ti.mt = r / p.ks;
+  ti.sp = r - ti.mt * p.ks;
+  ti.c0 = ti.sp * p.cps;
+  ti.c1 = min(p.nch, ti.c0 + p.cps);
+  ti.rt = ti.mt == p.nt - 1 ? p.rl : SL_ROWS;
+  return ti;
+}
+
+// MODE 1: band -> x (K = re n, im n stacked; B columns carry the signs of the
+// complex product).  MODE 2: x -> band (two planes).  C columns per slice and
+// MMA, P MMAs (parts) per K step.
+template <int MODE, int C, int P>
+__global__ void __launch_bounds__(SL_THREADS, 1) k_slice_gemm(const __grid_constant__ SliceParams p) {
+  constexpr int NAE = P == 1 ? C / 2 : C;        // complex columns
+  constexpr int NBOX = MODE == 1 ? SL_S : 2 * SL_S;
+  constexpr int N = SL_S * C;                    // MMA N
+  constexpr int PL = MODE == 2 && P == 1 ? 2 : 1;  // accumulators of their own per plane
+  constexpr int DCOLS = P * PL * N;
+  constexpr int ACC = 2 * DCOLS <= 512 ? 2 : 1;
+  constexpr uint32_t TCOLS = ACC * DCOLS <= 128 ? 128 : (ACC * DCOLS <= 256 ? 256 : 512);
+  constexpr uint32_t PROWS = 23 * C;             // 11 empty slices, 12 digit slices
+  constexpr uint32_t PITCH = P * PROWS * 16;     // bytes of a granule of B in shared memory
+  constexpr uint32_t IDESC0 = (1u << 4) | ((uint32_t)(SL_ROWS >> 4) << 24);
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const int S = p.stages;
+  const uint32_t slot_bytes = p.KC * PITCH, stage_bytes = p.KC * SL_ROWS * 16;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * slot_bytes + S * stage_bytes);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * SL_MAX_STAGES + 8);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const uint32_t b_smem = su32(smem), a_smem = b_smem + 2 * slot_bytes;
+  const uint32_t full0 = su32(bars), empty0 = full0 + 8 * SL_MAX_STAGES;
+  const uint32_t bfull0 = empty0 + 8 * SL_MAX_STAGES, bempty0 = bfull0 + 16, tfull0 = bempty0 + 16, tempty0 = tfull0 + 16;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  const int t0 = (int)((long long)p.ntiles * blockIdx.x / gridDim.x);
+  const int t1 = (int)((long long)p.ntiles * (blockIdx.x + 1) / gridDim.x);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S; ++s) {
+      mbar_init(full0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(bfull0 + 8 * b, 1);
+      mbar_init(bempty0 + 8 * b, 1);
+      mbar_init(tfull0 + 8 * b, 1);
+      mbar_init(tempty0 + 8 * b, 128);
+    }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(tmem_slot)), "r"(TCOLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  {  // the empty slices of B stay zero; A stages too when an odd granule count leaves one that is never
+     // written (it meets zero digits, but must hold finite ones)
+    const uint32_t zb = 2 * slot_bytes + ((p.G & 1) ? S * stage_bytes : 0);
+    for (uint32_t i = threadIdx.x * 16; i < zb; i += SL_THREADS * 16)
+      *reinterpret_cast<uint4*>(smem + i) = make_uint4(0, 0, 0, 0);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const bool keepb = p.nch == 1;  // one chunk: B stays while k does
+
+  if (warp == 0) {
+    // -------------------------------------------------------------- producer
+    uint32_t stage = 0, phase = 0, slot = 0, bphase = 0;
+    int armed[SL_MAX_STAGES], barmed[2] = {-1, -1};
+#pragma unroll
+    for (int s = 0; s < SL_MAX_STAGES; ++s) armed[s] = -1;
+    bool ok = true;
+    int lastk = -1;
+    for (int t = t0; t < t1 && ok; ++t) {
+      const SliceTile ti = slice_decode<MODE>(p, t);
+      const uint8_t* At = p.A + ((size_t)(ti.k + p.koff) * p.R + (size_t)SL_ROWS * ti.mt) * 16 * p.G * NBOX;
+      const uint8_t* Bk = p.B + (p.bshared ? 0 : (size_t)ti.k) * p.Ge * (P * N * 16);
+      for (int c = ti.c0; c < ti.c1 && ok; ++c) {
+        const int gc = min(p.KC, p.G - c * p.KC), gce = (gc + 1) & ~1;
+        if (!keepb || ti.k != lastk) {
+          ok = mbar_wait(bempty0 + 8 * slot, bphase ^ 1, abort_flag, TC_WAIT_CYCLES);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          if (lane == 0) mbar_expect_tx(bfull0 + 8 * slot, (uint32_t)gce * P * N * 16);
+          __syncwarp();
+          const uint8_t* src = Bk + (size_t)c * p.KC * (P * N * 16);
+          for (int i = lane; i < gce * P; i += 32)
+            bulk_load(b_smem + slot * slot_bytes + (i / P) * PITCH + ((i % P) * PROWS + 11 * C) * 16,
+                      src + (size_t)i * (N * 16), N * 16, bfull0 + 8 * slot);
+          barmed[slot] = (int)bphase;
+          slot ^= 1;
+          if (slot == 0) bphase ^= 1;
+          lastk = ti.k;
+        }
+        const uint32_t bytes = (uint32_t)gc * ti.rt * 16;
+        const uint8_t* src = At + (size_t)c * p.KC * ti.rt * 16 * NBOX;
+        for (int b = 0; b < NBOX; ++b) {
+          ok = mbar_wait(empty0 + 8 * stage, phase ^ 1, abort_flag, TC_WAIT_CYCLES);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          if (lane == 0) {
+            mbar_expect_tx(full0 + 8 * stage, bytes);
+            bulk_load(a_smem + stage * stage_bytes, src + (size_t)b * bytes, bytes, full0 + 8 * stage);
+          }
+          armed[stage] = (int)phase;
+          if (++stage == (uint32_t)S) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+      }
+    }
+    if (!ok && lane == 0) {
+      *abort_flag = 1;
+      atomicOr(p.err, 1);
+    }
+    // drain: never leave a bulk copy in flight
+    for (int s = 0; s < S; ++s)
+      if (armed[s] >= 0) {
+        const long long w0 = clock64();
+        while (!mbar_test(full0 + 8 * s, (uint32_t)armed[s]) && clock64() - w0 < TC_WAIT_CYCLES) {
+        }
+      }
+    for (int s = 0; s < 2; ++s)
+      if (barmed[s] >= 0) {
+        const long long w0 = clock64();
+        while (!mbar_test(bfull0 + 8 * s, (uint32_t)barmed[s]) && clock64() - w0 < TC_WAIT_CYCLES) {
+        }
+      }
+  } else if (warp == 1) {
+    // -------------------------------------------------------------- MMA issuer
+    // the whole warp runs the (warp-uniform) loop, one elected lane issues
+    uint32_t stage = 0, phase = 0, slot = 0, bphase = 0, acc = 0, acc_phase = 0;
+    int last_stage = -1;
+    uint32_t last_phase = 0;
+    bool ok = true;
+    int lastk = -1;
+    const bool leader = elect_one();
+    for (int t = t0; t < t1 && ok; ++t) {
+      const SliceTile ti = slice_decode<MODE>(p, t);
+      ok = __all_sync(0xffffffffu, mbar_wait(tempty0 + 8 * acc, acc_phase ^ 1, abort_flag, TC_WAIT_CYCLES));
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t dt = tmem_base + acc * DCOLS;
+      const uint32_t lba = (uint32_t)ti.rt * 16;
+      for (int c = ti.c0; c < ti.c1 && ok; ++c) {
+        const int gc = min(p.KC, p.G - c * p.KC), steps = (gc + 1) >> 1;
+        if (!keepb || ti.k != lastk) {
+          ok = __all_sync(0xffffffffu, mbar_wait(bfull0 + 8 * slot, bphase, abort_flag, TC_WAIT_CYCLES));
+          if (!ok) break;
+          lastk = ti.k;
+        }
+        for (int b = 0; b < NBOX; ++b) {
+          ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * stage, phase, abort_flag, TC_WAIT_CYCLES));
+          if (!ok) break;
+          tc_fence_after();
+          const int plane = b / SL_S, i = b - plane * SL_S;
+          uint32_t ad = plain_desc(a_smem + stage * stage_bytes, lba);
+          // the first i column groups of slice i only meet empty slices: N shrinks in steps of 16
+          const uint32_t ni = (uint32_t)((SL_S - i) * C + 15) & ~15u, off = N - ni;
+          const uint32_t idesc = IDESC0 | ((ni >> 3) << 17);
+          uint32_t bd = plain_desc(b_smem + slot * slot_bytes + ((11 - i) * C + off) * 16, PITCH);
+          const uint32_t d0 = dt + (PL == 2 ? plane * N : 0) + off;
+          // the first MMA of an accumulator overwrites it
+          uint32_t accum = (c > ti.c0 || (PL == 2 ? i > 0 : b > 0)) ? 1u : 0u;
+          if (leader) {
+#pragma unroll 4
+            for (int g = 0; g < steps; ++g) {
+#pragma unroll
+              for (int q = 0; q < P; ++q) {
+                const uint32_t part = MODE == 2 ? (uint32_t)(q ^ plane) : (uint32_t)q;  // im plane: parts swapped
+                const uint32_t neg = (MODE == 2 && P == 2 && q == 1 && plane == 1) ? (1u << 13) : 0u;
+                umma_fp8(d0 + q * N, ad, bd + (P == 2 ? part * PROWS : 0u), idesc | neg, accum);
+              }
+              accum = 1u;
+              ad += 2 * (lba >> 4);
+              bd += 2 * (PITCH >> 4);
+            }
+            umma_commit(empty0 + 8 * stage);
+          }
+          __syncwarp();
+          last_stage = (int)stage;
+          last_phase = phase;
+          if (++stage == (uint32_t)S) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+        if (!ok) break;
+        if (!keepb || t + 1 == t1 || slice_decode<MODE>(p, t + 1).k != ti.k) {
+          if (leader) umma_commit(bempty0 + 8 * slot);
+          slot ^= 1;
+          if (slot == 0) bphase ^= 1;
+        }
+      }
+      if (!ok) break;
+      if (leader) umma_commit(tfull0 + 8 * acc);
+      if (ACC == 2) acc ^= 1;
+      if (acc == 0) acc_phase ^= 1;
+    }
+    if (!ok && leader) {
+      *abort_flag = 1;
+      atomicOr(p.err, 2);
+    }
+    if (last_stage >= 0) {  // drain: every issued MMA finished reading shared memory
+      const long long w0 = clock64();
+      while (!mbar_test(empty0 + 8 * last_stage, last_phase) && clock64() - w0 < TC_WAIT_CYCLES) {
+      }
+    }
+  } else {
+    // -------------------------------------------------------------- epilogue
+    const int q4 = warp & 3;  // tensor-memory lane quadrant of this warp
+    const int row = q4 * 32 + lane;
+    uint32_t acc = 0, acc_phase = 0;
+    for (int t = t0; t < t1; ++t) {
+      const SliceTile ti = slice_decode<MODE>(p, t);
+      if (!mbar_wait(tfull0 + 8 * acc, acc_phase, abort_flag, TC_WAIT_CYCLES)) {
+        *abort_flag = 1;
+        atomicOr(p.err, 4);
+        break;
+      }
+      tc_fence_after();
+      const uint32_t ta = tmem_base + ((uint32_t)(q4 * 32) << 16) + acc * DCOLS;
+      long long hi[P][C], lo[P][C];
+#pragma unroll
+      for (int q = 0; q < P; ++q) {
+        add_groups<C>(ta + q * N, hi[q]);
+        add_groups<C>(ta + q * N + 6 * C, lo[q]);
+      }
+      if (PL == 2) {  // out = (re plane) phi' - i (im plane) phi'
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          long long (&o)[C] = h ? lo[0] : hi[0];
+          long long im[C];
+          add_groups<C>(ta + N + h * 6 * C, im);
+#pragma unroll
+          for (int a = 0; a < NAE; ++a) {
+            o[a] += im[(NAE + a) % C];
+            o[(NAE + a) % C] -= im[a];
+          }
+        }
+      }
+      tc_fence_before();
+      mbar_arrive(tempty0 + 8 * acc);
+      if (ACC == 2) acc ^= 1;
+      if (acc == 0) acc_phase ^= 1;
+      const int r = ti.mt * SL_ROWS + row;
+      if (r < p.rows) {
+        const int ea = p.eA[(size_t)(ti.k + p.koff) * p.rows + r];
+        const int* eb = p.eB + (p.bshared ? 0 : (size_t)ti.k) * NAE;
+#pragma unroll
+        for (int a = 0; a < NAE; ++a) {
+          if (p.spin >= 0 && (a & 1) != p.spin) continue;
+          const int e = eb[a];
+          constexpr int im0 = P == 1 ? NAE : 0;  // merged parts: im columns follow the re columns
+          double vr = fma((double)hi[0][a], 1073741824.0, (double)lo[0][a]);
+          double vi = fma((double)hi[P - 1][im0 + a], 1073741824.0, (double)lo[P - 1][im0 + a]);
+          if (ea == SL_NAN || e == SL_NAN) {
+            vr = vi = __longlong_as_double(0x7ff8000000000000ll);
+          } else {
+            vr = scale_pow2(vr, ea + e - 2 * SL_FRAC + 55);
+            vi = scale_pow2(vi, ea + e - 2 * SL_FRAC + 55);
+          }
+          if (MODE == 1) {
+            p.phi[((size_t)ti.k * p.rows + r) * NAE + a] = make_double2(vr, vi);
+          } else {
+            const int v = a / p.na;
+            double* out = p.part + (size_t)ti.sp * p.part_stride + (size_t)v * 2 * p.npsi;
+            const size_t idx = (size_t)r + (size_t)p.nb * ((size_t)ti.k + (size_t)p.nk * (a - v * p.na));
+            out[idx] = -vr;
+            out[p.npsi + idx] = -vi;
+          }
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TCOLS) : "memory");
+  }
+}
+
+// ------------------------------------------------------------- digit operands
+
+__device__ __forceinline__ unsigned exp_bits(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
+// exponent e of a row from the largest high word of its values: |v| < 2^e
+__device__ __forceinline__ int row_exp(unsigned hw) {
+  const int E = (int)(hw >> 20);
+  return E == 0x7ff ? SL_NAN : E - 1022;
+}
+// v 2^(59 - e) rounded to an integer, plus the digit bias (e = SL_NAN: zero digits)
+__device__ __forceinline__ unsigned long long fix_point(double v, int e) {
+  const long long b = __double_as_longlong(v);
+  const int ev = (int)((b >> 52) & 0x7ff);
+  unsigned long long m = (unsigned long long)b & 0xfffffffffffffull;
+  if (ev) m |= 1ull << 52;
+  const int s = max(ev, 1) - 1075 + SL_FRAC - e;
+  unsigned long long t = 0;
+  if (s >= 0) t = m << min(s, 6);  // s <= 6: |v| < 2^e
+  else if (s > -54) t = (m + (1ull << (-s - 1))) >> (-s);
+  if (e == SL_NAN) t = 0;
+  return SL_BIAS + (b < 0 ? 0ull - t : t);
+}
+// digit s (0 most significant) of a biased fixed-point value as an exact float
+__device__ __forceinline__ float digit_of(unsigned long long t, int s) {
+  unsigned r = (unsigned)(t >> (5 * (SL_S - 1 - s)));
+  if (s) r &= 31u;
+  return __int_as_float((int)(0x4B000000u | r)) - 8388624.0f;
+}
+__device__ __forceinline__ unsigned fp8x4(float a, float b, float c, float d) {
+  unsigned short lo, hi;
+  asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(lo) : "f"(b), "f"(a));
+  asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(hi) : "f"(d), "f"(c));
+  return (unsigned)lo | ((unsigned)hi << 16);
+}
+__device__ __forceinline__ unsigned digits4(const unsigned long long* t, int s) {
+  return fp8x4(digit_of(t[0], s), digit_of(t[1], s), digit_of(t[2], s), digit_of(t[3], s));
+}
+__device__ __forceinline__ uint4 digits16(const unsigned long long* t, int s) {
+  return make_uint4(digits4(t, s), digits4(t + 4, s), digits4(t + 8, s), digits4(t + 12, s));
+}
+
+// Row exponents of the band -> x operand: rows (k, x), over n.  One warp per row.
+// src: element (x, k, n) at x*sx + k*sk + n.
+__global__ void k_slice_exp_rows(const double2* __restrict__ u, size_t sx, size_t sk, int nb, int nk, int nx,
+                                 int* __restrict__ e) {
+  const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (w >= (long long)nk * nx) return;
+  const int k = (int)(w / nx), x = (int)(w % nx);
+  const double2* r = u + x * sx + k * sk;
+  unsigned m = 0;
+  for (int n = lane; n < nb; n += 32) m = max(m, max(exp_bits(r[n].x), exp_bits(r[n].y)));
+  m = __reduce_max_sync(0xffffffffu, m);
+  if (lane == 0) e[w] = row_exp(m);
+}
+
+// Row exponents of the x -> band operand: rows (k, n), over x.  Block (32 n, 8).
+__global__ void k_slice_exp_cols(const double2* __restrict__ u, size_t sx, size_t sk, int nb, int nk, int nx,
+                                 int* __restrict__ e) {
+  __shared__ unsigned sh[8][32];
+  const int n = blockIdx.x * 32 + threadIdx.x, k = blockIdx.y;
+  unsigned m = 0;
+  if (n < nb)
+    for (int x = threadIdx.y; x < nx; x += 8) {
+      const double2 v = u[x * sx + k * sk + n];
+      m = max(m, max(exp_bits(v.x), exp_bits(v.y)));
+    }
+  sh[threadIdx.y][threadIdx.x] = m;
+  __syncthreads();
+  if (threadIdx.y == 0 && n < nb) {
+    for (int i = 1; i < 8; ++i) m = max(m, sh[i][threadIdx.x]);
+    e[(size_t)k * nb + n] = row_exp(m);
+  }
+}
+
+// Where 16 digit bytes of (k, row, box, granule) go (see the file comment).
+__device__ __forceinline__ size_t slice_a_off(const SliceParams& p, int nbox, int k, int row, int box, int g) {
+  const int mt = row / SL_ROWS, rt = mt == p.nt - 1 ? p.rl : SL_ROWS;
+  const int c = g / p.KC, gc = min(p.KC, p.G - c * p.KC);
+  return ((size_t)k * p.R + (size_t)SL_ROWS * mt) * 16 * p.G * nbox +
+         ((size_t)c * p.KC * nbox + (size_t)box * gc + (g - c * p.KC)) * rt * 16 + (size_t)(row - mt * SL_ROWS) * 16;
+}
+
+// Digits of the band -> x operand; one thread per (k, granule, row), rows fastest.
+__global__ void k_slice_build_rows(const double2* __restrict__ u, size_t sx, size_t sk, int nb, const SliceParams p,
+                                   const int* __restrict__ e, uint8_t* __restrict__ A, int koff) {
+  const long long tot = (long long)p.nk * p.G * p.R;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < tot; i += (long long)gridDim.x * blockDim.x) {
+    const int row = (int)(i % p.R);
+    const int g = (int)((i / p.R) % p.G), k = (int)(i / ((long long)p.R * p.G));
+    unsigned long long t[16];
+    const bool in = row < p.rows;
+    const int er = in ? e[(size_t)k * p.rows + row] : 0;
+    const double2* r = u + (size_t)row * sx + (size_t)k * sk;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int K = 16 * g + j, n = K < nb ? K : K - nb;
+      t[j] = SL_BIAS;
+      if (in && K < 2 * nb) t[j] = fix_point(K < nb ? r[n].x : r[n].y, er);
+    }
+#pragma unroll 1
+    for (int s = 0; s < SL_S; ++s)
+      *reinterpret_cast<uint4*>(A + slice_a_off(p, SL_S, k + koff, row, s, g)) = digits16(t, s);
+  }
+}
+
+// Digits of the x -> band operand; one thread per (k, plane, granule of x, row n), rows fastest.
+__global__ void k_slice_build_cols(const double2* __restrict__ u, size_t sx, size_t sk, int nx, const SliceParams p,
+                                   const int* __restrict__ e, uint8_t* __restrict__ A, int koff) {
+  const long long tot = (long long)p.nk * 2 * p.G * p.R;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < tot; i += (long long)gridDim.x * blockDim.x) {
+    const int n = (int)(i % p.R);
+    const long long q = i / p.R;
+    const int g = (int)(q % p.G), plane = (int)((q / p.G) & 1), k = (int)(q / (2 * p.G));
+    unsigned long long t[16];
+    const bool in = n < p.rows;
+    const int er = in ? e[(size_t)k * p.rows + n] : 0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int x = 16 * g + j;
+      t[j] = SL_BIAS;
+      if (in && x < nx) {
+        const double2 v = u[(size_t)x * sx + (size_t)k * sk + n];
+        t[j] = fix_point(plane ? v.y : v.x, er);
+      }
+    }
+#pragma unroll 1
+    for (int s = 0; s < SL_S; ++s)
+      *reinterpret_cast<uint4*>(A + slice_a_off(p, 2 * SL_S, k + koff, n, plane * SL_S + s, g)) = digits16(t, s);
+  }
+}
+
+// psi operand of one k-point per CTA: q = allow o psi of nae columns t = (vector,
+// channel); column exponents, then digits of
+//   part 0 (Re phi): K = (re n) -> qr, (im n) -> -qi;  part 1 (Im phi): (re n) -> qi, (im n) -> qr.
+// merged: row order [slice][part][t], else [part][slice][t].
+__global__ void __launch_bounds__(256)
+    k_slice_prep_b1(const double* __restrict__ pr, const double* __restrict__ pi, size_t vstride,
+                    const double* __restrict__ allow, int nb, int nk, int na, int nae, int Ge, int merged,
+                    uint8_t* __restrict__ B, int* __restrict__ eB) {
+  __shared__ int se[OCN_MAX_NA];
+  const int k = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int t = warp; t < nae; t += 8) {
+    const int v = t / na, a = t - v * na;
+    const size_t base = (size_t)nb * ((size_t)k + (size_t)nk * a);
+    unsigned m = 0;
+    for (int n = lane; n < nb; n += 32) {
+      const double w = allow[base + n];
+      m = max(m, max(exp_bits(pr[v * vstride + base + n] * w), exp_bits(pi[v * vstride + base + n] * w)));
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (lane == 0) {
+      se[t] = row_exp(m);
+      eB[(size_t)k * nae + t] = se[t];
+    }
+  }
+  __syncthreads();
+  const int items = Ge * 2 * nae * 4;
+  for (int i = threadIdx.x; i < items; i += blockDim.x) {
+    const int qd = i & 3, r = i >> 2;
+    const int t = r % nae, part = (r / nae) & 1, g = r / (2 * nae);
+    const int v = t / na, a = t - v * na, e = se[t];
+    const size_t base = (size_t)nb * ((size_t)k + (size_t)nk * a);
+    unsigned long long f[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int K = 16 * g + 4 * qd + j, c = K >= nb, n = c ? K - nb : K;
+      f[j] = SL_BIAS;
+      if (K < 2 * nb) {
+        const double w = allow[base + n];
+        const double x = ((part ^ c) ? pi : pr)[v * vstride + base + n] * w;
+        f[j] = fix_point(part == 0 && c ? -x : x, e);
+      }
+    }
+    uint8_t* out = B + ((size_t)k * Ge + g) * 2 * SL_S * nae * 16 + 4 * qd;
+#pragma unroll 1
+    for (int s = 0; s < SL_S; ++s) {
+      const int row = merged ? (s * 2 + part) * nae + t : (part * SL_S + s) * nae + t;
+      *reinterpret_cast<unsigned*>(out + (size_t)row * 16) = digits4(f, s);
+    }
+  }
+}
+
+// phi' operand of one k-point per CTA from src[(k)*nx + x][t] (parts: re, im):
+// column exponents over x, then digits, rows as k_slice_prep_b1.
+__global__ void __launch_bounds__(512)
+    k_slice_prep_b2(const double2* __restrict__ src, int nx, int nae, int Ge, int merged, double sign,
+                    uint8_t* __restrict__ B,
+                    int* __restrict__ eB) {
+  __shared__ unsigned sm[OCN_MAX_NA];
+  const int k = blockIdx.x;
+  if (threadIdx.x < OCN_MAX_NA) sm[threadIdx.x] = 0;
+  __syncthreads();
+  const double2* f = src + (size_t)k * nx * nae;
+  {  // thread's column is fixed: its stride is a multiple of nae
+    const int step = (int)blockDim.x / nae * nae;
+    if ((int)threadIdx.x < step) {
+      unsigned m = 0;
+      for (int i = threadIdx.x; i < nx * nae; i += step) m = max(m, max(exp_bits(f[i].x), exp_bits(f[i].y)));
+      atomicMax(&sm[threadIdx.x % nae], m);
+    }
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < nae) eB[(size_t)k * nae + threadIdx.x] = row_exp(sm[threadIdx.x]);
+  const int items = Ge * nae * 4;
+  for (int i = threadIdx.x; i < items; i += blockDim.x) {
+    const int qd = i & 3, r = i >> 2;
+    const int t = r % nae, g = r / nae, e = row_exp(sm[t]);
+    unsigned long long fr[4], fi[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int x = 16 * g + 4 * qd + j;
+      fr[j] = fi[j] = SL_BIAS;
+      if (x < nx) {
+        const double2 v = f[(size_t)x * nae + t];
+        fr[j] = fix_point(sign * v.x, e);
+        fi[j] = fix_point(sign * v.y, e);
+      }
+    }
+    uint8_t* out = B + ((size_t)k * Ge + g) * 2 * SL_S * nae * 16 + (size_t)t * 16 + 4 * qd;
+#pragma unroll 1
+    for (int s = 0; s < SL_S; ++s) {
+      *reinterpret_cast<unsigned*>(out + (size_t)(merged ? 2 * s : s) * nae * 16) = digits4(fr, s);
+      *reinterpret_cast<unsigned*>(out + (size_t)(merged ? 2 * s + 1 : SL_S + s) * nae * 16) = digits4(fi, s);
+    }
+  }
+}
+
+typedef void (*SliceFn)(const SliceParams);
+SliceFn slice_fn(int mode, int nae) {
+  if (mode == 1) return nae == 4 ? k_slice_gemm<1, 8, 1> : (nae == 8 ? k_slice_gemm<1, 16, 1> : k_slice_gemm<1, 12, 2>);
+  return nae == 4 ? k_slice_gemm<2, 8, 1> : (nae == 8 ? k_slice_gemm<2, 16, 1> : k_slice_gemm<2, 12, 2>);
+}
+inline bool slice_merged(int nae) { return nae <= 8; }
+
+// One contraction: geometry, operand A (digits and exponents) and launch shape.
+struct SliceGemm {
+  SliceParams p{};
+  uint8_t* A = nullptr;
+  int* eA = nullptr;
+  int mode = 1, nbox = SL_S, nae = 4, grid = 1;
+  size_t smem = 0;
+  size_t a_bytes(int spins) const { return (size_t)spins * p.nk * p.R * 16 * p.G * nbox; }
+  size_t b_bytes() const { return (size_t)(p.bshared ? 1 : p.nk) * p.Ge * 2 * SL_S * nae * 16; }
+};
+
+// rows and summed index of a contraction; the largest K chunk whose two B slots
+// and at least four A stages fit in shared memory (16 granules at most for one
+// resident B operand, 12 for streamed ones).
+void slice_plan(SliceGemm* s, int mode, int nae, int nk, int rows, int K, int sm_count) {
+  SliceParams& p = s->p;
+  s->mode = mode;
+  s->nae = nae;
+  s->nbox = mode == 1 ? SL_S : 2 * SL_S;
+  p.nk = nk;
+  p.rows = rows;
+  p.nt = (rows + SL_ROWS - 1) / SL_ROWS;
+  p.rl = (rows - (p.nt - 1) * SL_ROWS + 7) / 8 * 8;
+  p.R = (p.nt - 1) * SL_ROWS + p.rl;
+  p.G = (K + 15) / 16;
+  p.Ge = (p.G + 1) & ~1;
+  const size_t pitch = (size_t)2 * 23 * nae * 16;
+  const int cap = mode == 1 ? 16 : 12;
+  int kc = std::min(cap, p.Ge);
+  while (kc > 2 && kc * (2 * pitch + 4 * SL_ROWS * 16) > SL_SMEM) kc -= 2;
+  p.KC = kc;
+  p.nch = (p.G + kc - 1) / kc;
+  p.stages = (int)std::min<size_t>(SL_MAX_STAGES, (SL_SMEM - 2 * kc * pitch) / ((size_t)kc * SL_ROWS * 16));
+  s->smem = 2 * kc * pitch + (size_t)p.stages * kc * SL_ROWS * 16 + 256;  // + barriers
+  p.ks = 1;
+  p.cps = p.nch;
+  if (mode == 2) {
+    // K splits: the fewest per cent of idle SM time in the last wave of tiles
+    // (each split costs a partial-sum slice, so a later candidate has to gain 3%),
+    // and K per accumulation within the exact range
+    const int most = SL_MAX_K / (16 * kc);  // chunks per accumulation
+    const int least = (p.nch + most - 1) / most;
+    double best = 1e30;
+    for (int r = least; r <= std::max(least, std::min(p.nch, 8)); ++r) {
+      const int cps = (p.nch + r - 1) / r, ks = (p.nch + cps - 1) / cps;
+      const long long tiles = (long long)nk * p.nt * ks;
+      const double t = (double)((tiles + sm_count - 1) / sm_count) * cps;
+      if (t < 0.97 * best) {
+        best = t;
+        p.ks = ks;
+        p.cps = cps;
+      }
+    }
+  }
+  p.ntiles = nk * p.nt * p.ks;
+  p.spin = -1;
+  s->grid = std::min(p.ntiles, sm_count);
+}
+
+}  // namespace
+
+struct SliceLR {
+  bool ready = false;
+  int nvs = 1;             // vectors per launch
+  SliceGemm g1, g2;        // band -> x, x -> band
+  uint8_t *b1 = nullptr, *b2 = nullptr;
+  int *e1 = nullptr, *e2 = nullptr;
+  int* d_err = nullptr;
+};
+
+namespace {
+
+template <typename T>
+int salloc(ocn_ctx* c, T** p, size_t n) {
+  cudaError_t e = cudaMalloc(reinterpret_cast<void**>(p), n * sizeof(T));
+  if (e != cudaSuccess) return set_err(c, OCN_ERR_ALLOC, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  return OCN_OK;
+}
+
+void slice_drop_a(SliceLR* s) {
+  for (SliceGemm* g : {&s->g1, &s->g2}) {
+    if (g->A) cudaFree(g->A);
+    if (g->eA) cudaFree(g->eA);
+    g->A = nullptr;
+    g->eA = nullptr;
+  }
+  s->ready = false;
+}
+
+int slice_launch(ocn_ctx* c, const SliceGemm& g, const uint8_t* B, const int* eB, double2* phi, double* part, int spin,
+                 int spins) {
+  SliceParams p = g.p;
+  p.A = g.A;
+  p.eA = g.eA;
+  p.B = B;
+  p.eB = eB;
+  p.phi = phi;
+  p.part = part;
+  p.part_stride = c->part_stride;
+  p.npsi = c->npsi;
+  p.na = c->na;
+  p.nb = c->nb;
+  p.err = c->slice->d_err;
+  p.koff = spin * p.nk;
+  p.spin = spins == 2 ? spin : -1;
+  slice_fn(g.mode, g.nae)<<<g.grid, SL_THREADS, g.smem, c->stream>>>(p);
+  ++c->launches;
+  OCN_CUDA(c, cudaGetLastError());
+  return OCN_OK;
+}
+
+}  // namespace
+
+// Geometry and vector-side buffers (before ocn_ctx_create sizes the partial sums).
+int slice_init(ocn_ctx* c) {
+  SliceLR* s = new (std::nothrow) SliceLR();
+  if (!s) return set_err(c, OCN_ERR_ALLOC, "host allocation failed");
+  c->slice = s;
+  slice_plan(&s->g1, 1, c->na, c->nk, c->nx, 2 * c->nb, c->sm_count);
+  slice_plan(&s->g2, 2, c->na, c->nk, c->nb, c->nx, c->sm_count);
+  c->lr_xsplit = s->g2.p.ks;
+  int rc;
+  if ((rc = salloc(c, &s->b1, s->g1.b_bytes())) || (rc = salloc(c, &s->b2, s->g2.b_bytes())) ||
+      (rc = salloc(c, &s->e1, (size_t)c->nk * c->na)) || (rc = salloc(c, &s->e2, (size_t)c->nk * c->na)) ||
+      (rc = salloc(c, &s->d_err, 1)))
+    return rc;
+  OCN_CUDA(c, cudaMemsetAsync(s->d_err, 0, sizeof(int), c->stream));
+  if ((rc = allow_max_smem(c, slice_fn(1, c->na))) || (rc = allow_max_smem(c, slice_fn(2, c->na)))) return rc;
+  return OCN_OK;
+}
+
+void slice_free(ocn_ctx* c) {
+  SliceLR* s = c->slice;
+  if (!s) return;
+  slice_drop_a(s);
+  for (void* q : {(void*)s->b1, (void*)s->b2, (void*)s->e1, (void*)s->e2, (void*)s->d_err})
+    if (q) cudaFree(q);
+  delete s;
+  c->slice = nullptr;
+}
+
+bool slice_ready(const ocn_ctx* c) { return c->slice && c->slice->ready; }
+
+// Digit operands from d_u.  They take 3 bytes for every 2 of u, twice; when that
+// is more than a quarter of the free device memory the context keeps the
+// FP64-pipe kernels, which need only u.
+int slice_set_bloch(ocn_ctx* c) {
+  SliceLR* s = c->slice;
+  if (!s) return OCN_OK;
+  const int ns = c->nspn;
+  if (!s->g1.A) {
+    size_t fr = 0, tot = 0;
+    OCN_CUDA(c, cudaMemGetInfo(&fr, &tot));
+    if (s->g1.a_bytes(ns) + s->g2.a_bytes(ns) > fr / 4) return OCN_OK;
+    if (salloc(c, &s->g1.A, s->g1.a_bytes(ns)) || salloc(c, &s->g2.A, s->g2.a_bytes(ns)) ||
+        salloc(c, &s->g1.eA, (size_t)ns * c->nk * c->nx) || salloc(c, &s->g2.eA, (size_t)ns * c->nk * c->nb)) {
+      slice_drop_a(s);
+      (void)cudaGetLastError();
+      c->err.clear();
+      return OCN_OK;
+    }
+  }
+  const size_t sx = (size_t)c->nk * c->nb, sk = c->nb;
+  const int blocks = 16 * c->sm_count;
+  for (int sp = 0; sp < ns; ++sp) {
+    const double2* u = c->d_u + (size_t)sp * c->nx * sx;
+    int* e1 = s->g1.eA + (size_t)sp * c->nk * c->nx;
+    int* e2 = s->g2.eA + (size_t)sp * c->nk * c->nb;
+    const long long warps = (long long)c->nk * c->nx;
+    k_slice_exp_rows<<<(unsigned)((warps + 7) / 8), 256, 0, c->stream>>>(u, sx, sk, c->nb, c->nk, c->nx, e1);
+    k_slice_build_rows<<<blocks, 256, 0, c->stream>>>(u, sx, sk, c->nb, s->g1.p, e1, s->g1.A, sp * c->nk);
+    k_slice_exp_cols<<<dim3((c->nb + 31) / 32, c->nk), dim3(32, 8), 0, c->stream>>>(u, sx, sk, c->nb, c->nk, c->nx, e2);
+    k_slice_build_cols<<<blocks, 256, 0, c->stream>>>(u, sx, sk, c->nx, s->g2.p, e2, s->g2.A, sp * c->nk);
+    c->launches += 4;
+    OCN_CUDA(c, cudaGetLastError());
+  }
+  OCN_CUDA(c, cudaStreamSynchronize(c->stream));
+  s->ready = true;
+  return OCN_OK;
+}
+
+// phi[k][x][a] of one vector (FP64 planes).
+int slice_band_to_x(ocn_ctx* c, const double* d_pr, const double* d_pi, double2* phi) {
+  SliceLR* s = c->slice;
+  {
+    TimedScope ts(c, T_LR_PREP);
+    k_slice_prep_b1<<<c->nk, 256, 0, c->stream>>>(d_pr, d_pi, 0, c->d_allow, c->nb, c->nk, c->na, c->na, s->g1.p.Ge,
+                                                  slice_merged(c->na) ? 1 : 0, s->b1, s->e1);
+    ++c->launches;
+    OCN_CUDA(c, cudaGetLastError());
+  }
+  TimedScope ts(c, T_LR_GEMM1);
+  for (int sp = 0; sp < c->nspn; ++sp)
+    if (int rc = slice_launch(c, s->g1, s->b1, s->e1, phi, nullptr, sp, c->nspn)) return rc;
+  return OCN_OK;
+}
+
+// d_accpart slices of one vector from phi'[k][x][a].
+int slice_x_to_band(ocn_ctx* c, const double2* phi) {
+  SliceLR* s = c->slice;
+  {
+    TimedScope ts(c, T_LR_PREP);
+    k_slice_prep_b2<<<c->nk, 512, 0, c->stream>>>(phi, c->nx, c->na, s->g2.p.Ge, slice_merged(c->na) ? 1 : 0, 1.0, s->b2, s->e2);
+    ++c->launches;
+    OCN_CUDA(c, cudaGetLastError());
+  }
+  TimedScope ts(c, T_LR_GEMM2);
+  for (int sp = 0; sp < c->nspn; ++sp)
+    if (int rc = slice_launch(c, s->g2, s->b2, s->e2, nullptr, c->d_accpart, sp, c->nspn)) return rc;
+  return OCN_OK;
+}
+
+// Reads and clears the device timeout flag (as mixed_check).
+int slice_check(ocn_ctx* c) {
+  if (!c->slice) return OCN_OK;
+  int err = 0;
+  OCN_CUDA(c, cudaMemcpyAsync(&err, c->slice->d_err, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+  OCN_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (!err) return OCN_OK;
+  OCN_CUDA(c, cudaMemset(c->slice->d_err, 0, sizeof(int)));
+  return set_err(c, OCN_ERR_TIMEOUT, "tensor-core pipeline timed out (mask " + std::to_string(err) + ")");
+}
+
+}  // namespace ocn
