@@ -29,6 +29,7 @@ SOURCES = {
     "ocn_gmres.cu": [],
     "ocn_mixed.cu": [],
     "ocn_slice.cu": [],
+    "ocn_fixfft.cu": [],
     "ocn_valence.cu": [],
     "ocn_setup.cpp": [],
     "ocn_io.cpp": [],
@@ -50,6 +51,7 @@ def _compile(src: str, extra: list[str], verbose: bool) -> str:
     srcp = os.path.join(CSRC, src)
     deps = [srcp, os.path.join(CSRC, "ocn_internal.h"), os.path.join(CSRC, "ocn_kmesh_dft.cuh"),
             os.path.join(CSRC, "ocn_df.cuh"), os.path.join(CSRC, "ocn_tc.cuh"),
+            os.path.join(CSRC, "ocn_fixed.cuh"),
             os.path.join(ROOT, "include", "ocean_gpu.h")]
     if os.path.exists(obj) and all(os.path.getmtime(obj) >= os.path.getmtime(d) for d in deps):
         return obj

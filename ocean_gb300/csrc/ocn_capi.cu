@@ -282,7 +282,7 @@ int ocn_ctx_create(const ocn_dims* d, ocn_ctx** out) {
   c->red_blocks = (int)std::min<size_t>(2 * (size_t)c->sm_count, std::max<size_t>(1, (c->npsi + 511) / 512));
   c->lr_xsplit = std::max(1, std::min((2 * c->sm_count + nk - 1) / nk, std::max(1, nx / 64)));
   int rc = OCN_OK;
-  if (d->precision == OCN_PREC_FP64 && (rc = slice_init(c))) return fail(rc);
+  if (d->precision == OCN_PREC_FP64 && ((rc = slice_init(c)) || (rc = fx_init(c)))) return fail(rc);
   if ((rc = dev_alloc(c, &c->d_er, c->npsi)) || (rc = dev_alloc(c, &c->d_ei, c->npsi)) ||
       (rc = dev_alloc(c, &c->d_allow, c->npsi)) ||
       (rc = dev_alloc(c, &c->d_u, (size_t)c->nb * nk * nx * c->nspn)) ||
@@ -314,7 +314,7 @@ int ocn_ctx_destroy(ocn_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   if (c->mixed) mixed_free(c);
   slice_free(c);
-  void* bufs[] = {c->d_er, c->d_ei, c->d_allow, c->d_u, c->d_W, c->d_tw, c->d_so, c->d_phi, c->d_acc,
+  void* bufs[] = {c->d_er, c->d_ei, c->d_allow, c->d_u, c->d_W, c->d_Wfx, c->d_Wexp, c->d_tw, c->d_so, c->d_phi, c->d_acc,
                   c->d_accpart, c->d_vec, c->d_red, c->d_scal, c->mult.mpc, c->mult.mpm, c->mult.mh,
                   c->mult.p_l, c->mult.p_m, c->mult.p_nu, c->mult.d_pfirst, c->mult.d_nproj,
                   c->mult.d_jbeg, c->mult.amp, c->mult.amp_part, c->mult.hamp, c->d_er_df, c->d_ei_df,
@@ -432,6 +432,7 @@ int ocn_lr_init(ocn_ctx* c, const ocn_lr_params* p) {
   c->have_bloch = true;
   c->have_W = true;
   if (c->dims.precision == OCN_PREC_MIXED) return mixed_set_bloch(c);
+  if ((rc = fx_set_w(c))) return rc;
   return slice_set_bloch(c);
 }
 
@@ -444,7 +445,7 @@ int ocn_set_W(ocn_ctx* c, const double* W) {
   OCN_CUDA(c, cudaStreamSynchronize(c->stream));
   c->have_W = true;
   if (c->dims.precision == OCN_PREC_MIXED && c->have_bloch) return mixed_set_bloch(c);
-  return OCN_OK;
+  return fx_set_w(c);
 }
 
 int ocn_get_W(ocn_ctx* c, double* W, int xshift[3], double tau_shifted[3]) {

@@ -110,6 +110,8 @@ struct ocn_ctx {
   float2* d_so_f = nullptr;
   double2* d_u = nullptr;    // phased Bloch functions, [s][x][k][n] complex (reference order)
   double* d_W = nullptr;     // (Nk, Nx): W[x*Nk + k]
+  long long* d_Wfx = nullptr;  // FP64 contexts: W / Nk as 62-bit integers, exponents per x in d_Wexp
+  int* d_Wexp = nullptr;
   double2* d_tw = nullptr;   // k-mesh twiddles exp(+2 pi i t / n_axis), [axis][t] (3 x OCN_MAX_KDIM)
   double2* d_so = nullptr;   // (Na,Na) somelr + i someli, [jc*Na + ic]
   std::vector<double> h_so_r, h_so_i;
@@ -354,13 +356,20 @@ int conv_check_launch(ocn_ctx* c, const double* ra, const double* ia, const doub
 int cf_eval_noalloc(const double* ra, const double* ia, const double* rb, int iter, double kpref,
                     const ocn_cf_params* p, double* out, std::string* err);
 
+// ---- FP64 k-mesh transform in 64-bit fixed point (ocn_fixfft.cu)
+int fx_init(ocn_ctx* c);
+int fx_set_w(ocn_ctx* c);          // integer copy of W / Nk from d_W
+bool fx_supported(const ocn_ctx* c);
+int fx_transform(ocn_ctx* c, double2* phi, int nt, unsigned* mx);  // phi[k][x][t] in place
+
 // ---- FP64 contractions on the tensor cores (ocn_slice.cu)
 int slice_init(ocn_ctx* c);        // geometry and vector-side buffers; sets lr_xsplit
 void slice_free(ocn_ctx* c);
 int slice_set_bloch(ocn_ctx* c);   // digit operands from d_u (not ready when they do not fit)
 bool slice_ready(const ocn_ctx* c);
 int slice_band_to_x(ocn_ctx* c, const double* d_pr, const double* d_pi, double2* phi);  // phi[k][x][a]
-int slice_x_to_band(ocn_ctx* c, const double2* phi);  // d_accpart slices from phi'[k][x][a]
+int slice_x_to_band(ocn_ctx* c, const double2* phi, bool have_max);  // d_accpart slices from phi'[k][x][a]
+unsigned* slice_maxima(ocn_ctx* c);  // [k][a] magnitude maxima of phi', cleared by slice_band_to_x
 int slice_check(ocn_ctx* c);       // reads and clears the device timeout flag
 
 // ---- mixed precision (ocn_mixed.cu)

@@ -1036,7 +1036,11 @@ int lr_apply_fp64(ocn_ctx* c, const double* d_pr, const double* d_pi) {
     ++c->launches;
     OCN_CUDA(c, cudaGetLastError());
   }
-  {
+  const bool fixed = fx_supported(c);
+  if (fixed) {
+    TimedScope ts(c, T_LR_FFT);
+    if (int rc = fx_transform(c, c->d_phi, na, sliced ? slice_maxima(c) : nullptr)) return rc;
+  } else {
     const KmeshGeom<double> g = kmesh_geom<double>(c->dims.kmesh, na);
     TimedScope ts(c, T_LR_FFT);
     CubeFnD f = nullptr;
@@ -1049,7 +1053,7 @@ int lr_apply_fp64(ocn_ctx* c, const double* d_pr, const double* d_pi) {
     ++c->launches;
     OCN_CUDA(c, cudaGetLastError());
   }
-  if (sliced) return slice_x_to_band(c, c->d_phi);
+  if (sliced) return slice_x_to_band(c, c->d_phi, fixed);
   {
     const int xs = c->lr_xsplit;
     const int xper = (nx + xs - 1) / xs;

@@ -39,8 +39,8 @@
 //
 // Measured, 8^3 k / 100 bands / 12^3 x, 1s: band -> x 4.3 ms on the FP64 pipe ->
 // 0.331 ms (2.2 GB, 6.7 TB/s), x -> band 5.9 ms -> 0.355 ms (6.2 TB/s): bound by
-// the read of A.  2p, 6^3 k / 64 bands / 10^3 x (12 columns): 0.093 and 0.123 ms
-// (3.6 and 2.5 TB/s): there the 144-column MMAs (72 cycles) and the epilogue's
+// the read of A.  2p, 6^3 k / 64 bands / 10^3 x (12 columns): 0.084 and 0.119 ms
+// (4.0 and 2.6 TB/s): there the 144-column MMAs (72 cycles) and the epilogue's
 // 288 integer columns per row weigh as much as the 0.3 GB read.
 #include <cuda_runtime.h>
 
@@ -49,6 +49,7 @@
 #include <new>
 #include <string>
 
+#include "ocn_fixed.cuh"
 #include "ocn_internal.h"
 #include "ocn_tc.cuh"
 
@@ -59,10 +60,12 @@ namespace {
 constexpr int SL_S = 12;           // digits per value
 constexpr int SL_FRAC = 59;        // fixed point: t = v 2^(59 - e), |v| < 2^e
 constexpr int SL_ROWS = 128;       // rows per tile (MMA M)
-constexpr int SL_THREADS = 192;
+// Two control warps and four epilogue warps; eight with 8 or 12 columns, half of the
+// columns each (band -> x of the 2p case: 113 us with four warps and 255 registers,
+// 84 us with eight).
+constexpr int slice_threads(int nae) { return nae == 4 ? 192 : 320; }
 constexpr int SL_MAX_STAGES = 8;
 constexpr size_t SL_SMEM = 222 * 1024;
-constexpr int SL_NAN = 0x40000000;  // exponent of a row that holds an Inf or NaN
 constexpr int SL_MAX_K = 2730;      // K per plane and accumulation: 2 * 2730 * 12 * 256 < 2^24
 constexpr unsigned long long SL_BIAS = 0x0842108421084210ull;  // sum of 16 * 32^i, i < 12
 
@@ -111,37 +114,37 @@ __device__ __forceinline__ bool elect_one() {
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
   return ok != 0;
 }
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
-  uint32_t r[8];
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+// A (4 or 6) consecutive accumulator columns of this thread's lane
+template <int A>
+__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, float* v) {
+  static_assert(A == 4 || A == 6, "4 or 6 columns");
+  uint32_t r[4];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
                : "r"(taddr));
 #pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+  for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
+  if constexpr (A == 6) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(taddr + 4));
+    v[4] = __uint_as_float(r[0]);
+    v[5] = __uint_as_float(r[1]);
+  }
 }
 
-// r 2^e for a finite r (r = 0 allowed)
-__device__ __forceinline__ double scale_pow2(double r, int e) {
-  const int hw = __double2hiint(r);
-  const int ne = ((hw >> 20) & 0x7ff) + e;
-  if (ne > 0 && ne < 2047 && (hw & 0x7ff00000)) return __hiloint2double(hw + (e << 20), __double2loint(r));
-  return ldexp(r, e);
-}
-
-// Six accumulator groups (most significant first) of C columns as integers.
-template <int C>
-__device__ __forceinline__ void add_groups(uint32_t ta, long long (&acc)[C]) {
-  float v[6 * C];
+// Six accumulator groups (most significant first, stride C columns) of A columns as integers.
+template <int A, int C>
+__device__ __forceinline__ void add_groups(uint32_t ta, long long (&acc)[A]) {
+  float v[6 * A];
 #pragma unroll
-  for (int c = 0; c < 6 * C; c += 8) tmem_ld8(ta + c, v + c);
+  for (int g = 0; g < 6; ++g) tmem_ld_cols<A>(ta + g * C, v + g * A);
   tmem_ld_wait();
 #pragma unroll
-  for (int c = 0; c < C; ++c) acc[c] = 0;
+  for (int c = 0; c < A; ++c) acc[c] = 0;
 #pragma unroll
   for (int g = 0; g < 6; ++g)
 #pragma unroll
-    for (int c = 0; c < C; ++c)
-      acc[c] += (long long)__float2int_rn(v[g * C + c]) * (long long)(1 << (5 * (5 - g)));
+    for (int c = 0; c < A; ++c)
+      acc[c] += (long long)__float2int_rn(v[g * A + c]) * (long long)(1 << (5 * (5 - g)));
 }
 
 struct SliceTile {
@@ -165,7 +168,7 @@ __device__ __forceinline__ SliceTile slice_decode(const SliceParams& p, int t) {
 // complex product).  MODE 2: x -> band (two planes).  C columns per slice and
 // MMA, P MMAs (parts) per K step.
 template <int MODE, int C, int P>
-__global__ void __launch_bounds__(SL_THREADS, 1) k_slice_gemm(const __grid_constant__ SliceParams p) {
+__global__ void __launch_bounds__(slice_threads(P == 1 ? C / 2 : C), 1) k_slice_gemm(const __grid_constant__ SliceParams p) {
   constexpr int NAE = P == 1 ? C / 2 : C;        // complex columns
   constexpr int NBOX = MODE == 1 ? SL_S : 2 * SL_S;
   constexpr int N = SL_S * C;                    // MMA N
@@ -198,7 +201,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_slice_gemm(const __grid_const
       mbar_init(bfull0 + 8 * b, 1);
       mbar_init(bempty0 + 8 * b, 1);
       mbar_init(tfull0 + 8 * b, 1);
-      mbar_init(tempty0 + 8 * b, 128);
+      mbar_init(tempty0 + 8 * b, (NAE == 4 ? 192 : 320) - 64);
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -211,7 +214,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_slice_gemm(const __grid_const
   {  // the empty slices of B stay zero; A stages too when an odd granule count leaves one that is never
      // written (it meets zero digits, but must hold finite ones)
     const uint32_t zb = 2 * slot_bytes + ((p.G & 1) ? S * stage_bytes : 0);
-    for (uint32_t i = threadIdx.x * 16; i < zb; i += SL_THREADS * 16)
+    for (uint32_t i = threadIdx.x * 16; i < zb; i += blockDim.x * 16)
       *reinterpret_cast<uint4*>(smem + i) = make_uint4(0, 0, 0, 0);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -366,8 +369,10 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_slice_gemm(const __grid_const
     }
   } else {
     // -------------------------------------------------------------- epilogue
+    constexpr int AH = NAE == 4 ? 4 : NAE / 2;       // columns of a thread
+    constexpr uint32_t PART = P == 1 ? NAE : N;      // accumulator columns between the parts
     const int q4 = warp & 3;  // tensor-memory lane quadrant of this warp
-    const int row = q4 * 32 + lane;
+    const int row = q4 * 32 + lane, h0 = ((warp - 2) >> 2) * AH;
     uint32_t acc = 0, acc_phase = 0;
     for (int t = t0; t < t1; ++t) {
       const SliceTile ti = slice_decode<MODE>(p, t);
@@ -377,24 +382,23 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_slice_gemm(const __grid_const
         break;
       }
       tc_fence_after();
-      const uint32_t ta = tmem_base + ((uint32_t)(q4 * 32) << 16) + acc * DCOLS;
-      long long hi[P][C], lo[P][C];
+      const uint32_t ta = tmem_base + ((uint32_t)(q4 * 32) << 16) + acc * DCOLS + h0;
+      long long hi[2][AH], lo[2][AH];
 #pragma unroll
-      for (int q = 0; q < P; ++q) {
-        add_groups<C>(ta + q * N, hi[q]);
-        add_groups<C>(ta + q * N + 6 * C, lo[q]);
+      for (int q = 0; q < 2; ++q) {
+        add_groups<AH, C>(ta + q * PART, hi[q]);
+        add_groups<AH, C>(ta + q * PART + 6 * C, lo[q]);
       }
       if (PL == 2) {  // out = (re plane) phi' - i (im plane) phi'
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          long long (&o)[C] = h ? lo[0] : hi[0];
-          long long im[C];
-          add_groups<C>(ta + N + h * 6 * C, im);
+        for (int q = 0; q < 2; ++q) {
+          long long im[AH];
+          add_groups<AH, C>(ta + N + (1 - q) * PART, im);
 #pragma unroll
-          for (int a = 0; a < NAE; ++a) {
-            o[a] += im[(NAE + a) % C];
-            o[(NAE + a) % C] -= im[a];
-          }
+          for (int a = 0; a < AH; ++a) hi[q][a] += q ? -im[a] : im[a];
+          add_groups<AH, C>(ta + N + (1 - q) * PART + 6 * C, im);
+#pragma unroll
+          for (int a = 0; a < AH; ++a) lo[q][a] += q ? -im[a] : im[a];
         }
       }
       tc_fence_before();
@@ -406,18 +410,14 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_slice_gemm(const __grid_const
         const int ea = p.eA[(size_t)(ti.k + p.koff) * p.rows + r];
         const int* eb = p.eB + (p.bshared ? 0 : (size_t)ti.k) * NAE;
 #pragma unroll
-        for (int a = 0; a < NAE; ++a) {
+        for (int j = 0; j < AH; ++j) {
+          const int a = h0 + j;
           if (p.spin >= 0 && (a & 1) != p.spin) continue;
           const int e = eb[a];
-          constexpr int im0 = P == 1 ? NAE : 0;  // merged parts: im columns follow the re columns
-          double vr = fma((double)hi[0][a], 1073741824.0, (double)lo[0][a]);
-          double vi = fma((double)hi[P - 1][im0 + a], 1073741824.0, (double)lo[P - 1][im0 + a]);
-          if (ea == SL_NAN || e == SL_NAN) {
-            vr = vi = __longlong_as_double(0x7ff8000000000000ll);
-          } else {
-            vr = scale_pow2(vr, ea + e - 2 * SL_FRAC + 55);
-            vi = scale_pow2(vi, ea + e - 2 * SL_FRAC + 55);
-          }
+          const int es = ea + e - 2 * SL_FRAC + 55;
+          double vr = fx_to_double(hi[0][j], lo[0][j], es);
+          double vi = fx_to_double(hi[1][j], lo[1][j], es);
+          if (ea == FX_NAN || e == FX_NAN) vr = vi = __longlong_as_double(0x7ff8000000000000ll);
           if (MODE == 1) {
             p.phi[((size_t)ti.k * p.rows + r) * NAE + a] = make_double2(vr, vi);
           } else {
@@ -440,24 +440,9 @@ __global__ void __launch_bounds__(SL_THREADS, 1) k_slice_gemm(const __grid_const
 
 // ------------------------------------------------------------- digit operands
 
-__device__ __forceinline__ unsigned exp_bits(double v) { return (unsigned)__double2hiint(v) & 0x7fffffffu; }
-// exponent e of a row from the largest high word of its values: |v| < 2^e
-__device__ __forceinline__ int row_exp(unsigned hw) {
-  const int E = (int)(hw >> 20);
-  return E == 0x7ff ? SL_NAN : E - 1022;
-}
-// v 2^(59 - e) rounded to an integer, plus the digit bias (e = SL_NAN: zero digits)
+// biased fixed point: the 60-bit integer plus 16 in every base-32 digit
 __device__ __forceinline__ unsigned long long fix_point(double v, int e) {
-  const long long b = __double_as_longlong(v);
-  const int ev = (int)((b >> 52) & 0x7ff);
-  unsigned long long m = (unsigned long long)b & 0xfffffffffffffull;
-  if (ev) m |= 1ull << 52;
-  const int s = max(ev, 1) - 1075 + SL_FRAC - e;
-  unsigned long long t = 0;
-  if (s >= 0) t = m << min(s, 6);  // s <= 6: |v| < 2^e
-  else if (s > -54) t = (m + (1ull << (-s - 1))) >> (-s);
-  if (e == SL_NAN) t = 0;
-  return SL_BIAS + (b < 0 ? 0ull - t : t);
+  return SL_BIAS + (unsigned long long)fx_from<SL_FRAC>(v, e);
 }
 // digit s (0 most significant) of a biased fixed-point value as an exact float
 __device__ __forceinline__ float digit_of(unsigned long long t, int s) {
@@ -488,9 +473,9 @@ __global__ void k_slice_exp_rows(const double2* __restrict__ u, size_t sx, size_
   const int k = (int)(w / nx), x = (int)(w % nx);
   const double2* r = u + x * sx + k * sk;
   unsigned m = 0;
-  for (int n = lane; n < nb; n += 32) m = max(m, max(exp_bits(r[n].x), exp_bits(r[n].y)));
+  for (int n = lane; n < nb; n += 32) m = max(m, max(fx_mag(r[n].x), fx_mag(r[n].y)));
   m = __reduce_max_sync(0xffffffffu, m);
-  if (lane == 0) e[w] = row_exp(m);
+  if (lane == 0) e[w] = fx_exp(m);
 }
 
 // Row exponents of the x -> band operand: rows (k, n), over x.  Block (32 n, 8).
@@ -502,13 +487,13 @@ __global__ void k_slice_exp_cols(const double2* __restrict__ u, size_t sx, size_
   if (n < nb)
     for (int x = threadIdx.y; x < nx; x += 8) {
       const double2 v = u[x * sx + k * sk + n];
-      m = max(m, max(exp_bits(v.x), exp_bits(v.y)));
+      m = max(m, max(fx_mag(v.x), fx_mag(v.y)));
     }
   sh[threadIdx.y][threadIdx.x] = m;
   __syncthreads();
   if (threadIdx.y == 0 && n < nb) {
     for (int i = 1; i < 8; ++i) m = max(m, sh[i][threadIdx.x]);
-    e[(size_t)k * nb + n] = row_exp(m);
+    e[(size_t)k * nb + n] = fx_exp(m);
   }
 }
 
@@ -569,27 +554,36 @@ __global__ void k_slice_build_cols(const double2* __restrict__ u, size_t sx, siz
   }
 }
 
+// x w for a mask weight w, without the FP64 pipe where w = 1
+__device__ __forceinline__ double weigh(double x, double w) {
+  const long long b = __double_as_longlong(w);
+  if (b == 0x3ff0000000000000ll) return x;
+  return x * w;
+}
+
 // psi operand of one k-point per CTA: q = allow o psi of nae columns t = (vector,
 // channel); column exponents, then digits of
 //   part 0 (Re phi): K = (re n) -> qr, (im n) -> -qi;  part 1 (Im phi): (re n) -> qi, (im n) -> qr.
-// merged: row order [slice][part][t], else [part][slice][t].
+// merged: row order [slice][part][t], else [part][slice][t].  Clears the maxima that
+// the k-mesh transform of this action collects (mx, may be null).
 __global__ void __launch_bounds__(256)
     k_slice_prep_b1(const double* __restrict__ pr, const double* __restrict__ pi, size_t vstride,
                     const double* __restrict__ allow, int nb, int nk, int na, int nae, int Ge, int merged,
-                    uint8_t* __restrict__ B, int* __restrict__ eB) {
+                    uint8_t* __restrict__ B, int* __restrict__ eB, unsigned* __restrict__ mx) {
   __shared__ int se[OCN_MAX_NA];
   const int k = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (mx && (int)threadIdx.x < nae) mx[(size_t)k * nae + threadIdx.x] = 0;
   for (int t = warp; t < nae; t += 8) {
     const int v = t / na, a = t - v * na;
     const size_t base = (size_t)nb * ((size_t)k + (size_t)nk * a);
     unsigned m = 0;
     for (int n = lane; n < nb; n += 32) {
       const double w = allow[base + n];
-      m = max(m, max(exp_bits(pr[v * vstride + base + n] * w), exp_bits(pi[v * vstride + base + n] * w)));
+      m = max(m, max(fx_mag(weigh(pr[v * vstride + base + n], w)), fx_mag(weigh(pi[v * vstride + base + n], w))));
     }
     m = __reduce_max_sync(0xffffffffu, m);
     if (lane == 0) {
-      se[t] = row_exp(m);
+      se[t] = fx_exp(m);
       eB[(size_t)k * nae + t] = se[t];
     }
   }
@@ -607,7 +601,7 @@ __global__ void __launch_bounds__(256)
       f[j] = SL_BIAS;
       if (K < 2 * nb) {
         const double w = allow[base + n];
-        const double x = ((part ^ c) ? pi : pr)[v * vstride + base + n] * w;
+        const double x = weigh(((part ^ c) ? pi : pr)[v * vstride + base + n], w);
         f[j] = fix_point(part == 0 && c ? -x : x, e);
       }
     }
@@ -620,48 +614,54 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// phi' operand of one k-point per CTA from src[(k)*nx + x][t] (parts: re, im):
-// column exponents over x, then digits, rows as k_slice_prep_b1.
+// Magnitude maxima mx[k][t] of src[k*nx + x][t] (k-meshes whose transform does not collect them).
 __global__ void __launch_bounds__(512)
-    k_slice_prep_b2(const double2* __restrict__ src, int nx, int nae, int Ge, int merged, double sign,
-                    uint8_t* __restrict__ B,
-                    int* __restrict__ eB) {
+    k_slice_col_max(const double2* __restrict__ src, int nx, int nae, unsigned* __restrict__ mx) {
   __shared__ unsigned sm[OCN_MAX_NA];
   const int k = blockIdx.x;
   if (threadIdx.x < OCN_MAX_NA) sm[threadIdx.x] = 0;
   __syncthreads();
   const double2* f = src + (size_t)k * nx * nae;
-  {  // thread's column is fixed: its stride is a multiple of nae
-    const int step = (int)blockDim.x / nae * nae;
-    if ((int)threadIdx.x < step) {
-      unsigned m = 0;
-      for (int i = threadIdx.x; i < nx * nae; i += step) m = max(m, max(exp_bits(f[i].x), exp_bits(f[i].y)));
-      atomicMax(&sm[threadIdx.x % nae], m);
-    }
+  const int step = (int)blockDim.x / nae * nae;  // a multiple of nae: a thread's column is fixed
+  if ((int)threadIdx.x < step) {
+    unsigned m = 0;
+    for (int i = threadIdx.x; i < nx * nae; i += step) m = max(m, max(fx_mag(f[i].x), fx_mag(f[i].y)));
+    atomicMax(&sm[threadIdx.x % nae], m);
   }
   __syncthreads();
-  if ((int)threadIdx.x < nae) eB[(size_t)k * nae + threadIdx.x] = row_exp(sm[threadIdx.x]);
-  const int items = Ge * nae * 4;
-  for (int i = threadIdx.x; i < items; i += blockDim.x) {
-    const int qd = i & 3, r = i >> 2;
-    const int t = r % nae, g = r / nae, e = row_exp(sm[t]);
-    unsigned long long fr[4], fi[4];
+  if ((int)threadIdx.x < nae) mx[(size_t)k * nae + threadIdx.x] = sm[threadIdx.x];
+}
+
+// phi' operand from src[k*nx + x][t] (parts: re, im) and its column maxima: digits,
+// rows as k_slice_prep_b1.  grid (ceil(items / block), Nk); a thread makes four x of
+// one column, both parts (reads 64-byte runs, writes 4-byte words of 64-byte runs).
+__global__ void __launch_bounds__(256)
+    k_slice_prep_b2(const double2* __restrict__ src, int nx, int nae, int Ge, int merged,
+                    const unsigned* __restrict__ mx, uint8_t* __restrict__ B, int* __restrict__ eB) {
+  const int k = blockIdx.y;
+  if (blockIdx.x == 0 && (int)threadIdx.x < nae)
+    eB[(size_t)k * nae + threadIdx.x] = fx_exp(mx[(size_t)k * nae + threadIdx.x]);
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= Ge * nae * 4) return;
+  const int qd = i & 3, r = i >> 2;
+  const int t = r % nae, g = r / nae, e = fx_exp(mx[(size_t)k * nae + t]);
+  const double2* f = src + (size_t)k * nx * nae + t;
+  unsigned long long fr[4], fi[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int x = 16 * g + 4 * qd + j;
-      fr[j] = fi[j] = SL_BIAS;
-      if (x < nx) {
-        const double2 v = f[(size_t)x * nae + t];
-        fr[j] = fix_point(sign * v.x, e);
-        fi[j] = fix_point(sign * v.y, e);
-      }
+  for (int j = 0; j < 4; ++j) {
+    const int x = 16 * g + 4 * qd + j;
+    fr[j] = fi[j] = SL_BIAS;
+    if (x < nx) {
+      const double2 v = f[(size_t)x * nae];
+      fr[j] = fix_point(v.x, e);
+      fi[j] = fix_point(v.y, e);
     }
-    uint8_t* out = B + ((size_t)k * Ge + g) * 2 * SL_S * nae * 16 + (size_t)t * 16 + 4 * qd;
-#pragma unroll 1
-    for (int s = 0; s < SL_S; ++s) {
-      *reinterpret_cast<unsigned*>(out + (size_t)(merged ? 2 * s : s) * nae * 16) = digits4(fr, s);
-      *reinterpret_cast<unsigned*>(out + (size_t)(merged ? 2 * s + 1 : SL_S + s) * nae * 16) = digits4(fi, s);
-    }
+  }
+  uint8_t* out = B + ((size_t)k * Ge + g) * 2 * SL_S * nae * 16 + (size_t)t * 16 + 4 * qd;
+#pragma unroll 4
+  for (int s = 0; s < SL_S; ++s) {
+    *reinterpret_cast<unsigned*>(out + (size_t)(merged ? 2 * s : s) * nae * 16) = digits4(fr, s);
+    *reinterpret_cast<unsigned*>(out + (size_t)(merged ? 2 * s + 1 : SL_S + s) * nae * 16) = digits4(fi, s);
   }
 }
 
@@ -739,6 +739,7 @@ struct SliceLR {
   SliceGemm g1, g2;        // band -> x, x -> band
   uint8_t *b1 = nullptr, *b2 = nullptr;
   int *e1 = nullptr, *e2 = nullptr;
+  unsigned* mx2 = nullptr;  // magnitude maxima of phi' per (k, column)
   int* d_err = nullptr;
 };
 
@@ -777,7 +778,7 @@ int slice_launch(ocn_ctx* c, const SliceGemm& g, const uint8_t* B, const int* eB
   p.err = c->slice->d_err;
   p.koff = spin * p.nk;
   p.spin = spins == 2 ? spin : -1;
-  slice_fn(g.mode, g.nae)<<<g.grid, SL_THREADS, g.smem, c->stream>>>(p);
+  slice_fn(g.mode, g.nae)<<<g.grid, slice_threads(g.nae), g.smem, c->stream>>>(p);
   ++c->launches;
   OCN_CUDA(c, cudaGetLastError());
   return OCN_OK;
@@ -796,6 +797,7 @@ int slice_init(ocn_ctx* c) {
   int rc;
   if ((rc = salloc(c, &s->b1, s->g1.b_bytes())) || (rc = salloc(c, &s->b2, s->g2.b_bytes())) ||
       (rc = salloc(c, &s->e1, (size_t)c->nk * c->na)) || (rc = salloc(c, &s->e2, (size_t)c->nk * c->na)) ||
+      (rc = salloc(c, &s->mx2, (size_t)c->nk * c->na)) ||
       (rc = salloc(c, &s->d_err, 1)))
     return rc;
   OCN_CUDA(c, cudaMemsetAsync(s->d_err, 0, sizeof(int), c->stream));
@@ -807,7 +809,7 @@ void slice_free(ocn_ctx* c) {
   SliceLR* s = c->slice;
   if (!s) return;
   slice_drop_a(s);
-  for (void* q : {(void*)s->b1, (void*)s->b2, (void*)s->e1, (void*)s->e2, (void*)s->d_err})
+  for (void* q : {(void*)s->b1, (void*)s->b2, (void*)s->e1, (void*)s->e2, (void*)s->mx2, (void*)s->d_err})
     if (q) cudaFree(q);
   delete s;
   c->slice = nullptr;
@@ -859,7 +861,7 @@ int slice_band_to_x(ocn_ctx* c, const double* d_pr, const double* d_pi, double2*
   {
     TimedScope ts(c, T_LR_PREP);
     k_slice_prep_b1<<<c->nk, 256, 0, c->stream>>>(d_pr, d_pi, 0, c->d_allow, c->nb, c->nk, c->na, c->na, s->g1.p.Ge,
-                                                  slice_merged(c->na) ? 1 : 0, s->b1, s->e1);
+                                                  slice_merged(c->na) ? 1 : 0, s->b1, s->e1, s->mx2);
     ++c->launches;
     OCN_CUDA(c, cudaGetLastError());
   }
@@ -869,12 +871,21 @@ int slice_band_to_x(ocn_ctx* c, const double* d_pr, const double* d_pi, double2*
   return OCN_OK;
 }
 
-// d_accpart slices of one vector from phi'[k][x][a].
-int slice_x_to_band(ocn_ctx* c, const double2* phi) {
+// The maxima that slice_x_to_band scales its operand by, cleared by slice_band_to_x.
+unsigned* slice_maxima(ocn_ctx* c) { return c->slice->mx2; }
+
+// d_accpart slices of one vector from phi'[k][x][a]; have_max: the maxima were collected.
+int slice_x_to_band(ocn_ctx* c, const double2* phi, bool have_max) {
   SliceLR* s = c->slice;
   {
     TimedScope ts(c, T_LR_PREP);
-    k_slice_prep_b2<<<c->nk, 512, 0, c->stream>>>(phi, c->nx, c->na, s->g2.p.Ge, slice_merged(c->na) ? 1 : 0, 1.0, s->b2, s->e2);
+    if (!have_max) {
+      k_slice_col_max<<<c->nk, 512, 0, c->stream>>>(phi, c->nx, c->na, s->mx2);
+      ++c->launches;
+    }
+    const int items = s->g2.p.Ge * c->na * 4;
+    k_slice_prep_b2<<<dim3((items + 255) / 256, c->nk), 256, 0, c->stream>>>(
+        phi, c->nx, c->na, s->g2.p.Ge, slice_merged(c->na) ? 1 : 0, s->mx2, s->b2, s->e2);
     ++c->launches;
     OCN_CUDA(c, cudaGetLastError());
   }

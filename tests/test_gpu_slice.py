@@ -1,4 +1,5 @@
-"""FP64 contractions on the FP8 tensor cores (digit slices) against the oracle.
+"""FP64 contractions on the FP8 tensor cores (digit slices) and the fixed-point
+k-mesh transform against the oracle.
 
 The digit sums are exact up to 2^-60 of a row's largest element, so the
 difference is the oracle's own rounding: a sum of K products in binary64 is off by
@@ -37,6 +38,17 @@ CASES = [  # kmesh, bands, xmesh, core_l, nspn
     ((2, 1, 3), 128, (7, 9, 4), 0, 2),    # two spins, a full band tile
     ((2, 2, 1), 137, (6, 6, 8), 1, 2),    # a second band tile of 9 rows
     ((2, 1, 1), 300, (10, 7, 20), 0, 1),  # several K chunks in both contractions, three band tiles
+    # the fixed-point k-mesh transform: every line length, cubic and mixed meshes
+    ((7, 5, 3), 6, (3, 2, 2), 0, 1),
+    ((8, 4, 6), 5, (2, 3, 2), 1, 1),
+    ((1, 8, 7), 5, (2, 2, 3), 0, 1),
+    ((3, 3, 3), 7, (2, 2, 3), 0, 1),
+    ((4, 4, 4), 7, (2, 2, 3), 1, 1),
+    ((5, 5, 5), 7, (2, 2, 3), 0, 1),
+    ((6, 6, 6), 7, (2, 2, 3), 0, 1),
+    ((7, 7, 7), 5, (2, 2, 2), 0, 1),
+    ((8, 8, 8), 5, (2, 2, 2), 1, 1),
+    ((9, 2, 3), 5, (2, 2, 2), 0, 1),      # an axis beyond 8: the FP64-pipe transform
 ]
 
 
