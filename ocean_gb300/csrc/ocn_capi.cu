@@ -52,6 +52,19 @@ int require(ocn_ctx* c) {
   return OCN_OK;
 }
 
+// Multiplet and long-range terms of an FP64 vector, into d_acc and d_accpart.
+int terms_fp64(ocn_ctx* c, const double* pr, const double* pi, bool mult_on, bool lr_on) {
+  int rc;
+  const bool sliced = mult_on && slice_mult_ready(c);
+  if (sliced) {
+    if ((rc = slice_prep_psi(c, pr, pi)) || (rc = slice_mult_apply(c))) return rc;
+  } else if (mult_on) {
+    if ((rc = zero_acc(c, 1)) || (rc = mult_apply(c, pr, pi, c->d_acc))) return rc;
+    c->acc_valid = true;
+  }
+  return lr_on ? lr_apply_fp64(c, pr, pi, sliced) : OCN_OK;
+}
+
 }  // namespace
 
 // H*psi on device vectors (OCEAN_xact, OCEAN_action.f90:286-618).
@@ -64,10 +77,14 @@ int apply_H_impl(ocn_ctx* c, const double* ir, const double* ii, double* orr, do
   c->acc_valid = false;
   const bool mult_on = c->sys.mult && hflag[4] == 1 && c->have_mult;
   const bool lr_on = c->sys.long_range && hflag[0] == 1;
-  if (c->mult_parts > 0) {  // mixed precision with tensor-core multiplet: one psi operand for both
+  if (c->mixed && c->mult_parts > 0) {  // mixed precision with tensor-core multiplet: one psi operand for both
     if ((mult_on || lr_on) && (rc = mixed_prep_b1(c, ir, ii, 0, 1))) return rc;
     if (mult_on && (rc = mult_apply_mixed(c, ir, ii, 0, 1, true))) return rc;
     if (lr_on && (rc = lr_apply_mixed(c, ir, ii, 0, 1, true))) return rc;
+    return combine(c, 1, ir, ii, orr, oi, 0, hflag, backwards);
+  }
+  if (c->dims.precision != OCN_PREC_MIXED) {
+    if ((rc = terms_fp64(c, ir, ii, mult_on, lr_on))) return rc;
     return combine(c, 1, ir, ii, orr, oi, 0, hflag, backwards);
   }
   if (mult_on) {
@@ -75,11 +92,7 @@ int apply_H_impl(ocn_ctx* c, const double* ir, const double* ii, double* orr, do
     if ((rc = mult_apply(c, ir, ii, c->d_acc))) return rc;
     c->acc_valid = true;
   }
-  if (lr_on) {
-    if (c->dims.precision == OCN_PREC_MIXED) rc = lr_apply_mixed(c, ir, ii, 0, 1);
-    else rc = lr_apply_fp64(c, ir, ii);
-    if (rc) return rc;
-  }
+  if (lr_on && (rc = lr_apply_mixed(c, ir, ii, 0, 1))) return rc;
   return combine(c, 1, ir, ii, orr, oi, 0, hflag, backwards);
 }
 
@@ -106,7 +119,7 @@ int apply_H_block_impl(ocn_ctx* c, int nv, const double* in, double* out, const 
   const bool mult_on = c->sys.mult && hflag[4] == 1 && c->have_mult;
   const bool lr_on = c->sys.long_range && hflag[0] == 1;
   bool b1_ready = false;
-  if (c->mult_parts > 0 && mult_on) {
+  if (c->mult_parts > 0 && mult_on) {  // (mixed: FP64 contexts returned above)
     if ((rc = mixed_prep_b1(c, in, in + n, 2 * n, nv)) || (rc = mult_apply_mixed(c, in, in + n, 2 * n, nv, true)))
       return rc;
     b1_ready = true;
@@ -610,8 +623,9 @@ int ocn_set_mult(ocn_ctx* c, const ocn_mult_data* m) {
   OCN_CUDA(c, cudaMemcpy(d.d_nproj, nproj.data(), nl * sizeof(int), cudaMemcpyHostToDevice));
   OCN_CUDA(c, cudaMemcpy(d.d_jbeg, jbeg.data(), nl * sizeof(long long), cudaMemcpyHostToDevice));
   c->have_mult = true;
-  // mixed precision: the projector contractions run on the tensor cores
+  // the projector contractions run on the tensor cores (split BF16, or digit slices in FP64)
   if (c->mixed && (rc = mixed_set_mult(c))) return rc;
+  if ((rc = slice_set_mult(c))) return rc;
   return OCN_OK;
 }
 
@@ -659,23 +673,16 @@ int haydock_iteration(ocn_ctx* c, int nv, double* old, double* psi, double* h, d
   if (mixed_parts(c)) mixed_defer_advance(c, c->d_iter);
   else if ((rc = advance_iter(c, c->d_iter))) return rc;
   c->acc_valid = false;
-  if (c->sys.mult && c->sys.nhflag[4] == 1 && c->have_mult) {
-    if (c->mult_parts > 0) {  // tensor cores; the psi operand was built with the last normalisation
-      if ((rc = mult_apply_mixed(c, psi, psi + n, 2 * n, nv, true))) return rc;
-    } else {
-      if (mixed_parts(c))  // the FP64 multiplet kernels cannot read the double-float vectors
-        return set_err(c, OCN_ERR_STATE, "mixed-precision multiplet operands not built");
-      if ((rc = zero_acc(c, nv))) return rc;
-      for (int v = 0; v < nv; ++v)
-        if ((rc = mult_apply(c, psi + 2 * v * n, psi + 2 * v * n + n, c->d_acc + 2 * v * n))) return rc;
-      c->acc_valid = true;
-    }
-  }
-  if (c->sys.long_range && c->sys.nhflag[0] == 1) {
-    // mixed: the psi operand was built by the previous normalisation (or before the loop)
-    rc = (c->dims.precision == OCN_PREC_MIXED) ? lr_apply_mixed(c, psi, psi + n, 2 * n, nv, true)
-                                               : lr_apply_fp64(c, psi, psi + n);
-    if (rc) return rc;
+  const bool mult_on = c->sys.mult && c->sys.nhflag[4] == 1 && c->have_mult;
+  const bool lr_on = c->sys.long_range && c->sys.nhflag[0] == 1;
+  if (!mixed_parts(c)) {
+    if ((rc = terms_fp64(c, psi, psi + n, mult_on, lr_on))) return rc;
+  } else {
+    // the psi operand was built by the previous normalisation (or before the loop)
+    if (mult_on && c->mult_parts == 0)  // the FP64 multiplet kernels cannot read the double-float vectors
+      return set_err(c, OCN_ERR_STATE, "mixed-precision multiplet operands not built");
+    if (mult_on && (rc = mult_apply_mixed(c, psi, psi + n, 2 * n, nv, true))) return rc;
+    if (lr_on && (rc = lr_apply_mixed(c, psi, psi + n, 2 * n, nv, true))) return rc;
   }
   if (mixed_take_advance(c) && (rc = advance_iter(c, c->d_iter))) return rc;  // no term ran a contraction
   rc = lanczos_launch(c, nv, old, psi, h, ra, ia, rb, cstride, c->d_iter);

@@ -127,7 +127,7 @@ struct ocn_ctx {
   double* d_acc = nullptr;         // full-store accumulator: re plane then im plane (npsi each)
   double* d_accpart = nullptr;     // long-range partials [split][vector][re|im][npsi]
   int lr_xsplit = 1;
-  int mult_parts = 0;              // multiplet partial slices after the LR ones (mixed precision)
+  int mult_parts = 0;              // multiplet partial slices after the LR ones (tensor-core multiplet)
   size_t part_stride = 0;          // elements between two splits of d_accpart
   int nvec = 1;                    // largest psi block
   double* d_vec = nullptr;         // general vector pool (see ocn_solvers.cu)
@@ -249,7 +249,8 @@ double gaunt_threey(int ll, int ml, int lm, int mm, int lr, int mr, int conjug);
 
 // ---- FP64 kernels (ocn_kernels.cu)
 int upload_twiddles(ocn_ctx* c);
-int lr_apply_fp64(ocn_ctx* c, const double* d_pr, const double* d_pi);  // adds into d_acc
+// long-range partials into d_accpart; b1_ready: the digit operand of psi was built
+int lr_apply_fp64(ocn_ctx* c, const double* d_pr, const double* d_pi, bool b1_ready = false);
 int mult_apply(ocn_ctx* c, const double* d_pr, const double* d_pi, double* acc);  // adds into acc
 int mult_hamp(ocn_ctx* c, const double2* amp, double2* hamp);  // one vector, [p][a]
 // base: binary32 partials on the mixed path, FP64 otherwise
@@ -367,9 +368,13 @@ int slice_init(ocn_ctx* c);        // geometry and vector-side buffers; sets lr_
 void slice_free(ocn_ctx* c);
 int slice_set_bloch(ocn_ctx* c);   // digit operands from d_u (not ready when they do not fit)
 bool slice_ready(const ocn_ctx* c);
-int slice_band_to_x(ocn_ctx* c, const double* d_pr, const double* d_pi, double2* phi);  // phi[k][x][a]
+int slice_prep_psi(ocn_ctx* c, const double* d_pr, const double* d_pi);  // operand of the next two
+int slice_band_to_x(ocn_ctx* c, double2* phi);  // phi[k][x][a]
 int slice_x_to_band(ocn_ctx* c, const double2* phi, bool have_max);  // d_accpart slices from phi'[k][x][a]
-unsigned* slice_maxima(ocn_ctx* c);  // [k][a] magnitude maxima of phi', cleared by slice_band_to_x
+unsigned* slice_maxima(ocn_ctx* c);  // [k][a] magnitude maxima of phi', cleared by slice_prep_psi
+int slice_set_mult(ocn_ctx* c);    // digit operands of the projectors (after ocn_set_mult)
+bool slice_mult_ready(const ocn_ctx* c);
+int slice_mult_apply(ocn_ctx* c);  // multiplet term of the prepared psi, into its d_accpart slices
 int slice_check(ocn_ctx* c);       // reads and clears the device timeout flag
 
 // ---- mixed precision (ocn_mixed.cu)
@@ -392,7 +397,7 @@ int haydock_to_df(ocn_ctx* c, double* buf, int nv);
 int mixed_norm_prep(ocn_ctx* c, int nv, const double* psi, double* h, double* ra, double* ia, double* rb,
                     size_t cstride, const int* itp);
 int mixed_check(ocn_ctx* c);       // reads and clears the device timeout flag
-inline int tc_check(ocn_ctx* c) { return c->mixed ? mixed_check(c) : (slice_ready(c) ? slice_check(c) : OCN_OK); }
+inline int tc_check(ocn_ctx* c) { return c->mixed ? mixed_check(c) : (slice_ready(c) || slice_mult_ready(c) ? slice_check(c) : OCN_OK); }
 int mixed_set_starve(ocn_ctx* c, int on);  // test hook of ocn_test_starve_tc
 // multiplet on the tensor cores: operands from c->mult (after ocn_set_mult), and
 // the action's multiplet term of nv vectors into its d_accpart slices

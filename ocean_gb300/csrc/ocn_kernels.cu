@@ -1022,11 +1022,13 @@ int zero_acc(ocn_ctx* c, int nv) {
   return OCN_OK;
 }
 
-int lr_apply_fp64(ocn_ctx* c, const double* d_pr, const double* d_pi) {
+int lr_apply_fp64(ocn_ctx* c, const double* d_pr, const double* d_pi, bool b1_ready) {
   const int nb = c->nb, nk = c->nk, nx = c->nx, na = c->na;
   const bool sliced = slice_ready(c);
   if (sliced) {
-    if (int rc = slice_band_to_x(c, d_pr, d_pi, c->d_phi)) return rc;
+    if (!b1_ready)
+      if (int rc = slice_prep_psi(c, d_pr, d_pi)) return rc;
+    if (int rc = slice_band_to_x(c, c->d_phi)) return rc;
   } else {
     const size_t sm = sizeof(double2) * ((size_t)c->nspn * G1_N * (G1_X + 1) + (size_t)na * G1_N);
     dim3 grid((nx + G1_X - 1) / G1_X, nk);
@@ -1081,7 +1083,9 @@ int lr_wgrad_fp64(ocn_ctx* c, const double* x, const double* y, double2* phi, do
   double2* phy = phi + (size_t)nk * nx * na;
   if (slice_ready(c)) {
     int rc;
-    if ((rc = slice_band_to_x(c, x, x + n, phx)) || (rc = slice_band_to_x(c, y, y + n, phy))) return rc;
+    if ((rc = slice_prep_psi(c, x, x + n)) || (rc = slice_band_to_x(c, phx)) || (rc = slice_prep_psi(c, y, y + n)) ||
+        (rc = slice_band_to_x(c, phy)))
+      return rc;
   } else {
     const size_t sm = sizeof(double2) * ((size_t)c->nspn * G1_N * (G1_X + 1) + (size_t)na * G1_N);
     const dim3 grid((nx + G1_X - 1) / G1_X, nk);

@@ -82,6 +82,7 @@ struct SliceParams {
   double* part;              // x -> band: [split][vector][re|im][npsi]
   size_t part_stride, npsi;
   int nb;
+  int negate;                // x -> band: the long-range term subtracts, the multiplet back-projection adds
   int* err;
 };
 
@@ -424,8 +425,8 @@ __global__ void __launch_bounds__(slice_threads(P == 1 ? C / 2 : C), 1) k_slice_
             const int v = a / p.na;
             double* out = p.part + (size_t)ti.sp * p.part_stride + (size_t)v * 2 * p.npsi;
             const size_t idx = (size_t)r + (size_t)p.nb * ((size_t)ti.k + (size_t)p.nk * (a - v * p.na));
-            out[idx] = -vr;
-            out[p.npsi + idx] = -vi;
+            out[idx] = p.negate ? -vr : vr;
+            out[p.npsi + idx] = p.negate ? -vi : vi;
           }
         }
       }
@@ -665,6 +666,30 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// amp[i] = sum_k part[k][i], i < n (OCEAN_multiplet.f90:1730-1783's sum over k): a CTA
+// owns 32 outputs, its 16 warps take every 16th k, warp 0 adds the partials in order.
+__global__ void __launch_bounds__(512)
+    k_slice_amp_reduce(const double2* __restrict__ part, double2* __restrict__ amp, int nk, int n) {
+  __shared__ double2 sh[16][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
+  double2 s = make_double2(0.0, 0.0);
+  if (i < n)
+    for (int k = w; k < nk; k += 16) {
+      const double2 v = part[(size_t)k * n + i];
+      s.x += v.x;
+      s.y += v.y;
+    }
+  sh[w][lane] = s;
+  __syncthreads();
+  if (w == 0 && i < n) {
+    for (int g = 1; g < 16; ++g) {
+      s.x += sh[g][lane].x;
+      s.y += sh[g][lane].y;
+    }
+    amp[i] = s;
+  }
+}
+
 typedef void (*SliceFn)(const SliceParams);
 SliceFn slice_fn(int mode, int nae) {
   if (mode == 1) return nae == 4 ? k_slice_gemm<1, 8, 1> : (nae == 8 ? k_slice_gemm<1, 16, 1> : k_slice_gemm<1, 12, 2>);
@@ -740,6 +765,13 @@ struct SliceLR {
   uint8_t *b1 = nullptr, *b2 = nullptr;
   int *e1 = nullptr, *e2 = nullptr;
   unsigned* mx2 = nullptr;  // magnitude maxima of phi' per (k, column)
+  // multiplet projectors (fg_combo): amplitudes and back-projection
+  bool mult_ready = false;
+  SliceGemm gm1, gm2;
+  uint8_t* bm = nullptr;
+  int* em = nullptr;
+  unsigned* mxm = nullptr;
+  double2* amp_part = nullptr;  // [k][p][a]
   int* d_err = nullptr;
 };
 
@@ -762,6 +794,54 @@ void slice_drop_a(SliceLR* s) {
   s->ready = false;
 }
 
+void slice_drop_mult(SliceLR* s) {
+  for (SliceGemm* g : {&s->gm1, &s->gm2}) {
+    if (g->A) cudaFree(g->A);
+    if (g->eA) cudaFree(g->eA);
+    g->A = nullptr;
+    g->eA = nullptr;
+  }
+  for (void* q : {(void*)s->bm, (void*)s->em, (void*)s->mxm, (void*)s->amp_part})
+    if (q) cudaFree(q);
+  s->bm = nullptr;
+  s->em = nullptr;
+  s->mxm = nullptr;
+  s->amp_part = nullptr;
+  s->mult_ready = false;
+}
+
+// Digits and exponents of both operands of one spin from src (element (x, k, n) at x*sx + k*sk + n).
+int slice_build(ocn_ctx* c, const double2* src, size_t sx, size_t sk, int nx, const SliceGemm& g1, const SliceGemm& g2,
+                int spin) {
+  const int nk = c->nk, nb = c->nb, blocks = 16 * c->sm_count;
+  int* e1 = g1.eA + (size_t)spin * nk * nx;
+  int* e2 = g2.eA + (size_t)spin * nk * nb;
+  const long long warps = (long long)nk * nx;
+  k_slice_exp_rows<<<(unsigned)((warps + 7) / 8), 256, 0, c->stream>>>(src, sx, sk, nb, nk, nx, e1);
+  k_slice_build_rows<<<blocks, 256, 0, c->stream>>>(src, sx, sk, nb, g1.p, e1, g1.A, spin * nk);
+  k_slice_exp_cols<<<dim3((nb + 31) / 32, nk), dim3(32, 8), 0, c->stream>>>(src, sx, sk, nb, nk, nx, e2);
+  k_slice_build_cols<<<blocks, 256, 0, c->stream>>>(src, sx, sk, nx, g2.p, e2, g2.A, spin * nk);
+  c->launches += 4;
+  OCN_CUDA(c, cudaGetLastError());
+  return OCN_OK;
+}
+
+// Allocates the A operands of both contractions; false (nothing kept) when they
+// would take more than a quarter of the free device memory.
+bool slice_alloc_a(ocn_ctx* c, SliceGemm* g1, SliceGemm* g2, int nx) {
+  const int ns = c->nspn;
+  size_t fr = 0, tot = 0;
+  if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return false;
+  if (g1->a_bytes(ns) + g2->a_bytes(ns) > fr / 4) return false;
+  if (salloc(c, &g1->A, g1->a_bytes(ns)) || salloc(c, &g2->A, g2->a_bytes(ns)) ||
+      salloc(c, &g1->eA, (size_t)ns * c->nk * nx) || salloc(c, &g2->eA, (size_t)ns * c->nk * c->nb)) {
+    (void)cudaGetLastError();
+    c->err.clear();
+    return false;
+  }
+  return true;
+}
+
 int slice_launch(ocn_ctx* c, const SliceGemm& g, const uint8_t* B, const int* eB, double2* phi, double* part, int spin,
                  int spins) {
   SliceParams p = g.p;
@@ -778,6 +858,7 @@ int slice_launch(ocn_ctx* c, const SliceGemm& g, const uint8_t* B, const int* eB
   p.err = c->slice->d_err;
   p.koff = spin * p.nk;
   p.spin = spins == 2 ? spin : -1;
+  p.negate = p.bshared ? 0 : 1;
   slice_fn(g.mode, g.nae)<<<g.grid, slice_threads(g.nae), g.smem, c->stream>>>(p);
   ++c->launches;
   OCN_CUDA(c, cudaGetLastError());
@@ -809,6 +890,7 @@ void slice_free(ocn_ctx* c) {
   SliceLR* s = c->slice;
   if (!s) return;
   slice_drop_a(s);
+  slice_drop_mult(s);
   for (void* q : {(void*)s->b1, (void*)s->b2, (void*)s->e1, (void*)s->e2, (void*)s->mx2, (void*)s->d_err})
     if (q) cudaFree(q);
   delete s;
@@ -823,55 +905,104 @@ bool slice_ready(const ocn_ctx* c) { return c->slice && c->slice->ready; }
 int slice_set_bloch(ocn_ctx* c) {
   SliceLR* s = c->slice;
   if (!s) return OCN_OK;
-  const int ns = c->nspn;
-  if (!s->g1.A) {
-    size_t fr = 0, tot = 0;
-    OCN_CUDA(c, cudaMemGetInfo(&fr, &tot));
-    if (s->g1.a_bytes(ns) + s->g2.a_bytes(ns) > fr / 4) return OCN_OK;
-    if (salloc(c, &s->g1.A, s->g1.a_bytes(ns)) || salloc(c, &s->g2.A, s->g2.a_bytes(ns)) ||
-        salloc(c, &s->g1.eA, (size_t)ns * c->nk * c->nx) || salloc(c, &s->g2.eA, (size_t)ns * c->nk * c->nb)) {
-      slice_drop_a(s);
-      (void)cudaGetLastError();
-      c->err.clear();
-      return OCN_OK;
-    }
+  if (!s->g1.A && !slice_alloc_a(c, &s->g1, &s->g2, c->nx)) {
+    slice_drop_a(s);
+    return OCN_OK;
   }
   const size_t sx = (size_t)c->nk * c->nb, sk = c->nb;
-  const int blocks = 16 * c->sm_count;
-  for (int sp = 0; sp < ns; ++sp) {
-    const double2* u = c->d_u + (size_t)sp * c->nx * sx;
-    int* e1 = s->g1.eA + (size_t)sp * c->nk * c->nx;
-    int* e2 = s->g2.eA + (size_t)sp * c->nk * c->nb;
-    const long long warps = (long long)c->nk * c->nx;
-    k_slice_exp_rows<<<(unsigned)((warps + 7) / 8), 256, 0, c->stream>>>(u, sx, sk, c->nb, c->nk, c->nx, e1);
-    k_slice_build_rows<<<blocks, 256, 0, c->stream>>>(u, sx, sk, c->nb, s->g1.p, e1, s->g1.A, sp * c->nk);
-    k_slice_exp_cols<<<dim3((c->nb + 31) / 32, c->nk), dim3(32, 8), 0, c->stream>>>(u, sx, sk, c->nb, c->nk, c->nx, e2);
-    k_slice_build_cols<<<blocks, 256, 0, c->stream>>>(u, sx, sk, c->nx, s->g2.p, e2, s->g2.A, sp * c->nk);
-    c->launches += 4;
-    OCN_CUDA(c, cudaGetLastError());
-  }
+  for (int sp = 0; sp < c->nspn; ++sp)
+    if (int rc = slice_build(c, c->d_u + (size_t)sp * c->nx * sx, sx, sk, c->nx, s->g1, s->g2, sp)) return rc;
   OCN_CUDA(c, cudaStreamSynchronize(c->stream));
   s->ready = true;
   return OCN_OK;
 }
 
-// phi[k][x][a] of one vector (FP64 planes).
-int slice_band_to_x(ocn_ctx* c, const double* d_pr, const double* d_pi, double2* phi) {
+// Digit operands of the projector coefficients c->mult.mpc [s][p][k*Nb + n]: the
+// amplitudes are the band -> x contraction with the projectors in place of x, the
+// back-projection the x -> band one with an operand shared by every k.  Grows the
+// partial sums by the back-projection's slices.  Without the memory the context
+// keeps the FP64-pipe multiplet kernels.  2p, 6^3 k / 64 bands / 128 projectors: the
+// whole term 1200 us on the FP64 pipe (170 M complex multiply-adds) -> 92 us, a
+// quarter of it the direct and exchange matrices (k_mult_hamp).
+int slice_set_mult(ocn_ctx* c) {
   SliceLR* s = c->slice;
-  {
-    TimedScope ts(c, T_LR_PREP);
-    k_slice_prep_b1<<<c->nk, 256, 0, c->stream>>>(d_pr, d_pi, 0, c->d_allow, c->nb, c->nk, c->na, c->na, s->g1.p.Ge,
-                                                  slice_merged(c->na) ? 1 : 0, s->b1, s->e1, s->mx2);
-    ++c->launches;
-    OCN_CUDA(c, cudaGetLastError());
+  if (!s) return OCN_OK;
+  slice_drop_mult(s);
+  c->mult_parts = 0;
+  const int np = c->mult.np;
+  if (np == 0) return OCN_OK;
+  slice_plan(&s->gm1, 1, c->na, c->nk, np, 2 * c->nb, c->sm_count);
+  slice_plan(&s->gm2, 2, c->na, c->nk, c->nb, np, c->sm_count);
+  s->gm2.p.bshared = 1;
+  double* parts = nullptr;
+  if (!slice_alloc_a(c, &s->gm1, &s->gm2, np) || salloc(c, &s->bm, s->gm2.b_bytes()) || salloc(c, &s->em, c->na) ||
+      salloc(c, &s->mxm, c->na) || salloc(c, &s->amp_part, (size_t)c->nk * np * c->na) ||
+      salloc(c, &parts, (size_t)(c->lr_xsplit + s->gm2.p.ks) * c->part_stride)) {
+    slice_drop_mult(s);
+    (void)cudaGetLastError();
+    c->err.clear();
+    return OCN_OK;
   }
+  OCN_CUDA(c, cudaStreamSynchronize(c->stream));
+  cudaFree(c->d_accpart);
+  c->d_accpart = parts;
+  c->mult_parts = s->gm2.p.ks;
+  const size_t nbk = (size_t)c->nb * c->nk;
+  for (int sp = 0; sp < c->nspn; ++sp)
+    if (int rc = slice_build(c, c->mult.mpc + (size_t)sp * np * nbk, nbk, c->nb, np, s->gm1, s->gm2, sp)) return rc;
+  OCN_CUDA(c, cudaStreamSynchronize(c->stream));
+  s->mult_ready = true;
+  return OCN_OK;
+}
+
+bool slice_mult_ready(const ocn_ctx* c) { return c->slice && c->slice->mult_ready; }
+
+// psi operand of one vector (FP64 planes), shared by the amplitudes and band -> x.
+int slice_prep_psi(ocn_ctx* c, const double* d_pr, const double* d_pi) {
+  SliceLR* s = c->slice;
+  TimedScope ts(c, T_LR_PREP);
+  k_slice_prep_b1<<<c->nk, 256, 0, c->stream>>>(d_pr, d_pi, 0, c->d_allow, c->nb, c->nk, c->na, c->na, s->g1.p.Ge,
+                                                slice_merged(c->na) ? 1 : 0, s->b1, s->e1, s->mx2);
+  ++c->launches;
+  OCN_CUDA(c, cudaGetLastError());
+  return OCN_OK;
+}
+
+// The multiplet term of the vector whose operand is in b1, into its d_accpart slices.
+int slice_mult_apply(ocn_ctx* c) {
+  SliceLR* s = c->slice;
+  MultDev& m = c->mult;
+  TimedScope ts(c, T_MULT);
+  int rc;
+  for (int sp = 0; sp < c->nspn; ++sp)
+    if ((rc = slice_launch(c, s->gm1, s->b1, s->e1, s->amp_part, nullptr, sp, c->nspn))) return rc;
+  const int n = m.np * c->na;
+  k_slice_amp_reduce<<<(n + 31) / 32, 512, 0, c->stream>>>(s->amp_part, m.amp, c->nk, n);
+  ++c->launches;
+  OCN_CUDA(c, cudaGetLastError());
+  if ((rc = mult_hamp(c, m.amp, m.hamp))) return rc;
+  k_slice_col_max<<<1, 512, 0, c->stream>>>(m.hamp, m.np, c->na, s->mxm);
+  const int items = s->gm2.p.Ge * c->na * 4;
+  k_slice_prep_b2<<<dim3((items + 255) / 256, 1), 256, 0, c->stream>>>(m.hamp, m.np, c->na, s->gm2.p.Ge,
+                                                                      slice_merged(c->na) ? 1 : 0, s->mxm, s->bm, s->em);
+  c->launches += 2;
+  OCN_CUDA(c, cudaGetLastError());
+  double* part = c->d_accpart + (size_t)c->lr_xsplit * c->part_stride;
+  for (int sp = 0; sp < c->nspn; ++sp)
+    if ((rc = slice_launch(c, s->gm2, s->bm, s->em, nullptr, part, sp, c->nspn))) return rc;
+  return OCN_OK;
+}
+
+// phi[k][x][a] of the vector whose operand is in b1.
+int slice_band_to_x(ocn_ctx* c, double2* phi) {
+  SliceLR* s = c->slice;
   TimedScope ts(c, T_LR_GEMM1);
   for (int sp = 0; sp < c->nspn; ++sp)
     if (int rc = slice_launch(c, s->g1, s->b1, s->e1, phi, nullptr, sp, c->nspn)) return rc;
   return OCN_OK;
 }
 
-// The maxima that slice_x_to_band scales its operand by, cleared by slice_band_to_x.
+// The maxima that slice_x_to_band scales its operand by, cleared by slice_prep_psi.
 unsigned* slice_maxima(ocn_ctx* c) { return c->slice->mx2; }
 
 // d_accpart slices of one vector from phi'[k][x][a]; have_max: the maxima were collected.
