@@ -31,6 +31,7 @@ SOURCES = {
     "ocn_slice.cu": [],
     "ocn_fixfft.cu": [],
     "ocn_valence.cu": [],
+    "ocn_val_fx.cu": [],
     "ocn_setup.cpp": [],
     "ocn_io.cpp": [],
 }

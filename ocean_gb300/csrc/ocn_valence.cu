@@ -72,6 +72,9 @@ struct ocn_val_ctx {
   float2* d_val32 = nullptr;
   void* d_valT = nullptr;     // [y][v][k], double2 or float2
   void* d_lad = nullptr;      // [y][x][k], double or float
+  bool fx = false;            // FP64 direct term in fixed point: d_valT holds split halves, d_lad integers
+  int* d_eV = nullptr;        // fx: exponents of val per (spin, y) and of the ladder per (y, x)
+  int* d_eL = nullptr;
   double* d_bub = nullptr;    // [x]
   double* d_fxc = nullptr;    // [x] ALDA kernel; set: the f_xc term is on (OCEAN_fxc_act)
   bool have_fxc = false;
@@ -903,32 +906,7 @@ cudaError_t raise_smem_limit(const void* fn, size_t optin) {
   return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room);
 }
 
-// y-tile from the shared-memory budget (two CTAs per SM where it fits), and
-// enough y-ranges per x-point for about two waves of CTAs.
-template <typename R>
-int plan_ladder(ocn_val_ctx* c) {
-  int ytile = 16;
-  // cubic kernel: in FP32 two x-points per CTA and the largest y-tile that
-  // leaves two CTAs per SM (measured on the 8^3 k-mesh, 10^3 x-mesh case: 5.9 ms
-  // per H psi with one x-point and 56 KB, 5.2 ms with two and 56 KB, 5.0 ms with
-  // two and 110 KB); in FP64 two x-points spill registers (85 -> 104 ms), so one
-  c->xper = (use_cube_kernel(c) && c->nx >= 2 && sizeof(R) == 4) ? 2 : 1;
-  const size_t target = std::min<size_t>(c->smem_optin, 110 * 1024);
-  // two x-points' A must fit with at least a one-y tile, else one x-point per CTA
-  if (c->xper == 2 && ladder_smem<R>(c, 1) > c->smem_optin) c->xper = 1;
-  while (ytile > 1 && ladder_smem<R>(c, ytile) > target) --ytile;
-  if (ladder_smem<R>(c, ytile) > c->smem_optin)
-    return vset_err(c, OCN_ERR_UNSUPPORTED,
-                    "ocn_val: Nv*Nk too large for the direct-term kernel's shared memory");
-  c->ytile = ytile;
-  c->lad_smem = ladder_smem<R>(c, ytile);
-  const bool cube = use_cube_kernel(c);
-  const void* fn = cube ? (const void*)ladder_cube_fn<R>(c) : (const void*)ladder_fn<R>(c);
-  cudaError_t e = raise_smem_limit(fn, c->smem_optin);
-  if (e != cudaSuccess) return vcuda(c, e, "cudaFuncSetAttribute(kv_ladder)");
-  int per_sm = 1;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, VAL_THREADS, c->lad_smem);
-  if (e != cudaSuccess) return vcuda(c, e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor(kv_ladder)");
+int plan_yranges(ocn_val_ctx* c, int per_sm, int ytile) {
   // y-ranges per x-point: the split (up to 8, ranges no shorter than a tile)
   // whose CTA count fills the last wave best
   const double slots = (double)std::max(1, per_sm) * c->sm_count;
@@ -947,6 +925,44 @@ int plan_ladder(ocn_val_ctx* c) {
   c->yper = (c->nx + best - 1) / best;
   c->ysplit = (c->nx + c->yper - 1) / c->yper;
   return OCN_OK;
+}
+
+// y-tile from the shared-memory budget (two CTAs per SM where it fits), and
+// enough y-ranges per x-point for about two waves of CTAs.
+template <typename R>
+int plan_ladder(ocn_val_ctx* c) {
+  int ytile = 16;
+  int per_sm = 1;
+  c->fx = sizeof(R) == 8 && ocn::val_fx_supported(c->dims.kmesh, c->nv, c->smem_optin);
+  if (c->fx) {
+    c->xper = 1;
+    ytile = 4;
+    c->ytile = ytile;
+    cudaError_t e = ocn::val_fx_plan(c->dims.kmesh, c->nv, c->smem_optin, &per_sm);
+    if (e != cudaSuccess) return vcuda(c, e, "plan of the fixed-point direct term");
+    return plan_yranges(c, per_sm, ytile);
+  }
+  // cubic kernel: in FP32 two x-points per CTA and the largest y-tile that
+  // leaves two CTAs per SM (measured on the 8^3 k-mesh, 10^3 x-mesh case: 5.9 ms
+  // per H psi with one x-point and 56 KB, 5.2 ms with two and 56 KB, 5.0 ms with
+  // two and 110 KB); in FP64 two x-points spill registers (85 -> 104 ms), so one
+  c->xper = (use_cube_kernel(c) && c->nx >= 2 && sizeof(R) == 4) ? 2 : 1;
+  const size_t target = std::min<size_t>(c->smem_optin, 110 * 1024);
+  // two x-points' A must fit with at least a one-y tile, else one x-point per CTA
+  if (c->xper == 2 && ladder_smem<R>(c, 1) > c->smem_optin) c->xper = 1;
+  while (ytile > 1 && ladder_smem<R>(c, ytile) > target) --ytile;
+  if (ladder_smem<R>(c, ytile) > c->smem_optin)
+    return vset_err(c, OCN_ERR_UNSUPPORTED,
+                    "ocn_val: Nv*Nk too large for the direct-term kernel's shared memory");
+  c->ytile = ytile;
+  c->lad_smem = ladder_smem<R>(c, ytile);
+  const bool cube = use_cube_kernel(c);
+  const void* fn = cube ? (const void*)ladder_cube_fn<R>(c) : (const void*)ladder_fn<R>(c);
+  cudaError_t e = raise_smem_limit(fn, c->smem_optin);
+  if (e != cudaSuccess) return vcuda(c, e, "cudaFuncSetAttribute(kv_ladder)");
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, VAL_THREADS, c->lad_smem);
+  if (e != cudaSuccess) return vcuda(c, e, "cudaOccupancyMaxActiveBlocksPerMultiprocessor(kv_ladder)");
+  return plan_yranges(c, per_sm, ytile);
 }
 
 size_t final_xchunk(const ocn_val_ctx* c) {
@@ -1031,7 +1047,11 @@ int apply_impl(ocn_val_ctx* c, const double* d_in, double* d_out, const int flag
         const CT* tw;
         if constexpr (sizeof(R) == 4) tw = c->d_twk32;
         else tw = c->d_twk;
-        if (use_cube_kernel(c))
+        if (c->fx) {
+          if constexpr (sizeof(R) == 8)
+            ocn::val_fx_apply(c->dims.kmesh, c->nv, c->nx, c->yper, c->ysplit, A, valT_s(sv), c->d_eV + (size_t)sv * c->nx,
+                              c->d_lad, c->d_eL, Bp + b * bp_blk, c->stream);
+        } else if (use_cube_kernel(c))
           ladder_cube_fn<R>(c)<<<dim3((c->nx + c->xper - 1) / c->xper, c->ysplit), VAL_THREADS, c->lad_smem,
                                  c->stream>>>(A, valT_s(sv), static_cast<const R*>(c->d_lad), Bp + b * bp_blk, c->nv,
                                               c->nx, c->ytile, c->yper, tw);
@@ -1142,6 +1162,8 @@ int ocn_val_create(const ocn_val_dims* d, ocn_val_ctx** out) {
                    nxk * c->nv * c->ysplit * cs * c->vspin * c->vspin)) ||
       (rc = valloc(c, &c->d_vec, 8 * c->npsi)) || (rc = valloc(c, &c->d_red, 4 * (size_t)c->red_blocks)))
     return fail(rc);
+  if (c->fx && ((rc = valloc(c, &c->d_eV, (size_t)c->nx * c->nspn)) || (rc = valloc(c, &c->d_eL, (size_t)c->nx * c->nx))))
+    return fail(rc);
   if (c->mixed && ((rc = valloc(c, &c->d_con32, nxk * c->nc * c->nspn)) ||
                    (rc = valloc(c, &c->d_val32, nxk * c->nv * c->nspn))))
     return fail(rc);
@@ -1180,7 +1202,7 @@ int ocn_val_destroy(ocn_val_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   void* bufs[] = {c->d_er, c->d_ei, c->d_allow, c->d_con, c->d_val, c->d_con32, c->d_val32, c->d_valT, c->d_lad, c->d_bub,
                   c->d_fxc, c->d_twk, c->d_twk32, c->d_twx, c->d_lp, c->d_s, c->d_A, c->d_Bp, c->d_vec, c->d_red,
-                  c->d_coef};
+                  c->d_coef, c->d_eV, c->d_eL};
   for (void* p : bufs)
     if (p) cudaFree(p);
   if (c->stream) cudaStreamDestroy(c->stream);
@@ -1282,6 +1304,10 @@ static int set_states_impl(ocn_val_ctx* c, const double* conr, const double* con
     kv_to_float<<<g, 256, 0, c->stream>>>(reinterpret_cast<const double*>(c->d_val), 2 * nval,
                                           reinterpret_cast<float*>(c->d_val32));
   }
+  else if (c->fx)
+    for (int sp = 0; sp < c->nspn; ++sp)
+      ocn::val_fx_states(c->d_val + sp * nval1, c->nv, c->nk, c->nx, static_cast<double2*>(c->d_valT) + sp * nval1,
+                         c->d_eV + (size_t)sp * c->nx, c->stream);
   else
     for (int sp = 0; sp < c->nspn; ++sp)
       kv_transpose_val<double><<<g, 256, 0, c->stream>>>(c->d_val + sp * nval1, c->nv, c->nk, c->nx,
@@ -1317,6 +1343,10 @@ static int set_ladder_impl(ocn_val_ctx* c, const double* lad, bool on_device) {
   if (!c->mixed) {
     VCUDA(c, cudaMemcpyAsync(c->d_lad, lad, sizeof(double) * n,
                              on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, c->stream));
+    if (c->fx) {
+      ocn::val_fx_ladder(static_cast<double*>(c->d_lad), (size_t)c->nx * c->nx, c->nk, c->d_eL, c->sm_count, c->stream);
+      VCUDA(c, cudaGetLastError());
+    }
   } else if (on_device) {
     kv_to_float<<<4 * c->sm_count, 256, 0, c->stream>>>(lad, n, static_cast<float*>(c->d_lad));
     VCUDA(c, cudaGetLastError());
