@@ -504,7 +504,8 @@ __device__ __forceinline__ void combine_df_body(const float2* __restrict__ pr, c
 }
 
 template <int NA, bool SO>
-__global__ void __launch_bounds__(LZ_DF_THREADS)
+// two CTAs per SM: at 101 registers one fitted, and the kernel waits on memory
+__global__ void __launch_bounds__(LZ_DF_THREADS, 2)
     k_combine_df(const float2* __restrict__ pr, const float2* __restrict__ pi, const float2* __restrict__ er,
                  const float2* __restrict__ ei, const float* __restrict__ allow, const float* __restrict__ part,
                  int nparts, const float2* __restrict__ so, float2* __restrict__ outr, float2* __restrict__ outi,
@@ -520,7 +521,7 @@ __global__ void __launch_bounds__(LZ_DF_THREADS)
 // contexts); every context keeps the block partition (and so the reduction
 // order) of its own launches.
 template <int NA, bool SO>
-__global__ void __launch_bounds__(LZ_DF_THREADS) k_combine_df_group(const CombineArgs* __restrict__ tab) {
+__global__ void __launch_bounds__(LZ_DF_THREADS, 2) k_combine_df_group(const CombineArgs* __restrict__ tab) {
   const CombineArgs& a = tab[blockIdx.z];
   if ((int)blockIdx.y >= a.nv || (int)blockIdx.x >= a.nblk) return;
   combine_df_body<NA, SO>(reinterpret_cast<const float2*>(a.pr), reinterpret_cast<const float2*>(a.pi), a.er_df,

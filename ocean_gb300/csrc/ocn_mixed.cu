@@ -467,6 +467,13 @@ __device__ __forceinline__ uint32_t pack_bf16(__nv_bfloat16 a, __nv_bfloat16 b) 
   return (uint32_t)__bfloat16_as_ushort(a) | ((uint32_t)__bfloat16_as_ushort(b) << 16);
 }
 
+// (a, b) split: hi = (bf16(a), bf16(b)) in the (low, high) half words, lo the same of the residuals
+__device__ __forceinline__ void split_bf16x2(float a, float b, uint32_t& hi, uint32_t& lo) {
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(b), "f"(a));
+  const float ra = a - __uint_as_float(hi << 16), rb = b - __uint_as_float(hi & 0xffff0000u);
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(rb), "f"(ra));
+}
+
 // UA_s[k][x][K1]: K < Nb -> Re u(n=K), else Im u(n=K-Nb)   (from u [x][k][n])
 __global__ void k_build_ua(const double2* __restrict__ u, __nv_bfloat16* __restrict__ hi,
                            __nv_bfloat16* __restrict__ lo, int nb, int nk, int nx, int p1) {
@@ -657,8 +664,10 @@ __global__ void k_prep_b3(const double2* __restrict__ hamp, __nv_bfloat16* __res
 // combine's double-float partials, a + i ia = <h|psi> and b_i^2 = |h - a psi|^2 =
 // |h|^2 - 2 a Re<h|psi> + a^2 |psi|^2 (formed in FP64 by one thread and broadcast,
 // so h is read once); psi = (h - a psi) / b_i written in place of h, and B1 rows of
-// vector v built from allow o psi.  One thread per (n, k) covers both K = n and
-// K = Nb + n for every alpha.  Every CTA sums the partials in the same order.
+// vector v built from allow o psi.  One thread per (n, k, alpha) covers both K = n
+// and K = Nb + n; its first element is loaded before the partials are added, so the
+// two latencies overlap (a thread per (n, k) that walked the alphas one after another
+// left two thirds of the grid idle).  Every CTA sums the partials in the same order.
 __device__ __forceinline__ void norm_prep_body(const double* __restrict__ red1, int nblk, size_t rstride,
                             double* __restrict__ hbase, const double* __restrict__ pbase, size_t vstride,
                             size_t npsi, const float* __restrict__ allow, __nv_bfloat16* __restrict__ b1, int nb,
@@ -668,14 +677,29 @@ __device__ __forceinline__ void norm_prep_body(const double* __restrict__ red1, 
   __shared__ float2 sh[4][32];
   __shared__ float2 s_am, s_inv;
   const int vv = by;
+  float2* hr = reinterpret_cast<float2*>(hbase + (size_t)vv * vstride);
+  float2* hi = hr + npsi;
+  const float2* pr = reinterpret_cast<const float2*>(pbase + (size_t)vv * vstride);
+  const float2* pi = pr + npsi;
+  const int n_all = (int)npsi, stride = nbx * blockDim.x;
+  int i = bx * blockDim.x + threadIdx.x;
+  float2 h0r{0.0f, 0.0f}, h0i{0.0f, 0.0f}, p0r{0.0f, 0.0f}, p0i{0.0f, 0.0f};
+  float m0 = 0.0f;
+  if (i < n_all) {
+    h0r = hr[i];
+    h0i = hi[i];
+    p0r = pr[i];
+    p0i = pi[i];
+    m0 = allow[i];
+  }
   const float2* r1 = reinterpret_cast<const float2*>(red1 + (size_t)vv * rstride);  // <h|psi> pairs
   const float2* r2 = r1 + 2 * nblk;                                                // |h|^2, |psi|^2 pairs
   df q[4] = {df{0.0f, 0.0f}, df{0.0f, 0.0f}, df{0.0f, 0.0f}, df{0.0f, 0.0f}};
-  for (int i = threadIdx.x; i < nblk; i += blockDim.x) {
-    q[0] = df_add(q[0], df{r1[2 * i].x, r1[2 * i].y});
-    q[1] = df_add(q[1], df{r1[2 * i + 1].x, r1[2 * i + 1].y});
-    q[2] = df_add(q[2], df{r2[2 * i].x, r2[2 * i].y});
-    q[3] = df_add(q[3], df{r2[2 * i + 1].x, r2[2 * i + 1].y});
+  for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
+    q[0] = df_add(q[0], df{r1[2 * b].x, r1[2 * b].y});
+    q[1] = df_add(q[1], df{r1[2 * b + 1].x, r1[2 * b + 1].y});
+    q[2] = df_add(q[2], df{r2[2 * b].x, r2[2 * b].y});
+    q[3] = df_add(q[3], df{r2[2 * b + 1].x, r2[2 * b + 1].y});
   }
 #pragma unroll
   for (int j = 0; j < 4; ++j)
@@ -710,37 +734,36 @@ __device__ __forceinline__ void norm_prep_body(const double* __restrict__ red1, 
   }
   __syncthreads();
   const df am{s_am.x, s_am.y}, inv{s_inv.x, s_inv.y};
-  float2* hr = reinterpret_cast<float2*>(hbase + (size_t)vv * vstride);
-  float2* hi = hr + npsi;
-  const float2* pr = reinterpret_cast<const float2*>(pbase + (size_t)vv * vstride);
-  const float2* pi = pr + npsi;
-  const int g4 = 4 * na;
-  const int total = nb * nk;
-  for (int i = bx * blockDim.x + threadIdx.x; i < total; i += nbx * blockDim.x) {
-    const int n = i % nb;
-    const int k = i / nb;
-    __nv_bfloat16* base = b1 + (size_t)k * ncol * p1 + (size_t)vv * g4 * p1;
-    for (int a = 0; a < na; ++a) {
-      const size_t idx = (size_t)i + (size_t)total * a;
-      const df r = df_mul(df_add(df_ld(hr, idx), df_mul(am, df_ld(pr, idx))), inv);
-      const df im = df_mul(df_add(df_ld(hi, idx), df_mul(am, df_ld(pi, idx))), inv);
-      df_st(hr, idx, r);
-      df_st(hi, idx, im);
-      const float m = allow[idx];
-      const float qr = df_to_float(r) * m, qi = df_to_float(im) * m;
-      __nv_bfloat16 h0, l0, h1, l1, h2, l2;
-      split_bf16(qr, h0, l0);
-      split_bf16(qi, h1, l1);
-      split_bf16(-qi, h2, l2);
-      // K = n (c = 0): part 0 <- qr, part 1 <- qi;  K = Nb + n (c = 1): part 0 <- -qi, part 1 <- qr
-      base[(size_t)(a)*p1 + n] = h0;
-      base[(size_t)(na + a) * p1 + n] = h1;
-      base[(size_t)(2 * na + a) * p1 + n] = l0;
-      base[(size_t)(3 * na + a) * p1 + n] = l1;
-      base[(size_t)(a)*p1 + nb + n] = h2;
-      base[(size_t)(na + a) * p1 + nb + n] = h0;
-      base[(size_t)(2 * na + a) * p1 + nb + n] = l2;
-      base[(size_t)(3 * na + a) * p1 + nb + n] = l0;
+  const int g4 = 4 * na, total = nb * nk;
+  while (i < n_all) {
+    const int a = i / total, e = i - a * total;
+    const int k = e / nb, n = e - k * nb;
+    const df r = df_mul(df_add(df{h0r.x, h0r.y}, df_mul(am, df{p0r.x, p0r.y})), inv);
+    const df im = df_mul(df_add(df{h0i.x, h0i.y}, df_mul(am, df{p0i.x, p0i.y})), inv);
+    df_st(hr, i, r);
+    df_st(hi, i, im);
+    const float qr = df_to_float(r) * m0, qi = df_to_float(im) * m0;
+    __nv_bfloat16 h0, l0, h1, l1;
+    split_bf16(qr, h0, l0);
+    split_bf16(qi, h1, l1);
+    // K = n (c = 0): part 0 <- qr, part 1 <- qi;  K = Nb + n (c = 1): part 0 <- -qi, part 1 <- qr
+    __nv_bfloat16* base = b1 + (size_t)k * ncol * p1 + ((size_t)vv * g4 + a) * p1 + n;
+    const size_t rp = (size_t)na * p1;  // between the (split, part) groups of rows
+    base[0] = h0;
+    base[rp] = h1;
+    base[2 * rp] = l0;
+    base[3 * rp] = l1;
+    base[nb] = __hneg(h1);
+    base[rp + nb] = h0;
+    base[2 * rp + nb] = __hneg(l1);
+    base[3 * rp + nb] = l0;
+    i += stride;
+    if (i < n_all) {
+      h0r = hr[i];
+      h0i = hi[i];
+      p0r = pr[i];
+      p0i = pi[i];
+      m0 = allow[i];
     }
   }
 }
@@ -968,11 +991,19 @@ __device__ __forceinline__ void fft_b2_cube_body(const float2* __restrict__ phi,
   __syncthreads();
   // E: forward along k1 and the B2 columns.  Lane q of a group of 4 writes word q
   // = (split s, part) = (q / 2, q % 2) of the group's 4 alphas: for Na = 4 the 4
-  // lanes write one 32-byte row segment.  Every lane of the warp takes part in
-  // the shuffles (tasks is a multiple of 4; idle lanes carry zeros).
+  // lanes write one 32-byte row segment.  Every lane splits its own transform once,
+  // packs (re, im) of the high and of the low halves in a word each, and gets the
+  // other three transforms' words of its split s by a 4 x 4 exchange (3 shuffles); byte
+  // permutes then pick re or im, and the sign of -re is a bit flip.  (Splitting all
+  // four transforms in every lane took four times the conversions: 32 -> 27 us for
+  // the 6912 transforms of the 8^3 k / 12^3 x case.)  Every lane of the warp takes
+  // part in the shuffles (tasks is a multiple of 4; idle lanes carry zeros).
   const float norm = 1.0f / (float)NK;
   const int row_x = ((x >> 6) << 7) + (x & 63);
   const int lane = threadIdx.x & 31, q = lane & 3, s = q >> 1, part = q & 1;
+  const uint32_t sel0 = part ? 0x3276u : 0x5410u;  // c = 0: re (part 0) or im (part 1) of two transforms
+  const uint32_t sel1 = part ? 0x1054u : 0x7632u;  // c = 1: im or re
+  const uint32_t flip = part ? 0x80008000u : 0u;   //        -re
   for (int base = 0; base < tasks; base += blockDim.x) {
     const int task = base + threadIdx.x;
     const bool on = task < tasks;
@@ -991,28 +1022,19 @@ __device__ __forceinline__ void fft_b2_cube_body(const float2* __restrict__ phi,
     __nv_bfloat16* col = b2 + (size_t)vv * 4 * na + s * 2 * na + part * na + a0;
 #pragma unroll
     for (int k1 = 0; k1 < N; ++k1) {
-      float2 f[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        f[j].x = __shfl_sync(0xffffffffu, v[k1].x, (lane & ~3) + j);
-        f[j].y = __shfl_sync(0xffffffffu, v[k1].y, (lane & ~3) + j);
-      }
+      uint32_t hw, lw;
+      split_bf16x2(v[k1].x * norm, v[k1].y * norm, hw, lw);
+      const uint32_t keep = s ? lw : hw;                                              // transform q
+      const uint32_t recv = __shfl_xor_sync(0xffffffffu, s ? hw : lw, 2);             // q ^ 2
+      const uint32_t nk = __shfl_xor_sync(0xffffffffu, keep, 1);                      // q ^ 1
+      const uint32_t nr = __shfl_xor_sync(0xffffffffu, recv, 1);                      // q ^ 3
+      // this lane's transform order is (own pair, neighbour): sel0/sel1 put it in ascending order
+      const uint32_t x0 = s ? recv : keep, x1 = s ? nr : nk, y0 = s ? keep : recv, y1 = s ? nk : nr;
       if (!on) continue;
-      const size_t k = (size_t)k1 * N2 + r;
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        __nv_bfloat16 e[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float re = f[j].x * norm, im = f[j].y * norm;
-          const float val = part == 0 ? (c == 0 ? re : im) : (c == 0 ? im : -re);
-          __nv_bfloat16 hv, lv;
-          split_bf16(val, hv, lv);
-          e[j] = s == 0 ? hv : lv;
-        }
-        *reinterpret_cast<uint2*>(col + (k * k2ext + row_x + 64 * c) * ncol) =
-            make_uint2(pack_bf16(e[0], e[1]), pack_bf16(e[2], e[3]));
-      }
+      __nv_bfloat16* o = col + ((size_t)(k1 * N2 + r) * k2ext + row_x) * ncol;
+      *reinterpret_cast<uint2*>(o) = make_uint2(__byte_perm(x0, x1, sel0), __byte_perm(y0, y1, sel0));
+      *reinterpret_cast<uint2*>(o + (size_t)64 * ncol) =
+          make_uint2(__byte_perm(x0, x1, sel1) ^ flip, __byte_perm(y0, y1, sel1) ^ flip);
     }
   }
 }
