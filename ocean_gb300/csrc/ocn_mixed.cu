@@ -222,7 +222,7 @@ __device__ __forceinline__ void lr_tc_body(const TcParams& p, const Src& src) {
   const uint32_t full0 = su32(bars), empty0 = su32(bars + TC_MAX_STAGES);
   const uint32_t tfull0 = su32(bars + 2 * TC_MAX_STAGES), tempty0 = su32(bars + 2 * TC_MAX_STAGES + 2);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   if (p.inc && blockIdx.x == 0 && threadIdx.x == 0) *p.inc += 1;  // nothing in this launch reads it
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
@@ -300,58 +300,63 @@ __device__ __forceinline__ void lr_tc_body(const TcParams& p, const Src& src) {
         }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ------------------------------------------------------------ MMA issuer
-      uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
-      int last_stage = -1;
-      uint32_t last_phase = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < p.ntiles && ok; t += gridDim.x) {
-        int lt;
-        const int ii = src.inst(t, &lt);
-        const TcParams& tp = src.par(ii);
-        const TileInfo ti = decode(tp, lt);
-        if (!mbar_wait(tempty0 + 8 * acc, acc_phase ^ 1, abort_flag, TC_WAIT_CYCLES)) {
-          ok = false;
-          break;
-        }
+    // -------------------------------------------------------------- MMA issuer
+    // the whole warp runs the (warp-uniform) loop, one elected lane issues, and the
+    // descriptors advance by constants: a single lane that built every descriptor
+    // issued an MMA per ~140 cycles
+    uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
+    int last_stage = -1;
+    uint32_t last_phase = 0;
+    bool ok = true;
+    const bool leader = elect_one();
+    for (int t = blockIdx.x; t < p.ntiles && ok; t += gridDim.x) {
+      int lt;
+      const int ii = src.inst(t, &lt);
+      const TcParams& tp = src.par(ii);
+      const TileInfo ti = decode(tp, lt);
+      const uint32_t idesc = tp.idesc;
+      const bool bmn = tp.bmn != 0;
+      ok = __all_sync(0xffffffffu, mbar_wait(tempty0 + 8 * acc, acc_phase ^ 1, abort_flag, TC_WAIT_CYCLES));
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t dt = tmem_base + acc * (uint32_t)p.ncol;
+      for (int c = ti.c0; c < ti.c1; ++c) {
+        ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * stage, phase, abort_flag, TC_WAIT_CYCLES));
+        if (!ok) break;
         tc_fence_after();
-        const uint32_t dt = tmem_base + acc * (uint32_t)p.ncol;
-        for (int c = ti.c0; c < ti.c1; ++c) {
-          if (!mbar_wait(full0 + 8 * stage, phase, abort_flag, TC_WAIT_CYCLES)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t sa = su32(smem + stage * stage_bytes);
+        const uint32_t sa = su32(smem) + stage * stage_bytes;
+        if (leader) {
+          const uint64_t ah = sw128_desc(sa), al = sw128_desc(sa + a_bytes);
+          const uint64_t b0 = bmn ? sw32_mn_desc(sa + 2 * a_bytes) : sw128_desc(sa + 2 * a_bytes);
+          const uint32_t bstep = bmn ? 512 >> 4 : 32 >> 4;  // addresses stay below 2^18: the low word advances alone
 #pragma unroll
           for (int kk = 0; kk < TC_BK / 16; ++kk) {
-            const uint64_t bd =
-                tp.bmn ? sw32_mn_desc(sa + 2 * a_bytes + kk * 512) : sw128_desc(sa + 2 * a_bytes + kk * 32);
-            umma_bf16(dt, sw128_desc(sa + kk * 32), bd, tp.idesc, (c > ti.c0 || kk > 0) ? 1u : 0u);
-            umma_bf16(dt, sw128_desc(sa + a_bytes + kk * 32), bd, tp.idesc, 1u);
+            const uint64_t bd = b0 + kk * bstep;
+            umma_bf16(dt, ah + kk * (32 >> 4), bd, idesc, (c > ti.c0 || kk > 0) ? 1u : 0u);
+            umma_bf16(dt, al + kk * (32 >> 4), bd, idesc, 1u);
           }
           umma_commit(empty0 + 8 * stage);
-          last_stage = (int)stage;
-          last_phase = phase;
-          if (++stage == (uint32_t)S) {
-            stage = 0;
-            phase ^= 1;
-          }
         }
-        if (!ok) break;
-        umma_commit(tfull0 + 8 * acc);
-        acc ^= 1;
-        if (acc == 0) acc_phase ^= 1;
-      }
-      if (!ok) {
-        *abort_flag = 1;
-        atomicOr(p.err, 2);
-      }
-      if (last_stage >= 0) {  // drain: every issued MMA finished reading shared memory
-        const long long t0 = clock64();
-        while (!mbar_test(empty0 + 8 * last_stage, last_phase) && clock64() - t0 < TC_WAIT_CYCLES) {
+        __syncwarp();
+        last_stage = (int)stage;
+        last_phase = phase;
+        if (++stage == (uint32_t)S) {
+          stage = 0;
+          phase ^= 1;
         }
+      }
+      if (!ok) break;
+      if (leader) umma_commit(tfull0 + 8 * acc);
+      acc ^= 1;
+      if (acc == 0) acc_phase ^= 1;
+    }
+    if (!ok && leader) {
+      *abort_flag = 1;
+      atomicOr(p.err, 2);
+    }
+    if (last_stage >= 0) {  // drain: every issued MMA finished reading shared memory
+      const long long t0 = clock64();
+      while (!mbar_test(empty0 + 8 * last_stage, last_phase) && clock64() - t0 < TC_WAIT_CYCLES) {
       }
     }
   } else {

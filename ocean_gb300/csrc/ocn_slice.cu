@@ -110,11 +110,6 @@ __device__ __forceinline__ void umma_fp8(uint32_t dtmem, uint32_t adesc, uint32_
       "r"(adesc), "r"(bdesc), "r"(idesc), "r"(accumulate), "r"(PLAIN_DESC_HI)
       : "memory");
 }
-__device__ __forceinline__ bool elect_one() {
-  uint32_t ok;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
-  return ok != 0;
-}
 // A (4 or 6) consecutive accumulator columns of this thread's lane
 template <int A>
 __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, float* v) {
