@@ -205,6 +205,56 @@ struct TcGroup {
   __device__ __forceinline__ const CUtensorMap* map(int i, int w) const { return &maps->m[i][w]; }
 };
 
+// Epilogue of one tile row (accumulator lane): the NA channels of every vector of
+// the block, to the staging row wr (mode 1, staged), phi (mode 1) or the partial sums
+// (mode 2).  NA is a compile-time count so that a vector's 4 NA columns stay in
+// registers: indexed at run time they went through local memory, 2.2 us per tile of
+// 12 complex columns, which bounded band->x below 70 bands.
+template <int NA>
+__device__ __forceinline__ void tc_drain(const TcParams& p, const TcParams& tp, const TileInfo& ti, uint32_t ta, int row,
+                                         float2* wr) {
+  for (int vv = 0; vv < tp.nv; ++vv) {
+    float v[4 * NA];
+#pragma unroll
+    for (int c = 0; c < 4 * NA; c += 16) tmem_ld16(ta + vv * 4 * NA + c, v + c);
+    tmem_ld_wait();
+    if (tp.mode == 1) {
+      const int x = ti.row0 + row;
+      if (p.estg && tp.spin < 0) {
+#pragma unroll
+        for (int a = 0; a < NA; ++a)
+          wr[vv * NA + a] = make_float2(v[a] + v[2 * NA + a], v[NA + a] + v[3 * NA + a]);
+      } else if (x < tp.nx) {
+        float2* o = tp.phi + ((size_t)ti.k * tp.nx + x) * (tp.nv * NA) + vv * NA;
+        if (tp.spin < 0) {  // 16-byte aligned: NA is a multiple of 4
+#pragma unroll
+          for (int a = 0; a < NA; a += 2)
+            *reinterpret_cast<float4*>(o + a) =
+                make_float4(v[a] + v[2 * NA + a], v[NA + a] + v[3 * NA + a], v[a + 1] + v[2 * NA + a + 1],
+                            v[NA + a + 1] + v[3 * NA + a + 1]);
+        } else {
+#pragma unroll
+          for (int a = 0; a < NA; ++a)
+            if ((a & 1) == tp.spin) o[a] = make_float2(v[a] + v[2 * NA + a], v[NA + a] + v[3 * NA + a]);
+        }
+      }
+    } else {
+      const int n = ti.row0 + row;
+      if (n < tp.nb) {
+        float* pr = tp.part + ((size_t)ti.sp * tp.nvmax + vv) * 2 * tp.npsi + (size_t)n + (size_t)tp.nb * ti.k;
+        float* pim = pr + tp.npsi;
+        const size_t da = (size_t)tp.nb * tp.nk;
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+          if (tp.spin >= 0 && (a & 1) != tp.spin) continue;
+          pr[a * da] = -(v[a] + v[2 * NA + a]);
+          pim[a * da] = -(v[NA + a] + v[3 * NA + a]);
+        }
+      }
+    }
+  }
+}
+
 // p: launch-wide values (tile count, pipeline depth, shared-memory stage layout
 // and accumulator stride for the largest N, tensor-memory columns, error flag).
 template <class Src>
@@ -364,7 +414,6 @@ __device__ __forceinline__ void lr_tc_body(const TcParams& p, const Src& src) {
     const int q = warp & 3;  // TMEM lane quadrant this warp may access
     const int row = q * 32 + lane;
     uint32_t acc = 0, acc_phase = 0;
-    float v[48];  // one vector's 4 Na columns
     // mode-1 staging: this warp's 32 rows of (vector, alpha) values, row pitch wld
     const int wld = p.ncol / 4 + 1;
     float2* wst = reinterpret_cast<float2*>(smem + S * stage_bytes + 256) + (size_t)(warp - 2) * 32 * wld;
@@ -373,7 +422,7 @@ __device__ __forceinline__ void lr_tc_body(const TcParams& p, const Src& src) {
       const int ii = src.inst(t, &lt);
       const TcParams& tp = src.par(ii);
       const TileInfo ti = decode(tp, lt);
-      const int na = tp.na, g4 = 4 * na;
+      const int na = tp.na;
       if (!mbar_wait(tfull0 + 8 * acc, acc_phase, abort_flag, TC_WAIT_CYCLES)) {
         *abort_flag = 1;
         atomicOr(p.err, 4);
@@ -381,34 +430,8 @@ __device__ __forceinline__ void lr_tc_body(const TcParams& p, const Src& src) {
       }
       tc_fence_after();
       const uint32_t ta = tmem_base + ((uint32_t)(q * 32) << 16) + acc * (uint32_t)p.ncol;
-      for (int vv = 0; vv < tp.nv; ++vv) {
-        for (int c16 = 0; c16 < g4; c16 += 16) tmem_ld16(ta + vv * g4 + c16, v + c16);
-        tmem_ld_wait();
-        if (tp.mode == 1) {
-          const int x = ti.row0 + row;
-          if (p.estg && tp.spin < 0) {
-            float2* wr = wst + lane * wld + vv * na;
-            for (int a = 0; a < na; ++a) wr[a] = make_float2(v[a] + v[2 * na + a], v[na + a] + v[3 * na + a]);
-          } else if (x < tp.nx) {
-            float2* o = tp.phi + ((size_t)ti.k * tp.nx + x) * (tp.nv * na) + vv * na;
-            for (int a = 0; a < na; ++a)
-              if (tp.spin < 0 || (a & 1) == tp.spin)
-                o[a] = make_float2(v[a] + v[2 * na + a], v[na + a] + v[3 * na + a]);
-          }
-        } else {
-          const int n = ti.row0 + row;
-          if (n < tp.nb) {
-            float* pr = tp.part + ((size_t)ti.sp * tp.nvmax + vv) * 2 * tp.npsi;
-            float* pim = pr + tp.npsi;
-            for (int a = 0; a < na; ++a) {
-              if (tp.spin >= 0 && (a & 1) != tp.spin) continue;
-              const size_t idx = (size_t)n + (size_t)tp.nb * ((size_t)ti.k + (size_t)tp.nk * a);
-              pr[idx] = -(v[a] + v[2 * na + a]);
-              pim[idx] = -(v[na + a] + v[3 * na + a]);
-            }
-          }
-        }
-      }
+      if (na == 4) tc_drain<4>(p, tp, ti, ta, row, wst + lane * wld);
+      else tc_drain<12>(p, tp, ti, ta, row, wst + lane * wld);
       tc_fence_before();
       mbar_arrive(tempty0 + 8 * acc);
       if (tp.mode == 1 && p.estg && tp.spin < 0) {
