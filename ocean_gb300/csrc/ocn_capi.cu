@@ -52,17 +52,21 @@ int require(ocn_ctx* c) {
   return OCN_OK;
 }
 
-// Multiplet and long-range terms of an FP64 vector, into d_acc and d_accpart.
-int terms_fp64(ocn_ctx* c, const double* pr, const double* pi, bool mult_on, bool lr_on) {
+// Multiplet and long-range terms of nv <= fp64_nv FP64 vectors (vector v: planes at
+// pr + v*vstride, pi + v*vstride), into d_acc and d_accpart.
+int terms_fp64(ocn_ctx* c, const double* pr, const double* pi, size_t vstride, int nv, bool mult_on, bool lr_on) {
   int rc;
   const bool sliced = mult_on && slice_mult_ready(c);
   if (sliced) {
-    if ((rc = slice_prep_psi(c, pr, pi)) || (rc = slice_mult_apply(c))) return rc;
+    for (int v = 0; v < nv; ++v)
+      if ((rc = slice_prep_psi(c, pr + v * vstride, pi + v * vstride, 0, 1)) || (rc = slice_mult_apply(c, v))) return rc;
   } else if (mult_on) {
-    if ((rc = zero_acc(c, 1)) || (rc = mult_apply(c, pr, pi, c->d_acc))) return rc;
+    if ((rc = zero_acc(c, nv))) return rc;
+    for (int v = 0; v < nv; ++v)
+      if ((rc = mult_apply(c, pr + v * vstride, pi + v * vstride, c->d_acc + 2 * v * c->npsi))) return rc;
     c->acc_valid = true;
   }
-  return lr_on ? lr_apply_fp64(c, pr, pi, sliced) : OCN_OK;
+  return lr_on ? lr_apply_fp64(c, pr, pi, vstride, nv, sliced && nv == 1) : OCN_OK;
 }
 
 }  // namespace
@@ -84,7 +88,7 @@ int apply_H_impl(ocn_ctx* c, const double* ir, const double* ii, double* orr, do
     return combine(c, 1, ir, ii, orr, oi, 0, hflag, backwards);
   }
   if (c->dims.precision != OCN_PREC_MIXED) {
-    if ((rc = terms_fp64(c, ir, ii, mult_on, lr_on))) return rc;
+    if ((rc = terms_fp64(c, ir, ii, 0, 1, mult_on, lr_on))) return rc;
     return combine(c, 1, ir, ii, orr, oi, 0, hflag, backwards);
   }
   if (mult_on) {
@@ -96,21 +100,13 @@ int apply_H_impl(ocn_ctx* c, const double* ir, const double* ii, double* orr, do
   return combine(c, 1, ir, ii, orr, oi, 0, hflag, backwards);
 }
 
-// H on a block of nv vectors (vector v at in + 2*v*npsi) -- mixed precision reads
-// the Bloch functions once for the block; the FP64 path acts vector by vector.
+// H on a block of nv vectors (vector v at in + 2*v*npsi): the Bloch functions are
+// read once for the block in mixed precision, once per fp64_nv vectors in FP64.
 // back_each (may be NULL): the backwards switch of each vector (H or H^dagger).
 int apply_H_block_impl(ocn_ctx* c, int nv, const double* in, double* out, const int* hflag_in,
                        int backwards, const int* back_each) {
   const size_t n = c->npsi;
   if (nv < 1 || nv > c->nvec) return set_err(c, OCN_ERR_ARG, "block size must be in 1..nvec");
-  if (c->dims.precision != OCN_PREC_MIXED) {
-    for (int v = 0; v < nv; ++v) {
-      int rc = apply_H_impl(c, in + 2 * v * n, in + 2 * v * n + n, out + 2 * v * n, out + 2 * v * n + n,
-                            hflag_in, back_each ? back_each[v] : backwards);
-      if (rc) return rc;
-    }
-    return OCN_OK;
-  }
   int hflag[6];
   for (int i = 0; i < 6; ++i) hflag[i] = hflag_in ? hflag_in[i] : c->sys.nhflag[i];
   int rc = require(c);
@@ -118,8 +114,26 @@ int apply_H_block_impl(ocn_ctx* c, int nv, const double* in, double* out, const 
   c->acc_valid = false;
   const bool mult_on = c->sys.mult && hflag[4] == 1 && c->have_mult;
   const bool lr_on = c->sys.long_range && hflag[0] == 1;
+  if (c->dims.precision != OCN_PREC_MIXED) {
+    for (int v0 = 0; v0 < nv; v0 += c->fp64_nv) {
+      const int w = std::min(c->fp64_nv, nv - v0);
+      const double* pin = in + 2 * v0 * n;
+      double* pout = out + 2 * v0 * n;
+      c->acc_valid = false;
+      if ((rc = terms_fp64(c, pin, pin + n, 2 * n, w, mult_on, lr_on))) return rc;
+      if (!back_each) {
+        if ((rc = combine(c, w, pin, pin + n, pout, pout + n, 2 * n, hflag, backwards))) return rc;
+        continue;
+      }
+      for (int v = 0; v < w; ++v)
+        if ((rc = combine(c, 1, pin + 2 * v * n, pin + 2 * v * n + n, pout + 2 * v * n, pout + 2 * v * n + n, 2 * n, hflag,
+                          back_each[v0 + v], v)))
+          return rc;
+    }
+    return OCN_OK;
+  }
   bool b1_ready = false;
-  if (c->mult_parts > 0 && mult_on) {  // (mixed: FP64 contexts returned above)
+  if (c->mult_parts > 0 && mult_on) {
     if ((rc = mixed_prep_b1(c, in, in + n, 2 * n, nv)) || (rc = mult_apply_mixed(c, in, in + n, 2 * n, nv, true)))
       return rc;
     b1_ready = true;
@@ -306,8 +320,9 @@ int ocn_ctx_create(const ocn_dims* d, ocn_ctx** out) {
       (rc = dev_alloc(c, &c->d_scal, 64)))
     return fail(rc);
   if (d->precision == OCN_PREC_FP64) {
-    c->part_stride = 2 * c->npsi;  // the FP64 path acts on one vector at a time
-    if ((rc = dev_alloc(c, &c->d_phi, (size_t)nk * nx * c->na)) ||
+    c->fp64_nv = slice_width(c);
+    c->part_stride = (size_t)c->fp64_nv * 2 * c->npsi;
+    if ((rc = dev_alloc(c, &c->d_phi, (size_t)nk * nx * c->na * c->fp64_nv)) ||
         (rc = dev_alloc(c, &c->d_accpart, (size_t)c->lr_xsplit * c->part_stride)))
       return fail(rc);
   }
@@ -676,7 +691,7 @@ int haydock_iteration(ocn_ctx* c, int nv, double* old, double* psi, double* h, d
   const bool mult_on = c->sys.mult && c->sys.nhflag[4] == 1 && c->have_mult;
   const bool lr_on = c->sys.long_range && c->sys.nhflag[0] == 1;
   if (!mixed_parts(c)) {
-    if ((rc = terms_fp64(c, psi, psi + n, mult_on, lr_on))) return rc;
+    if ((rc = terms_fp64(c, psi, psi + n, 2 * n, nv, mult_on, lr_on))) return rc;
   } else {
     // the psi operand was built by the previous normalisation (or before the loop)
     if (mult_on && c->mult_parts == 0)  // the FP64 multiplet kernels cannot read the double-float vectors
@@ -725,9 +740,10 @@ unsigned long long haydock_key(const ocn_ctx* c, int nv) {
   return k;
 }
 
-// Chains held at once by the Haydock buffers: a block in mixed precision, one
-// chain in FP64 (the FP64 block driver runs its chains one after another).
-int haydock_chains(const ocn_ctx* c) { return c->dims.precision == OCN_PREC_MIXED ? c->nvec : 1; }
+// Chains held at once by the Haydock buffers: a block in mixed precision, the
+// vectors that share the contractions in FP64 (the block driver runs further ones
+// after them).
+int haydock_chains(const ocn_ctx* c) { return c->dims.precision == OCN_PREC_MIXED ? c->nvec : c->fp64_nv; }
 
 // Buffers of one Haydock run of nv chains on a context (see haydock_prepare).
 struct HayRun {
@@ -977,18 +993,17 @@ int haydock_run(ocn_ctx* c, int nv, const double* p0r, const double* p0i, size_t
   return rc ? rc : rf;
 }
 
-// Block Haydock on device psi0 planes; FP64 contexts run the chains one by one.
+// Block Haydock on device psi0 planes, haydock_chains at a time.
 int haydock_block_impl(ocn_ctx* c, int nv, const double* d_psi0, int niter, double* real_a, double* imag_a,
                        double* real_b, int* niter_done) {
   const size_t n = c->npsi;
   if (nv < 1 || nv > std::max(c->nvec, 1)) return set_err(c, OCN_ERR_ARG, "block size must be in 1..nvec");
-  if (haydock_chains(c) >= nv)
-    return haydock_run(c, nv, d_psi0, d_psi0 + n, 2 * n, niter, real_a, imag_a, real_b, niter_done);
   const size_t out1 = (size_t)niter + 1;
+  const int hv = haydock_chains(c);
   int rc = OCN_OK;
-  for (int v = 0; v < nv; ++v) {
-    const int r = haydock_run(c, 1, d_psi0 + 2 * v * n, d_psi0 + 2 * v * n + n, 0, niter, real_a + v * out1,
-                              imag_a ? imag_a + v * out1 : nullptr, real_b + v * out1,
+  for (int v = 0; v < nv; v += hv) {
+    const int r = haydock_run(c, std::min(hv, nv - v), d_psi0 + 2 * v * n, d_psi0 + 2 * v * n + n, 2 * n, niter,
+                              real_a + v * out1, imag_a ? imag_a + v * out1 : nullptr, real_b + v * out1,
                               niter_done ? niter_done + v : nullptr);
     if (r == OCN_ERR_NAN) rc = r;
     else if (r) return r;
@@ -1087,6 +1102,8 @@ int ocn_haydock_batch(ocn_ctx* const* ctxs, int nctx, const int* nv, const doubl
   std::vector<HayRun> R(nctx);
   for (int i = 0; i < nctx; ++i) {
     ocn_ctx* c = ctxs[i];
+    if (c->dims.precision == OCN_PREC_FP64 && nv[i] != 1)
+      return set_err(c, OCN_ERR_ARG, "ocn_haydock_batch: FP64 contexts run one chain");
     const int rc = haydock_prepare(c, nv[i], d_psi0[i], d_psi0[i] + c->npsi, 2 * c->npsi, niter, &R[i]);
     if (rc) return rc;
   }

@@ -123,7 +123,8 @@ struct ocn_ctx {
   double tau_shifted[3] = {0, 0, 0};
 
   // work buffers
-  double2* d_phi = nullptr;        // FP64 path: [k][x][a]
+  double2* d_phi = nullptr;        // FP64 path: [k][x][t] of fp64_nv vectors
+  int fp64_nv = 1;                 // FP64 contexts: vectors of a block that act together
   double* d_acc = nullptr;         // full-store accumulator: re plane then im plane (npsi each)
   double* d_accpart = nullptr;     // long-range partials [split][vector][re|im][npsi]
   int lr_xsplit = 1;
@@ -249,8 +250,9 @@ double gaunt_threey(int ll, int ml, int lm, int mm, int lr, int mr, int conjug);
 
 // ---- FP64 kernels (ocn_kernels.cu)
 int upload_twiddles(ocn_ctx* c);
-// long-range partials into d_accpart; b1_ready: the digit operand of psi was built
-int lr_apply_fp64(ocn_ctx* c, const double* d_pr, const double* d_pi, bool b1_ready = false);
+// long-range partials of nv <= fp64_width vectors (stride vstride) into d_accpart;
+// b1_ready: the digit operand of the one psi was built
+int lr_apply_fp64(ocn_ctx* c, const double* d_pr, const double* d_pi, size_t vstride, int nv, bool b1_ready = false);
 int mult_apply(ocn_ctx* c, const double* d_pr, const double* d_pi, double* acc);  // adds into acc
 int mult_hamp(ocn_ctx* c, const double2* amp, double2* hamp);  // one vector, [p][a]
 // base: binary32 partials on the mixed path, FP64 otherwise
@@ -376,13 +378,15 @@ int slice_init(ocn_ctx* c);        // geometry and vector-side buffers; sets lr_
 void slice_free(ocn_ctx* c);
 int slice_set_bloch(ocn_ctx* c);   // digit operands from d_u (not ready when they do not fit)
 bool slice_ready(const ocn_ctx* c);
-int slice_prep_psi(ocn_ctx* c, const double* d_pr, const double* d_pi);  // operand of the next two
-int slice_band_to_x(ocn_ctx* c, double2* phi);  // phi[k][x][a]
-int slice_x_to_band(ocn_ctx* c, const double2* phi, bool have_max);  // d_accpart slices from phi'[k][x][a]
+int slice_width(const ocn_ctx* c); // vectors that share a launch (12 columns at most)
+int slice_prep_psi(ocn_ctx* c, const double* d_pr, const double* d_pi, size_t vstride, int nv);  // operand of:
+int slice_band_to_x(ocn_ctx* c, double2* phi, int nv);  // phi[k][x][t], t = v*Na + a
+// d_accpart slices of vectors v0 .. v0 + nv - 1 from phi'[k][x][t]
+int slice_x_to_band(ocn_ctx* c, const double2* phi, int nv, int v0, bool have_max);
 unsigned* slice_maxima(ocn_ctx* c);  // [k][a] magnitude maxima of phi', cleared by slice_prep_psi
 int slice_set_mult(ocn_ctx* c);    // digit operands of the projectors (after ocn_set_mult)
 bool slice_mult_ready(const ocn_ctx* c);
-int slice_mult_apply(ocn_ctx* c);  // multiplet term of the prepared psi, into its d_accpart slices
+int slice_mult_apply(ocn_ctx* c, int v);  // multiplet term of the one prepared psi, into vector v's slices
 int slice_check(ocn_ctx* c);       // reads and clears the device timeout flag
 
 // ---- mixed precision (ocn_mixed.cu)

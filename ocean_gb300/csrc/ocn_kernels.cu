@@ -167,7 +167,7 @@ WgradFnD wgrad_fn(int n) {
 constexpr int G2_XC = 32;
 __global__ void k_lr_gemm2_fp64(const double2* __restrict__ u, const double2* __restrict__ phi,
                                 double* __restrict__ part, int nb, int nk, int nx, int na, int nspn,
-                                int xper, size_t npsi) {
+                                int xper, size_t pstride, size_t npsi) {
   __shared__ double2 fs[G2_XC * OCN_MAX_NA];
   const int k = blockIdx.x;
   const int split = blockIdx.y;
@@ -199,7 +199,7 @@ __global__ void k_lr_gemm2_fp64(const double2* __restrict__ u, const double2* __
     }
   }
   if (n < nb) {
-    double* pr = part + (size_t)split * 2 * npsi;
+    double* pr = part + (size_t)split * pstride;
     double* pim = pr + npsi;
 #pragma unroll
     for (int a = 0; a < OCN_MAX_NA; ++a)
@@ -1023,48 +1023,60 @@ int zero_acc(ocn_ctx* c, int nv) {
   return OCN_OK;
 }
 
-int lr_apply_fp64(ocn_ctx* c, const double* d_pr, const double* d_pi, bool b1_ready) {
+int lr_apply_fp64(ocn_ctx* c, const double* d_pr, const double* d_pi, size_t vstride, int nv, bool b1_ready) {
   const int nb = c->nb, nk = c->nk, nx = c->nx, na = c->na;
-  const bool sliced = slice_ready(c);
-  if (sliced) {
-    if (!b1_ready)
-      if (int rc = slice_prep_psi(c, d_pr, d_pi)) return rc;
-    if (int rc = slice_band_to_x(c, c->d_phi)) return rc;
-  } else {
-    const size_t sm = sizeof(double2) * ((size_t)c->nspn * G1_N * (G1_X + 1) + (size_t)na * G1_N);
-    dim3 grid((nx + G1_X - 1) / G1_X, nk);
-    TimedScope ts(c, T_LR_GEMM1);
-    k_lr_gemm1_fp64<<<grid, G1_X, sm, c->stream>>>(c->d_u, d_pr, d_pi, c->d_allow, c->d_phi, nb, nk,
-                                                   nx, na, c->nspn);
-    ++c->launches;
-    OCN_CUDA(c, cudaGetLastError());
+  if (nv < 1 || nv > c->fp64_nv) return set_err(c, OCN_ERR_ARG, "FP64 block wider than its buffers");
+  if (slice_ready(c) && fx_supported(c)) {  // all nv vectors in one set of launches
+    int rc;
+    if (!b1_ready && (rc = slice_prep_psi(c, d_pr, d_pi, vstride, nv))) return rc;
+    if ((rc = slice_band_to_x(c, c->d_phi, nv))) return rc;
+    {
+      TimedScope ts(c, T_LR_FFT);
+      if ((rc = fx_transform(c, c->d_phi, na * nv, slice_maxima(c)))) return rc;
+    }
+    return slice_x_to_band(c, c->d_phi, nv, 0, true);
   }
-  const bool fixed = fx_supported(c);
-  if (fixed) {
-    TimedScope ts(c, T_LR_FFT);
-    if (int rc = fx_transform(c, c->d_phi, na, sliced ? slice_maxima(c) : nullptr)) return rc;
-  } else {
-    const KmeshGeom<double> g = kmesh_geom<double>(c->dims.kmesh, na);
-    TimedScope ts(c, T_LR_FFT);
-    CubeFnD f = nullptr;
-    if (kmesh_cube_supported(c->dims.kmesh)) OCN_CUBE_DISPATCH(k_fft_cube_fp64, c->dims.kmesh[0], na, f);
-    if (f)
-      f<<<nx, 128, kmesh_cube_smem<double>(c->dims.kmesh[0], na), c->stream>>>(c->d_phi, c->d_W, nx, na,
-                                                                               c->d_tw);
-    else
-      k_lr_fft_w_fp64<<<nx, 256, kmesh_smem(g), c->stream>>>(c->d_phi, c->d_W, nx, g, c->d_tw);
-    ++c->launches;
-    OCN_CUDA(c, cudaGetLastError());
-  }
-  if (sliced) return slice_x_to_band(c, c->d_phi, fixed);
-  {
+  for (int v = 0; v < nv; ++v) {
+    const double *pr = d_pr + v * vstride, *pi = d_pi + v * vstride;
+    const bool sliced = slice_ready(c);  // k-mesh without the fixed-point transform: one vector at a time
+    if (sliced) {
+      int rc;
+      if (!b1_ready && (rc = slice_prep_psi(c, pr, pi, 0, 1))) return rc;
+      if ((rc = slice_band_to_x(c, c->d_phi, 1))) return rc;
+    } else {
+      const size_t sm = sizeof(double2) * ((size_t)c->nspn * G1_N * (G1_X + 1) + (size_t)na * G1_N);
+      dim3 grid((nx + G1_X - 1) / G1_X, nk);
+      TimedScope ts(c, T_LR_GEMM1);
+      k_lr_gemm1_fp64<<<grid, G1_X, sm, c->stream>>>(c->d_u, pr, pi, c->d_allow, c->d_phi, nb, nk, nx, na, c->nspn);
+      ++c->launches;
+      OCN_CUDA(c, cudaGetLastError());
+    }
+    if (fx_supported(c)) {
+      TimedScope ts(c, T_LR_FFT);
+      if (int rc = fx_transform(c, c->d_phi, na, nullptr)) return rc;
+    } else {
+      const KmeshGeom<double> g = kmesh_geom<double>(c->dims.kmesh, na);
+      TimedScope ts(c, T_LR_FFT);
+      CubeFnD f = nullptr;
+      if (kmesh_cube_supported(c->dims.kmesh)) OCN_CUBE_DISPATCH(k_fft_cube_fp64, c->dims.kmesh[0], na, f);
+      if (f)
+        f<<<nx, 128, kmesh_cube_smem<double>(c->dims.kmesh[0], na), c->stream>>>(c->d_phi, c->d_W, nx, na, c->d_tw);
+      else
+        k_lr_fft_w_fp64<<<nx, 256, kmesh_smem(g), c->stream>>>(c->d_phi, c->d_W, nx, g, c->d_tw);
+      ++c->launches;
+      OCN_CUDA(c, cudaGetLastError());
+    }
+    if (sliced) {
+      if (int rc = slice_x_to_band(c, c->d_phi, 1, v, false)) return rc;
+      continue;
+    }
     const int xs = c->lr_xsplit;
     const int xper = (nx + xs - 1) / xs;
     const int block = ((nb + 31) / 32) * 32;
     dim3 grid(nk, xs);
     TimedScope ts(c, T_LR_GEMM2);
-    k_lr_gemm2_fp64<<<grid, block, 0, c->stream>>>(c->d_u, c->d_phi, c->d_accpart, nb, nk, nx, na,
-                                                   c->nspn, xper, c->npsi);
+    k_lr_gemm2_fp64<<<grid, block, 0, c->stream>>>(c->d_u, c->d_phi, c->d_accpart + (size_t)v * 2 * c->npsi, nb, nk, nx, na,
+                                                   c->nspn, xper, c->part_stride, c->npsi);
     ++c->launches;
     OCN_CUDA(c, cudaGetLastError());
   }
@@ -1084,8 +1096,8 @@ int lr_wgrad_fp64(ocn_ctx* c, const double* x, const double* y, double2* phi, do
   double2* phy = phi + (size_t)nk * nx * na;
   if (slice_ready(c)) {
     int rc;
-    if ((rc = slice_prep_psi(c, x, x + n)) || (rc = slice_band_to_x(c, phx)) || (rc = slice_prep_psi(c, y, y + n)) ||
-        (rc = slice_band_to_x(c, phy)))
+    if ((rc = slice_prep_psi(c, x, x + n, 0, 1)) || (rc = slice_band_to_x(c, phx, 1)) ||
+        (rc = slice_prep_psi(c, y, y + n, 0, 1)) || (rc = slice_band_to_x(c, phy, 1)))
       return rc;
   } else {
     const size_t sm = sizeof(double2) * ((size_t)c->nspn * G1_N * (G1_X + 1) + (size_t)na * G1_N);

@@ -703,10 +703,11 @@ struct SliceGemm {
   size_t b_bytes() const { return (size_t)(p.bshared ? 1 : p.nk) * p.Ge * 2 * SL_S * nae * 16; }
 };
 
-// rows and summed index of a contraction; the largest K chunk whose two B slots
-// and at least four A stages fit in shared memory (16 granules at most for one
-// resident B operand, 12 for streamed ones).
-void slice_plan(SliceGemm* s, int mode, int nae, int nk, int rows, int K, int sm_count) {
+// rows and summed index of a contraction of nae columns; the largest K chunk whose
+// two B slots and at least four A stages fit in shared memory (16 granules at most
+// for one resident B operand, 12 for streamed ones) with the widest columns, nae_max,
+// that share the A operand: its order depends on the chunks.
+void slice_plan(SliceGemm* s, int mode, int nae, int nae_max, int nk, int rows, int K, int sm_count) {
   SliceParams& p = s->p;
   s->mode = mode;
   s->nae = nae;
@@ -718,10 +719,10 @@ void slice_plan(SliceGemm* s, int mode, int nae, int nk, int rows, int K, int sm
   p.R = (p.nt - 1) * SL_ROWS + p.rl;
   p.G = (K + 15) / 16;
   p.Ge = (p.G + 1) & ~1;
-  const size_t pitch = (size_t)2 * 23 * nae * 16;
+  const size_t pitch = (size_t)2 * 23 * nae * 16, pitch_max = (size_t)2 * 23 * nae_max * 16;
   const int cap = mode == 1 ? 16 : 12;
   int kc = std::min(cap, p.Ge);
-  while (kc > 2 && kc * (2 * pitch + 4 * SL_ROWS * 16) > SL_SMEM) kc -= 2;
+  while (kc > 2 && kc * (2 * pitch_max + 4 * SL_ROWS * 16) > SL_SMEM) kc -= 2;
   p.KC = kc;
   p.nch = (p.G + kc - 1) / kc;
   p.stages = (int)std::min<size_t>(SL_MAX_STAGES, (SL_SMEM - 2 * kc * pitch) / ((size_t)kc * SL_ROWS * 16));
@@ -755,8 +756,8 @@ void slice_plan(SliceGemm* s, int mode, int nae, int nk, int rows, int K, int sm
 
 struct SliceLR {
   bool ready = false;
-  int nvs = 1;             // vectors per launch
-  SliceGemm g1, g2;        // band -> x, x -> band
+  int nvs = 1;             // most vectors per launch (12 columns)
+  SliceGemm g1[3], g2[3];  // band -> x, x -> band of 1, 2, 3 vectors; A is held by [0] and shared
   uint8_t *b1 = nullptr, *b2 = nullptr;
   int *e1 = nullptr, *e2 = nullptr;
   unsigned* mx2 = nullptr;  // magnitude maxima of phi' per (k, column)
@@ -780,7 +781,7 @@ int salloc(ocn_ctx* c, T** p, size_t n) {
 }
 
 void slice_drop_a(SliceLR* s) {
-  for (SliceGemm* g : {&s->g1, &s->g2}) {
+  for (SliceGemm* g : {&s->g1[0], &s->g2[0]}) {
     if (g->A) cudaFree(g->A);
     if (g->eA) cudaFree(g->eA);
     g->A = nullptr;
@@ -837,11 +838,12 @@ bool slice_alloc_a(ocn_ctx* c, SliceGemm* g1, SliceGemm* g2, int nx) {
   return true;
 }
 
-int slice_launch(ocn_ctx* c, const SliceGemm& g, const uint8_t* B, const int* eB, double2* phi, double* part, int spin,
-                 int spins) {
+// g: the launch's geometry, a: the holder of its A operand
+int slice_launch(ocn_ctx* c, const SliceGemm& g, const SliceGemm& a, const uint8_t* B, const int* eB, double2* phi,
+                 double* part, int spin, int spins) {
   SliceParams p = g.p;
-  p.A = g.A;
-  p.eA = g.eA;
+  p.A = a.A;
+  p.eA = a.eA;
   p.B = B;
   p.eB = eB;
   p.phi = phi;
@@ -867,19 +869,27 @@ int slice_init(ocn_ctx* c) {
   SliceLR* s = new (std::nothrow) SliceLR();
   if (!s) return set_err(c, OCN_ERR_ALLOC, "host allocation failed");
   c->slice = s;
-  slice_plan(&s->g1, 1, c->na, c->nk, c->nx, 2 * c->nb, c->sm_count);
-  slice_plan(&s->g2, 2, c->na, c->nk, c->nb, c->nx, c->sm_count);
-  c->lr_xsplit = s->g2.p.ks;
+  s->nvs = std::max(1, std::min(c->nvec, 12 / c->na));
   int rc;
-  if ((rc = salloc(c, &s->b1, s->g1.b_bytes())) || (rc = salloc(c, &s->b2, s->g2.b_bytes())) ||
-      (rc = salloc(c, &s->e1, (size_t)c->nk * c->na)) || (rc = salloc(c, &s->e2, (size_t)c->nk * c->na)) ||
-      (rc = salloc(c, &s->mx2, (size_t)c->nk * c->na)) ||
+  for (int w = 1; w <= s->nvs; ++w) {
+    const int nae = w * c->na, most = s->nvs * c->na;
+    slice_plan(&s->g1[w - 1], 1, nae, most, c->nk, c->nx, 2 * c->nb, c->sm_count);
+    slice_plan(&s->g2[w - 1], 2, nae, most, c->nk, c->nb, c->nx, c->sm_count);
+    if ((rc = allow_max_smem(c, slice_fn(1, nae))) || (rc = allow_max_smem(c, slice_fn(2, nae)))) return rc;
+  }
+  c->lr_xsplit = s->g2[0].p.ks;
+  const SliceGemm &w1 = s->g1[s->nvs - 1], &w2 = s->g2[s->nvs - 1];
+  const size_t cols = (size_t)c->nk * c->na * s->nvs;
+  if ((rc = salloc(c, &s->b1, w1.b_bytes())) || (rc = salloc(c, &s->b2, w2.b_bytes())) ||
+      (rc = salloc(c, &s->e1, cols)) || (rc = salloc(c, &s->e2, cols)) || (rc = salloc(c, &s->mx2, cols)) ||
       (rc = salloc(c, &s->d_err, 1)))
     return rc;
   OCN_CUDA(c, cudaMemsetAsync(s->d_err, 0, sizeof(int), c->stream));
-  if ((rc = allow_max_smem(c, slice_fn(1, c->na))) || (rc = allow_max_smem(c, slice_fn(2, c->na)))) return rc;
   return OCN_OK;
 }
+
+// Vectors that one action's contractions take together.
+int slice_width(const ocn_ctx* c) { return c->slice ? c->slice->nvs : 1; }
 
 void slice_free(ocn_ctx* c) {
   SliceLR* s = c->slice;
@@ -900,13 +910,13 @@ bool slice_ready(const ocn_ctx* c) { return c->slice && c->slice->ready; }
 int slice_set_bloch(ocn_ctx* c) {
   SliceLR* s = c->slice;
   if (!s) return OCN_OK;
-  if (!s->g1.A && !slice_alloc_a(c, &s->g1, &s->g2, c->nx)) {
+  if (!s->g1[0].A && !slice_alloc_a(c, &s->g1[0], &s->g2[0], c->nx)) {
     slice_drop_a(s);
     return OCN_OK;
   }
   const size_t sx = (size_t)c->nk * c->nb, sk = c->nb;
   for (int sp = 0; sp < c->nspn; ++sp)
-    if (int rc = slice_build(c, c->d_u + (size_t)sp * c->nx * sx, sx, sk, c->nx, s->g1, s->g2, sp)) return rc;
+    if (int rc = slice_build(c, c->d_u + (size_t)sp * c->nx * sx, sx, sk, c->nx, s->g1[0], s->g2[0], sp)) return rc;
   OCN_CUDA(c, cudaStreamSynchronize(c->stream));
   s->ready = true;
   return OCN_OK;
@@ -926,8 +936,8 @@ int slice_set_mult(ocn_ctx* c) {
   c->mult_parts = 0;
   const int np = c->mult.np;
   if (np == 0) return OCN_OK;
-  slice_plan(&s->gm1, 1, c->na, c->nk, np, 2 * c->nb, c->sm_count);
-  slice_plan(&s->gm2, 2, c->na, c->nk, c->nb, np, c->sm_count);
+  slice_plan(&s->gm1, 1, c->na, c->na, c->nk, np, 2 * c->nb, c->sm_count);
+  slice_plan(&s->gm2, 2, c->na, c->na, c->nk, c->nb, np, c->sm_count);
   s->gm2.p.bshared = 1;
   double* parts = nullptr;
   if (!slice_alloc_a(c, &s->gm1, &s->gm2, np) || salloc(c, &s->bm, s->gm2.b_bytes()) || salloc(c, &s->em, c->na) ||
@@ -952,25 +962,27 @@ int slice_set_mult(ocn_ctx* c) {
 
 bool slice_mult_ready(const ocn_ctx* c) { return c->slice && c->slice->mult_ready; }
 
-// psi operand of one vector (FP64 planes), shared by the amplitudes and band -> x.
-int slice_prep_psi(ocn_ctx* c, const double* d_pr, const double* d_pi) {
+// psi operand of nv vectors (FP64 planes at stride vstride), shared by the amplitudes
+// (nv = 1) and band -> x.
+int slice_prep_psi(ocn_ctx* c, const double* d_pr, const double* d_pi, size_t vstride, int nv) {
   SliceLR* s = c->slice;
+  const int nae = c->na * nv;
   TimedScope ts(c, T_LR_PREP);
-  k_slice_prep_b1<<<c->nk, 256, 0, c->stream>>>(d_pr, d_pi, 0, c->d_allow, c->nb, c->nk, c->na, c->na, s->g1.p.Ge,
-                                                slice_merged(c->na) ? 1 : 0, s->b1, s->e1, s->mx2);
+  k_slice_prep_b1<<<c->nk, 256, 0, c->stream>>>(d_pr, d_pi, vstride, c->d_allow, c->nb, c->nk, c->na, nae, s->g1[0].p.Ge,
+                                                slice_merged(nae) ? 1 : 0, s->b1, s->e1, s->mx2);
   ++c->launches;
   OCN_CUDA(c, cudaGetLastError());
   return OCN_OK;
 }
 
-// The multiplet term of the vector whose operand is in b1, into its d_accpart slices.
-int slice_mult_apply(ocn_ctx* c) {
+// The multiplet term of the one vector whose operand is in b1, into the d_accpart slices of vector v.
+int slice_mult_apply(ocn_ctx* c, int v) {
   SliceLR* s = c->slice;
   MultDev& m = c->mult;
   TimedScope ts(c, T_MULT);
   int rc;
   for (int sp = 0; sp < c->nspn; ++sp)
-    if ((rc = slice_launch(c, s->gm1, s->b1, s->e1, s->amp_part, nullptr, sp, c->nspn))) return rc;
+    if ((rc = slice_launch(c, s->gm1, s->gm1, s->b1, s->e1, s->amp_part, nullptr, sp, c->nspn))) return rc;
   const int n = m.np * c->na;
   k_slice_amp_reduce<<<(n + 31) / 32, 512, 0, c->stream>>>(s->amp_part, m.amp, c->nk, n);
   ++c->launches;
@@ -982,42 +994,44 @@ int slice_mult_apply(ocn_ctx* c) {
                                                                       slice_merged(c->na) ? 1 : 0, s->mxm, s->bm, s->em);
   c->launches += 2;
   OCN_CUDA(c, cudaGetLastError());
-  double* part = c->d_accpart + (size_t)c->lr_xsplit * c->part_stride;
+  double* part = c->d_accpart + (size_t)c->lr_xsplit * c->part_stride + (size_t)v * 2 * c->npsi;
   for (int sp = 0; sp < c->nspn; ++sp)
-    if ((rc = slice_launch(c, s->gm2, s->bm, s->em, nullptr, part, sp, c->nspn))) return rc;
+    if ((rc = slice_launch(c, s->gm2, s->gm2, s->bm, s->em, nullptr, part, sp, c->nspn))) return rc;
   return OCN_OK;
 }
 
-// phi[k][x][a] of the vector whose operand is in b1.
-int slice_band_to_x(ocn_ctx* c, double2* phi) {
+// phi[k][x][t] of the nv vectors whose operand is in b1, t = v*Na + a.
+int slice_band_to_x(ocn_ctx* c, double2* phi, int nv) {
   SliceLR* s = c->slice;
   TimedScope ts(c, T_LR_GEMM1);
   for (int sp = 0; sp < c->nspn; ++sp)
-    if (int rc = slice_launch(c, s->g1, s->b1, s->e1, phi, nullptr, sp, c->nspn)) return rc;
+    if (int rc = slice_launch(c, s->g1[nv - 1], s->g1[0], s->b1, s->e1, phi, nullptr, sp, c->nspn)) return rc;
   return OCN_OK;
 }
 
 // The maxima that slice_x_to_band scales its operand by, cleared by slice_prep_psi.
 unsigned* slice_maxima(ocn_ctx* c) { return c->slice->mx2; }
 
-// d_accpart slices of one vector from phi'[k][x][a]; have_max: the maxima were collected.
-int slice_x_to_band(ocn_ctx* c, const double2* phi, bool have_max) {
+// d_accpart slices of vectors v0 .. v0 + nv - 1 from phi'[k][x][t]; have_max: the maxima were collected.
+int slice_x_to_band(ocn_ctx* c, const double2* phi, int nv, int v0, bool have_max) {
   SliceLR* s = c->slice;
+  const SliceGemm& g = s->g2[nv - 1];
+  const int nae = c->na * nv;
   {
     TimedScope ts(c, T_LR_PREP);
     if (!have_max) {
-      k_slice_col_max<<<c->nk, 512, 0, c->stream>>>(phi, c->nx, c->na, s->mx2);
+      k_slice_col_max<<<c->nk, 512, 0, c->stream>>>(phi, c->nx, nae, s->mx2);
       ++c->launches;
     }
-    const int items = s->g2.p.Ge * c->na * 4;
-    k_slice_prep_b2<<<dim3((items + 255) / 256, c->nk), 256, 0, c->stream>>>(
-        phi, c->nx, c->na, s->g2.p.Ge, slice_merged(c->na) ? 1 : 0, s->mx2, s->b2, s->e2);
+    const int items = g.p.Ge * nae * 4;
+    k_slice_prep_b2<<<dim3((items + 255) / 256, c->nk), 256, 0, c->stream>>>(phi, c->nx, nae, g.p.Ge,
+                                                                            slice_merged(nae) ? 1 : 0, s->mx2, s->b2, s->e2);
     ++c->launches;
     OCN_CUDA(c, cudaGetLastError());
   }
   TimedScope ts(c, T_LR_GEMM2);
   for (int sp = 0; sp < c->nspn; ++sp)
-    if (int rc = slice_launch(c, s->g2, s->b2, s->e2, nullptr, c->d_accpart, sp, c->nspn)) return rc;
+    if (int rc = slice_launch(c, g, s->g2[0], s->b2, s->e2, nullptr, c->d_accpart + (size_t)v0 * 2 * c->npsi, sp, c->nspn)) return rc;
   return OCN_OK;
 }
 

@@ -112,3 +112,30 @@ def test_non_finite_input_stays_visible(built, bad):
         assert np.all(np.isfinite(good[0])) and np.all(np.isfinite(good[1]))
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("kmesh,nb,xmesh,nspn,nvec,nv", [
+    ((3, 2, 4), 19, (5, 4, 3), 1, 3, 3),   # 12 columns in one launch
+    ((4, 4, 4), 11, (4, 4, 4), 2, 2, 2),   # 8 columns, two spins
+    ((2, 2, 3), 21, (4, 3, 3), 1, 5, 5),   # groups of three and two
+    ((9, 2, 1), 7, (3, 2, 2), 1, 2, 2),    # FP64-pipe transform: vector by vector
+])
+def test_block_of_vectors(built, kmesh, nb, xmesh, nspn, nvec, nv):
+    """Vectors that share launches give the action of each alone, bit for bit, and match the oracle."""
+    _, O = built
+    w = WL.make("batch", seed=nb, nb=nb, kmesh=kmesh, xmesh=xmesh, core_l=0, with_mult=False, nspn=nspn)
+    w.er[:] = 0.0
+    P = O.OracleProblem(w)
+    rng = np.random.default_rng(9)
+    pr, pi = rng.standard_normal((nv, w.npsi)), rng.standard_normal((nv, w.npsi))
+    pr[1] *= 1e-30
+    pi[1] *= 1e-30
+    ctx = capi.Context(w, nvec=nvec)
+    try:
+        br, bi = ctx.apply_H_block(pr, pi)
+        for v in range(nv):
+            sr, si = ctx.apply_H(pr[v], pi[v])
+            assert np.array_equal(br[v], sr) and np.array_equal(bi[v], si)
+            assert _rel((br[v], bi[v]), P.xact(pr[v], pi[v])) < TOL
+    finally:
+        ctx.close()
