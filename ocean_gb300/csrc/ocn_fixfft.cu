@@ -21,8 +21,9 @@
 // conflicts).  W / Nk is kept as 62-bit integers with one exponent per x-point, so
 // the normalisation costs nothing.  The pass maxima that set the shifts are
 // OR-reductions over the four lanes' classes (t = lane mod 4) and four shared words.
-// The result's maxima per (k, t), which scale the next contraction's operand, are
-// collected on the way out.
+// For the digit contractions the result stays integers, with one exponent per (x, t)
+// and the exponent maxima per (k, t) that scale the next operand collected on the way
+// out: rounding to binary64 and back took an eighth of the instructions.
 //
 // Measured: 319 -> 70 us (8^3, 6912 transforms), 766 -> 59 us (6^3, 12000), 375 ->
 // 62 us (7x6x5, 3960).  Bound by integer issue (about 3400 instructions per thread,
@@ -45,7 +46,8 @@ struct FxParams {
   double2* phi;                 // [k][x][t], transformed in place
   const long long* W;           // [x][k]: W / Nk = W 2^(we - 62)
   const int* we;                // [x]
-  unsigned* mx;                 // [k][t] largest magnitude word of phi' (may be null)
+  int* ex;                      // integer output: phi' = int 2^ex[x][t], ...
+  int* mx;                      // ... and running maxima over x of the exponents e, |phi'(k,x,t)| <= 2^e, [k][t]
   int nx, ld;
   int n1, n2, n3;
 };
@@ -99,8 +101,9 @@ __device__ __forceinline__ void store_line(const cfx (&v)[N], cfx* p, int st) {
   for (int j = 0; j < N; ++j) p[j * st] = v[j];
 }
 
-// N1, N2, N3: mesh extents known at compile time (0: from p)
-template <int N1, int N2, int N3>
+// N1, N2, N3: mesh extents known at compile time (0: from p).  INT: phi' stays integers
+// (re, im as 64-bit words in phi's place) for the digit operand of the next contraction.
+template <int N1, int N2, int N3, bool INT>
 __global__ void __launch_bounds__(256, 3) k_fx_transform(const FxParams p) {
   extern __shared__ __align__(16) unsigned char fxsm[];
   unsigned (*mx)[4] = reinterpret_cast<unsigned (*)[4]>(fxsm);  // [pass][transform]
@@ -214,33 +217,39 @@ __global__ void __launch_bounds__(256, 3) k_fx_transform(const FxParams p) {
     fx_dft<N>(v);
     const bool bad = e0 == FX_NAN || we == FX_NAN;
     const int e = e0 - FX_BITS + we + pass_shift(mx[1][t]) + pass_shift(mx[2][t]) + s3 + pass_shift(mx[4][t]) + s5;
+    if (INT && r == 0) p.ex[(size_t)x * p.ld + tg] = bad ? FX_NAN : e;
 #pragma unroll
     for (int j = 0; j < N; ++j) {
-      double2 o = make_double2(fx_to_double(v[j].y, e), fx_to_double(v[j].x, e));
-      if (bad) o.x = o.y = __longlong_as_double(0x7ff8000000000000ll);
       const int k = j * n23 + r;
-      p.phi[((size_t)k * p.nx + x) * p.ld + tg] = o;
-      if (p.mx) {  // the running maximum rarely grows: look before the atomic
-        unsigned* d = p.mx + (size_t)k * p.ld + tg;
-        const unsigned m = max(fx_mag(o.x), fx_mag(o.y));
-        if (m > __ldcg(d)) atomicMax(d, m);
+      const size_t o = ((size_t)k * p.nx + x) * p.ld + tg;
+      if constexpr (INT) {
+        reinterpret_cast<longlong2*>(p.phi)[o] = make_longlong2(v[j].y, v[j].x);
+        const unsigned long long m = (unsigned long long)((v[j].x ^ (v[j].x >> 63)) | (v[j].y ^ (v[j].y >> 63)));
+        const int em = bad ? FX_NAN : e + 64 - __clzll((long long)m);
+        int* d = p.mx + (size_t)k * p.ld + tg;  // the running maximum rarely grows: look before the atomic
+        if (em > __ldcg(d)) atomicMax(d, em);
+      } else {
+        double2 z = make_double2(fx_to_double(v[j].y, e), fx_to_double(v[j].x, e));
+        if (bad) z.x = z.y = __longlong_as_double(0x7ff8000000000000ll);
+        p.phi[o] = z;
       }
     }
   });
 }
 
 typedef void (*FxFn)(const FxParams);
+template <bool INT>
 FxFn fx_fn(const int n[3]) {
   if (n[0] == n[1] && n[1] == n[2]) switch (n[0]) {
-      case 2: return k_fx_transform<2, 2, 2>;
-      case 3: return k_fx_transform<3, 3, 3>;
-      case 4: return k_fx_transform<4, 4, 4>;
-      case 5: return k_fx_transform<5, 5, 5>;
-      case 6: return k_fx_transform<6, 6, 6>;
-      case 7: return k_fx_transform<7, 7, 7>;
-      case 8: return k_fx_transform<8, 8, 8>;
+      case 2: return k_fx_transform<2, 2, 2, INT>;
+      case 3: return k_fx_transform<3, 3, 3, INT>;
+      case 4: return k_fx_transform<4, 4, 4, INT>;
+      case 5: return k_fx_transform<5, 5, 5, INT>;
+      case 6: return k_fx_transform<6, 6, 6, INT>;
+      case 7: return k_fx_transform<7, 7, 7, INT>;
+      case 8: return k_fx_transform<8, 8, 8, INT>;
     }
-  return k_fx_transform<0, 0, 0>;
+  return k_fx_transform<0, 0, 0, INT>;
 }
 
 // W / Nk as 62-bit integers, one exponent per x-point (a CTA each).
@@ -283,7 +292,8 @@ int fx_init(ocn_ctx* c) {
   cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&c->d_Wfx), (size_t)c->nk * c->nx * sizeof(long long));
   if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&c->d_Wexp), (size_t)c->nx * sizeof(int));
   if (e != cudaSuccess) return set_err(c, OCN_ERR_ALLOC, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-  return allow_max_smem(c, fx_fn(c->dims.kmesh));
+  if (int rc = allow_max_smem(c, fx_fn<true>(c->dims.kmesh))) return rc;
+  return allow_max_smem(c, fx_fn<false>(c->dims.kmesh));
 }
 
 int fx_set_w(ocn_ctx* c) {
@@ -295,12 +305,13 @@ int fx_set_w(ocn_ctx* c) {
   return OCN_OK;
 }
 
-// phi[k][x][t], t < nt, in place; mx (may be null): [k][t] magnitude maxima of the result.
-int fx_transform(ocn_ctx* c, double2* phi, int nt, unsigned* mx) {
+// phi[k][x][t], t < nt, in place.  ex, mx null: binary64; else integers with exponents
+// ex[x][t] and column maxima mx[k][t] (cleared by the caller).
+int fx_transform(ocn_ctx* c, double2* phi, int nt, int* ex, int* mx) {
   const int* n = c->dims.kmesh;
-  const FxParams p = {phi, c->d_Wfx, c->d_Wexp, mx, c->nx, nt, n[0], n[1], n[2]};
+  const FxParams p = {phi, c->d_Wfx, c->d_Wexp, ex, mx, c->nx, nt, n[0], n[1], n[2]};
   const int lines = std::max({n[1] * n[2], n[0] * n[2], n[0] * n[1]});
-  fx_fn(n)<<<dim3(c->nx, nt / 4), (4 * lines + 31) / 32 * 32, fx_smem(n), c->stream>>>(p);
+  (ex ? fx_fn<true>(n) : fx_fn<false>(n))<<<dim3(c->nx, nt / 4), (4 * lines + 31) / 32 * 32, fx_smem(n), c->stream>>>(p);
   ++c->launches;
   OCN_CUDA(c, cudaGetLastError());
   return OCN_OK;

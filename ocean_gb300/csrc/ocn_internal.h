@@ -363,7 +363,8 @@ int cf_eval_noalloc(const double* ra, const double* ia, const double* rb, int it
 int fx_init(ocn_ctx* c);
 int fx_set_w(ocn_ctx* c);          // integer copy of W / Nk from d_W
 bool fx_supported(const ocn_ctx* c);
-int fx_transform(ocn_ctx* c, double2* phi, int nt, unsigned* mx);  // phi[k][x][t] in place
+// phi[k][x][t] in place: binary64 (ex, mx null) or integers with exponents ex[x][t], maxima mx[k][t]
+int fx_transform(ocn_ctx* c, double2* phi, int nt, int* ex, int* mx);
 
 // ---- FP64 direct term of the valence action in 64-bit fixed point (ocn_val_fx.cu)
 bool val_fx_supported(const int kmesh[3], int nv, size_t smem_optin);
@@ -382,8 +383,8 @@ int slice_width(const ocn_ctx* c); // vectors that share a launch (12 columns at
 int slice_prep_psi(ocn_ctx* c, const double* d_pr, const double* d_pi, size_t vstride, int nv);  // operand of:
 int slice_band_to_x(ocn_ctx* c, double2* phi, int nv);  // phi[k][x][t], t = v*Na + a
 // d_accpart slices of vectors v0 .. v0 + nv - 1 from phi'[k][x][t]
-int slice_x_to_band(ocn_ctx* c, const double2* phi, int nv, int v0, bool have_max);
-unsigned* slice_maxima(ocn_ctx* c);  // [k][a] magnitude maxima of phi', cleared by slice_prep_psi
+int slice_x_to_band(ocn_ctx* c, const double2* phi, int nv, int v0, bool integers);
+void slice_exponents(ocn_ctx* c, int** ex, int** mx);  // of phi' in integers
 int slice_set_mult(ocn_ctx* c);    // digit operands of the projectors (after ocn_set_mult)
 bool slice_mult_ready(const ocn_ctx* c);
 int slice_mult_apply(ocn_ctx* c, int v);  // multiplet term of the one prepared psi, into vector v's slices

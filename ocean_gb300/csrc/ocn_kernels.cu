@@ -1032,7 +1032,9 @@ int lr_apply_fp64(ocn_ctx* c, const double* d_pr, const double* d_pi, size_t vst
     if ((rc = slice_band_to_x(c, c->d_phi, nv))) return rc;
     {
       TimedScope ts(c, T_LR_FFT);
-      if ((rc = fx_transform(c, c->d_phi, na * nv, slice_maxima(c)))) return rc;
+      int *ex, *mx;
+      slice_exponents(c, &ex, &mx);
+      if ((rc = fx_transform(c, c->d_phi, na * nv, ex, mx))) return rc;
     }
     return slice_x_to_band(c, c->d_phi, nv, 0, true);
   }
@@ -1053,7 +1055,7 @@ int lr_apply_fp64(ocn_ctx* c, const double* d_pr, const double* d_pi, size_t vst
     }
     if (fx_supported(c)) {
       TimedScope ts(c, T_LR_FFT);
-      if (int rc = fx_transform(c, c->d_phi, na, nullptr)) return rc;
+      if (int rc = fx_transform(c, c->d_phi, na, nullptr, nullptr)) return rc;
     } else {
       const KmeshGeom<double> g = kmesh_geom<double>(c->dims.kmesh, na);
       TimedScope ts(c, T_LR_FFT);

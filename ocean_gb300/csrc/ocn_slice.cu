@@ -64,7 +64,8 @@ constexpr int SL_ROWS = 128;       // rows per tile (MMA M)
 // columns each (band -> x of the 2p case: 113 us with four warps and 255 registers,
 // 84 us with eight).
 constexpr int slice_threads(int nae) { return nae == 4 ? 192 : 320; }
-constexpr int SL_MAX_STAGES = 8;
+// (1s case of 512 k / 100 bands, x -> band: 355 us with six stages, 369 us with seven)
+constexpr int SL_MAX_STAGES = 6;
 constexpr size_t SL_SMEM = 222 * 1024;
 constexpr int SL_MAX_K = 2730;      // K per plane and accumulation: 2 * 2730 * 12 * 256 < 2^24
 constexpr unsigned long long SL_BIAS = 0x0842108421084210ull;  // sum of 16 * 32^i, i < 12
@@ -76,6 +77,8 @@ struct SliceParams {
   int G, Ge, KC, nch;        // 16-wide K granules (A; B padded to even), granules per chunk, chunks
   int ks, cps;               // K splits, chunks per split
   int ntiles, stages;
+  int sb;                    // boxes (slices) per pipeline stage, a divisor of 12
+  uint32_t stage_bytes;
   int bshared, koff, spin;   // B one k slice for all k; added to k for A; -1 or the spin whose columns are written
   int na, nvw;               // channels per vector; vectors written
   double2* phi;              // band -> x: [k][row][t]
@@ -177,7 +180,7 @@ __global__ void __launch_bounds__(slice_threads(P == 1 ? C / 2 : C), 1) k_slice_
   constexpr uint32_t IDESC0 = (1u << 4) | ((uint32_t)(SL_ROWS >> 4) << 24);
   extern __shared__ __align__(1024) uint8_t smem[];
   const int S = p.stages;
-  const uint32_t slot_bytes = p.KC * PITCH, stage_bytes = p.KC * SL_ROWS * 16;
+  const uint32_t slot_bytes = p.KC * PITCH, stage_bytes = p.stage_bytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * slot_bytes + S * stage_bytes);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * SL_MAX_STAGES + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -248,9 +251,9 @@ __global__ void __launch_bounds__(slice_threads(P == 1 ? C / 2 : C), 1) k_slice_
           if (slot == 0) bphase ^= 1;
           lastk = ti.k;
         }
-        const uint32_t bytes = (uint32_t)gc * ti.rt * 16;
+        const uint32_t bytes = (uint32_t)gc * ti.rt * 16 * p.sb;
         const uint8_t* src = At + (size_t)c * p.KC * ti.rt * 16 * NBOX;
-        for (int b = 0; b < NBOX; ++b) {
+        for (int b = 0; b < NBOX / p.sb; ++b) {
           ok = mbar_wait(empty0 + 8 * stage, phase ^ 1, abort_flag, TC_WAIT_CYCLES);
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
@@ -306,34 +309,36 @@ __global__ void __launch_bounds__(slice_threads(P == 1 ? C / 2 : C), 1) k_slice_
           if (!ok) break;
           lastk = ti.k;
         }
-        for (int b = 0; b < NBOX; ++b) {
+        for (int b0 = 0; b0 < NBOX; b0 += p.sb) {
           ok = __all_sync(0xffffffffu, mbar_wait(full0 + 8 * stage, phase, abort_flag, TC_WAIT_CYCLES));
           if (!ok) break;
           tc_fence_after();
-          const int plane = b / SL_S, i = b - plane * SL_S;
-          uint32_t ad = plain_desc(a_smem + stage * stage_bytes, lba);
-          // the first i column groups of slice i only meet empty slices: N shrinks in steps of 16
-          const uint32_t ni = (uint32_t)((SL_S - i) * C + 15) & ~15u, off = N - ni;
-          const uint32_t idesc = IDESC0 | ((ni >> 3) << 17);
-          uint32_t bd = plain_desc(b_smem + slot * slot_bytes + ((11 - i) * C + off) * 16, PITCH);
-          const uint32_t d0 = dt + (PL == 2 ? plane * N : 0) + off;
-          // the first MMA of an accumulator overwrites it
-          uint32_t accum = (c > ti.c0 || (PL == 2 ? i > 0 : b > 0)) ? 1u : 0u;
-          if (leader) {
+          for (int b = b0; b < b0 + p.sb; ++b) {
+            const int plane = b / SL_S, i = b - plane * SL_S;
+            uint32_t ad = plain_desc(a_smem + stage * stage_bytes + (b - b0) * gc * lba, lba);
+            // the first i column groups of slice i only meet empty slices: N shrinks in steps of 16
+            const uint32_t ni = (uint32_t)((SL_S - i) * C + 15) & ~15u, off = N - ni;
+            const uint32_t idesc = IDESC0 | ((ni >> 3) << 17);
+            uint32_t bd = plain_desc(b_smem + slot * slot_bytes + ((11 - i) * C + off) * 16, PITCH);
+            const uint32_t d0 = dt + (PL == 2 ? plane * N : 0) + off;
+            // the first MMA of an accumulator overwrites it
+            uint32_t accum = (c > ti.c0 || (PL == 2 ? i > 0 : b > 0)) ? 1u : 0u;
+            if (leader) {
 #pragma unroll 4
-            for (int g = 0; g < steps; ++g) {
+              for (int g = 0; g < steps; ++g) {
 #pragma unroll
-              for (int q = 0; q < P; ++q) {
-                const uint32_t part = MODE == 2 ? (uint32_t)(q ^ plane) : (uint32_t)q;  // im plane: parts swapped
-                const uint32_t neg = (MODE == 2 && P == 2 && q == 1 && plane == 1) ? (1u << 13) : 0u;
-                umma_fp8(d0 + q * N, ad, bd + (P == 2 ? part * PROWS : 0u), idesc | neg, accum);
+                for (int q = 0; q < P; ++q) {
+                  const uint32_t part = MODE == 2 ? (uint32_t)(q ^ plane) : (uint32_t)q;  // im plane: parts swapped
+                  const uint32_t neg = (MODE == 2 && P == 2 && q == 1 && plane == 1) ? (1u << 13) : 0u;
+                  umma_fp8(d0 + q * N, ad, bd + (P == 2 ? part * PROWS : 0u), idesc | neg, accum);
+                }
+                accum = 1u;
+                ad += 2 * (lba >> 4);
+                bd += 2 * (PITCH >> 4);
               }
-              accum = 1u;
-              ad += 2 * (lba >> 4);
-              bd += 2 * (PITCH >> 4);
             }
-            umma_commit(empty0 + 8 * stage);
           }
+          if (leader) umma_commit(empty0 + 8 * stage);
           __syncwarp();
           last_stage = (int)stage;
           last_phase = phase;
@@ -561,14 +566,14 @@ __device__ __forceinline__ double weigh(double x, double w) {
 // channel); column exponents, then digits of
 //   part 0 (Re phi): K = (re n) -> qr, (im n) -> -qi;  part 1 (Im phi): (re n) -> qi, (im n) -> qr.
 // merged: row order [slice][part][t], else [part][slice][t].  Clears the maxima that
-// the k-mesh transform of this action collects (mx, may be null).
+// the k-mesh transform of this action collects.
 __global__ void __launch_bounds__(256)
     k_slice_prep_b1(const double* __restrict__ pr, const double* __restrict__ pi, size_t vstride,
                     const double* __restrict__ allow, int nb, int nk, int na, int nae, int Ge, int merged,
-                    uint8_t* __restrict__ B, int* __restrict__ eB, unsigned* __restrict__ mx) {
+                    uint8_t* __restrict__ B, int* __restrict__ eB, int* __restrict__ mx) {
   __shared__ int se[OCN_MAX_NA];
   const int k = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (mx && (int)threadIdx.x < nae) mx[(size_t)k * nae + threadIdx.x] = 0;
+  if ((int)threadIdx.x < nae) mx[(size_t)k * nae + threadIdx.x] = -FX_NAN;
   for (int t = warp; t < nae; t += 8) {
     const int v = t / na, a = t - v * na;
     const size_t base = (size_t)nb * ((size_t)k + (size_t)nk * a);
@@ -610,9 +615,10 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Magnitude maxima mx[k][t] of src[k*nx + x][t] (k-meshes whose transform does not collect them).
+// Exponent maxima mx[k][t] of src[k*nx + x][t] (operands that do not come from the
+// fixed-point k-mesh transform).
 __global__ void __launch_bounds__(512)
-    k_slice_col_max(const double2* __restrict__ src, int nx, int nae, unsigned* __restrict__ mx) {
+    k_slice_col_max(const double2* __restrict__ src, int nx, int nae, int* __restrict__ mx) {
   __shared__ unsigned sm[OCN_MAX_NA];
   const int k = blockIdx.x;
   if (threadIdx.x < OCN_MAX_NA) sm[threadIdx.x] = 0;
@@ -625,22 +631,31 @@ __global__ void __launch_bounds__(512)
     atomicMax(&sm[threadIdx.x % nae], m);
   }
   __syncthreads();
-  if ((int)threadIdx.x < nae) mx[(size_t)k * nae + threadIdx.x] = sm[threadIdx.x];
+  if ((int)threadIdx.x < nae) mx[(size_t)k * nae + threadIdx.x] = fx_exp(sm[threadIdx.x]);
 }
 
-// phi' operand from src[k*nx + x][t] (parts: re, im) and its column maxima: digits,
-// rows as k_slice_prep_b1.  grid (ceil(items / block), Nk); a thread makes four x of
-// one column, both parts (reads 64-byte runs, writes 4-byte words of 64-byte runs).
+// int 2^s rounded to nearest, plus the digit bias; |int 2^s| <= 2^59
+__device__ __forceinline__ unsigned long long fix_int(long long v, int s) {
+  if (s >= 0) return SL_BIAS + ((unsigned long long)v << s);
+  const int r = min(-s, 63);
+  return SL_BIAS + (unsigned long long)((v + (1ll << (r - 1))) >> r);
+}
+
+// phi' operand from src[k*nx + x][t] (parts: re, im) and its column exponents: digits,
+// rows as k_slice_prep_b1.  INT: src holds integers with exponents ex[x][t], else
+// binary64.  grid (ceil(items / block), Nk); a thread makes four x of one column, both
+// parts (reads 64-byte runs, writes 4-byte words of 64-byte runs).
+template <bool INT>
 __global__ void __launch_bounds__(256)
-    k_slice_prep_b2(const double2* __restrict__ src, int nx, int nae, int Ge, int merged,
-                    const unsigned* __restrict__ mx, uint8_t* __restrict__ B, int* __restrict__ eB) {
+    k_slice_prep_b2(const double2* __restrict__ src, const int* __restrict__ ex, int nx, int nae, int Ge, int merged,
+                    const int* __restrict__ mx, uint8_t* __restrict__ B, int* __restrict__ eB) {
   const int k = blockIdx.y;
   if (blockIdx.x == 0 && (int)threadIdx.x < nae)
-    eB[(size_t)k * nae + threadIdx.x] = fx_exp(mx[(size_t)k * nae + threadIdx.x]);
+    eB[(size_t)k * nae + threadIdx.x] = mx[(size_t)k * nae + threadIdx.x];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= Ge * nae * 4) return;
   const int qd = i & 3, r = i >> 2;
-  const int t = r % nae, g = r / nae, e = fx_exp(mx[(size_t)k * nae + t]);
+  const int t = r % nae, g = r / nae, e = mx[(size_t)k * nae + t];
   const double2* f = src + (size_t)k * nx * nae + t;
   unsigned long long fr[4], fi[4];
 #pragma unroll
@@ -648,9 +663,18 @@ __global__ void __launch_bounds__(256)
     const int x = 16 * g + 4 * qd + j;
     fr[j] = fi[j] = SL_BIAS;
     if (x < nx) {
-      const double2 v = f[(size_t)x * nae];
-      fr[j] = fix_point(v.x, e);
-      fi[j] = fix_point(v.y, e);
+      if constexpr (INT) {
+        const longlong2 v = reinterpret_cast<const longlong2*>(f)[(size_t)x * nae];
+        if (e < FX_NAN) {
+          const int s = ex[(size_t)x * nae + t] + SL_FRAC - e;
+          fr[j] = fix_int(v.x, s);
+          fi[j] = fix_int(v.y, s);
+        }
+      } else {
+        const double2 v = f[(size_t)x * nae];
+        fr[j] = fix_point(v.x, e);
+        fi[j] = fix_point(v.y, e);
+      }
     }
   }
   uint8_t* out = B + ((size_t)k * Ge + g) * 2 * SL_S * nae * 16 + (size_t)t * 16 + 4 * qd;
@@ -707,7 +731,8 @@ struct SliceGemm {
 // two B slots and at least four A stages fit in shared memory (16 granules at most
 // for one resident B operand, 12 for streamed ones) with the widest columns, nae_max,
 // that share the A operand: its order depends on the chunks.
-void slice_plan(SliceGemm* s, int mode, int nae, int nae_max, int nk, int rows, int K, int sm_count) {
+void slice_plan(SliceGemm* s, int mode, int nae, int nae_max, int nk, int rows, int K, int sm_count,
+                double cost_split) {
   SliceParams& p = s->p;
   s->mode = mode;
   s->nae = nae;
@@ -724,29 +749,45 @@ void slice_plan(SliceGemm* s, int mode, int nae, int nae_max, int nk, int rows, 
   int kc = std::min(cap, p.Ge);
   while (kc > 2 && kc * (2 * pitch_max + 4 * SL_ROWS * 16) > SL_SMEM) kc -= 2;
   p.KC = kc;
-  p.nch = (p.G + kc - 1) / kc;
-  p.stages = (int)std::min<size_t>(SL_MAX_STAGES, (SL_SMEM - 2 * kc * pitch) / ((size_t)kc * SL_ROWS * 16));
-  s->smem = 2 * kc * pitch + (size_t)p.stages * kc * SL_ROWS * 16 + 256;  // + barriers
   p.ks = 1;
-  p.cps = p.nch;
   if (mode == 2) {
-    // K splits: the fewest per cent of idle SM time in the last wave of tiles
-    // (each split costs a partial-sum slice, so a later candidate has to gain 3%),
-    // and K per accumulation within the exact range
-    const int most = SL_MAX_K / (16 * kc);  // chunks per accumulation
-    const int least = (p.nch + most - 1) / most;
+    // K chunk and splits: the least modelled time of the busiest SM's share of A at
+    // 45 GB/s per SM, 0.6 us per chunk and the partial sums' round trip (cost_split
+    // seconds per slice); a smaller chunk or another split has to gain 3% (1s case of
+    // 512 k / 100 bands: 12 granules in 3 splits 358 us, 6 in 2 splits 371 us; 64 k /
+    // 32 bands: 12 in 2 splits 22 us, 8 in 2 splits 18 us).  K per accumulation
+    // stays within the exact range.
+    const double a_gran = (double)(p.nt > 1 ? SL_ROWS : p.rl) * 16 * s->nbox / 45e9;
     double best = 1e30;
-    for (int r = least; r <= std::max(least, std::min(p.nch, 8)); ++r) {
-      const int cps = (p.nch + r - 1) / r, ks = (p.nch + cps - 1) / cps;
-      const long long tiles = (long long)nk * p.nt * ks;
-      const double t = (double)((tiles + sm_count - 1) / sm_count) * cps;
-      if (t < 0.97 * best) {
-        best = t;
-        p.ks = ks;
-        p.cps = cps;
+    for (int q = kc; q >= std::min(kc, 4); q -= 2) {
+      const int nch = (p.G + q - 1) / q, most = SL_MAX_K / (16 * q), least = (nch + most - 1) / most;
+      for (int r = least; r <= std::max(least, std::min(nch, 8)); ++r) {
+        const int cps = (nch + r - 1) / r, ks = (nch + cps - 1) / cps;
+        const long long tiles = (long long)nk * p.nt * ks;
+        const double waves = (double)((tiles + sm_count - 1) / sm_count);
+        const double t = waves * (std::min(cps * q, p.G) * a_gran + cps * 0.6e-6) + ks * cost_split;
+        if (t < 0.97 * best) {
+          best = t;
+          p.KC = q;
+          p.ks = ks;
+        }
       }
     }
   }
+  p.nch = (p.G + p.KC - 1) / p.KC;
+  p.cps = (p.nch + p.ks - 1) / p.ks;
+  // boxes per stage: up to 32 KB in one copy and one wait (short rows or few granules
+  // make small boxes), with four stages at least.  An MMA reads 128 rows: behind the
+  // last box of a tile of fewer rows that runs past the data by up to 127 rows.
+  const int rt = p.nt > 1 ? SL_ROWS : p.rl;
+  const size_t box = (size_t)p.KC * rt * 16, room = SL_SMEM - 2 * p.KC * pitch;
+  for (int sb : {12, 6, 4, 3, 2, 1}) {
+    p.sb = sb;
+    p.stage_bytes = (uint32_t)((sb * box + (size_t)(SL_ROWS - rt) * 16 + 127) / 128 * 128);
+    if (sb == 1 || (sb * box <= 32 * 1024 && 4 * (size_t)p.stage_bytes <= room)) break;
+  }
+  p.stages = (int)std::min<size_t>(SL_MAX_STAGES, room / p.stage_bytes);
+  s->smem = 2 * p.KC * pitch + (size_t)p.stages * p.stage_bytes + 256;  // + barriers
   p.ntiles = nk * p.nt * p.ks;
   p.spin = -1;
   s->grid = std::min(p.ntiles, sm_count);
@@ -760,13 +801,14 @@ struct SliceLR {
   SliceGemm g1[3], g2[3];  // band -> x, x -> band of 1, 2, 3 vectors; A is held by [0] and shared
   uint8_t *b1 = nullptr, *b2 = nullptr;
   int *e1 = nullptr, *e2 = nullptr;
-  unsigned* mx2 = nullptr;  // magnitude maxima of phi' per (k, column)
+  int* mx2 = nullptr;      // exponent maxima of phi' per (k, column)
+  int* ex2 = nullptr;      // exponents of phi' per (x, column)
   // multiplet projectors (fg_combo): amplitudes and back-projection
   bool mult_ready = false;
   SliceGemm gm1, gm2;
   uint8_t* bm = nullptr;
   int* em = nullptr;
-  unsigned* mxm = nullptr;
+  int* mxm = nullptr;
   double2* amp_part = nullptr;  // [k][p][a]
   int* d_err = nullptr;
 };
@@ -873,8 +915,9 @@ int slice_init(ocn_ctx* c) {
   int rc;
   for (int w = 1; w <= s->nvs; ++w) {
     const int nae = w * c->na, most = s->nvs * c->na;
-    slice_plan(&s->g1[w - 1], 1, nae, most, c->nk, c->nx, 2 * c->nb, c->sm_count);
-    slice_plan(&s->g2[w - 1], 2, nae, most, c->nk, c->nb, c->nx, c->sm_count);
+    const double cost = 32.0 * c->npsi / 6e12;  // the same splits for every width: results do not depend on it
+    slice_plan(&s->g1[w - 1], 1, nae, most, c->nk, c->nx, 2 * c->nb, c->sm_count, 0.0);
+    slice_plan(&s->g2[w - 1], 2, nae, most, c->nk, c->nb, c->nx, c->sm_count, cost);
     if ((rc = allow_max_smem(c, slice_fn(1, nae))) || (rc = allow_max_smem(c, slice_fn(2, nae)))) return rc;
   }
   c->lr_xsplit = s->g2[0].p.ks;
@@ -882,6 +925,7 @@ int slice_init(ocn_ctx* c) {
   const size_t cols = (size_t)c->nk * c->na * s->nvs;
   if ((rc = salloc(c, &s->b1, w1.b_bytes())) || (rc = salloc(c, &s->b2, w2.b_bytes())) ||
       (rc = salloc(c, &s->e1, cols)) || (rc = salloc(c, &s->e2, cols)) || (rc = salloc(c, &s->mx2, cols)) ||
+      (rc = salloc(c, &s->ex2, (size_t)c->nx * c->na * s->nvs)) ||
       (rc = salloc(c, &s->d_err, 1)))
     return rc;
   OCN_CUDA(c, cudaMemsetAsync(s->d_err, 0, sizeof(int), c->stream));
@@ -896,7 +940,7 @@ void slice_free(ocn_ctx* c) {
   if (!s) return;
   slice_drop_a(s);
   slice_drop_mult(s);
-  for (void* q : {(void*)s->b1, (void*)s->b2, (void*)s->e1, (void*)s->e2, (void*)s->mx2, (void*)s->d_err})
+  for (void* q : {(void*)s->b1, (void*)s->b2, (void*)s->e1, (void*)s->e2, (void*)s->mx2, (void*)s->ex2, (void*)s->d_err})
     if (q) cudaFree(q);
   delete s;
   c->slice = nullptr;
@@ -936,8 +980,8 @@ int slice_set_mult(ocn_ctx* c) {
   c->mult_parts = 0;
   const int np = c->mult.np;
   if (np == 0) return OCN_OK;
-  slice_plan(&s->gm1, 1, c->na, c->na, c->nk, np, 2 * c->nb, c->sm_count);
-  slice_plan(&s->gm2, 2, c->na, c->na, c->nk, c->nb, np, c->sm_count);
+  slice_plan(&s->gm1, 1, c->na, c->na, c->nk, np, 2 * c->nb, c->sm_count, 0.0);
+  slice_plan(&s->gm2, 2, c->na, c->na, c->nk, c->nb, np, c->sm_count, 32.0 * c->npsi / 6e12);
   s->gm2.p.bshared = 1;
   double* parts = nullptr;
   if (!slice_alloc_a(c, &s->gm1, &s->gm2, np) || salloc(c, &s->bm, s->gm2.b_bytes()) || salloc(c, &s->em, c->na) ||
@@ -990,7 +1034,7 @@ int slice_mult_apply(ocn_ctx* c, int v) {
   if ((rc = mult_hamp(c, m.amp, m.hamp))) return rc;
   k_slice_col_max<<<1, 512, 0, c->stream>>>(m.hamp, m.np, c->na, s->mxm);
   const int items = s->gm2.p.Ge * c->na * 4;
-  k_slice_prep_b2<<<dim3((items + 255) / 256, 1), 256, 0, c->stream>>>(m.hamp, m.np, c->na, s->gm2.p.Ge,
+  k_slice_prep_b2<false><<<dim3((items + 255) / 256, 1), 256, 0, c->stream>>>(m.hamp, nullptr, m.np, c->na, s->gm2.p.Ge,
                                                                       slice_merged(c->na) ? 1 : 0, s->mxm, s->bm, s->em);
   c->launches += 2;
   OCN_CUDA(c, cudaGetLastError());
@@ -1009,29 +1053,37 @@ int slice_band_to_x(ocn_ctx* c, double2* phi, int nv) {
   return OCN_OK;
 }
 
-// The maxima that slice_x_to_band scales its operand by, cleared by slice_prep_psi.
-unsigned* slice_maxima(ocn_ctx* c) { return c->slice->mx2; }
+// Exponents per (x, t) and maxima per (k, t) that fx_transform leaves with phi' in
+// integers; the maxima are cleared by slice_prep_psi.
+void slice_exponents(ocn_ctx* c, int** ex, int** mx) {
+  *ex = c->slice->ex2;
+  *mx = c->slice->mx2;
+}
 
-// d_accpart slices of vectors v0 .. v0 + nv - 1 from phi'[k][x][t]; have_max: the maxima were collected.
-int slice_x_to_band(ocn_ctx* c, const double2* phi, int nv, int v0, bool have_max) {
+// d_accpart slices of vectors v0 .. v0 + nv - 1 from phi'[k][x][t], in integers with
+// slice_exponents or (not integers) in binary64.
+int slice_x_to_band(ocn_ctx* c, const double2* phi, int nv, int v0, bool integers) {
   SliceLR* s = c->slice;
   const SliceGemm& g = s->g2[nv - 1];
   const int nae = c->na * nv;
   {
     TimedScope ts(c, T_LR_PREP);
-    if (!have_max) {
+    const int items = g.p.Ge * nae * 4, merged = slice_merged(nae) ? 1 : 0;
+    const dim3 grid((items + 255) / 256, c->nk);
+    if (integers) {
+      k_slice_prep_b2<true><<<grid, 256, 0, c->stream>>>(phi, s->ex2, c->nx, nae, g.p.Ge, merged, s->mx2, s->b2, s->e2);
+    } else {
       k_slice_col_max<<<c->nk, 512, 0, c->stream>>>(phi, c->nx, nae, s->mx2);
       ++c->launches;
+      k_slice_prep_b2<false><<<grid, 256, 0, c->stream>>>(phi, nullptr, c->nx, nae, g.p.Ge, merged, s->mx2, s->b2, s->e2);
     }
-    const int items = g.p.Ge * nae * 4;
-    k_slice_prep_b2<<<dim3((items + 255) / 256, c->nk), 256, 0, c->stream>>>(phi, c->nx, nae, g.p.Ge,
-                                                                            slice_merged(nae) ? 1 : 0, s->mx2, s->b2, s->e2);
     ++c->launches;
     OCN_CUDA(c, cudaGetLastError());
   }
   TimedScope ts(c, T_LR_GEMM2);
   for (int sp = 0; sp < c->nspn; ++sp)
-    if (int rc = slice_launch(c, g, s->g2[0], s->b2, s->e2, nullptr, c->d_accpart + (size_t)v0 * 2 * c->npsi, sp, c->nspn)) return rc;
+    if (int rc = slice_launch(c, g, s->g2[0], s->b2, s->e2, nullptr, c->d_accpart + (size_t)v0 * 2 * c->npsi, sp, c->nspn))
+      return rc;
   return OCN_OK;
 }
 
