@@ -31,6 +31,12 @@
 // GB300 runs at 64x its FP64 rate; the normal equations, the solve and the
 // residual norms stay FP64.
 //
+// A step on a small problem is bound by launches and waits, not by its passes: the
+// combine g += sum c au also forms the next u, |g|^2 and pg, the passes reduce their
+// sums themselves and write them to pinned memory, and the next step starts before
+// |g|^2 is read where the normal equations put it above the threshold (4^3 k / 32
+// bands, FP64: 160 -> 111 us per step).
+//
 // Energy lanes.  With ocn_gmres_set_lanes the energy list is split into
 // contiguous chunks, one per lane; each lane runs the reference's recycled
 // sweep over its chunk and the lanes advance in lockstep, so one block action
@@ -44,6 +50,7 @@
 #include <complex>
 #include <cstring>
 #include <functional>
+#include <type_traits>
 #include <vector>
 
 #include "ocn_df.cuh"
@@ -56,7 +63,9 @@ namespace {
 typedef std::complex<double> cd;
 constexpr double EV2HA = 0.036749322175666;
 constexpr int GM_THREADS = 256;
-constexpr int GM_CTAS_PER_SM = 4;  // target CTAs per SM of the Gram and recycle passes
+constexpr int GM_CTAS_PER_SM = 4;  // target CTAs per SM of the recycle pass
+constexpr int GM_GRAM_PER_SM = 3;  // CTAs per SM of the Gram pass (its launch bound): one wave,
+                                   // 8^3 k / 40 bands, mixed: a sweep of 4 energies 66 -> 60 ms
 constexpr int GM_NQ = 10;          // real sums per basis vector in the Gram pass
 
 // double-float helpers: ocn_df.cuh
@@ -74,7 +83,8 @@ struct Pol<false> {  // FP64, complex interleaved
     __device__ __forceinline__ void zero() { v = 0.0; }
     __device__ __forceinline__ void fma(R a, R b) { v = __fma_rn(a, b, v); }
     __device__ __forceinline__ double value() const { return v; }
-    __device__ __forceinline__ void shfl_add(int o) { v += __shfl_down_sync(0xffffffffu, v, o); }
+    // this plus the other lane's o
+    __device__ __forceinline__ void xchg_add(const Acc& o, int lane) { v += __shfl_xor_sync(0xffffffffu, o.v, lane); }
   };
   static __device__ __forceinline__ E pack(double re, double im) { return make_double2(re, im); }
   static __device__ __forceinline__ R re(const E& e) { return e.x; }
@@ -95,9 +105,9 @@ struct Pol<true> {  // double-float: (re hi, re lo, im hi, im lo)
     __device__ __forceinline__ void zero() { h = l = 0.0f; }
     __device__ __forceinline__ void fma(R a, R b) { df_fma(h, l, a, b); }
     __device__ __forceinline__ double value() const { return (double)h + (double)l; }
-    __device__ __forceinline__ void shfl_add(int o) {
-      const float bh = __shfl_down_sync(0xffffffffu, h, o);
-      const float bl = __shfl_down_sync(0xffffffffu, l, o);
+    __device__ __forceinline__ void xchg_add(const Acc& o, int lane) {
+      const float bh = __shfl_xor_sync(0xffffffffu, o.h, lane);
+      const float bl = __shfl_xor_sync(0xffffffffu, o.l, lane);
       df_add(h, l, bh, bl);
     }
   };
@@ -139,17 +149,43 @@ __device__ __forceinline__ void caxpy(typename Pol<DF>::Acc& sr, typename Pol<DF
   si.fma(P::im(c), P::re(v));
 }
 
+// Warp sums of K accumulators: each exchange hands the other lane the half of the sums
+// that this lane gives up, so ten sums take 12 additions instead of 50 (the additions of
+// a shuffle tree per sum were more FP64 work than the products of a Gram pass over 8192
+// elements and 49 basis vectors: 42 us; 29 us with this and 24 us with the CTAs in one
+// wave, where the 8 M products take 14 us of the FP64 pipe).  Returns in acc[0] the sum whose
+// index is the returned value.
+template <int K, int O, typename A>
+__device__ __forceinline__ void warp_sums(A* acc, int* id) {
+  if constexpr (O > 0) {
+    constexpr int H = (K + 1) / 2;
+    const bool up = (threadIdx.x & O) != 0;
+#pragma unroll
+    for (int q = 0; q < H; ++q) {
+      const bool pair = q + H < K;
+      const A give = pair && !up ? acc[pair ? q + H : q] : acc[q];
+      if (pair && up) {
+        acc[q] = acc[q + H];
+        id[q] = id[q + H];
+      }
+      acc[q].xchg_add(give, O);
+    }
+    warp_sums<H, O / 2>(acc, id);
+  }
+}
+
 // Block reduction of K accumulators per thread into K doubles written by
-// threads 0..K-1 to out[0..K-1] (fixed order: shuffle tree, then warps in order).
+// threads 0..K-1 to out[0..K-1] (fixed order: exchange tree, then warps in order).
 template <bool DF, int K>
 __device__ __forceinline__ void block_reduce_out(typename Pol<DF>::Acc (&acc)[K], double* sh, double* out,
                                                  int kvalid) {
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  static_assert(K <= 32, "one sum per lane at the end of the tree");
+  const int w = threadIdx.x >> 5;
+  int id[K];
 #pragma unroll
-  for (int q = 0; q < K; ++q) {
-    for (int o = 16; o > 0; o >>= 1) acc[q].shfl_add(o);
-    if (l == 0) sh[w * K + q] = acc[q].value();
-  }
+  for (int q = 0; q < K; ++q) id[q] = q;
+  warp_sums<K, 16>(acc, id);
+  sh[w * K + id[0]] = acc[0].value();
   __syncthreads();
   const int nw = blockDim.x >> 5;
   for (int q = threadIdx.x; q < kvalid; q += blockDim.x) {
@@ -157,6 +193,34 @@ __device__ __forceinline__ void block_reduce_out(typename Pol<DF>::Acc (&acc)[K]
     for (int i = 0; i < nw; ++i) s += sh[i * K + q];
     out[q] = s;
   }
+}
+
+// out[i] = sum_b part[b*stride + i], i < nout, by one CTA in the fixed order of k_gm_reduce.
+__device__ __forceinline__ void sum_parts(const double* part, int nblk, size_t stride, int nout, double* out) {
+  const int lane = threadIdx.x & 31;
+  for (int i = threadIdx.x >> 5; i < nout; i += blockDim.x >> 5) {
+    double s = 0.0;
+    for (int b = lane; b < nblk; b += 32) s += __ldcg(part + (size_t)b * stride + i);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) out[i] = s;
+  }
+}
+
+// The last CTA of a group of nblk (by ticket, which it resets) sums the group's partial
+// sums.  In place of a k_gm_reduce launch after the pass.  out may be host memory.
+__device__ __forceinline__ void last_block_sum(const double* part, int nblk, size_t stride, int nout, double* out,
+                                               unsigned int* ticket) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(ticket, 1u) == (unsigned int)nblk - 1;
+    if (last) *ticket = 0u;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  sum_parts(part, nblk, stride, nout, out);
 }
 
 // ------------------------------------------------------------------ kernels
@@ -196,7 +260,9 @@ __global__ void __launch_bounds__(GM_THREADS)
 // basis vector j = blockIdx.y <= m and the element chunk blockIdx.x, partial
 // sums of
 //   <au_j|au_m>, <au_j|u_m>, <au_m|u_j>, <u_j|u_m>, <au_j|g>   (re, im each)
-// into part[(chunk*(m+1) + j)*10 + q].  u_m and au_m were stored by the two
+// into part[(chunk*(m+1) + j)*10 + q], summed over the chunks into out[j*10 + q] by the
+// last CTA of each j.  red != NULL: a last row of CTAs also sums the nred partials that the
+// combine before it left.  u_m and au_m were stored by the two
 // kernels before this one; for j == m their values are reused.  The next
 // element's five loads are issued before the current element's products (the
 // pass is bound by issue and load latency; measured on the 8^3 k / 100-band
@@ -204,12 +270,17 @@ __global__ void __launch_bounds__(GM_THREADS)
 // CTA and no prefetch).
 template <bool DF>
 __global__ void __launch_bounds__(GM_THREADS, 3)
-    k_gm_gram(const typename Pol<DF>::E* __restrict__ ub, const typename Pol<DF>::E* __restrict__ aub, int m,
-              size_t n, size_t chunk, const typename Pol<DF>::E* __restrict__ gs, double* __restrict__ part) {
+    k_gm_gram(const double* __restrict__ red, int nred, double* red_out, const typename Pol<DF>::E* __restrict__ ub, const typename Pol<DF>::E* __restrict__ aub, int m,
+              size_t n, size_t chunk, const typename Pol<DF>::E* __restrict__ gs, double* part, double* out,
+              unsigned int* ticket) {
   typedef Pol<DF> P;
   typedef typename P::E E;
   __shared__ double sh[(GM_THREADS / 32) * GM_NQ];
   const int j = blockIdx.y;
+  if (j > m) {  // the combine's partial sums, when it left them (see combine_into)
+    if (blockIdx.x == 0) sum_parts(red, nred, 3, 3, red_out);
+    return;
+  }
   const bool self = j == m;
   const size_t e0 = blockIdx.x * chunk;
   const size_t e1 = min(n, e0 + chunk);
@@ -251,6 +322,7 @@ __global__ void __launch_bounds__(GM_THREADS, 3)
     Aj = Aj2;
   }
   block_reduce_out<DF, GM_NQ>(acc, sh, part + ((size_t)blockIdx.x * (m + 1) + j) * GM_NQ, GM_NQ);
+  last_block_sum(part + (size_t)j * GM_NQ, gridDim.x, (size_t)(m + 1) * GM_NQ, GM_NQ, out + (size_t)j * GM_NQ, ticket + j);
 }
 
 // make_recycle (au_j += dw u_j, OCEAN_gmres.f90:233-236) fused with the
@@ -278,31 +350,84 @@ __global__ void __launch_bounds__(GM_THREADS)
   block_reduce_out<DF, 2>(acc, sh, part + ((size_t)blockIdx.x * P + j) * 2, 2);
 }
 
-// y += sum_j c_j v_j over nvec basis vectors (coefficients in basis format),
-// then partial sums over this CTA's elements of |y|^2 and <rhs|y> into
-// red[block*3 + q] (when red != NULL).
-template <bool DF>
+struct alignas(16) Coef16 {
+  unsigned char b[16];
+};
+// Coefficients of up to GM_NCOEF basis vectors travel as a launch parameter (a copy of a
+// few hundred bytes ahead of the kernel costs more than the kernel's own work on a small
+// problem); longer lists are read from device memory.
+constexpr int GM_NCOEF = 128;
+struct GmCoef {
+  Coef16 c[GM_NCOEF];
+};
+
+// y += sum_j c_j v_j over nvec basis vectors (coefficients in basis format), then,
+// when red != NULL, the sums |y|^2 and <rhs|y> into out[0..2] (partials in red, the last
+// CTA sums them).  With PREC, y is the residual and the next step's preconditioned
+// residual pg = y o pcdiv (OCEAN_psi_3element_mult, OCEAN_gmres.f90:689), basis vector u
+// and residual in basis format are written as k_gm_prec would; the partials stay in red for
+// the Gram pass to sum.
+// A CTA covers blockDim/js elements with js groups of threads, each taking every js-th
+// basis vector: a small problem has too few elements to fill the chip, and one thread
+// per element walks the basis as one chain of loads.
+template <bool DF, bool PREC>
 __global__ void __launch_bounds__(GM_THREADS)
-    k_gm_combine(const typename Pol<DF>::E* __restrict__ vb, int nvec, const typename Pol<DF>::E* __restrict__ coef,
-                 double* __restrict__ y, size_t n, const double* __restrict__ rhs, double* __restrict__ red) {
+    k_gm_combine(const typename Pol<DF>::E* __restrict__ vb, int nvec, const __grid_constant__ GmCoef cp,
+                 const typename Pol<DF>::E* __restrict__ coef, int js, double* __restrict__ y, size_t n,
+                 const double* __restrict__ rhs, double* red, double* out, unsigned int* ticket,
+                 const double* __restrict__ pcdiv, double* __restrict__ pg, typename Pol<DF>::E* __restrict__ u,
+                 typename Pol<DF>::E* __restrict__ gs) {
   typedef Pol<DF> P;
   typedef typename P::E E;
   extern __shared__ __align__(16) unsigned char gm_sm[];
   E* sc = reinterpret_cast<E*>(gm_sm);
-  for (int j = threadIdx.x; j < nvec; j += blockDim.x) sc[j] = coef[j];
+  double2* sp = reinterpret_cast<double2*>(gm_sm) + nvec;  // js > 1: one sum per thread
+  const E* pc = reinterpret_cast<const E*>(&cp);
+  for (int j = threadIdx.x; j < nvec; j += blockDim.x) sc[j] = nvec <= GM_NCOEF ? pc[j] : coef[j];
   __syncthreads();
+  const int ec = GM_THREADS / js, grp = threadIdx.x / ec, le = threadIdx.x - grp * ec;
   double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
+  for (size_t e0 = (size_t)blockIdx.x * ec; e0 < n; e0 += (size_t)gridDim.x * ec) {
+    const size_t e = e0 + le;
     typename P::Acc ar, ai;
     ar.zero();
     ai.zero();
-#pragma unroll 4
-    for (int j = 0; j < nvec; ++j) caxpy<DF>(ar, ai, sc[j], vb[(size_t)j * n + e]);
-    const double yr = y[e] + ar.value();
-    const double yi = y[n + e] + ai.value();
+    if (e < n) {
+      for (int j = grp; j < nvec; j += 8 * js) {  // eight loads in flight, also in the last round
+        E v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (j + q * js < nvec) v[q] = vb[(size_t)(j + q * js) * n + e];
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (j + q * js < nvec) caxpy<DF>(ar, ai, sc[j + q * js], v[q]);
+      }
+    }
+    double vr = ar.value(), vi = ai.value();
+    if (js > 1) {
+      if (grp > 0) sp[threadIdx.x] = make_double2(vr, vi);
+      __syncthreads();
+      if (grp == 0)
+        for (int q = 1; q < js; ++q) {
+          vr += sp[q * ec + le].x;
+          vi += sp[q * ec + le].y;
+        }
+      __syncthreads();
+    }
+    if (grp > 0 || e >= n) continue;
+    const double yr = y[e] + vr;
+    const double yi = y[n + e] + vi;
     if (nvec > 0) {
       y[e] = yr;
       y[n + e] = yi;
+    }
+    if (PREC) {
+      const double c = pcdiv[e], d = pcdiv[n + e];
+      const double zr = yr * c - yi * d, zi = yr * d + yi * c;
+      pg[e] = zr;
+      pg[n + e] = zi;
+      u[e] = P::pack(zr, zi);
+      gs[e] = P::pack(yr, yi);
     }
     if (red) {
       s0 += yr * yr + yi * yi;
@@ -320,6 +445,7 @@ __global__ void __launch_bounds__(GM_THREADS)
   acc[1].v = s1;
   acc[2].v = s2;
   block_reduce_out<false, 3>(acc, shr, red + (size_t)blockIdx.x * 3, 3);
+  if (!PREC) last_block_sum(red, gridDim.x, 3, 3, out, ticket);
 }
 
 // g = (er + i ei) x - t - rhs  (set_initial_vector: ax = (w + i G) x - H x,
@@ -441,9 +567,6 @@ struct Chol {
 };
 
 // Host split of a complex coefficient into the basis format of the kernels.
-struct Coef16 {
-  unsigned char b[16];
-};
 Coef16 pack_coef(bool dfmt, cd c) {
   Coef16 o;
   if (dfmt) {
@@ -464,6 +587,11 @@ int grid_n(int sm_count, size_t n) {
   const size_t b = (n + GM_THREADS - 1) / GM_THREADS;
   return (int)std::max<size_t>(1, std::min<size_t>(b, (size_t)4 * sm_count));
 }
+
+constexpr int GM_HOST_G = 4;  // doubles ahead of the Gram row in the pinned area
+// An inner step is started before |g|^2 of its residual is read back when the normal
+// equations put it above this multiple of the convergence threshold (see LP_ITER_RB).
+constexpr double GM_AHEAD = 2.0;
 
 enum LaneWait { LW_RUN, LW_H, LW_RB, LW_DONE };
 
@@ -488,8 +616,10 @@ struct Lane {
   // device
   double *x = nullptr, *g = nullptr, *pcdiv = nullptr;
   unsigned char *ub = nullptr, *aub = nullptr, *gs = nullptr, *coef = nullptr;
-  double *part = nullptr, *out = nullptr;
-  double* host = nullptr;   // pinned read-back area
+  double *part = nullptr, *red = nullptr;  // partial sums of the Gram and recycle passes; of combine and resid
+  int nred = 0;
+  unsigned int* ticket = nullptr;  // last-CTA tickets: one per basis vector, then the combine's
+  double* host = nullptr;   // pinned: GM_HOST_G sums of combine, resid; then the Gram row or recycled rhs
   Coef16* hcoef = nullptr;  // pinned coefficient staging
   // H slot of the current round
   int slot = -1;
@@ -499,6 +629,8 @@ struct Lane {
   int it = 0;       // current inner step (1-based)
   bool restarted = false;
   bool after_recycle = false;
+  bool ahead = false;   // this inner step was started before its residual's |g|^2 was read
+  bool gknown = false;  // gval is |g|^2 of the residual in g
   double ener = 0.0, prev_energy = -1.0e308;
   int complete_iter = 0, restarts = 0;
   double gval = 0.0, rval = 0.0, ival = 0.0;
@@ -530,8 +662,11 @@ int gmres_solve_op(const GmresOp& op, const double* d_rhs_in, double kpref, cons
   // Gram / recycle chunking: about GM_CTAS_PER_SM CTAs per SM over all basis vectors
   const size_t nchunk_max =
       std::max<size_t>(8, std::min<size_t>((n + 255) / 256, (size_t)GM_CTAS_PER_SM * SM));
-  const size_t part_doubles = std::max<size_t>(nchunk_max * (size_t)depth * GM_NQ, (size_t)4 * SM * 3);
-  const size_t rb_doubles = (size_t)depth * GM_NQ + 8;
+  // elements per Gram CTA at least: two per thread (the block reduction of one CTA costs as
+  // much FP64 work as one more element per thread)
+  const size_t gm_rows = 2 * GM_THREADS;
+  const size_t part_doubles = nchunk_max * (size_t)depth * GM_NQ, red_doubles = (size_t)4 * SM * 3;
+  const size_t rb_doubles = (size_t)depth * GM_NQ + GM_HOST_G;
   const size_t host_bytes = rb_doubles * sizeof(double) + (size_t)depth * sizeof(Coef16);
 
   std::vector<void*> owned;
@@ -565,7 +700,7 @@ int gmres_solve_op(const GmresOp& op, const double* d_rhs_in, double kpref, cons
     unsigned char* q = nullptr;
     const size_t vb = 2 * n * sizeof(double), eb = n * 16;
     const size_t bytes = 3 * vb + (2 * (size_t)depth + 1) * eb + (size_t)depth * 16 +
-                         (part_doubles + rb_doubles) * sizeof(double);
+                         (part_doubles + red_doubles) * sizeof(double) + ((size_t)depth + 1) * sizeof(unsigned int);
     if ((rc = alloc(bytes, (void**)&q))) break;
     ln.x = reinterpret_cast<double*>(q);
     ln.g = ln.x + 2 * n;
@@ -575,7 +710,12 @@ int gmres_solve_op(const GmresOp& op, const double* d_rhs_in, double kpref, cons
     ln.gs = ln.aub + (size_t)depth * eb;
     ln.coef = ln.gs + eb;
     ln.part = reinterpret_cast<double*>(ln.coef + (size_t)depth * 16);
-    ln.out = ln.part + part_doubles;
+    ln.red = ln.part + part_doubles;
+    ln.ticket = reinterpret_cast<unsigned int*>(ln.red + red_doubles);
+    if (cudaMemsetAsync(ln.ticket, 0, ((size_t)depth + 1) * sizeof(unsigned int), stream) != cudaSuccess) {
+      rc = op.err(OCN_ERR_CUDA, "cudaMemsetAsync (GMRES tickets)");
+      break;
+    }
     ln.C.assign((size_t)depth * depth, cd(0.0, 0.0));
     ln.A = ln.C;
     ln.S = ln.C;
@@ -607,38 +747,58 @@ int gmres_solve_op(const GmresOp& op, const double* d_rhs_in, double kpref, cons
     k_gm_reduce<<<(nout * 32 + 255) / 256, 256, 0, stream>>>(part, nblk, nout, dout);
     return launched();
   };
-  auto readback = [&](Lane& ln, const double* dsrc, int count) -> int {
-    GM_CUDA(cudaMemcpyAsync(ln.host, dsrc, count * sizeof(double), cudaMemcpyDeviceToHost, stream));
+  // The passes write their sums to the lane's pinned area themselves; the scheduler syncs
+  // the stream before the lane goes on.
+  auto readback = [&](Lane& ln) -> int {
     ln.wait = LW_RB;
     return OCN_OK;
   };
-  // y += sum_j coef_j v_j (coefficients staged through this lane's pinned
-  // buffer; every path syncs the stream between two of a lane's calls, so the
-  // previous copy out of it has completed); want: |y|^2 and <rhs|y> to ln.out
+  // y += sum_j coef_j v_j (a long list of coefficients is staged through this lane's pinned
+  // buffer; every path syncs the stream between two of a lane's calls, so the previous copy
+  // out of it has completed); want: |y|^2 and <rhs|y> to ln.host[0..2]; pg != NULL: y = g
+  // and the next step's u, gs and pg as well
   auto combine_into = [&](Lane& ln, const unsigned char* vb, const std::vector<cd>& cf, int nvec, double* y,
-                          bool want) -> int {
-    if (nvec > 0) {
+                          bool want, double* pg) -> int {
+    GmCoef cp;
+    if (nvec <= GM_NCOEF) {
+      for (int j = 0; j < nvec; ++j) cp.c[j] = pack_coef(dfmt, cf[j]);
+    } else {
       for (int j = 0; j < nvec; ++j) ln.hcoef[j] = pack_coef(dfmt, cf[j]);
       GM_CUDA(cudaMemcpyAsync(ln.coef, ln.hcoef, nvec * sizeof(Coef16), cudaMemcpyHostToDevice, stream));
     }
-    const int gb = grid_n(SM, n);
-    double* red = want ? ln.part : nullptr;
-    const size_t smem = (size_t)std::max(1, nvec) * 16;
-    if (dfmt)
-      k_gm_combine<true><<<gb, GM_THREADS, smem, stream>>>(reinterpret_cast<const float4*>(vb), nvec,
-                                                             reinterpret_cast<const float4*>(ln.coef), y, n,
-                                                             rhs, red);
-    else
-      k_gm_combine<false><<<gb, GM_THREADS, smem, stream>>>(reinterpret_cast<const double2*>(vb), nvec,
-                                                              reinterpret_cast<const double2*>(ln.coef), y, n,
-                                                              rhs, red);
-    int q = launched();
-    if (q || !want) return q;
-    return reduce_to(ln.part, gb, 3, ln.out);
+    // thread groups per element until the chip has a CTA per SM (64 k / 32 bands: 32 CTAs
+    // at one thread per element)
+    int js = 1;
+    while (js < 8 && n * js < (size_t)GM_THREADS * SM) js *= 2;
+    if ((size_t)nvec * 16 + GM_THREADS * 16 > 48 * 1024) js = 1;
+    const int ec = GM_THREADS / js;
+    const int gb = (int)std::max<size_t>(1, std::min<size_t>((n + ec - 1) / ec, (size_t)4 * SM));
+    double* red = want ? ln.red : nullptr;
+    ln.nred = gb;
+    const size_t smem = (size_t)std::max(1, nvec) * 16 + (js > 1 ? GM_THREADS * 16 : 0);
+    unsigned char* u = ln.ub + (size_t)nvec * n * 16;
+    auto go = [&](auto kern, auto* e) {
+      typedef std::remove_pointer_t<decltype(e)> E;
+      kern<<<gb, GM_THREADS, smem, stream>>>(reinterpret_cast<const E*>(vb), nvec, cp, reinterpret_cast<const E*>(ln.coef),
+                                             js, y, n, rhs, red, ln.host, ln.ticket + depth, ln.pcdiv, pg,
+                                             reinterpret_cast<E*>(u), reinterpret_cast<E*>(ln.gs));
+    };
+    if (dfmt) {
+      if (pg)
+        go(k_gm_combine<true, true>, (float4*)nullptr);
+      else
+        go(k_gm_combine<true, false>, (float4*)nullptr);
+    } else {
+      if (pg)
+        go(k_gm_combine<false, true>, (double2*)nullptr);
+      else
+        go(k_gm_combine<false, false>, (double2*)nullptr);
+    }
+    return launched();
   };
   // x += sum gamma_j u_j, gamma = 0 (the pending solution formed)
   auto form_x = [&](Lane& ln, bool want) -> int {
-    int q = combine_into(ln, ln.ub, ln.gam, ln.xpend ? ln.P : 0, ln.x, want);
+    int q = combine_into(ln, ln.ub, ln.gam, ln.xpend ? ln.P : 0, ln.x, want, nullptr);
     std::fill(ln.gam.begin(), ln.gam.end(), cd(0.0, 0.0));
     ln.xpend = false;
     return q;
@@ -649,14 +809,14 @@ int gmres_solve_op(const GmresOp& op, const double* d_rhs_in, double kpref, cons
     if (dfmt)
       k_gm_resid<true><<<gb, GM_THREADS, 0, stream>>>(xp, t, rhs, n, ln.ener, res, ln.g,
                                                          want_gs ? reinterpret_cast<float4*>(ln.gs) : nullptr,
-                                                         ln.part);
+                                                         ln.red);
     else
       k_gm_resid<false><<<gb, GM_THREADS, 0, stream>>>(xp, t, rhs, n, ln.ener, res, ln.g,
                                                           want_gs ? reinterpret_cast<double2*>(ln.gs) : nullptr,
-                                                          ln.part);
+                                                          ln.red);
     int q = launched();
     if (q) return q;
-    return reduce_to(ln.part, gb, 3, ln.out);
+    return reduce_to(ln.red, gb, 3, ln.host);
   };
   auto set_prec = [&](Lane& ln) -> int {
     ln.prev_energy = ln.ener;
@@ -695,7 +855,7 @@ int gmres_solve_op(const GmresOp& op, const double* d_rhs_in, double kpref, cons
     int q = form_x(ln, true);
     if (q) return q;
     ln.ph = LP_CONV_RB;
-    return readback(ln, ln.out, 3);
+    return readback(ln);
   };
   // after an inner step's residual is known and the test did not pass
   auto inner_continue = [&](Lane& ln) -> int {
@@ -725,6 +885,7 @@ int gmres_solve_op(const GmresOp& op, const double* d_rhs_in, double kpref, cons
         case LP_BEGIN: {
           ln.ener = elist[ln.s] * EV2HA;
           ln.complete_iter = 0;
+          ln.gknown = false;
           ln.restarts = 0;
           ln.restarted = false;
           if (ln.P == 0 && (q = set_prec(ln))) return q;
@@ -763,7 +924,7 @@ int gmres_solve_op(const GmresOp& op, const double* d_rhs_in, double kpref, cons
             k_gm_recycle<false><<<grid, GM_THREADS, 0, stream>>>(
                 reinterpret_cast<const double2*>(ln.ub), reinterpret_cast<double2*>(ln.aub), ln.P, n, chunk, dw,
                 reinterpret_cast<const double2*>(ln.gs), ln.part);
-          if ((q = launched()) || (q = reduce_to(ln.part, (int)nch, 2 * ln.P, ln.out))) return q;
+          if ((q = launched()) || (q = reduce_to(ln.part, (int)nch, 2 * ln.P, ln.host + GM_HOST_G))) return q;
           // the same shift on the host matrices: C += dw (A + A^H) + dw^2 S, A += dw S
           for (int i = 0; i < ln.P; ++i)
             for (int j = 0; j < ln.P; ++j) {
@@ -773,7 +934,7 @@ int gmres_solve_op(const GmresOp& op, const double* d_rhs_in, double kpref, cons
           for (int i = 0; i < ln.P; ++i)
             for (int j = 0; j < ln.P; ++j) ln.A[(size_t)i * depth + j] += dw * ln.S[(size_t)i * depth + j];
           ln.ph = LP_REC_RB;
-          return readback(ln, ln.out, 2 * ln.P);
+          return readback(ln);
         }
         case LP_REC_RB: {
           // the recycled solve (the P updates of :667-677 in one projection)
@@ -781,16 +942,17 @@ int gmres_solve_op(const GmresOp& op, const double* d_rhs_in, double kpref, cons
             if (ln.chol.add_row(i, ln.C))
               return op.err(OCN_ERR_SOLVE, "GMRES Gram matrix not positive definite");
           ln.r.assign(ln.P, cd(0.0, 0.0));
-          for (int j = 0; j < ln.P; ++j) ln.r[j] = -cd(ln.host[2 * j], ln.host[2 * j + 1]);
+          for (int j = 0; j < ln.P; ++j) ln.r[j] = -cd(ln.host[GM_HOST_G + 2 * j], ln.host[GM_HOST_G + 2 * j + 1]);
           ln.chol.solve(ln.P, ln.r);
           for (int j = 0; j < ln.P; ++j) ln.gam[j] += ln.r[j];
           ln.xpend = true;
-          if ((q = combine_into(ln, ln.aub, ln.r, ln.P, ln.g, true))) return q;
+          if ((q = combine_into(ln, ln.aub, ln.r, ln.P, ln.g, true, nullptr))) return q;
           ln.ph = LP_REC_G_RB;
-          return readback(ln, ln.out, 1);
+          return readback(ln);
         }
         case LP_REC_G_RB:
           ln.gval = ln.host[0];
+          ln.gknown = true;
           if (ln.gval < p->convergence) {
             ln.after_recycle = true;
             return conv_test(ln);
@@ -856,25 +1018,36 @@ int gmres_solve_op(const GmresOp& op, const double* d_rhs_in, double kpref, cons
                                                                reinterpret_cast<double2*>(ln.aub + (size_t)m * eb));
           if ((q = launched())) return q;
           const int ng = m + 1;
-          const size_t nch =
-              std::max<size_t>(1, std::min<size_t>(nchunk_max, ((size_t)GM_CTAS_PER_SM * SM + ng - 1) / ng));
+          const size_t nch = std::max<size_t>(
+              1, std::min<size_t>({nchunk_max, (size_t)GM_GRAM_PER_SM * SM / ng, (n + gm_rows - 1) / gm_rows}));
           const size_t chunk = (n + nch - 1) / nch;
-          const dim3 grid((unsigned)nch, (unsigned)ng);
+          const dim3 grid((unsigned)nch, (unsigned)(ng + (ln.ahead ? 1 : 0)));
           if (dfmt)
             k_gm_gram<true><<<grid, GM_THREADS, 0, stream>>>(
+                ln.red, ln.nred, ln.host,
                 reinterpret_cast<const float4*>(ln.ub), reinterpret_cast<const float4*>(ln.aub), m, n, chunk,
-                reinterpret_cast<const float4*>(ln.gs), ln.part);
+                reinterpret_cast<const float4*>(ln.gs), ln.part, ln.host + GM_HOST_G, ln.ticket);
           else
             k_gm_gram<false><<<grid, GM_THREADS, 0, stream>>>(
+                ln.red, ln.nred, ln.host,
                 reinterpret_cast<const double2*>(ln.ub), reinterpret_cast<const double2*>(ln.aub), m, n, chunk,
-                reinterpret_cast<const double2*>(ln.gs), ln.part);
-          if ((q = launched()) || (q = reduce_to(ln.part, (int)nch, (m + 1) * GM_NQ, ln.out))) return q;
+                reinterpret_cast<const double2*>(ln.gs), ln.part, ln.host + GM_HOST_G, ln.ticket);
+          if ((q = launched())) return q;
           ln.ph = LP_ITER_RB;
-          return readback(ln, ln.out, (m + 1) * GM_NQ);
+          return readback(ln);
         }
         case LP_ITER_RB: {
+          if (ln.ahead) {  // the last step's residual, read back with this step's Gram row
+            ln.ahead = false;
+            ln.gval = ln.host[0];
+            if (ln.gval < p->convergence) {  // it had converged: this step is void
+              ln.it = ln.P;
+              --ln.complete_iter;
+              return conv_test(ln);
+            }
+          }
           const int m = ln.it - 1;
-          const double* h = ln.host;
+          const double* h = ln.host + GM_HOST_G;
           for (int j = 0; j <= m; ++j) {
             const double* v = h + (size_t)j * GM_NQ;
             const cd cjm(v[0], v[1]), ajm(v[2], v[3]), amj(v[4], v[5]), sjm(v[6], v[7]);
@@ -899,9 +1072,24 @@ int gmres_solve_op(const GmresOp& op, const double* d_rhs_in, double kpref, cons
             ln.ph = LP_RESTART_H;
             return request_H(ln, ln.x);
           }
-          if ((q = combine_into(ln, ln.aub, ln.r, m + 1, ln.g, true))) return q;
+          // |g + sum r_j au_j|^2 = |g|^2 - Re sum conj(r_j) b_j with C r = b.  Well above the
+          // threshold the next step starts at once and the measured |g|^2 comes back with
+          // its Gram row (one wait per step instead of two; every decision is taken on the
+          // measured value).
+          double est = ln.gknown ? ln.gval : 0.0;
+          for (int j = 0; j <= m; ++j)
+            est += (std::conj(ln.r[j]) * cd(h[(size_t)j * GM_NQ + 8], h[(size_t)j * GM_NQ + 9])).real();
+          if (ln.gknown && est > GM_AHEAD * p->convergence) {
+            if ((q = combine_into(ln, ln.aub, ln.r, m + 1, ln.g, true, hin + (size_t)nreq * 2 * n))) return q;
+            ln.it = ln.P + 1;
+            ++ln.complete_iter;
+            ln.ahead = true;
+            ln.ph = LP_ITER_H;
+            return request_H(ln, nullptr);
+          }
+          if ((q = combine_into(ln, ln.aub, ln.r, m + 1, ln.g, true, nullptr))) return q;
           ln.ph = LP_G_RB;
-          return readback(ln, ln.out, 1);
+          return readback(ln);
         }
         case LP_RESTART_H:
           if ((q = resid(ln, ln.hout, false, false))) return q;
@@ -909,9 +1097,10 @@ int gmres_solve_op(const GmresOp& op, const double* d_rhs_in, double kpref, cons
           ln.P = 0;
           ln.restarted = true;
           ln.ph = LP_G_RB;
-          return readback(ln, ln.out, 1);
+          return readback(ln);
         case LP_G_RB:
           ln.gval = ln.host[0];
+          ln.gknown = true;
           if (ln.gval < p->convergence) return conv_test(ln);
           if ((q = inner_continue(ln))) return q;
           continue;
