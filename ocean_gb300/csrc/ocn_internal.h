@@ -153,6 +153,8 @@ struct ocn_ctx {
   int conv_cap_ne = 0, conv_cap_iter = 0;
 
   // Haydock loop: persistent buffers and the captured 3-iteration CUDA graph
+  double *xb = nullptr, *xb_host = nullptr;  // buffers of the action on host vectors (grow only)
+  size_t xb_len = 0, xb_host_len = 0;
   double* hay_vec = nullptr;   // old | psi | h, each 2*npsi
   double* hay_coef = nullptr;  // real_a | imag_a | real_b, each hay_cap+1
   int hay_cap = 0;
@@ -410,6 +412,12 @@ int haydock_to_df(ocn_ctx* c, double* buf, int nv);
 int mixed_norm_prep(ocn_ctx* c, int nv, const double* psi, double* h, double* ra, double* ia, double* rb,
                     size_t cstride, const int* itp);
 int mixed_check(ocn_ctx* c);       // reads and clears the device timeout flag
+// The error word that tc_check tests (device memory), or NULL.
+const int* mixed_err_word(const ocn_ctx* c);
+const int* slice_err_word(const ocn_ctx* c);
+inline const int* tc_err_word(const ocn_ctx* c) {
+  return c->mixed ? mixed_err_word(c) : (slice_ready(c) || slice_mult_ready(c) ? slice_err_word(c) : nullptr);
+}
 inline int tc_check(ocn_ctx* c) { return c->mixed ? mixed_check(c) : (slice_ready(c) || slice_mult_ready(c) ? slice_check(c) : OCN_OK); }
 int mixed_set_starve(ocn_ctx* c, int on);  // test hook of ocn_test_starve_tc
 // multiplet on the tensor cores: operands from c->mult (after ocn_set_mult), and

@@ -1641,6 +1641,8 @@ int mixed_set_starve(ocn_ctx* c, int on) {
   return OCN_OK;
 }
 
+const int* mixed_err_word(const ocn_ctx* c) { return c->mixed->d_err; }
+
 int mixed_check(ocn_ctx* c) {
   MixedLR* m = c->mixed;
   if (!m) return OCN_OK;

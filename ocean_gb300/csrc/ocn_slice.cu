@@ -1088,6 +1088,8 @@ int slice_x_to_band(ocn_ctx* c, const double2* phi, int nv, int v0, bool integer
 }
 
 // Reads and clears the device timeout flag (as mixed_check).
+const int* slice_err_word(const ocn_ctx* c) { return c->slice->d_err; }
+
 int slice_check(ocn_ctx* c) {
   if (!c->slice) return OCN_OK;
   int err = 0;
