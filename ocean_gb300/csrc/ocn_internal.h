@@ -256,7 +256,7 @@ int upload_twiddles(ocn_ctx* c);
 // b1_ready: the digit operand of the one psi was built
 int lr_apply_fp64(ocn_ctx* c, const double* d_pr, const double* d_pi, size_t vstride, int nv, bool b1_ready = false);
 int mult_apply(ocn_ctx* c, const double* d_pr, const double* d_pi, double* acc);  // adds into acc
-int mult_hamp(ocn_ctx* c, const double2* amp, double2* hamp);  // one vector, [p][a]
+int mult_hamp(ocn_ctx* c, const double2* amp, double2* hamp, int nv);  // [v][p][a]
 // base: binary32 partials on the mixed path, FP64 otherwise
 void active_parts(const ocn_ctx* c, const int* hflag, const void** base, int* count);
 int phase_bloch(ocn_ctx* c, const double* d_ur, const double* d_ui, const double* d_cos,

@@ -747,18 +747,28 @@ __global__ void k_mult_amp_reduce(const double2* __restrict__ part, double2* __r
   amp[i] = s;
 }
 
+constexpr int HAMP_THREADS = 64;
+
 // hamp(p,a) = mul * ( -sum_nu' mpm(nu,nu',l) amp((nu',m,l),a)
 //                     + sum_jj MH_l(ii(nu,m,a), jj) pw_l(jj) )
-// (OCEAN_multiplet.f90:1819-1936).  One warp per (p, a).
-__global__ void k_mult_hamp(const double2* __restrict__ amp, double2* __restrict__ hamp,
+// (OCEAN_multiplet.f90:1819-1936).  One warp per (p, a) and vector (blockIdx.y).  The
+// FP64 pipe bounds it (an instruction of a warp takes 16 cycles of an SM): four FMAs per
+// element of MH, one exchange tree for both sums, and neighbouring warps take rows that
+// lie gridDim.x apart, because a row of the largest l is 2l+1 times as long as one of
+// l = 0.  Eight elements are loaded ahead of their products.  128 projectors, 12 channels
+// (12 MB of MH): 24 us as a warp per row in order with six FP64 instructions per element,
+// 14 us so.
+__global__ void __launch_bounds__(HAMP_THREADS) k_mult_hamp(const double2* __restrict__ amp, double2* __restrict__ hamp,
                             const int* __restrict__ pl, const int* __restrict__ pm,
                             const int* __restrict__ pnu, const int* __restrict__ pfirst,
                             const double* __restrict__ mpm, const double2* __restrict__ mh,
                             const long long* __restrict__ jbeg, const int* __restrict__ nprojv,
                             int np, int na, int lmin, int npmax, double mul) {
-  const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int gw = blockIdx.x + (threadIdx.x >> 5) * gridDim.x;
   const int lane = threadIdx.x & 31;
   if (gw >= np * na) return;
+  amp += (size_t)blockIdx.y * np * na;
+  hamp += (size_t)blockIdx.y * np * na;
   const int p = gw / na, a = gw % na;
   const int l = pl[p], m = pm[p], nu = pnu[p];
   const int li = l - lmin;
@@ -770,28 +780,38 @@ __global__ void k_mult_hamp(const double2* __restrict__ amp, double2* __restrict
     const double mm = mpm[(size_t)nu + (size_t)npmax * ((size_t)nup + (size_t)npmax * li)];
     const int q = first + (m + l) * npl + nup;
     const double2 v = amp[(size_t)q * na + a];
-    s.x -= mm * v.x;
-    s.y -= mm * v.y;
+    s.x = __fma_rn(-mm, v.x, s.x);
+    s.y = __fma_rn(-mm, v.y, s.y);
   }
   // exchange term: pw_l(jj), jj = nu' + (m'+l) npl + a' (2l+1) npl
-  const int mham = na * (2 * l + 1) * npl;
-  const int ii = nu + (m + l) * npl + a * (2 * l + 1) * npl;
+  const int ml = (2 * l + 1) * npl, mham = na * ml;
+  const int ii = nu + (m + l) * npl + a * ml;
   const double2* row = mh + jbeg[li] + (size_t)ii * mham;
-  for (int jj = lane; jj < mham; jj += 32) {
-    const int nup = jj % npl;
-    const int mp = (jj / npl) % (2 * l + 1);
-    const int ap = jj / (npl * (2 * l + 1));
-    const int q = first + mp * npl + nup;
-    const double2 v = amp[(size_t)q * na + ap];
-    const double2 h = row[jj];
-    s.x += h.x * v.x - h.y * v.y;
-    s.y += h.x * v.y + h.y * v.x;
+  for (int j0 = lane; j0 < mham; j0 += 8 * 32) {
+    double2 h[8], v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int jj = j0 + 32 * u;
+      if (jj >= mham) continue;
+      const int ap = jj / ml, q = first + jj - ap * ml;
+      h[u] = row[jj];
+      v[u] = amp[(size_t)q * na + ap];
+    }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      if (j0 + 32 * u >= mham) continue;
+      s.x = __fma_rn(h[u].x, v[u].x, s.x);
+      s.y = __fma_rn(h[u].x, v[u].y, s.y);
+      s.x = __fma_rn(-h[u].y, v[u].y, s.x);
+      s.y = __fma_rn(h[u].y, v[u].x, s.y);
+    }
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    s.x += __shfl_down_sync(0xffffffffu, s.x, o);
-    s.y += __shfl_down_sync(0xffffffffu, s.y, o);
-  }
-  if (lane == 0) hamp[(size_t)p * na + a] = make_double2(s.x * mul, s.y * mul);
+  // lanes 0-15 go on with the real sum, 16-31 with the imaginary one
+  const bool up = lane >= 16;
+  double t = up ? s.y : s.x;
+  t += __shfl_xor_sync(0xffffffffu, up ? s.x : s.y, 16);
+  for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if ((lane & 15) == 0) reinterpret_cast<double*>(hamp + (size_t)p * na + a)[up ? 1 : 0] = t * mul;
 }
 
 // acc(e,a) += sum_p conj(mpc_s(p)(e)) hamp(p,a)   (OCEAN_multiplet.f90:1943-1998)
@@ -1118,14 +1138,13 @@ int lr_wgrad_fp64(ocn_ctx* c, const double* x, const double* y, double2* phi, do
   return OCN_OK;
 }
 
-// hamp = mul (-mpm amp + MH amp) of one vector (k_mult_hamp), amp/hamp [p][a]
-int mult_hamp(ocn_ctx* c, const double2* amp, double2* hamp) {
+// hamp = mul (-mpm amp + MH amp) of nv vectors (k_mult_hamp), amp/hamp [v][p][a]
+int mult_hamp(ocn_ctx* c, const double2* amp, double2* hamp, int nv) {
   MultDev& m = c->mult;
   const double mul = c->sys.interaction_scale / ((double)c->nk * c->sys.celvol);
   const int npa = m.np * c->na;
-  const int threads = 256;
-  const int blocks = (npa * 32 + threads - 1) / threads;
-  k_mult_hamp<<<blocks, threads, 0, c->stream>>>(amp, hamp, m.p_l, m.p_m, m.p_nu, m.d_pfirst, m.mpm, m.mh,
+  const int blocks = (npa * 32 + HAMP_THREADS - 1) / HAMP_THREADS;
+  k_mult_hamp<<<dim3(blocks, nv), HAMP_THREADS, 0, c->stream>>>(amp, hamp, m.p_l, m.p_m, m.p_nu, m.d_pfirst, m.mpm, m.mh,
                                                 m.d_jbeg, m.d_nproj, m.np, c->na, m.lmin, m.npmax, mul);
   ++c->launches;
   OCN_CUDA(c, cudaGetLastError());
@@ -1160,17 +1179,8 @@ int mult_apply(ocn_ctx* c, const double* d_pr, const double* d_pi, double* acc) 
   k_mult_amp_reduce<<<(npa + 127) / 128, 128, 0, c->stream>>>(m.amp_part, m.amp, nchunk, npa);
   ++c->launches;
   OCN_CUDA(c, cudaGetLastError());
-  {
-    const double mul = c->sys.interaction_scale / ((double)c->nk * c->sys.celvol);
-    const int warps = npa;
-    const int threads = 256;
-    const int blocks = (warps * 32 + threads - 1) / threads;
-    k_mult_hamp<<<blocks, threads, 0, c->stream>>>(m.amp, m.hamp, m.p_l, m.p_m, m.p_nu, m.d_pfirst,
-                                                  m.mpm, m.mh, m.d_jbeg, m.d_nproj, m.np, c->na,
-                                                  m.lmin, m.npmax, mul);
-    ++c->launches;
-    OCN_CUDA(c, cudaGetLastError());
-  }
+  int rc;
+  if ((rc = mult_hamp(c, m.amp, m.hamp, 1))) return rc;
   {
     const size_t sm = sizeof(double2) * (size_t)npa;
     const int block = 64;

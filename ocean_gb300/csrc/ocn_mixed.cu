@@ -1573,8 +1573,7 @@ int mult_apply_mixed(ocn_ctx* c, const double* d_pr, const double* d_pi, size_t 
                                                                                  np, na, nv);
   ++c->launches;
   OCN_CUDA(c, cudaGetLastError());
-  for (int v = 0; v < nv; ++v)
-    if ((rc = mult_hamp(c, m->amp + (size_t)v * np * na, m->hamp + (size_t)v * np * na))) return rc;
+  if ((rc = mult_hamp(c, m->amp, m->hamp, nv))) return rc;
   k_prep_b3<<<(nv * np * na + 127) / 128, 128, 0, c->stream>>>(m->hamp, m->b3, np, na, nv, m->p3);
   ++c->launches;
   for (int s = 0; s < ns; ++s) {

@@ -1031,7 +1031,7 @@ int slice_mult_apply(ocn_ctx* c, int v) {
   k_slice_amp_reduce<<<(n + 31) / 32, 512, 0, c->stream>>>(s->amp_part, m.amp, c->nk, n);
   ++c->launches;
   OCN_CUDA(c, cudaGetLastError());
-  if ((rc = mult_hamp(c, m.amp, m.hamp))) return rc;
+  if ((rc = mult_hamp(c, m.amp, m.hamp, 1))) return rc;
   k_slice_col_max<<<1, 512, 0, c->stream>>>(m.hamp, m.np, c->na, s->mxm);
   const int items = s->gm2.p.Ge * c->na * 4;
   k_slice_prep_b2<false><<<dim3((items + 255) / 256, 1), 256, 0, c->stream>>>(m.hamp, nullptr, m.np, c->na, s->gm2.p.Ge,
