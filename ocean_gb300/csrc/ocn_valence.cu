@@ -70,7 +70,7 @@ struct ocn_val_ctx {
   double2* d_val = nullptr;   // [k][v][x]
   float2* d_con32 = nullptr;  // FP32 copies (mixed precision)
   float2* d_val32 = nullptr;
-  void* d_valT = nullptr;     // [y][v][k], double2 or float2
+  void* d_valT = nullptr;     // [y][v][k], double2 or float2 (cubic kernel in FP32: val_line_at)
   void* d_lad = nullptr;      // [y][x][k], double or float
   bool fx = false;            // FP64 direct term in fixed point: d_valT holds split halves, d_lad integers
   int* d_eV = nullptr;        // fx: exponents of val per (spin, y) and of the ladder per (y, x)
@@ -401,15 +401,23 @@ __global__ void __launch_bounds__(VAL_THREADS)
   }
 }
 
-// N consecutive complex values; FP32 lines of even length (16-byte aligned:
-// every caller's offset is a multiple of N complex values) as 16-byte loads.
+// val of one (y, v) for the cubic kernel in FP32: the lines along k3 side by side, in
+// units of two k3 values (one for odd N), so that lanes on neighbouring lines load
+// neighbouring 16-byte words.  With a line's values together a warp's load met 16 cache
+// lines, and the val loads were half of the kernel's L1 cycles (8^3 k / 10^3 x / 4 bands:
+// an H psi 3.86 ms, now 3.15 ms).  Offset of value j of line ln within the N^3 values:
+template <int N>
+__host__ __device__ constexpr int val_line_at(int ln, int j) {
+  return N % 2 == 0 ? (j >> 1) * (2 * N * N) + 2 * ln + (j & 1) : j * (N * N) + ln;
+}
+
+// Line ln of one (y, v): FP64 lines are N consecutive values.
 template <typename CT, int N>
-__device__ __forceinline__ void load_line(const CT* __restrict__ p, CT (&v)[N]) {
+__device__ __forceinline__ void load_line(const CT* __restrict__ p, int ln, CT (&v)[N]) {
   if constexpr (sizeof(CT) == 8 && N % 2 == 0) {
-    const float4* q = reinterpret_cast<const float4*>(p);
 #pragma unroll
     for (int i = 0; i < N / 2; ++i) {
-      const float4 t = __ldg(q + i);
+      const float4 t = __ldg(reinterpret_cast<const float4*>(p + val_line_at<N>(ln, 2 * i)));
       v[2 * i].x = t.x;
       v[2 * i].y = t.y;
       v[2 * i + 1].x = t.z;
@@ -417,7 +425,7 @@ __device__ __forceinline__ void load_line(const CT* __restrict__ p, CT (&v)[N]) 
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < N; ++j) v[j] = p[j];
+    for (int j = 0; j < N; ++j) v[j] = p[sizeof(CT) == 8 ? val_line_at<N>(ln, j) : ln * N + j];
   }
 }
 
@@ -437,10 +445,13 @@ __global__ void __launch_bounds__(VAL_THREADS, (sizeof(R) == 4 && X == 1) ? 4 : 
   typedef typename C2<R>::T CT;
   constexpr int NK = N * N * N, NL = N * N, P3 = N + 1;
   constexpr int SLAB = ocn::cube_slab<CT>(N);
-  // FP32: the last backward transform is redone by each of the nv threads of a
-  // line in the B sum (saves a shared-memory pass); FP64 is FP64-pipe bound,
-  // so there it stays one shared pass (85 ms against 104 ms per H psi)
-  constexpr bool FUSE_K3 = sizeof(R) == 4;
+  // FP32, N = 8: the last backward transform is redone by each of the nv threads of a
+  // line in the B sum (saves a shared-memory pass).  Smaller N leave threads of the B sum
+  // idle and redo it in the others, FP64 is FP64-pipe bound: there it stays one shared
+  // pass (us per H psi, redone / pass, 8^3 x, 4 bands: N = 8 984 / 997, 6 862 / 729,
+  // 5 575 / 534, 3 232 / 217; FP64 N = 8 104 / 85 ms at 10^3 x)
+  constexpr bool FUSE_K3 = sizeof(R) == 4 && N == 8;
+  constexpr bool LINES = sizeof(R) == 4;  // val in the order of val_line_at
   extern __shared__ __align__(16) unsigned char vsm[];
   CT* tw = reinterpret_cast<CT*>(vsm);
   CT* As = tw + 3 * OCN_MAX_KDIM;        // [xi][(v N + k3) NL + line]
@@ -476,7 +487,7 @@ __global__ void __launch_bounds__(VAL_THREADS, (sizeof(R) == 4 && X == 1) ? 4 : 
     // T(x, y, k) for a k3 line, then the forward transform along k3
     for (int li = threadIdx.x; li < ny * NL; li += blockDim.x) {
       const int yl = li / NL, ln = li % NL;
-      const CT* vt = valT + (size_t)(y0 + yl) * nv * NK + ln * N;
+      const CT* vt = valT + (size_t)(y0 + yl) * nv * NK;
       CT v[X][N];
 #pragma unroll
       for (int xi = 0; xi < X; ++xi)
@@ -487,7 +498,7 @@ __global__ void __launch_bounds__(VAL_THREADS, (sizeof(R) == 4 && X == 1) ? 4 : 
         }
       for (int vv = 0; vv < nv; ++vv) {
         CT bl[N];
-        load_line<CT, N>(vt + (size_t)vv * NK, bl);
+        load_line<CT, N>(vt + (size_t)vv * NK, ln, bl);
 #pragma unroll
         for (int xi = 0; xi < X; ++xi) {
           const CT* as = As + xi * nv * NK + ln;
@@ -544,10 +555,10 @@ __global__ void __launch_bounds__(VAL_THREADS, (sizeof(R) == 4 && X == 1) ? 4 : 
     for (int q = 0; q < MAXC; ++q) {
       const int cb = threadIdx.x + q * VAL_THREADS;
       if (cb < ncomb) {
-        const int ln = cb / nv, vv = cb % nv;
+        const int ln = LINES ? cb % NL : cb / nv, vv = LINES ? cb / NL : cb % nv;
         for (int yl = 0; yl < ny; ++yl) {
           CT bl[N];
-          load_line<CT, N>(valT + ((size_t)(y0 + yl) * nv + vv) * NK + ln * N, bl);
+          load_line<CT, N>(valT + ((size_t)(y0 + yl) * nv + vv) * NK, ln, bl);
 #pragma unroll
           for (int xi = 0; xi < X; ++xi) {
             const CT* p = T + (yl * X + xi) * SLAB + ln * P3;
@@ -571,7 +582,7 @@ __global__ void __launch_bounds__(VAL_THREADS, (sizeof(R) == 4 && X == 1) ? 4 : 
   for (int q = 0; q < MAXC; ++q) {
     const int cb = threadIdx.x + q * VAL_THREADS;
     if (cb < ncomb) {
-      const int ln = cb / nv, vv = cb % nv;
+      const int ln = LINES ? cb % NL : cb / nv, vv = LINES ? cb / NL : cb % nv;
 #pragma unroll
       for (int xi = 0; xi < X; ++xi) {
         if (x0 + xi >= nx) continue;
@@ -684,13 +695,18 @@ __global__ void kv_interleave(const double* __restrict__ re, const double* __res
     out[i] = make_double2(re[i], im[i]);
 }
 
+// N > 0: the lines along k3 in the order of val_line_at<N>.
 template <typename R>
-__global__ void kv_transpose_val(const double2* __restrict__ val, int nv, int nk, int nx,
+__global__ void kv_transpose_val(const double2* __restrict__ val, int nv, int nk, int nx, int N,
                                  typename C2<R>::T* __restrict__ valT) {
   const size_t n = (size_t)nx * nv * nk;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const int k = (int)(i % nk);
+    int k = (int)(i % nk);
     const size_t r = i / nk;
+    if (N > 0) {
+      const int u = N % 2 == 0 ? 2 : 1, unit = k / u, ln = unit % (N * N);
+      k = ln * N + unit / (N * N) * u + k % u;
+    }
     const int v = (int)(r % nv);
     const int y = (int)(r / nv);
     const double2 t = val[((size_t)k * nv + v) * nx + y];
@@ -1298,6 +1314,7 @@ static int set_states_impl(ocn_val_ctx* c, const double* conr, const double* con
   if (c->mixed) {
     for (int sp = 0; sp < c->nspn; ++sp)
       kv_transpose_val<float><<<g, 256, 0, c->stream>>>(c->d_val + sp * nval1, c->nv, c->nk, c->nx,
+                                                        use_cube_kernel(c) ? c->dims.kmesh[0] : 0,
                                                         static_cast<float2*>(c->d_valT) + sp * nval1);
     kv_to_float<<<g, 256, 0, c->stream>>>(reinterpret_cast<const double*>(c->d_con), 2 * ncon,
                                           reinterpret_cast<float*>(c->d_con32));
@@ -1310,7 +1327,7 @@ static int set_states_impl(ocn_val_ctx* c, const double* conr, const double* con
                          c->d_eV + (size_t)sp * c->nx, c->stream);
   else
     for (int sp = 0; sp < c->nspn; ++sp)
-      kv_transpose_val<double><<<g, 256, 0, c->stream>>>(c->d_val + sp * nval1, c->nv, c->nk, c->nx,
+      kv_transpose_val<double><<<g, 256, 0, c->stream>>>(c->d_val + sp * nval1, c->nv, c->nk, c->nx, 0,
                                                          static_cast<double2*>(c->d_valT) + sp * nval1);
   {
     cudaError_t e = cudaGetLastError();
