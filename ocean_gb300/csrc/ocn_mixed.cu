@@ -919,7 +919,8 @@ __device__ __forceinline__ void store_b2_rows(const Get& get, float norm, __nv_b
   }
 }
 
-// FP32 k-mesh transform of one x-point per CTA (ocn_kmesh_dft.cuh), B2 rows out: generic meshes
+// FP32 k-mesh transform of one x-point per CTA (ocn_kmesh_dft.cuh), B2 rows out: meshes
+// with an axis beyond 8
 __global__ void k_fft_b2(const float2* __restrict__ phi, const float* __restrict__ W, int nx,
                          const KmeshGeom<float> g, const float2* __restrict__ twg, __nv_bfloat16* __restrict__ b2,
                          int na, int ncol, int k2ext) {
@@ -1093,6 +1094,177 @@ __global__ void k_fft_b2_cube_group(const FftGroupArgs* __restrict__ tab, int n)
                            a.k2ext);
 }
 typedef void (*CubeFnB2Group)(const FftGroupArgs*, int);
+
+// The same transform on a mesh without symmetry, axes of 1 to 8 points, in six phases over
+// shared memory: backward along k1 (from phi), k2, k3 (times W), forward along k1, k2, k3
+// (B2 columns out, as phase E of the cubic transform).  Every line is the direct sum of
+// dft_pass_fixed in the same order of passes, so the results are those of k_fft_b2, which
+// took a pass each for the load, W and the output and split every value twice: 120 k x
+// 720 x x 12 transforms, 44 us against 26 us.
+struct MeshGeom {
+  int n1, n2, n3, nk, P3, slab;
+};
+inline MeshGeom mesh_geom(const int n[3]) {
+  MeshGeom g{n[0], n[1], n[2], n[0] * n[1] * n[2], n[2] | 1, 0};
+  g.slab = (g.n1 * g.n2 * g.P3 + 15) / 16 * 16 + 4;
+  return g;
+}
+inline size_t mesh_smem(const MeshGeom& g, int nt) {
+  return sizeof(float2) * (3 * OCN_MAX_KDIM + (size_t)nt * g.slab);
+}
+inline bool mesh_supported(const int n[3], int nt) {
+  return n[0] <= 8 && n[1] <= 8 && n[2] <= 8 && nt % 4 == 0 && mesh_smem(mesh_geom(n), nt) <= 227u * 1024u;
+}
+
+template <int N>
+__device__ __forceinline__ void line_direct(float2 (&v)[N], const float2* __restrict__ tw, float sgn) {
+  if constexpr (N > 1) {
+    float2 w[N], out[N];
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+      w[t] = tw[t];
+      w[t].y *= sgn;
+    }
+#pragma unroll
+    for (int m = 0; m < N; ++m) {
+      float sr = v[0].x, si = v[0].y;
+#pragma unroll
+      for (int j = 1; j < N; ++j) {
+        const float2 ww = w[(j * m) % N];
+        sr += v[j].x * ww.x - v[j].y * ww.y;
+        si += v[j].x * ww.y + v[j].y * ww.x;
+      }
+      out[m].x = sr;
+      out[m].y = si;
+    }
+#pragma unroll
+    for (int m = 0; m < N; ++m) v[m] = out[m];
+  }
+}
+
+// In place along an axis: lines (o1, o2) of every transform, element i1 s1 + i2 s2 + j st;
+// ws (k-order, W of the x-point) multiplies the result when given (lines along k3 only).
+template <int N>
+__device__ __forceinline__ void mesh_pass(float2* buf, int nt, int slab, int o1, int o2, int s1, int s2, int st,
+                                          const float2* __restrict__ tw, float sgn, const float* __restrict__ ws) {
+  const int lines = o1 * o2;
+  for (int l = threadIdx.x; l < nt * lines; l += blockDim.x) {
+    const int t = l / lines, r = l - t * lines;
+    const int i1 = r / o2, i2 = r - i1 * o2;
+    float2* p = buf + t * slab + i1 * s1 + i2 * s2;
+    float2 v[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) v[j] = p[j * st];
+    line_direct<N>(v, tw, sgn);
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      if (ws) {
+        const float wv = ws[r * N + j];
+        v[j].x *= wv;
+        v[j].y *= wv;
+      }
+      p[j * st] = v[j];
+    }
+  }
+}
+template <int N>
+__device__ __forceinline__ void mesh_load(const float2* __restrict__ phi, int nx, int x, const MeshGeom& g, int nt,
+                                          float2* buf, const float2* __restrict__ tw) {
+  const int n23 = g.n2 * g.n3, tasks = n23 * nt;
+  for (int task = threadIdx.x; task < tasks; task += blockDim.x) {
+    const int r = task / nt, t = task - r * nt;
+    float2 v[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) v[j] = phi[((size_t)(j * n23 + r) * nx + x) * nt + t];
+    line_direct<N>(v, tw, 1.0f);
+    const int i2 = r / g.n3;
+    float2* dst = buf + t * g.slab + i2 * g.P3 + (r - i2 * g.n3);
+#pragma unroll
+    for (int j = 0; j < N; ++j) dst[j * g.n2 * g.P3] = v[j];
+  }
+}
+template <int N>
+__device__ __forceinline__ void mesh_out(const float2* buf, const MeshGeom& g, int nt, const float2* __restrict__ tw,
+                                         __nv_bfloat16* __restrict__ b2, int x, int na, int ncol, int k2ext) {
+  const float norm = 1.0f / (float)g.nk;
+  const int row_x = ((x >> 6) << 7) + (x & 63);
+  const int lane = threadIdx.x & 31, q = lane & 3, s = q >> 1, part = q & 1;
+  const uint32_t sel0 = part ? 0x3276u : 0x5410u, sel1 = part ? 0x1054u : 0x7632u, flip = part ? 0x80008000u : 0u;
+  const int tasks = g.n1 * g.n2 * nt;
+  for (int base = 0; base < tasks; base += blockDim.x) {
+    const int task = base + threadIdx.x;
+    const bool on = task < tasks;
+    const int r = on ? task / nt : 0, t = on ? task - r * nt : 0;
+    float2 v[N];
+    const float2* src = buf + t * g.slab + r * g.P3;
+#pragma unroll
+    for (int j = 0; j < N; ++j) v[j] = src[j];
+    line_direct<N>(v, tw, -1.0f);
+    const int tg = t & ~3, vv = tg / na, a0 = tg - vv * na;
+    __nv_bfloat16* col = b2 + ((size_t)r * N * k2ext + row_x) * ncol + (size_t)vv * 4 * na + s * 2 * na + part * na + a0;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      uint32_t hw, lw;
+      split_bf16x2(v[j].x * norm, v[j].y * norm, hw, lw);
+      const uint32_t keep = s ? lw : hw;
+      const uint32_t recv = __shfl_xor_sync(0xffffffffu, s ? hw : lw, 2);
+      const uint32_t nk = __shfl_xor_sync(0xffffffffu, keep, 1);
+      const uint32_t nr = __shfl_xor_sync(0xffffffffu, recv, 1);
+      const uint32_t x0 = s ? recv : keep, x1 = s ? nr : nk, y0 = s ? keep : recv, y1 = s ? nk : nr;
+      if (!on) continue;
+      __nv_bfloat16* o = col + (size_t)j * k2ext * ncol;
+      *reinterpret_cast<uint2*>(o) = make_uint2(__byte_perm(x0, x1, sel0), __byte_perm(y0, y1, sel0));
+      *reinterpret_cast<uint2*>(o + (size_t)64 * ncol) =
+          make_uint2(__byte_perm(x0, x1, sel1) ^ flip, __byte_perm(y0, y1, sel1) ^ flip);
+    }
+  }
+}
+
+#define OCN_MESH_LEN(n, CALL)        \
+  switch (n) {                       \
+    case 1: CALL(1); break;          \
+    case 2: CALL(2); break;          \
+    case 3: CALL(3); break;          \
+    case 4: CALL(4); break;          \
+    case 5: CALL(5); break;          \
+    case 6: CALL(6); break;          \
+    case 7: CALL(7); break;          \
+    default: CALL(8); break;         \
+  }
+
+__global__ void __launch_bounds__(256, 3)
+    k_fft_b2_mesh(const float2* __restrict__ phi, const float* __restrict__ W, int nx, int nt, const MeshGeom g,
+                  const float2* __restrict__ twg, __nv_bfloat16* __restrict__ b2, int na, int ncol, int k2ext) {
+  extern __shared__ float2 fsm[];
+  float2 *tw1 = fsm, *tw3 = fsm + 2 * OCN_MAX_KDIM, *buf = fsm + 3 * OCN_MAX_KDIM;
+  const int x = blockIdx.x, n23 = g.n2 * g.P3;
+  for (int i = threadIdx.x; i < 3 * OCN_MAX_KDIM; i += blockDim.x) fsm[i] = twg[i];
+  __syncthreads();
+#define OCN_LOAD(N) mesh_load<N>(phi, nx, x, g, nt, buf, tw1)
+  OCN_MESH_LEN(g.n1, OCN_LOAD)
+  __syncthreads();
+#pragma unroll 1
+  for (int dir = 0; dir < 2; ++dir) {  // (backward k2, k3 times W), then (forward k1, k2)
+    const float sgn = dir ? -1.0f : 1.0f;
+#pragma unroll 1
+    for (int i = 0; i < 2; ++i) {
+      const int ax = dir ? i : i + 1;
+      const int n = ax == 0 ? g.n1 : (ax == 1 ? g.n2 : g.n3);
+      const int o1 = ax == 0 ? g.n2 : g.n1, o2 = ax == 2 ? g.n2 : g.n3;
+      const int s1 = ax == 0 ? g.P3 : n23, s2 = ax == 2 ? g.P3 : 1, st = ax == 0 ? n23 : (ax == 1 ? g.P3 : 1);
+      const float* ws = ax == 2 ? W + (size_t)x * g.nk : nullptr;
+      const float2* tw = fsm + ax * OCN_MAX_KDIM;
+#define OCN_PASS(N) mesh_pass<N>(buf, nt, g.slab, o1, o2, s1, s2, st, tw, sgn, ws)
+      OCN_MESH_LEN(n, OCN_PASS)
+      __syncthreads();
+    }
+  }
+#define OCN_OUT(N) mesh_out<N>(buf, g, nt, tw3, b2, x, na, ncol, k2ext)
+  OCN_MESH_LEN(g.n3, OCN_OUT)
+#undef OCN_LOAD
+#undef OCN_PASS
+#undef OCN_OUT
+}
 
 __global__ void k_w_to_f32(const double* __restrict__ W, float* __restrict__ Wf, size_t n) {
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
@@ -1315,6 +1487,7 @@ int mixed_init(ocn_ctx* c) {
   if ((rc = mixed_configure(c, cfg))) return rc;
   if (int rc_ = allow_max_smem(c, k_lr_tc)) return rc_;
   if (int rc_ = allow_max_smem(c, k_fft_b2)) return rc_;
+  if (int rc_ = allow_max_smem(c, k_fft_b2_mesh)) return rc_;
   if (cube) {
     // the three instantiations a call can select (nt = 4, 12, other)
     for (int nt : {4, 12, 1}) {
@@ -1713,6 +1886,10 @@ int lr_apply_mixed(ocn_ctx* c, const double* d_pr, const double* d_pi, size_t vs
       const int th = m->cfg[5] ? m->cfg[5] : 128;
       f<<<dim3(nx, ntot / tc), th, fft_b2_smem(c->dims.kmesh[0], tc), c->stream>>>(
           m->phi, m->Wf, nx, tc, ntot, m->twf, m->b2, na, m->ncol, m->p2);
+    } else if (mesh_supported(c->dims.kmesh, na * nv)) {
+      const MeshGeom g = mesh_geom(c->dims.kmesh);
+      k_fft_b2_mesh<<<nx, 256, mesh_smem(g, na * nv), c->stream>>>(m->phi, m->Wf, nx, na * nv, g, m->twf, m->b2, na,
+                                                                   m->ncol, m->p2);
     } else {
       const KmeshGeom<float> g = kmesh_geom<float>(c->dims.kmesh, na * nv);
       k_fft_b2<<<nx, 256, kmesh_smem(g), c->stream>>>(m->phi, m->Wf, nx, g, m->twf, m->b2, na, m->ncol, m->p2);
