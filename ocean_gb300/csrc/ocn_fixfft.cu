@@ -25,9 +25,9 @@
 // and the exponent maxima per (k, t) that scale the next operand collected on the way
 // out: rounding to binary64 and back took an eighth of the instructions.
 //
-// Measured: 319 -> 70 us (8^3, 6912 transforms), 766 -> 59 us (6^3, 12000), 375 ->
-// 62 us (7x6x5, 3960).  Bound by integer issue (about 3400 instructions per thread,
-// ALU pipe 56 %), not by the 114 MB it moves.
+// Measured: 319 -> 60 us (8^3, 6912 transforms), 766 -> 53 us (6^3, 12000), 375 ->
+// 32 us (7x6x5, 3960 of the 11880 of three vectors).  Bound by integer issue (about 3000
+// instructions per thread), not by the 114 MB it moves.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -63,9 +63,8 @@ namespace {
 typedef std::complex<double> cd;
 constexpr double EV2HA = 0.036749322175666;
 constexpr int GM_THREADS = 256;
-constexpr int GM_CTAS_PER_SM = 4;  // target CTAs per SM of the recycle pass
-constexpr int GM_GRAM_PER_SM = 3;  // CTAs per SM of the Gram pass (its launch bound): one wave,
-                                   // 8^3 k / 40 bands, mixed: a sweep of 4 energies 66 -> 60 ms
+constexpr int GM_CTAS_PER_SM = 4;  // target CTAs per SM of the Gram (double-float) and recycle passes
+constexpr int GM_GRAM_PER_SM = 3;  // FP64 Gram pass: CTAs per SM by its launch bound, one wave
 constexpr int GM_NQ = 10;          // real sums per basis vector in the Gram pass
 
 // double-float helpers: ocn_df.cuh
@@ -766,10 +765,12 @@ int gmres_solve_op(const GmresOp& op, const double* d_rhs_in, double kpref, cons
       for (int j = 0; j < nvec; ++j) ln.hcoef[j] = pack_coef(dfmt, cf[j]);
       GM_CUDA(cudaMemcpyAsync(ln.coef, ln.hcoef, nvec * sizeof(Coef16), cudaMemcpyHostToDevice, stream));
     }
-    // thread groups per element until the chip has a CTA per SM (64 k / 32 bands: 32 CTAs
-    // at one thread per element)
+    // FP64: thread groups per element until the chip has a CTA per SM (64 k / 32 bands: 32
+    // CTAs at one thread per element).  The double-float basis keeps one order of summation
+    // here and in the Gram pass whatever the tiling: the mixed action rounds its input to
+    // two bf16, so another last bit of g comes back as 1e-6 of the spectrum.
     int js = 1;
-    while (js < 8 && n * js < (size_t)GM_THREADS * SM) js *= 2;
+    while (!dfmt && js < 8 && n * js < (size_t)GM_THREADS * SM) js *= 2;
     if ((size_t)nvec * 16 + GM_THREADS * 16 > 48 * 1024) js = 1;
     const int ec = GM_THREADS / js;
     const int gb = (int)std::max<size_t>(1, std::min<size_t>((n + ec - 1) / ec, (size_t)4 * SM));
@@ -1019,7 +1020,8 @@ int gmres_solve_op(const GmresOp& op, const double* d_rhs_in, double kpref, cons
           if ((q = launched())) return q;
           const int ng = m + 1;
           const size_t nch = std::max<size_t>(
-              1, std::min<size_t>({nchunk_max, (size_t)GM_GRAM_PER_SM * SM / ng, (n + gm_rows - 1) / gm_rows}));
+              1, dfmt ? std::min<size_t>(nchunk_max, ((size_t)GM_CTAS_PER_SM * SM + ng - 1) / ng)
+                      : std::min<size_t>({nchunk_max, (size_t)GM_GRAM_PER_SM * SM / ng, (n + gm_rows - 1) / gm_rows}));
           const size_t chunk = (n + nch - 1) / nch;
           const dim3 grid((unsigned)nch, (unsigned)(ng + (ln.ahead ? 1 : 0)));
           if (dfmt)

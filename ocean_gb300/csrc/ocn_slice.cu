@@ -39,8 +39,8 @@
 //
 // Measured, 8^3 k / 100 bands / 12^3 x, 1s: band -> x 4.3 ms on the FP64 pipe ->
 // 0.331 ms (2.2 GB, 6.7 TB/s), x -> band 5.9 ms -> 0.355 ms (6.2 TB/s): bound by
-// the read of A.  2p, 6^3 k / 64 bands / 10^3 x (12 columns): 0.084 and 0.119 ms
-// (4.0 and 2.6 TB/s): there the 144-column MMAs (72 cycles) and the epilogue's
+// the read of A.  2p, 6^3 k / 64 bands / 10^3 x (12 columns): 0.084 and 0.108 ms
+// (4.0 and 2.9 TB/s): there the 144-column MMAs (72 cycles) and the epilogue's
 // 288 integer columns per row weigh as much as the 0.3 GB read.
 #include <cuda_runtime.h>
 
@@ -971,8 +971,8 @@ int slice_set_bloch(ocn_ctx* c) {
 // back-projection the x -> band one with an operand shared by every k.  Grows the
 // partial sums by the back-projection's slices.  Without the memory the context
 // keeps the FP64-pipe multiplet kernels.  2p, 6^3 k / 64 bands / 128 projectors: the
-// whole term 1200 us on the FP64 pipe (170 M complex multiply-adds) -> 92 us, a
-// quarter of it the direct and exchange matrices (k_mult_hamp).
+// whole term 1200 us on the FP64 pipe (170 M complex multiply-adds) -> 80 us, a
+// sixth of it the direct and exchange matrices (k_mult_hamp).
 int slice_set_mult(ocn_ctx* c) {
   SliceLR* s = c->slice;
   if (!s) return OCN_OK;
