@@ -190,6 +190,15 @@ int apply_host(ocn_ctx* c, int nv, const double* ir, const double* ii, double* o
   double *in = c->xb, *out = c->xb + half, *hb = c->xb_host ? c->xb_host + 1 : nullptr;
   int* herr = reinterpret_cast<int*>(c->xb_host);
   if (herr) *herr = 0;
+  // one strided copy per plane, or one per vector where the pitch is beyond the copy's limit
+  auto plane = [&](double* dst, size_t dp, const double* src, size_t sp, cudaMemcpyKind kind) {
+    if (2 * row <= 0x7fffffffu) return cudaMemcpy2DAsync(dst, dp, src, sp, row, nv, kind, c->stream);
+    cudaError_t r = cudaSuccess;
+    for (int v = 0; v < nv && r == cudaSuccess; ++v)
+      r = cudaMemcpyAsync(reinterpret_cast<char*>(dst) + v * dp, reinterpret_cast<const char*>(src) + v * sp, row, kind,
+                          c->stream);
+    return r;
+  };
   cudaError_t e = cudaSuccess;
   if (pinned) {
     for (int v = 0; v < nv; ++v) {
@@ -197,9 +206,9 @@ int apply_host(ocn_ctx* c, int nv, const double* ir, const double* ii, double* o
       std::memcpy(hb + 2 * v * n + n, ii + v * n, n * sizeof(double));
     }
     e = cudaMemcpyAsync(in, hb, half * sizeof(double), cudaMemcpyHostToDevice, c->stream);
-  } else {  // one strided copy per plane
-    e = cudaMemcpy2DAsync(in, 2 * row, ir, row, row, nv, cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess) e = cudaMemcpy2DAsync(in + n, 2 * row, ii, row, row, nv, cudaMemcpyHostToDevice, c->stream);
+  } else {
+    e = plane(in, 2 * row, ir, row, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = plane(in + n, 2 * row, ii, row, cudaMemcpyHostToDevice);
   }
   rc = e == cudaSuccess ? act(in, out) : OCN_OK;
   const bool ok = e == cudaSuccess && rc == OCN_OK;
@@ -208,9 +217,9 @@ int apply_host(ocn_ctx* c, int nv, const double* ir, const double* ii, double* o
   if (ok && pinned && e == cudaSuccess)
     e = cudaMemcpyAsync(hb + half, out, half * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
   if (ok && !pinned && e == cudaSuccess)
-    e = cudaMemcpy2DAsync(orr, row, out, 2 * row, row, nv, cudaMemcpyDeviceToHost, c->stream);
+    e = plane(orr, row, out, 2 * row, cudaMemcpyDeviceToHost);
   if (ok && !pinned && e == cudaSuccess)
-    e = cudaMemcpy2DAsync(oi, row, out + n, 2 * row, row, nv, cudaMemcpyDeviceToHost, c->stream);
+    e = plane(oi, row, out + n, 2 * row, cudaMemcpyDeviceToHost);
   const cudaError_t es = cudaStreamSynchronize(c->stream);
   if (e == cudaSuccess) e = es;
   if (e != cudaSuccess) return cuda_fail(c, e, what);
