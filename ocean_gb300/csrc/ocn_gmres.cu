@@ -1151,9 +1151,15 @@ int gmres_solve_op(const GmresOp& op, const double* d_rhs_in, double kpref, cons
           if ((q = op.Hblock(nb, hin + (size_t)v0 * 2 * n, hout + (size_t)v0 * 2 * n))) return q;
         }
       }
-      for (Lane* lp : hq) lp->wait = LW_RUN;
+      // A lane that starts a step early may hold a lower slot than a lane ahead of it in the
+      // list, and the new round's requests go to slot 0 upwards: every input slot that is
+      // still to be read (H pg and pg form au) is read before any lane may request again.
+      const std::vector<Lane*> served(hq);
       hq.clear();
       nreq = 0;
+      for (Lane* lp : served) lp->wait = LW_RUN;
+      for (Lane* lp : served)
+        if (lp->ph == LP_ITER_H && (q = advance(*lp))) return q;
     }
     return OCN_OK;
   };
