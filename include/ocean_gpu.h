@@ -603,6 +603,17 @@ int ocn_get_tiles(const ocn_ctx* ctx, int tiles[7]);
  * normal operation; the context stays usable.  Mixed precision only. */
 int ocn_test_starve_tc(ocn_ctx* ctx, int on);
 
+/* FP64 contexts: where the contractions run.  The long-range (bit 0 of mask) and the
+ * multiplet contractions (bit 1) run on digit operands on the tensor cores when these
+ * fit (about four times the memory of the Bloch functions, at most a quarter of the
+ * device memory that is free at ocn_lr_init and ocn_set_mult), else on the FP64 pipe,
+ * an order of magnitude slower on large problems and different in the last bits.
+ * ocn_fp64_digits tells which ones do (0 in mixed precision).  ocn_set_fp64_digits
+ * declines them where a bit is 0 (default 3): a run is then the same whatever else
+ * holds device memory; the operands are freed or built by the call. */
+int ocn_set_fp64_digits(ocn_ctx* ctx, int mask);
+int ocn_fp64_digits(const ocn_ctx* ctx, int* mask);
+
 /* Per-kernel device timing with CUDA events recorded on the context stream
  * (replaces the wall-clock buckets of OCEAN_timekeeper, OCEAN_timekeeper.f90:13-168).
  * Classes: 0 LR band->x contraction, 1 LR k-mesh transform x W, 2 LR x->band

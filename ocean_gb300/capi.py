@@ -96,6 +96,7 @@ EXPORTS = [
     "ocn_val_apply_H", "ocn_val_apply_H_dev", "ocn_val_haydock", "ocn_val_haydock_dev",
     "ocn_val_spectrum", "ocn_val_optical_constants", "ocn_write_opcons", "ocn_val_set_fxc",
     "ocn_val_fxc_from_rho", "ocn_read_val_u2", "ocn_val_pair_energies", "ocn_test_starve_tc",
+    "ocn_set_fp64_digits", "ocn_fp64_digits",
     "ocn_gmres_set_lanes", "ocn_set_haydock_conv", "ocn_read_haydockconv",
     "ocn_read_u2par", "ocn_read_con_u2", "ocn_read_obf_control",
     "ocn_mult_exchange", "ocn_threey", "ocn_read_slater", "ocn_val_gmres",
@@ -316,6 +317,16 @@ class Context:
 
     def timing(self, on: bool = True):
         self._chk(self.lib.ocn_timing_enable(self.ptr, int(on)))
+
+    def set_fp64_digits(self, mask: int):
+        """FP64: bit 0 long-range, bit 1 multiplet contractions on digit operands where they fit; else the FP64 pipe."""
+        self._chk(self.lib.ocn_set_fp64_digits(self.ptr, int(mask)))
+
+    def fp64_digits(self) -> int:
+        """The contractions that run on digit operands (bits as set_fp64_digits)."""
+        m = C.c_int(0)
+        self._chk(self.lib.ocn_fp64_digits(self.ptr, C.byref(m)))
+        return m.value
 
     def starve_tc(self, on: bool = True):
         """Test hook: the tensor-core contractions' load warp issues nothing, so

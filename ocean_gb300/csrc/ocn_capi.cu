@@ -286,6 +286,27 @@ int ocn_test_starve_tc(ocn_ctx* c, int on) {
   return mixed_set_starve(c, on);
 }
 
+int ocn_set_fp64_digits(ocn_ctx* c, int mask) {
+  if (!c) return OCN_ERR_ARG;
+  if (c->dims.precision != OCN_PREC_FP64)
+    return set_err(c, OCN_ERR_UNSUPPORTED, "ocn_set_fp64_digits: FP64 contexts only");
+  if (mask < 0 || mask > 3) return set_err(c, OCN_ERR_ARG, "ocn_set_fp64_digits: mask must be in 0..3");
+  cudaSetDevice(c->device);
+  OCN_CUDA(c, cudaStreamSynchronize(c->stream));
+  drop_haydock_graph(c);
+  c->digits = mask;
+  int rc = OCN_OK;
+  if (c->have_bloch) rc = slice_set_bloch(c);
+  if (rc == OCN_OK && c->have_mult) rc = slice_set_mult(c);
+  return rc;
+}
+
+int ocn_fp64_digits(const ocn_ctx* c, int* mask) {
+  if (!c || !mask) return OCN_ERR_ARG;
+  *mask = (slice_ready(c) ? 1 : 0) | (slice_mult_ready(c) ? 2 : 0);
+  return OCN_OK;
+}
+
 int ocn_get_tiles(const ocn_ctx* c, int tiles[7]) {
   if (!c || !tiles) return OCN_ERR_ARG;
   return c->mixed ? mixed_config(c, tiles) : OCN_ERR_UNSUPPORTED;
@@ -390,7 +411,7 @@ int ocn_ctx_create(const ocn_dims* d, ocn_ctx** out) {
   // small vectors (about two elements per thread); each block's partial is
   // re-reduced by every block of the next stage, so extra blocks cost.
   c->red_blocks = (int)std::min<size_t>(2 * (size_t)c->sm_count, std::max<size_t>(1, (c->npsi + 511) / 512));
-  c->lr_xsplit = std::max(1, std::min((2 * c->sm_count + nk - 1) / nk, std::max(1, nx / 64)));
+  c->lr_xsplit = c->lr_xsplit_pipe = std::max(1, std::min((2 * c->sm_count + nk - 1) / nk, std::max(1, nx / 64)));
   int rc = OCN_OK;
   if (d->precision == OCN_PREC_FP64 && ((rc = slice_init(c)) || (rc = fx_init(c)))) return fail(rc);
   if ((rc = dev_alloc(c, &c->d_er, c->npsi)) || (rc = dev_alloc(c, &c->d_ei, c->npsi)) ||
@@ -406,7 +427,7 @@ int ocn_ctx_create(const ocn_dims* d, ocn_ctx** out) {
     c->fp64_nv = slice_width(c);
     c->part_stride = (size_t)c->fp64_nv * 2 * c->npsi;
     if ((rc = dev_alloc(c, &c->d_phi, (size_t)nk * nx * c->na * c->fp64_nv)) ||
-        (rc = dev_alloc(c, &c->d_accpart, (size_t)c->lr_xsplit * c->part_stride)))
+        (rc = dev_alloc(c, &c->d_accpart, (size_t)std::max(c->lr_xsplit_pipe, slice_splits(c)) * c->part_stride)))
       return fail(rc);
   }
   cudaMemsetAsync(c->d_ei, 0, sizeof(double) * c->npsi, c->stream);
@@ -545,6 +566,7 @@ int ocn_lr_init(ocn_ctx* c, const ocn_lr_params* p) {
   c->have_W = true;
   if (c->dims.precision == OCN_PREC_MIXED) return mixed_set_bloch(c);
   if ((rc = fx_set_w(c))) return rc;
+  drop_haydock_graph(c);  // a captured graph holds the kernels of the path in use
   return slice_set_bloch(c);
 }
 

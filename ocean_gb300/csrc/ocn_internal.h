@@ -127,7 +127,9 @@ struct ocn_ctx {
   int fp64_nv = 1;                 // FP64 contexts: vectors of a block that act together
   double* d_acc = nullptr;         // full-store accumulator: re plane then im plane (npsi each)
   double* d_accpart = nullptr;     // long-range partials [split][vector][re|im][npsi]
-  int lr_xsplit = 1;
+  int lr_xsplit = 1;               // x-splits of the x->band contraction in use
+  int lr_xsplit_pipe = 1;          // FP64 contexts: those of the FP64-pipe kernels
+  int digits = 3;                  // FP64 contexts: digit operands allowed (1 long range, 2 multiplet)
   int mult_parts = 0;              // multiplet partial slices after the LR ones (tensor-core multiplet)
   size_t part_stride = 0;          // elements between two splits of d_accpart
   int nvec = 1;                    // largest psi block
@@ -377,9 +379,10 @@ void val_fx_apply(const int kmesh[3], int nv, int nx, int yper, int ysplit, cons
                   const int* eV, const void* lad, const int* eL, double2* Bp, cudaStream_t s);
 
 // ---- FP64 contractions on the tensor cores (ocn_slice.cu)
-int slice_init(ocn_ctx* c);        // geometry and vector-side buffers; sets lr_xsplit
+int slice_init(ocn_ctx* c);        // geometry and vector-side buffers
+int slice_splits(const ocn_ctx* c);  // x-splits of the x->band contraction
 void slice_free(ocn_ctx* c);
-int slice_set_bloch(ocn_ctx* c);   // digit operands from d_u (not ready when they do not fit)
+int slice_set_bloch(ocn_ctx* c);   // digit operands from d_u (not ready when they do not fit); sets lr_xsplit
 bool slice_ready(const ocn_ctx* c);
 int slice_width(const ocn_ctx* c); // vectors that share a launch (12 columns at most)
 int slice_prep_psi(ocn_ctx* c, const double* d_pr, const double* d_pi, size_t vstride, int nv);  // operand of:

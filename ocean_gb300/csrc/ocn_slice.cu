@@ -822,7 +822,8 @@ int salloc(ocn_ctx* c, T** p, size_t n) {
   return OCN_OK;
 }
 
-void slice_drop_a(SliceLR* s) {
+void slice_drop_a(ocn_ctx* c) {
+  SliceLR* s = c->slice;
   for (SliceGemm* g : {&s->g1[0], &s->g2[0]}) {
     if (g->A) cudaFree(g->A);
     if (g->eA) cudaFree(g->eA);
@@ -830,9 +831,11 @@ void slice_drop_a(SliceLR* s) {
     g->eA = nullptr;
   }
   s->ready = false;
+  c->lr_xsplit = c->lr_xsplit_pipe;
 }
 
-void slice_drop_mult(SliceLR* s) {
+void slice_drop_mult(ocn_ctx* c) {
+  SliceLR* s = c->slice;
   for (SliceGemm* g : {&s->gm1, &s->gm2}) {
     if (g->A) cudaFree(g->A);
     if (g->eA) cudaFree(g->eA);
@@ -846,6 +849,7 @@ void slice_drop_mult(SliceLR* s) {
   s->mxm = nullptr;
   s->amp_part = nullptr;
   s->mult_ready = false;
+  c->mult_parts = 0;
 }
 
 // Digits and exponents of both operands of one spin from src (element (x, k, n) at x*sx + k*sk + n).
@@ -920,7 +924,6 @@ int slice_init(ocn_ctx* c) {
     slice_plan(&s->g2[w - 1], 2, nae, most, c->nk, c->nb, c->nx, c->sm_count, cost);
     if ((rc = allow_max_smem(c, slice_fn(1, nae))) || (rc = allow_max_smem(c, slice_fn(2, nae)))) return rc;
   }
-  c->lr_xsplit = s->g2[0].p.ks;
   const SliceGemm &w1 = s->g1[s->nvs - 1], &w2 = s->g2[s->nvs - 1];
   const size_t cols = (size_t)c->nk * c->na * s->nvs;
   if ((rc = salloc(c, &s->b1, w1.b_bytes())) || (rc = salloc(c, &s->b2, w2.b_bytes())) ||
@@ -932,14 +935,16 @@ int slice_init(ocn_ctx* c) {
   return OCN_OK;
 }
 
+int slice_splits(const ocn_ctx* c) { return c->slice ? c->slice->g2[0].p.ks : 1; }
+
 // Vectors that one action's contractions take together.
 int slice_width(const ocn_ctx* c) { return c->slice ? c->slice->nvs : 1; }
 
 void slice_free(ocn_ctx* c) {
   SliceLR* s = c->slice;
   if (!s) return;
-  slice_drop_a(s);
-  slice_drop_mult(s);
+  slice_drop_a(c);
+  slice_drop_mult(c);
   for (void* q : {(void*)s->b1, (void*)s->b2, (void*)s->e1, (void*)s->e2, (void*)s->mx2, (void*)s->ex2, (void*)s->d_err})
     if (q) cudaFree(q);
   delete s;
@@ -949,13 +954,13 @@ void slice_free(ocn_ctx* c) {
 bool slice_ready(const ocn_ctx* c) { return c->slice && c->slice->ready; }
 
 // Digit operands from d_u.  They take 3 bytes for every 2 of u, twice; when that
-// is more than a quarter of the free device memory the context keeps the
-// FP64-pipe kernels, which need only u.
+// is more than a quarter of the free device memory, or the caller declined them
+// (ocn_set_fp64_digits), the context keeps the FP64-pipe kernels, which need only u.
 int slice_set_bloch(ocn_ctx* c) {
   SliceLR* s = c->slice;
   if (!s) return OCN_OK;
-  if (!s->g1[0].A && !slice_alloc_a(c, &s->g1[0], &s->g2[0], c->nx)) {
-    slice_drop_a(s);
+  if (!(c->digits & 1) || (!s->g1[0].A && !slice_alloc_a(c, &s->g1[0], &s->g2[0], c->nx))) {
+    slice_drop_a(c);
     return OCN_OK;
   }
   const size_t sx = (size_t)c->nk * c->nb, sk = c->nb;
@@ -963,6 +968,7 @@ int slice_set_bloch(ocn_ctx* c) {
     if (int rc = slice_build(c, c->d_u + (size_t)sp * c->nx * sx, sx, sk, c->nx, s->g1[0], s->g2[0], sp)) return rc;
   OCN_CUDA(c, cudaStreamSynchronize(c->stream));
   s->ready = true;
+  c->lr_xsplit = s->g2[0].p.ks;
   return OCN_OK;
 }
 
@@ -976,18 +982,17 @@ int slice_set_bloch(ocn_ctx* c) {
 int slice_set_mult(ocn_ctx* c) {
   SliceLR* s = c->slice;
   if (!s) return OCN_OK;
-  slice_drop_mult(s);
-  c->mult_parts = 0;
+  slice_drop_mult(c);
   const int np = c->mult.np;
-  if (np == 0) return OCN_OK;
+  if (np == 0 || !(c->digits & 2)) return OCN_OK;
   slice_plan(&s->gm1, 1, c->na, c->na, c->nk, np, 2 * c->nb, c->sm_count, 0.0);
   slice_plan(&s->gm2, 2, c->na, c->na, c->nk, c->nb, np, c->sm_count, 32.0 * c->npsi / 6e12);
   s->gm2.p.bshared = 1;
   double* parts = nullptr;
   if (!slice_alloc_a(c, &s->gm1, &s->gm2, np) || salloc(c, &s->bm, s->gm2.b_bytes()) || salloc(c, &s->em, c->na) ||
       salloc(c, &s->mxm, c->na) || salloc(c, &s->amp_part, (size_t)c->nk * np * c->na) ||
-      salloc(c, &parts, (size_t)(c->lr_xsplit + s->gm2.p.ks) * c->part_stride)) {
-    slice_drop_mult(s);
+      salloc(c, &parts, (size_t)(std::max(c->lr_xsplit_pipe, slice_splits(c)) + s->gm2.p.ks) * c->part_stride)) {
+    slice_drop_mult(c);
     (void)cudaGetLastError();
     c->err.clear();
     return OCN_OK;
