@@ -600,7 +600,7 @@ int ocn_get_tiles(const ocn_ctx* ctx, int tiles[7]);
  * warp issues no loads, so the MMA warp's first bounded wait (about 1 s) runs
  * out with no copy or MMA in flight; the kernel records it, frees its tensor
  * memory and returns, and the call reports OCN_ERR_TIMEOUT.  on = 0 restores
- * normal operation; the context stays usable.  Mixed precision only. */
+ * normal operation; the context stays usable. */
 int ocn_test_starve_tc(ocn_ctx* ctx, int on);
 
 /* FP64 contexts: where the contractions run.  The long-range (bit 0 of mask) and the

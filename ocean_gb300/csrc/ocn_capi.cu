@@ -278,12 +278,10 @@ int ocn_set_tiles(ocn_ctx* c, const int tiles[7]) {
 
 int ocn_test_starve_tc(ocn_ctx* c, int on) {
   if (!c) return OCN_ERR_ARG;
-  if (c->dims.precision != OCN_PREC_MIXED || !c->mixed)
-    return set_err(c, OCN_ERR_UNSUPPORTED, "ocn_test_starve_tc: mixed-precision contexts only");
   cudaSetDevice(c->device);
   OCN_CUDA(c, cudaStreamSynchronize(c->stream));
   drop_haydock_graph(c);  // a captured graph holds the launch parameters
-  return mixed_set_starve(c, on);
+  return c->mixed ? mixed_set_starve(c, on) : slice_set_starve(c, on);
 }
 
 int ocn_set_fp64_digits(ocn_ctx* c, int mask) {

@@ -394,6 +394,7 @@ int slice_set_mult(ocn_ctx* c);    // digit operands of the projectors (after oc
 bool slice_mult_ready(const ocn_ctx* c);
 int slice_mult_apply(ocn_ctx* c, int v);  // multiplet term of the one prepared psi, into vector v's slices
 int slice_check(ocn_ctx* c);       // reads and clears the device timeout flag
+int slice_set_starve(ocn_ctx* c, int on);  // test hook of ocn_test_starve_tc
 
 // ---- mixed precision (ocn_mixed.cu)
 int mixed_init(ocn_ctx* c);

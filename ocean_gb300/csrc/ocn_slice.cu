@@ -86,6 +86,7 @@ struct SliceParams {
   size_t part_stride, npsi;
   int nb;
   int negate;                // x -> band: the long-range term subtracts, the multiplet back-projection adds
+  int starve;                // test hook: the load warp issues nothing, so the MMA warp's bounded wait runs out
   int* err;
 };
 
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(slice_threads(P == 1 ? C / 2 : C), 1) k_slice_
     for (int s = 0; s < SL_MAX_STAGES; ++s) armed[s] = -1;
     bool ok = true;
     int lastk = -1;
-    for (int t = t0; t < t1 && ok; ++t) {
+    for (int t = t0; t < t1 && ok && !p.starve; ++t) {
       const SliceTile ti = slice_decode<MODE>(p, t);
       const uint8_t* At = p.A + ((size_t)(ti.k + p.koff) * p.R + (size_t)SL_ROWS * ti.mt) * 16 * p.G * NBOX;
       const uint8_t* Bk = p.B + (p.bshared ? 0 : (size_t)ti.k) * p.Ge * (P * N * 16);
@@ -811,6 +812,7 @@ struct SliceLR {
   int* mxm = nullptr;
   double2* amp_part = nullptr;  // [k][p][a]
   int* d_err = nullptr;
+  int starve = 0;
 };
 
 namespace {
@@ -902,6 +904,7 @@ int slice_launch(ocn_ctx* c, const SliceGemm& g, const SliceGemm& a, const uint8
   p.koff = spin * p.nk;
   p.spin = spins == 2 ? spin : -1;
   p.negate = p.bshared ? 0 : 1;
+  p.starve = c->slice->starve;
   slice_fn(g.mode, g.nae)<<<g.grid, slice_threads(g.nae), g.smem, c->stream>>>(p);
   ++c->launches;
   OCN_CUDA(c, cudaGetLastError());
@@ -1092,9 +1095,15 @@ int slice_x_to_band(ocn_ctx* c, const double2* phi, int nv, int v0, bool integer
   return OCN_OK;
 }
 
-// Reads and clears the device timeout flag (as mixed_check).
+int slice_set_starve(ocn_ctx* c, int on) {
+  if (!c->slice) return set_err(c, OCN_ERR_STATE, "no FP64 tensor-core path");
+  c->slice->starve = on ? 1 : 0;
+  return OCN_OK;
+}
+
 const int* slice_err_word(const ocn_ctx* c) { return c->slice->d_err; }
 
+// Reads and clears the device timeout flag (as mixed_check).
 int slice_check(ocn_ctx* c) {
   if (!c->slice) return OCN_OK;
   int err = 0;
