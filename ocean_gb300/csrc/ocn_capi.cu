@@ -357,7 +357,7 @@ int ocn_ctx_create(const ocn_dims* d, ocn_ctx** out) {
       return set_err(nullptr, OCN_ERR_ARG, "kmesh extent out of range 1..32");
     if (d->xmesh[i] < 1) return set_err(nullptr, OCN_ERR_ARG, "xmesh extent must be >= 1");
   }
-  if (d->num_bands < 1 || d->num_bands > 1024)
+  if (d->num_bands < 1 || d->num_bands > OCN_MAX_NB)
     return set_err(nullptr, OCN_ERR_ARG, "num_bands must be in 1..1024");
   if (d->core_l < 0 || d->core_l > 1) return set_err(nullptr, OCN_ERR_ARG, "core_l must be 0 or 1");
   if (d->nalpha != 4 * (2 * d->core_l + 1))

@@ -11,6 +11,7 @@
 #include "../../include/ocean_gpu.h"
 
 #define OCN_MAX_NA 12       // 4*(2*l_c+1) for l_c <= 1 (1s, 2p edges)
+#define OCN_MAX_NB 1024     // most bands of a core context
 #define OCN_MAX_KDIM 32     // largest k-mesh extent along one axis handled by the FFT kernels
 #define OCN_MAX_NK 4096     // largest k-mesh size (shared-memory FFT)
 #define LZ_THREADS 256      // threads of the Lanczos-step kernels

@@ -11,8 +11,9 @@
 // S = 12 signed base-32 digits (|d| <= 16, exact in E4M3), and
 //   sum a b = 2^(ea + eb - 118) sum_(i,j) 32^(22-i-j) sum_K d_i(a) d_j(b)
 // is formed on the tensor cores.  |d_i d_j| <= 256, so the FP32 accumulator of a
-// group i + j is an exact integer while K * pairs * 256 <= 2^24 (checked where
-// the K splits are chosen); the groups i + j <= 11 are added in 64-bit integers
+// group i + j is an exact integer while K * pairs * 256 <= 2^24 (x -> band: kept by
+// the choice of the K splits; band -> x, which has none: by the largest number of
+// bands, asserted below); the groups i + j <= 11 are added in 64-bit integers
 // and rounded to binary64 once.  What is left out (digits below 2^-60 of a row's
 // largest element, pairs with i + j > 11) is below the rounding error of an FP64
 // sum: 2-norm error 5e-17 against 3e-16 (100 bands) and 1.4e-15 (1728 x-points)
@@ -68,6 +69,7 @@ constexpr int slice_threads(int nae) { return nae == 4 ? 192 : 320; }
 constexpr int SL_MAX_STAGES = 6;
 constexpr size_t SL_SMEM = 222 * 1024;
 constexpr int SL_MAX_K = 2730;      // K per plane and accumulation: 2 * 2730 * 12 * 256 < 2^24
+static_assert(OCN_MAX_NB <= SL_MAX_K, "band -> x sums 2 Nb products (re n, im n) in one accumulation");
 constexpr unsigned long long SL_BIAS = 0x0842108421084210ull;  // sum of 16 * 32^i, i < 12
 
 struct SliceParams {
