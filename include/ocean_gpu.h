@@ -605,8 +605,8 @@ int ocn_test_starve_tc(ocn_ctx* ctx, int on);
 
 /* FP64 contexts: where the contractions run.  The long-range (bit 0 of mask) and the
  * multiplet contractions (bit 1) run on digit operands on the tensor cores when these
- * fit (about four times the memory of the Bloch functions, at most a quarter of the
- * device memory that is free at ocn_lr_init and ocn_set_mult), else on the FP64 pipe,
+ * fit (about three times the memory of the Bloch functions on top of it, at most a quarter
+ * of the device memory that is free at ocn_lr_init and ocn_set_mult), else on the FP64 pipe,
  * an order of magnitude slower on large problems and different in the last bits.
  * ocn_fp64_digits tells which ones do (0 in mixed precision).  ocn_set_fp64_digits
  * declines them where a bit is 0 (default 3): a run is then the same whatever else

@@ -59,7 +59,9 @@ int terms_fp64(ocn_ctx* c, const double* pr, const double* pi, size_t vstride, i
   const bool sliced = mult_on && slice_mult_ready(c);
   if (sliced) {
     for (int v = 0; v < nv; ++v)
-      if ((rc = slice_prep_psi(c, pr + v * vstride, pi + v * vstride, 0, 1)) || (rc = slice_mult_apply(c, v))) return rc;
+      if ((rc = slice_prep_psi(c, pr + v * vstride, pi + v * vstride, 0, 1)) ||
+          (rc = slice_mult_apply(c, pr + v * vstride, pi + v * vstride, v)))
+        return rc;
   } else if (mult_on) {
     if ((rc = zero_acc(c, nv))) return rc;
     for (int v = 0; v < nv; ++v)

@@ -54,7 +54,7 @@ __device__ __forceinline__ double fx_to_double(long long v, int e) {
   }
   return fx_ldexp(v < 0 ? -(long long)m : (long long)m, e + 11 - lz);
 }
-// (h 2^30 + l) 2^e rounded to binary64; |h| < 2^50, |l| < 2^52
+// (h 2^30 + l) 2^e rounded to binary64; |h| < 2^56, |l| < 2^55
 __device__ __forceinline__ double fx_to_double(long long h, long long l, int e) {
   h += l >> 30;
   unsigned ul = (unsigned)(l & 0x3fffffff);

@@ -387,13 +387,15 @@ int slice_set_bloch(ocn_ctx* c);   // digit operands from d_u (not ready when th
 bool slice_ready(const ocn_ctx* c);
 int slice_width(const ocn_ctx* c); // vectors that share a launch (12 columns at most)
 int slice_prep_psi(ocn_ctx* c, const double* d_pr, const double* d_pi, size_t vstride, int nv);  // operand of:
-int slice_band_to_x(ocn_ctx* c, double2* phi, int nv);  // phi[k][x][t], t = v*Na + a
+// phi[k][x][t], t = v*Na + a, of the vectors that slice_prep_psi was given
+int slice_band_to_x(ocn_ctx* c, const double* d_pr, const double* d_pi, size_t vstride, double2* phi, int nv);
 // d_accpart slices of vectors v0 .. v0 + nv - 1 from phi'[k][x][t]
 int slice_x_to_band(ocn_ctx* c, const double2* phi, int nv, int v0, bool integers);
 void slice_exponents(ocn_ctx* c, int** ex, int** mx);  // of phi' in integers
 int slice_set_mult(ocn_ctx* c);    // digit operands of the projectors (after ocn_set_mult)
 bool slice_mult_ready(const ocn_ctx* c);
-int slice_mult_apply(ocn_ctx* c, int v);  // multiplet term of the one prepared psi, into vector v's slices
+// multiplet term of the one psi that slice_prep_psi was given, into vector v's slices
+int slice_mult_apply(ocn_ctx* c, const double* d_pr, const double* d_pi, int v);
 int slice_check(ocn_ctx* c);       // reads and clears the device timeout flag
 int slice_set_starve(ocn_ctx* c, int on);  // test hook of ocn_test_starve_tc
 

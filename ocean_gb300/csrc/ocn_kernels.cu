@@ -1049,7 +1049,7 @@ int lr_apply_fp64(ocn_ctx* c, const double* d_pr, const double* d_pi, size_t vst
   if (slice_ready(c) && fx_supported(c)) {  // all nv vectors in one set of launches
     int rc;
     if (!b1_ready && (rc = slice_prep_psi(c, d_pr, d_pi, vstride, nv))) return rc;
-    if ((rc = slice_band_to_x(c, c->d_phi, nv))) return rc;
+    if ((rc = slice_band_to_x(c, d_pr, d_pi, vstride, c->d_phi, nv))) return rc;
     {
       TimedScope ts(c, T_LR_FFT);
       int *ex, *mx;
@@ -1064,7 +1064,7 @@ int lr_apply_fp64(ocn_ctx* c, const double* d_pr, const double* d_pi, size_t vst
     if (sliced) {
       int rc;
       if (!b1_ready && (rc = slice_prep_psi(c, pr, pi, 0, 1))) return rc;
-      if ((rc = slice_band_to_x(c, c->d_phi, 1))) return rc;
+      if ((rc = slice_band_to_x(c, pr, pi, 0, c->d_phi, 1))) return rc;
     } else {
       const size_t sm = sizeof(double2) * ((size_t)c->nspn * G1_N * (G1_X + 1) + (size_t)na * G1_N);
       dim3 grid((nx + G1_X - 1) / G1_X, nk);
@@ -1118,8 +1118,8 @@ int lr_wgrad_fp64(ocn_ctx* c, const double* x, const double* y, double2* phi, do
   double2* phy = phi + (size_t)nk * nx * na;
   if (slice_ready(c)) {
     int rc;
-    if ((rc = slice_prep_psi(c, x, x + n, 0, 1)) || (rc = slice_band_to_x(c, phx, 1)) ||
-        (rc = slice_prep_psi(c, y, y + n, 0, 1)) || (rc = slice_band_to_x(c, phy, 1)))
+    if ((rc = slice_prep_psi(c, x, x + n, 0, 1)) || (rc = slice_band_to_x(c, x, x + n, 0, phx, 1)) ||
+        (rc = slice_prep_psi(c, y, y + n, 0, 1)) || (rc = slice_band_to_x(c, y, y + n, 0, phy, 1)))
       return rc;
   } else {
     const size_t sm = sizeof(double2) * ((size_t)c->nspn * G1_N * (G1_X + 1) + (size_t)na * G1_N);

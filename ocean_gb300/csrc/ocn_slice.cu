@@ -13,39 +13,50 @@
 // is formed on the tensor cores.  |d_i d_j| <= 256, so the FP32 accumulator of a
 // group i + j is an exact integer while K * pairs * 256 <= 2^24 (x -> band: kept by
 // the choice of the K splits; band -> x, which has none: by the largest number of
-// bands, asserted below); the groups i + j <= 11 are added in 64-bit integers
-// and rounded to binary64 once.  What is left out (digits below 2^-60 of a row's
-// largest element, pairs with i + j > 11) is below the rounding error of an FP64
-// sum: 2-norm error 5e-17 against 3e-16 (100 bands) and 1.4e-15 (1728 x-points)
-// for binary64 multiply-adds on Gaussian rows, and still below it for rows that
-// spread over six decades (with S = 11 it is not).  The sums are exact, so results
-// do not depend on tiling, splits or the number of vectors sharing a launch.
+// bands, asserted below); the groups i + j <= 12 are added in 64-bit integers
+// and rounded to binary64 once (per K split).
+//
+// Accuracy.  What is left out are digits below 2^-60 of a row's largest element and
+// pairs with i + j > 12.  For rows whose elements are of one size that is a tenth of
+// the rounding error of an FP64 sum; where a row is small at the K at which the column
+// is large it would not be.  The epilogue checks every sum (see check_part) and forms
+// those that the digits do not hold as well in binary64.  An action is therefore as
+// accurate as an FP64 one element by element, not only in the norm.  (With the groups
+// i + j <= 11 the check left many sums over preconditioned GMRES residuals open, which
+// are peaked over the bands: the 64 k / 32 bands gradient took 220 ms, now 130.)
+//
+// The sums of a K split are exact; splits are rounded and added one after another, and
+// chunks and splits follow the context's largest block (nvec), so results do not depend
+// on the vectors that share a launch, but may differ in the last bit between contexts.
 //
 // Layout.  The digits of u are stored in the order in which the kernel consumes
 // them, as no-swizzle K-major core matrices ([granule of 16 K][row][16 bytes]), so
 // every pipeline stage is one contiguous bulk copy:
 //   A[spin][k][row tile of 128][K chunk][box][granule][row][16]
 // box = slice (band -> x: K runs over re n then im n) or plane * 12 + slice (x ->
-// band: re and im planes of u, K over x).  12 bytes per real against 8 for FP64.
+// band: re and im planes of u, K over x).  12 bytes per real against 8 for FP64, and
+// one byte per complex element of magnitudes for the check.
 // The vector side is small and rebuilt per action:
 //   B[k][granule][part][slice][column][16]
 // In shared memory each granule's digit rows follow 11 empty slices, so the
 // operand of slice i of A is the same buffer read from row (11 - i) C: its digit j
-// meets output column group i + j, and one MMA of N = 12 C columns per (slice, 32
-// K) adds every pair of that slice.  part: re/im columns; both in one MMA when
-// 24 C' <= 256 (band -> x of up to two 1s vectors), else one MMA per part (x ->
-// band swaps the parts between the planes and negates A for the last of the four).
+// meets output column group i + j, and one MMA of N = 13 C columns per (slice, 32
+// K) adds every pair of that slice.  part: re/im columns; both in one MMA (C = 2
+// columns each) with up to 8 columns, else one MMA per part (x -> band swaps the
+// parts between the planes and negates A for the last of the four).
 // The kernel is persistent and warp-specialised like k_lr_tc; CTAs take
 // contiguous tile ranges so that the B operand of a k-point is read once.
 //
 // Measured, 8^3 k / 100 bands / 12^3 x, 1s: band -> x 4.3 ms on the FP64 pipe ->
-// 0.331 ms (2.2 GB, 6.7 TB/s), x -> band 5.9 ms -> 0.355 ms (6.2 TB/s): bound by
-// the read of A.  2p, 6^3 k / 64 bands / 10^3 x (12 columns): 0.084 and 0.108 ms
-// (4.0 and 2.9 TB/s): there the 144-column MMAs (72 cycles) and the epilogue's
-// 288 integer columns per row weigh as much as the 0.3 GB read.
+// 0.345 ms (2.3 GB, 6.7 TB/s), x -> band 5.9 ms -> 0.355 ms (6.4 TB/s): bound by
+// the read of A.  2p, 6^3 k / 64 bands / 10^3 x (12 columns): 0.099 and 0.108 ms
+// (3.5 and 3.2 TB/s): there the 160-column MMAs (80 cycles) and the epilogue's
+// 312 integer columns per row weigh as much as the 0.33 GB read.  Without the group
+// i + j = 12 and the check the four took 0.331, 0.355, 0.083 and 0.104 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <new>
 #include <string>
@@ -61,6 +72,11 @@ namespace {
 constexpr int SL_S = 12;           // digits per value
 constexpr int SL_FRAC = 59;        // fixed point: t = v 2^(59 - e), |v| < 2^e
 constexpr int SL_ROWS = 128;       // rows per tile (MMA M)
+// MMA N: the 13 groups i + j <= 12 of C columns, in steps of 16
+__host__ __device__ constexpr int slice_n(int C) { return (13 * C + 15) / 16 * 16; }
+// Rows of a granule of B in shared memory: 11 empty and 12 digit slices per part, and empty rows
+// to the end of the last part's widest operand (the other part's ends in the next empty slices)
+__host__ __device__ constexpr int slice_rows(int C, int P) { return (P - 1) * 23 * C + 11 * C + slice_n(C); }
 // Two control warps and four epilogue warps; eight with 8 or 12 columns, half of the
 // columns each (band -> x of the 2p case: 113 us with four warps and 255 registers,
 // 84 us with eight).
@@ -69,6 +85,9 @@ constexpr int slice_threads(int nae) { return nae == 4 ? 192 : 320; }
 constexpr int SL_MAX_STAGES = 6;
 constexpr size_t SL_SMEM = 222 * 1024;
 constexpr int SL_MAX_K = 2730;      // K per plane and accumulation: 2 * 2730 * 12 * 256 < 2^24
+// Most products of a sum: an epilogue that forms all sums of a tile in binary64 (3072 clocks
+// a product with 12 columns) stays below half of the pipeline's time limit.
+constexpr int SL_MAX_SUM = 1 << 18;
 static_assert(OCN_MAX_NB <= SL_MAX_K, "band -> x sums 2 Nb products (re n, im n) in one accumulation");
 constexpr unsigned long long SL_BIAS = 0x0842108421084210ull;  // sum of 16 * 32^i, i < 12
 
@@ -90,6 +109,17 @@ struct SliceParams {
   int negate;                // x -> band: the long-range term subtracts, the multiplet back-projection adds
   int starve;                // test hook: the load warp issues nothing, so the MMA warp's bounded wait runs out
   int* err;
+  // the check of the sums and its binary64 fallback
+  const uint4* A8;           // magnitudes of u (k_slice_build_mag)
+  const uint2* B8;           // and of the columns, [k][t][32 S8 bytes]
+  int K, S8;                 // complex products of a sum; steps of 32 of them
+  int sample, least;         // steps of the first pass and the least sum that clears
+  const double2* u;          // of this spin, element (x, k, n) at x*ux + k*uk + n
+  size_t ux, uk;
+  const double *pr, *pi, *allow;  // band -> x: psi of the columns
+  size_t vstride;
+  const double2* f;          // x -> band: [k][x][t], integers with exponents ex[x][t] or binary64
+  const int* ex;
 };
 
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
@@ -133,20 +163,20 @@ __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, float* v) {
   }
 }
 
-// Six accumulator groups (most significant first, stride C columns) of A columns as integers.
-template <int A, int C>
+// NG accumulator groups (most significant first, stride C columns) of A columns as integers.
+template <int A, int C, int NG>
 __device__ __forceinline__ void add_groups(uint32_t ta, long long (&acc)[A]) {
-  float v[6 * A];
+  float v[NG * A];
 #pragma unroll
-  for (int g = 0; g < 6; ++g) tmem_ld_cols<A>(ta + g * C, v + g * A);
+  for (int g = 0; g < NG; ++g) tmem_ld_cols<A>(ta + g * C, v + g * A);
   tmem_ld_wait();
 #pragma unroll
   for (int c = 0; c < A; ++c) acc[c] = 0;
 #pragma unroll
-  for (int g = 0; g < 6; ++g)
+  for (int g = 0; g < NG; ++g)
 #pragma unroll
     for (int c = 0; c < A; ++c)
-      acc[c] += (long long)__float2int_rn(v[g * A + c]) * (long long)(1 << (5 * (5 - g)));
+      acc[c] += (long long)__float2int_rn(v[g * A + c]) * (long long)(1 << (5 * (NG - 1 - g)));
 }
 
 struct SliceTile {
@@ -166,6 +196,214 @@ __device__ __forceinline__ SliceTile slice_decode(const SliceParams& p, int t) {
   return ti;
 }
 
+// x w for a mask weight w, without the FP64 pipe where w = 1
+__device__ __forceinline__ double weigh(double x, double w) {
+  const long long b = __double_as_longlong(w);
+  if (b == 0x3ff0000000000000ll) return x;
+  return x * w;
+}
+
+// ------------------------------------------------------ graded rows and columns
+
+// The digits of a row and of a column end at 2^-60 of their largest elements.  A sum whose
+// terms are all small against the product of the two maxima -- row and column graded
+// oppositely -- would be less accurate than in binary64.  The epilogue bounds sum |a||b| of
+// every sum from below by 8-bit magnitudes, and the sums that the bound does not clear are
+// formed in binary64 from u and the column instead.
+//
+// The error of a digit sum of K complex products is sqrt(2) 2^-60.8 (2^eb |a|_2 + 2^ea |b|_2)
+// (the two in quadrature; rounding of the elements) and 2^-64.8 sqrt(2 K) 2^(ea + eb) (pairs
+// left out) per part.  A sum is cleared when this is at most a quarter of 2^-53 sum |a||b|;
+// sums of products in binary64 are off by 0.3 to 0.5 of that (K = 4..1000).  In magnitudes m
+// (2^e = 256): (sum m(a) m(b))^2 >= 42 (sum m(a)^2 + sum m(b)^2) + 10100 K.  Ungraded Gaussian
+// rows have 18 (K = 1) to 150 (K = 500) times the square root of that, rows graded oppositely
+// over two decades about as much.
+constexpr float SL_CHECK_M = 42.0f, SL_CHECK_K = 10100.0f;
+
+__device__ __forceinline__ void mma_u8(int (&c)[4], const uint4& a, const uint2& b) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+      : "r"(a.x), "r"(a.z), "r"(a.y), "r"(a.w), "r"(b.x), "r"(b.y));
+}
+// exponent of a row or column whose sums are checked: not of zeros (or subnormal), Inf or NaN
+__device__ __forceinline__ bool plain_exp(int e) { return e > -1022 && e != FX_NAN; }
+// A warp checks the AH <= 8 columns from h0 on that its threads drain, one column tile of the MMA.
+template <int NAE, int AH>
+__device__ __forceinline__ unsigned plain_columns(const SliceParams& p, int k, int h0) {
+  const int lane = threadIdx.x & 31, t = h0 + min(lane, AH - 1);
+  const int e = p.eB[(p.bshared ? 0 : (size_t)k) * NAE + t];
+  return __ballot_sync(0xffffffffu, lane < AH && plain_exp(e) && (p.spin < 0 || (t & 1) == p.spin));
+}
+// this lane's words of its column; columns beyond the last repeat it
+template <int NAE, int AH>
+__device__ __forceinline__ const uint2* check_column(const SliceParams& p, int k, int h0) {
+  const int lane = threadIdx.x & 31;
+  return p.B8 + ((p.bshared ? 0 : (size_t)k) * NAE + h0 + min(lane >> 2, AH - 1)) * p.S8 * 4 + (lane & 3);
+}
+
+// First pass, by a warp for the 32 rows of group rg: part of K (p.sample steps of 32) against
+// the largest error that any row and column of K elements can have, (sum)^2 >= K (2 * 42 *
+// 255^2 + 10100).  A partial sum bounds the whole from below; ungraded rows pass about ten
+// times over, so the magnitudes are read in part (512 k / 100 bands / 12^3 x: 57 and 17 of
+// 113 and 88 MB) while the tile's digits are still on their way.  As a kernel of its own
+// after the contraction the check took 18 and 10 us and a launch each.
+template <int NAE, int AH>
+__device__ __forceinline__ bool check_part(const SliceParams& p, int k, int rg, int h0) {
+  const int lane = threadIdx.x & 31, lg = lane >> 2, lq = lane & 3, ngrp = (p.rows + 31) / 32;
+  if (rg >= ngrp) return true;
+  const uint4* A = p.A8 + ((size_t)(k + p.koff) * ngrp + rg) * 2 * p.S8 * 32 + lane;
+  const uint2* B = check_column<NAE, AH>(p, k, h0);
+  const int ea = rg * 32 + lane < p.rows ? p.eA[(size_t)(k + p.koff) * p.rows + rg * 32 + lane] : FX_NAN;
+  int d[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};  // [h][q]: row 16 h + lg (+ 8 for q >= 2), column 2 lq (+ 1 for odd q)
+#pragma unroll 4
+  for (int c = 0; c < p.sample; ++c) {
+    const int st = (int)((long long)c * p.S8 / p.sample);
+    const uint4 a0 = __ldg(A + (size_t)st * 32), a1 = __ldg(A + (size_t)(p.S8 + st) * 32);
+    const uint2 b = __ldg(B + (size_t)st * 4);
+    mma_u8(d[0], a0, b);
+    mma_u8(d[1], a1, b);
+  }
+  const unsigned rows = __ballot_sync(0xffffffffu, plain_exp(ea)), cols = plain_columns<NAE, AH>(p, k, h0);
+  bool low = false;
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int r = 16 * h + lg + (q >= 2 ? 8 : 0), t = 2 * lq + (q & 1);
+      low |= ((rows >> r) & (cols >> t) & 1u) && d[h][q] < p.least;
+    }
+  return !__any_sync(0xffffffffu, low);
+}
+
+// Second pass: all of K and the norms.  The columns (bit t: h0 + t) of this lane's row (32 rg +
+// lane) that stay open.
+template <int NAE, int AH>
+__device__ __noinline__ unsigned check_whole(const SliceParams& p, int k, int rg, int h0) {
+  const int lane = threadIdx.x & 31, ngrp = (p.rows + 31) / 32;
+  const uint4* A = p.A8 + ((size_t)(k + p.koff) * ngrp + rg) * 2 * p.S8 * 32 + lane;
+  const uint2* B = check_column<NAE, AH>(p, k, h0);
+  float s[2][4] = {{0.0f, 0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f, 0.0f}}, qa[4] = {0.0f, 0.0f, 0.0f, 0.0f}, qb = 0.0f;
+  for (int c0 = 0; c0 < p.S8; c0 += 512) {  // 512 steps of 32 products below 2^16 fit in 31 bits
+    int d[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
+    unsigned da[4] = {0, 0, 0, 0}, db = 0;
+#pragma unroll 4
+    for (int st = c0; st < min(p.S8, c0 + 512); ++st) {
+      const uint4 a0 = __ldg(A + (size_t)st * 32), a1 = __ldg(A + (size_t)(p.S8 + st) * 32);
+      const uint2 b = __ldg(B + (size_t)st * 4);
+      mma_u8(d[0], a0, b);
+      mma_u8(d[1], a1, b);
+      db = __dp4a(b.x, b.x, __dp4a(b.y, b.y, db));
+      da[0] = __dp4a(a0.x, a0.x, __dp4a(a0.y, a0.y, da[0]));
+      da[1] = __dp4a(a0.z, a0.z, __dp4a(a0.w, a0.w, da[1]));
+      da[2] = __dp4a(a1.x, a1.x, __dp4a(a1.y, a1.y, da[2]));
+      da[3] = __dp4a(a1.z, a1.z, __dp4a(a1.w, a1.w, da[3]));
+    }
+    qb += (float)db;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      qa[q] += (float)da[q];
+      s[0][q] += (float)d[0][q];
+      s[1][q] += (float)d[1][q];
+    }
+  }
+#pragma unroll
+  for (int o = 1; o < 4; o <<= 1) {
+    qb += __shfl_xor_sync(0xffffffffu, qb, o);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) qa[q] += __shfl_xor_sync(0xffffffffu, qa[q], o);
+  }
+  // from the accumulators' places to a row per lane
+  const int quarter = lane >> 3, from = (lane & 7) * 4;  // rows 8 quarter ..
+  float a2 = 0.0f;
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float v = __shfl_sync(0xffffffffu, qa[q], from);
+    if (q == quarter) a2 = v;
+  }
+  const int row = 32 * rg + lane;
+  const bool on = row < p.rows && plain_exp(p.eA[(size_t)(k + p.koff) * p.rows + min(row, p.rows - 1)]);
+  const unsigned cols = plain_columns<NAE, AH>(p, k, h0);
+  unsigned bits = 0;
+#pragma unroll
+  for (int t = 0; t < AH; ++t) {
+    float ab = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float v = __shfl_sync(0xffffffffu, s[q >> 1][2 * (q & 1) + (t & 1)], from + (t >> 1));
+      if (q == quarter) ab = v;
+    }
+    const float b2 = __shfl_sync(0xffffffffu, qb, t * 4);
+    if (on && ((cols >> t) & 1u) && !(ab * ab >= SL_CHECK_M * (a2 + b2) + SL_CHECK_K * (float)p.K)) bits |= 1u << t;
+  }
+  return bits;
+}
+
+// Columns h0 .. h0 + AH - 1 of the 32 rows of a warp in binary64, those in bits (bit j: h0 + j)
+// of this lane's row (clamped to the last) stored.  All columns at once, so that an element of
+// u is read for 4 AH products, and a column's element is fetched and converted by one lane:
+// bound by the FP64 pipe.  With every x -> band sum open, 512 k / 100 bands / 8^3 x: 2.3 ms for
+// that contraction (0.12 with none; the FP64-pipe kernel 1.75), the action 2.5 ms (pipe: 3.2).
+template <int MODE, int NAE, int AH>
+__device__ __noinline__ void sum_binary64(const SliceParams& p, int k, int row, int h0, unsigned bits) {
+  constexpr int NI = 32 / AH;  // products in flight: a lane holds the column element of one (i, j)
+  const int lane = threadIdx.x & 31, li = lane / AH, lj = lane - li * AH, r = min(row, p.rows - 1);
+  const int t = h0 + lj, v = t / p.na;
+  const double2* u = p.u + (size_t)k * p.uk + (MODE == 1 ? (size_t)r * p.ux : (size_t)r);
+  double2 z[AH];
+#pragma unroll
+  for (int j = 0; j < AH; ++j) z[j] = make_double2(0.0, 0.0);
+  for (int i0 = 0; i0 < p.K; i0 += NI) {
+    double2 a[NI], b = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int q = 0; q < NI; ++q) {
+      const int i = min(i0 + q, p.K - 1);
+      a[q] = u[MODE == 1 ? (size_t)i : (size_t)i * p.ux];
+    }
+    const int i = i0 + li;
+    if (li < NI && i < p.K) {
+      if (MODE == 1) {
+        const size_t o = (size_t)i + (size_t)p.nb * ((size_t)k + (size_t)p.nk * (t - v * p.na));
+        const double w = p.allow[o];
+        b = make_double2(weigh(p.pr[v * p.vstride + o], w), weigh(p.pi[v * p.vstride + o], w));
+      } else {
+        b = p.f[((p.bshared ? 0 : (size_t)k) * p.K + i) * NAE + t];
+        if (p.ex) {
+          const int e = p.ex[(size_t)i * NAE + t];
+          b = make_double2(fx_to_double(__double_as_longlong(b.x), e), fx_to_double(__double_as_longlong(b.y), e));
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < NI; ++q) {
+      if (i0 + q >= p.K) break;
+#pragma unroll
+      for (int j = 0; j < AH; ++j) {
+        const double br = __shfl_sync(0xffffffffu, b.x, q * AH + j), bi = __shfl_sync(0xffffffffu, b.y, q * AH + j);
+        if (MODE == 1) {
+          z[j].x += a[q].x * br - a[q].y * bi;
+          z[j].y += a[q].x * bi + a[q].y * br;
+        } else {
+          z[j].x += a[q].x * br + a[q].y * bi;
+          z[j].y += a[q].x * bi - a[q].y * br;
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < AH; ++j) {
+    if (!((bits >> j) & 1u)) continue;
+    if (MODE == 1) {
+      p.phi[((size_t)k * p.rows + row) * NAE + h0 + j] = z[j];
+    } else {
+      const int vj = (h0 + j) / p.na;
+      double* out = p.part + (size_t)vj * 2 * p.npsi + (size_t)row +
+                    (size_t)p.nb * ((size_t)k + (size_t)p.nk * (h0 + j - vj * p.na));
+      out[0] = p.negate ? -z[j].x : z[j].x;
+      out[p.npsi] = p.negate ? -z[j].y : z[j].y;
+    }
+  }
+}
+
 // MODE 1: band -> x (K = re n, im n stacked; B columns carry the signs of the
 // complex product).  MODE 2: x -> band (two planes).  C columns per slice and
 // MMA, P MMAs (parts) per K step.
@@ -173,13 +411,14 @@ template <int MODE, int C, int P>
 __global__ void __launch_bounds__(slice_threads(P == 1 ? C / 2 : C), 1) k_slice_gemm(const __grid_constant__ SliceParams p) {
   constexpr int NAE = P == 1 ? C / 2 : C;        // complex columns
   constexpr int NBOX = MODE == 1 ? SL_S : 2 * SL_S;
-  constexpr int N = SL_S * C;                    // MMA N
+  constexpr int ND = SL_S * C;                   // digit rows of a part
+  constexpr int N = slice_n(C);                  // MMA N
   constexpr int PL = MODE == 2 && P == 1 ? 2 : 1;  // accumulators of their own per plane
   constexpr int DCOLS = P * PL * N;
   constexpr int ACC = 2 * DCOLS <= 512 ? 2 : 1;
   constexpr uint32_t TCOLS = ACC * DCOLS <= 128 ? 128 : (ACC * DCOLS <= 256 ? 256 : 512);
   constexpr uint32_t PROWS = 23 * C;             // 11 empty slices, 12 digit slices
-  constexpr uint32_t PITCH = P * PROWS * 16;     // bytes of a granule of B in shared memory
+  constexpr uint32_t PITCH = slice_rows(C, P) * 16;  // bytes of a granule of B in shared memory
   constexpr uint32_t IDESC0 = (1u << 4) | ((uint32_t)(SL_ROWS >> 4) << 24);
   extern __shared__ __align__(1024) uint8_t smem[];
   const int S = p.stages;
@@ -236,19 +475,19 @@ __global__ void __launch_bounds__(slice_threads(P == 1 ? C / 2 : C), 1) k_slice_
     for (int t = t0; t < t1 && ok && !p.starve; ++t) {
       const SliceTile ti = slice_decode<MODE>(p, t);
       const uint8_t* At = p.A + ((size_t)(ti.k + p.koff) * p.R + (size_t)SL_ROWS * ti.mt) * 16 * p.G * NBOX;
-      const uint8_t* Bk = p.B + (p.bshared ? 0 : (size_t)ti.k) * p.Ge * (P * N * 16);
+      const uint8_t* Bk = p.B + (p.bshared ? 0 : (size_t)ti.k) * p.Ge * (P * ND * 16);
       for (int c = ti.c0; c < ti.c1 && ok; ++c) {
         const int gc = min(p.KC, p.G - c * p.KC), gce = (gc + 1) & ~1;
         if (!keepb || ti.k != lastk) {
           ok = mbar_wait(bempty0 + 8 * slot, bphase ^ 1, abort_flag, TC_WAIT_CYCLES);
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
-          if (lane == 0) mbar_expect_tx(bfull0 + 8 * slot, (uint32_t)gce * P * N * 16);
+          if (lane == 0) mbar_expect_tx(bfull0 + 8 * slot, (uint32_t)gce * P * ND * 16);
           __syncwarp();
-          const uint8_t* src = Bk + (size_t)c * p.KC * (P * N * 16);
+          const uint8_t* src = Bk + (size_t)c * p.KC * (P * ND * 16);
           for (int i = lane; i < gce * P; i += 32)
             bulk_load(b_smem + slot * slot_bytes + (i / P) * PITCH + ((i % P) * PROWS + 11 * C) * 16,
-                      src + (size_t)i * (N * 16), N * 16, bfull0 + 8 * slot);
+                      src + (size_t)i * (ND * 16), ND * 16, bfull0 + 8 * slot);
           barmed[slot] = (int)bphase;
           slot ^= 1;
           if (slot == 0) bphase ^= 1;
@@ -320,7 +559,7 @@ __global__ void __launch_bounds__(slice_threads(P == 1 ? C / 2 : C), 1) k_slice_
             const int plane = b / SL_S, i = b - plane * SL_S;
             uint32_t ad = plain_desc(a_smem + stage * stage_bytes + (b - b0) * gc * lba, lba);
             // the first i column groups of slice i only meet empty slices: N shrinks in steps of 16
-            const uint32_t ni = (uint32_t)((SL_S - i) * C + 15) & ~15u, off = N - ni;
+            const uint32_t ni = (uint32_t)(N - i * C + 15) & ~15u, off = N - ni;
             const uint32_t idesc = IDESC0 | ((ni >> 3) << 17);
             uint32_t bd = plain_desc(b_smem + slot * slot_bytes + ((11 - i) * C + off) * 16, PITCH);
             const uint32_t d0 = dt + (PL == 2 ? plane * N : 0) + off;
@@ -380,7 +619,12 @@ __global__ void __launch_bounds__(slice_threads(P == 1 ? C / 2 : C), 1) k_slice_
     uint32_t acc = 0, acc_phase = 0;
     for (int t = t0; t < t1; ++t) {
       const SliceTile ti = slice_decode<MODE>(p, t);
-      if (!mbar_wait(tfull0 + 8 * acc, acc_phase, abort_flag, TC_WAIT_CYCLES)) {
+      __syncwarp();
+      const int rg = ti.mt * (SL_ROWS / 32) + q4;
+      unsigned open = 0;  // columns (from h0) of this row that the digits are not accurate enough for
+      if (!check_part<NAE, AH>(p, ti.k, rg, h0)) open = check_whole<NAE, AH>(p, ti.k, rg, h0);
+      // every lane the same way: the loop's warp-wide steps need all of them
+      if (!__all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * acc, acc_phase, abort_flag, TC_WAIT_CYCLES))) {
         *abort_flag = 1;
         atomicOr(p.err, 4);
         break;
@@ -390,17 +634,17 @@ __global__ void __launch_bounds__(slice_threads(P == 1 ? C / 2 : C), 1) k_slice_
       long long hi[2][AH], lo[2][AH];
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
-        add_groups<AH, C>(ta + q * PART, hi[q]);
-        add_groups<AH, C>(ta + q * PART + 6 * C, lo[q]);
+        add_groups<AH, C, 7>(ta + q * PART, hi[q]);
+        add_groups<AH, C, 6>(ta + q * PART + 7 * C, lo[q]);
       }
       if (PL == 2) {  // out = (re plane) phi' - i (im plane) phi'
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
           long long im[AH];
-          add_groups<AH, C>(ta + N + (1 - q) * PART, im);
+          add_groups<AH, C, 7>(ta + N + (1 - q) * PART, im);
 #pragma unroll
           for (int a = 0; a < AH; ++a) hi[q][a] += q ? -im[a] : im[a];
-          add_groups<AH, C>(ta + N + (1 - q) * PART + 6 * C, im);
+          add_groups<AH, C, 6>(ta + N + (1 - q) * PART + 7 * C, im);
 #pragma unroll
           for (int a = 0; a < AH; ++a) lo[q][a] += q ? -im[a] : im[a];
         }
@@ -418,10 +662,14 @@ __global__ void __launch_bounds__(slice_threads(P == 1 ? C / 2 : C), 1) k_slice_
           const int a = h0 + j;
           if (p.spin >= 0 && (a & 1) != p.spin) continue;
           const int e = eb[a];
-          const int es = ea + e - 2 * SL_FRAC + 55;
+          const int es = ea + e - 2 * SL_FRAC + 50;
           double vr = fx_to_double(hi[0][j], lo[0][j], es);
           double vi = fx_to_double(hi[1][j], lo[1][j], es);
           if (ea == FX_NAN || e == FX_NAN) vr = vi = __longlong_as_double(0x7ff8000000000000ll);
+          if ((open >> j) & 1u) {  // the whole sum goes to the first split, below
+            if (MODE == 1 || ti.sp == 0) continue;
+            vr = vi = 0.0;
+          }
           if (MODE == 1) {
             p.phi[((size_t)ti.k * p.rows + r) * NAE + a] = make_double2(vr, vi);
           } else {
@@ -433,6 +681,7 @@ __global__ void __launch_bounds__(slice_threads(P == 1 ? C / 2 : C), 1) k_slice_
           }
         }
       }
+      if (__any_sync(0xffffffffu, open != 0) && ti.sp == 0) sum_binary64<MODE, NAE, AH>(p, ti.k, r, h0, open);
     }
   }
   __syncthreads();
@@ -558,22 +807,25 @@ __global__ void k_slice_build_cols(const double2* __restrict__ u, size_t sx, siz
   }
 }
 
-// x w for a mask weight w, without the FP64 pipe where w = 1
-__device__ __forceinline__ double weigh(double x, double w) {
-  const long long b = __double_as_longlong(w);
-  if (b == 0x3ff0000000000000ll) return x;
-  return x * w;
+// 8-bit magnitude of a complex element against its block exponent, rounded down: the larger
+// part is at least m 2^(e - 8).
+__device__ __forceinline__ unsigned mag8(long long re, long long im) {
+  const long long a = max(re < 0 ? -re : re, im < 0 ? -im : im);
+  return min((unsigned)(a >> (SL_FRAC - 8)), 255u);
+}
+__device__ __forceinline__ unsigned mag8(double re, double im, int e) {
+  return mag8(fx_from<SL_FRAC>(re, e), fx_from<SL_FRAC>(im, e));
 }
 
 // psi operand of one k-point per CTA: q = allow o psi of nae columns t = (vector,
 // channel); column exponents, then digits of
 //   part 0 (Re phi): K = (re n) -> qr, (im n) -> -qi;  part 1 (Im phi): (re n) -> qi, (im n) -> qr.
-// merged: row order [slice][part][t], else [part][slice][t].  Clears the maxima that
-// the k-mesh transform of this action collects.
+// merged: row order [slice][part][t], else [part][slice][t].  M: magnitudes [k][t][32 S8].
+// Clears the maxima that the k-mesh transform of this action collects.
 __global__ void __launch_bounds__(256)
     k_slice_prep_b1(const double* __restrict__ pr, const double* __restrict__ pi, size_t vstride,
                     const double* __restrict__ allow, int nb, int nk, int na, int nae, int Ge, int merged,
-                    uint8_t* __restrict__ B, int* __restrict__ eB, int* __restrict__ mx) {
+                    uint8_t* __restrict__ B, int* __restrict__ eB, int* __restrict__ mx, uint8_t* __restrict__ M, int S8) {
   __shared__ int se[OCN_MAX_NA];
   const int k = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if ((int)threadIdx.x < nae) mx[(size_t)k * nae + threadIdx.x] = -FX_NAN;
@@ -616,6 +868,19 @@ __global__ void __launch_bounds__(256)
       *reinterpret_cast<unsigned*>(out + (size_t)row * 16) = digits4(f, s);
     }
   }
+  for (int i = threadIdx.x; i < nae * S8 * 8; i += blockDim.x) {
+    const int t = i / (8 * S8), n0 = 4 * (i - t * 8 * S8), v = t / na, a = t - v * na;
+    const size_t base = (size_t)nb * ((size_t)k + (size_t)nk * a);
+    unsigned m = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int n = n0 + j;
+      if (n >= nb) break;
+      const double w = allow[base + n];
+      m |= mag8(weigh(pr[v * vstride + base + n], w), weigh(pi[v * vstride + base + n], w), se[t]) << (8 * j);
+    }
+    *reinterpret_cast<unsigned*>(M + ((size_t)k * nae + t) * 32 * S8 + n0) = m;
+  }
 }
 
 // Exponent maxima mx[k][t] of src[k*nx + x][t] (operands that do not come from the
@@ -645,13 +910,14 @@ __device__ __forceinline__ unsigned long long fix_int(long long v, int s) {
 }
 
 // phi' operand from src[k*nx + x][t] (parts: re, im) and its column exponents: digits,
-// rows as k_slice_prep_b1.  INT: src holds integers with exponents ex[x][t], else
+// rows and M as k_slice_prep_b1.  INT: src holds integers with exponents ex[x][t], else
 // binary64.  grid (ceil(items / block), Nk); a thread makes four x of one column, both
 // parts (reads 64-byte runs, writes 4-byte words of 64-byte runs).
 template <bool INT>
 __global__ void __launch_bounds__(256)
     k_slice_prep_b2(const double2* __restrict__ src, const int* __restrict__ ex, int nx, int nae, int Ge, int merged,
-                    const int* __restrict__ mx, uint8_t* __restrict__ B, int* __restrict__ eB) {
+                    const int* __restrict__ mx, uint8_t* __restrict__ B, int* __restrict__ eB, uint8_t* __restrict__ M,
+                    int S8) {
   const int k = blockIdx.y;
   if (blockIdx.x == 0 && (int)threadIdx.x < nae)
     eB[(size_t)k * nae + threadIdx.x] = mx[(size_t)k * nae + threadIdx.x];
@@ -686,6 +952,36 @@ __global__ void __launch_bounds__(256)
     *reinterpret_cast<unsigned*>(out + (size_t)(merged ? 2 * s : s) * nae * 16) = digits4(fr, s);
     *reinterpret_cast<unsigned*>(out + (size_t)(merged ? 2 * s + 1 : SL_S + s) * nae * 16) = digits4(fi, s);
   }
+  {
+    unsigned m = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) m |= mag8((long long)(fr[j] - SL_BIAS), (long long)(fi[j] - SL_BIAS)) << (8 * j);
+    *reinterpret_cast<unsigned*>(M + ((size_t)k * nae + t) * 32 * S8 + 16 * g + 4 * qd) = m;
+  }
+}
+
+// Magnitudes of the u operand in the order in which check_part's lanes hold them, [spin k]
+// [group of 32 rows][half][32 K][lane][16 bytes]: lane 4 g + q has K = 8 q .. 8 q + 7 of rows g
+// and g + 8 of its half.  One thread per 16 bytes.  MODE 1: rows x over n; MODE 2: rows n over x.
+template <int MODE>
+__global__ void k_slice_build_mag(const double2* __restrict__ u, size_t sx, size_t sk, int nk, int rows, int K,
+                                  const int* __restrict__ e, uint4* __restrict__ M, int koff) {
+  const int ngrp = (rows + 31) / 32, S = (K + 31) / 32;
+  const long long tot = (long long)nk * ngrp * 2 * S * 32;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < tot; i += (long long)gridDim.x * blockDim.x) {
+    const int lane = (int)(i & 31), st = (int)((i >> 5) % S);
+    const long long h = (i >> 5) / S;  // (k ngrp + group) 2 + half
+    const int k = (int)(h / (2 * ngrp)), row0 = (int)(h % (2 * ngrp)) * 16 + (lane >> 2);
+    unsigned w[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int row = row0 + (j >= 8 ? 8 : 0), c = 32 * st + 8 * (lane & 3) + (j & 7);
+      if (row >= rows || c >= K) continue;
+      const double2 v = MODE == 1 ? u[(size_t)row * sx + (size_t)k * sk + c] : u[(size_t)c * sx + (size_t)k * sk + row];
+      w[j >> 2] |= mag8(v.x, v.y, e[(size_t)k * rows + row]) << (8 * (j & 3));
+    }
+    M[((size_t)koff * ngrp * 2 * S) * 32 + i] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
 }
 
 // amp[i] = sum_k part[k][i], i < n (OCEAN_multiplet.f90:1730-1783's sum over k): a CTA
@@ -718,19 +1014,30 @@ SliceFn slice_fn(int mode, int nae) {
   return nae == 4 ? k_slice_gemm<2, 8, 1> : (nae == 8 ? k_slice_gemm<2, 16, 1> : k_slice_gemm<2, 12, 2>);
 }
 inline bool slice_merged(int nae) { return nae <= 8; }
+// bytes of a granule of B in shared memory
+size_t slice_pitch(int nae) {
+  const int C = slice_merged(nae) ? 2 * nae : nae, P = slice_merged(nae) ? 1 : 2;
+  return (size_t)slice_rows(C, P) * 16;
+}
 
 // One contraction: geometry, operand A (digits and exponents) and launch shape.
 struct SliceGemm {
   SliceParams p{};
   uint8_t* A = nullptr;
+  uint8_t* A8 = nullptr;     // magnitudes (k_slice_build_mag)
   int* eA = nullptr;
   int mode = 1, nbox = SL_S, nae = 4, grid = 1;
+  int K = 1;                 // complex products of a sum
   size_t smem = 0;
   size_t a_bytes(int spins) const { return (size_t)spins * p.nk * p.R * 16 * p.G * nbox; }
+  int s8() const { return (K + 31) / 32; }  // steps of 32 K of the magnitudes
+  size_t a8_bytes(int spins) const { return (size_t)spins * p.nk * ((p.rows + 31) / 32) * 32 * 32 * s8(); }
+  size_t b8_bytes() const { return (size_t)(p.bshared ? 1 : p.nk) * nae * 32 * s8(); }
   size_t b_bytes() const { return (size_t)(p.bshared ? 1 : p.nk) * p.Ge * 2 * SL_S * nae * 16; }
 };
 
-// rows and summed index of a contraction of nae columns; the largest K chunk whose
+// rows and summed index of a contraction of nae columns (K complex products, stacked as re
+// and im for band -> x); the largest K chunk whose
 // two B slots and at least four A stages fit in shared memory (16 granules at most
 // for one resident B operand, 12 for streamed ones) with the widest columns, nae_max,
 // that share the A operand: its order depends on the chunks.
@@ -740,6 +1047,8 @@ void slice_plan(SliceGemm* s, int mode, int nae, int nae_max, int nk, int rows, 
   s->mode = mode;
   s->nae = nae;
   s->nbox = mode == 1 ? SL_S : 2 * SL_S;
+  s->K = K;
+  if (mode == 1) K *= 2;
   p.nk = nk;
   p.rows = rows;
   p.nt = (rows + SL_ROWS - 1) / SL_ROWS;
@@ -747,7 +1056,7 @@ void slice_plan(SliceGemm* s, int mode, int nae, int nae_max, int nk, int rows, 
   p.R = (p.nt - 1) * SL_ROWS + p.rl;
   p.G = (K + 15) / 16;
   p.Ge = (p.G + 1) & ~1;
-  const size_t pitch = (size_t)2 * 23 * nae * 16, pitch_max = (size_t)2 * 23 * nae_max * 16;
+  const size_t pitch = slice_pitch(nae), pitch_max = slice_pitch(nae_max);
   const int cap = mode == 1 ? 16 : 12;
   int kc = std::min(cap, p.Ge);
   while (kc > 2 && kc * (2 * pitch_max + 4 * SL_ROWS * 16) > SL_SMEM) kc -= 2;
@@ -803,6 +1112,7 @@ struct SliceLR {
   int nvs = 1;             // most vectors per launch (12 columns)
   SliceGemm g1[3], g2[3];  // band -> x, x -> band of 1, 2, 3 vectors; A is held by [0] and shared
   uint8_t *b1 = nullptr, *b2 = nullptr;
+  uint8_t *m1 = nullptr, *m2 = nullptr;  // magnitudes of the columns
   int *e1 = nullptr, *e2 = nullptr;
   int* mx2 = nullptr;      // exponent maxima of phi' per (k, column)
   int* ex2 = nullptr;      // exponents of phi' per (x, column)
@@ -810,6 +1120,7 @@ struct SliceLR {
   bool mult_ready = false;
   SliceGemm gm1, gm2;
   uint8_t* bm = nullptr;
+  uint8_t* mm = nullptr;
   int* em = nullptr;
   int* mxm = nullptr;
   double2* amp_part = nullptr;  // [k][p][a]
@@ -830,8 +1141,9 @@ void slice_drop_a(ocn_ctx* c) {
   SliceLR* s = c->slice;
   for (SliceGemm* g : {&s->g1[0], &s->g2[0]}) {
     if (g->A) cudaFree(g->A);
+    if (g->A8) cudaFree(g->A8);
     if (g->eA) cudaFree(g->eA);
-    g->A = nullptr;
+    g->A = g->A8 = nullptr;
     g->eA = nullptr;
   }
   s->ready = false;
@@ -842,13 +1154,14 @@ void slice_drop_mult(ocn_ctx* c) {
   SliceLR* s = c->slice;
   for (SliceGemm* g : {&s->gm1, &s->gm2}) {
     if (g->A) cudaFree(g->A);
+    if (g->A8) cudaFree(g->A8);
     if (g->eA) cudaFree(g->eA);
-    g->A = nullptr;
+    g->A = g->A8 = nullptr;
     g->eA = nullptr;
   }
-  for (void* q : {(void*)s->bm, (void*)s->em, (void*)s->mxm, (void*)s->amp_part})
+  for (void* q : {(void*)s->bm, (void*)s->mm, (void*)s->em, (void*)s->mxm, (void*)s->amp_part})
     if (q) cudaFree(q);
-  s->bm = nullptr;
+  s->bm = s->mm = nullptr;
   s->em = nullptr;
   s->mxm = nullptr;
   s->amp_part = nullptr;
@@ -867,7 +1180,9 @@ int slice_build(ocn_ctx* c, const double2* src, size_t sx, size_t sk, int nx, co
   k_slice_build_rows<<<blocks, 256, 0, c->stream>>>(src, sx, sk, nb, g1.p, e1, g1.A, spin * nk);
   k_slice_exp_cols<<<dim3((nb + 31) / 32, nk), dim3(32, 8), 0, c->stream>>>(src, sx, sk, nb, nk, nx, e2);
   k_slice_build_cols<<<blocks, 256, 0, c->stream>>>(src, sx, sk, nx, g2.p, e2, g2.A, spin * nk);
-  c->launches += 4;
+  k_slice_build_mag<1><<<blocks, 256, 0, c->stream>>>(src, sx, sk, nk, nx, nb, e1, reinterpret_cast<uint4*>(g1.A8), spin * nk);
+  k_slice_build_mag<2><<<blocks, 256, 0, c->stream>>>(src, sx, sk, nk, nb, nx, e2, reinterpret_cast<uint4*>(g2.A8), spin * nk);
+  c->launches += 6;
   OCN_CUDA(c, cudaGetLastError());
   return OCN_OK;
 }
@@ -878,8 +1193,9 @@ bool slice_alloc_a(ocn_ctx* c, SliceGemm* g1, SliceGemm* g2, int nx) {
   const int ns = c->nspn;
   size_t fr = 0, tot = 0;
   if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return false;
-  if (g1->a_bytes(ns) + g2->a_bytes(ns) > fr / 4) return false;
+  if (g1->a_bytes(ns) + g2->a_bytes(ns) + g1->a8_bytes(ns) + g2->a8_bytes(ns) > fr / 4) return false;
   if (salloc(c, &g1->A, g1->a_bytes(ns)) || salloc(c, &g2->A, g2->a_bytes(ns)) ||
+      salloc(c, &g1->A8, g1->a8_bytes(ns)) || salloc(c, &g2->A8, g2->a8_bytes(ns)) ||
       salloc(c, &g1->eA, (size_t)ns * c->nk * nx) || salloc(c, &g2->eA, (size_t)ns * c->nk * c->nb)) {
     (void)cudaGetLastError();
     c->err.clear();
@@ -888,9 +1204,19 @@ bool slice_alloc_a(ocn_ctx* c, SliceGemm* g1, SliceGemm* g2, int nx) {
   return true;
 }
 
-// g: the launch's geometry, a: the holder of its A operand
-int slice_launch(ocn_ctx* c, const SliceGemm& g, const SliceGemm& a, const uint8_t* B, const int* eB, double2* phi,
-                 double* part, int spin, int spins) {
+// Where the columns of a contraction come from: psi (band -> x) or f (x -> band).
+struct SliceColumns {
+  const double *pr = nullptr, *pi = nullptr;
+  size_t vstride = 0;
+  const double2* f = nullptr;
+  const int* ex = nullptr;
+};
+
+// The contraction of both spins.  g: the launch's geometry, a: the holder of its A operand; B,
+// M, eB: the columns' digits, magnitudes and exponents; u: element (spin, x, k, n) at
+// spin*us + x*ux + k*uk + n, what the digits of a were built from.
+int slice_contract(ocn_ctx* c, const SliceGemm& g, const SliceGemm& a, const uint8_t* B, const uint8_t* M, const int* eB,
+                   const SliceColumns& col, const double2* u, size_t us, size_t ux, size_t uk, double2* phi, double* part) {
   SliceParams p = g.p;
   p.A = a.A;
   p.eA = a.eA;
@@ -903,13 +1229,31 @@ int slice_launch(ocn_ctx* c, const SliceGemm& g, const SliceGemm& a, const uint8
   p.na = c->na;
   p.nb = c->nb;
   p.err = c->slice->d_err;
-  p.koff = spin * p.nk;
-  p.spin = spins == 2 ? spin : -1;
   p.negate = p.bshared ? 0 : 1;
   p.starve = c->slice->starve;
-  slice_fn(g.mode, g.nae)<<<g.grid, slice_threads(g.nae), g.smem, c->stream>>>(p);
-  ++c->launches;
-  OCN_CUDA(c, cudaGetLastError());
+  p.A8 = reinterpret_cast<const uint4*>(a.A8);
+  p.B8 = reinterpret_cast<const uint2*>(M);
+  p.K = g.K;
+  p.S8 = g.s8();
+  const double rk = std::sqrt((double)g.K);
+  p.sample = std::min(p.S8, (int)std::ceil(6.0 * rk / 32.0));  // ungraded rows: ten times the least sum
+  p.least = (int)std::ceil(std::sqrt(2.0 * SL_CHECK_M * 255.0 * 255.0 + SL_CHECK_K) * rk);
+  p.ux = ux;
+  p.uk = uk;
+  p.pr = col.pr;
+  p.pi = col.pi;
+  p.allow = c->d_allow;
+  p.vstride = col.vstride;
+  p.f = col.f;
+  p.ex = col.ex;
+  for (int sp = 0; sp < c->nspn; ++sp) {
+    p.koff = sp * p.nk;
+    p.spin = c->nspn == 2 ? sp : -1;
+    p.u = u + sp * us;
+    slice_fn(g.mode, g.nae)<<<g.grid, slice_threads(g.nae), g.smem, c->stream>>>(p);
+    ++c->launches;
+    OCN_CUDA(c, cudaGetLastError());
+  }
   return OCN_OK;
 }
 
@@ -924,14 +1268,15 @@ int slice_init(ocn_ctx* c) {
   int rc;
   for (int w = 1; w <= s->nvs; ++w) {
     const int nae = w * c->na, most = s->nvs * c->na;
-    const double cost = 32.0 * c->npsi / 6e12;  // the same splits for every width: results do not depend on it
-    slice_plan(&s->g1[w - 1], 1, nae, most, c->nk, c->nx, 2 * c->nb, c->sm_count, 0.0);
+    const double cost = 32.0 * c->npsi / 6e12;  // the same splits for every width of this context: results do not depend on it
+    slice_plan(&s->g1[w - 1], 1, nae, most, c->nk, c->nx, c->nb, c->sm_count, 0.0);
     slice_plan(&s->g2[w - 1], 2, nae, most, c->nk, c->nb, c->nx, c->sm_count, cost);
     if ((rc = allow_max_smem(c, slice_fn(1, nae))) || (rc = allow_max_smem(c, slice_fn(2, nae)))) return rc;
   }
   const SliceGemm &w1 = s->g1[s->nvs - 1], &w2 = s->g2[s->nvs - 1];
   const size_t cols = (size_t)c->nk * c->na * s->nvs;
   if ((rc = salloc(c, &s->b1, w1.b_bytes())) || (rc = salloc(c, &s->b2, w2.b_bytes())) ||
+      (rc = salloc(c, &s->m1, w1.b8_bytes())) || (rc = salloc(c, &s->m2, w2.b8_bytes())) ||
       (rc = salloc(c, &s->e1, cols)) || (rc = salloc(c, &s->e2, cols)) || (rc = salloc(c, &s->mx2, cols)) ||
       (rc = salloc(c, &s->ex2, (size_t)c->nx * c->na * s->nvs)) ||
       (rc = salloc(c, &s->d_err, 1)))
@@ -950,7 +1295,7 @@ void slice_free(ocn_ctx* c) {
   if (!s) return;
   slice_drop_a(c);
   slice_drop_mult(c);
-  for (void* q : {(void*)s->b1, (void*)s->b2, (void*)s->e1, (void*)s->e2, (void*)s->mx2, (void*)s->ex2, (void*)s->d_err})
+  for (void* q : {(void*)s->b1, (void*)s->b2, (void*)s->m1, (void*)s->m2, (void*)s->e1, (void*)s->e2, (void*)s->mx2, (void*)s->ex2, (void*)s->d_err})
     if (q) cudaFree(q);
   delete s;
   c->slice = nullptr;
@@ -964,7 +1309,7 @@ bool slice_ready(const ocn_ctx* c) { return c->slice && c->slice->ready; }
 int slice_set_bloch(ocn_ctx* c) {
   SliceLR* s = c->slice;
   if (!s) return OCN_OK;
-  if (!(c->digits & 1) || (!s->g1[0].A && !slice_alloc_a(c, &s->g1[0], &s->g2[0], c->nx))) {
+  if (!(c->digits & 1) || c->nx > SL_MAX_SUM || (!s->g1[0].A && !slice_alloc_a(c, &s->g1[0], &s->g2[0], c->nx))) {
     slice_drop_a(c);
     return OCN_OK;
   }
@@ -990,11 +1335,12 @@ int slice_set_mult(ocn_ctx* c) {
   slice_drop_mult(c);
   const int np = c->mult.np;
   if (np == 0 || !(c->digits & 2)) return OCN_OK;
-  slice_plan(&s->gm1, 1, c->na, c->na, c->nk, np, 2 * c->nb, c->sm_count, 0.0);
+  slice_plan(&s->gm1, 1, c->na, c->na, c->nk, np, c->nb, c->sm_count, 0.0);
   slice_plan(&s->gm2, 2, c->na, c->na, c->nk, c->nb, np, c->sm_count, 32.0 * c->npsi / 6e12);
   s->gm2.p.bshared = 1;
   double* parts = nullptr;
-  if (!slice_alloc_a(c, &s->gm1, &s->gm2, np) || salloc(c, &s->bm, s->gm2.b_bytes()) || salloc(c, &s->em, c->na) ||
+  if (!slice_alloc_a(c, &s->gm1, &s->gm2, np) || salloc(c, &s->bm, s->gm2.b_bytes()) ||
+      salloc(c, &s->mm, s->gm2.b8_bytes()) || salloc(c, &s->em, c->na) ||
       salloc(c, &s->mxm, c->na) || salloc(c, &s->amp_part, (size_t)c->nk * np * c->na) ||
       salloc(c, &parts, (size_t)(std::max(c->lr_xsplit_pipe, slice_splits(c)) + s->gm2.p.ks) * c->part_stride)) {
     slice_drop_mult(c);
@@ -1023,20 +1369,25 @@ int slice_prep_psi(ocn_ctx* c, const double* d_pr, const double* d_pi, size_t vs
   const int nae = c->na * nv;
   TimedScope ts(c, T_LR_PREP);
   k_slice_prep_b1<<<c->nk, 256, 0, c->stream>>>(d_pr, d_pi, vstride, c->d_allow, c->nb, c->nk, c->na, nae, s->g1[0].p.Ge,
-                                                slice_merged(nae) ? 1 : 0, s->b1, s->e1, s->mx2);
+                                                slice_merged(nae) ? 1 : 0, s->b1, s->e1, s->mx2, s->m1, s->g1[0].s8());
   ++c->launches;
   OCN_CUDA(c, cudaGetLastError());
   return OCN_OK;
 }
 
 // The multiplet term of the one vector whose operand is in b1, into the d_accpart slices of vector v.
-int slice_mult_apply(ocn_ctx* c, int v) {
+int slice_mult_apply(ocn_ctx* c, const double* d_pr, const double* d_pi, int v) {
   SliceLR* s = c->slice;
   MultDev& m = c->mult;
   TimedScope ts(c, T_MULT);
   int rc;
-  for (int sp = 0; sp < c->nspn; ++sp)
-    if ((rc = slice_launch(c, s->gm1, s->gm1, s->b1, s->e1, s->amp_part, nullptr, sp, c->nspn))) return rc;
+  const size_t nbk = (size_t)c->nb * c->nk;
+  SliceColumns psi, hamp;
+  psi.pr = d_pr;
+  psi.pi = d_pi;
+  hamp.f = m.hamp;
+  if ((rc = slice_contract(c, s->gm1, s->gm1, s->b1, s->m1, s->e1, psi, m.mpc, m.np * nbk, nbk, c->nb, s->amp_part, nullptr)))
+    return rc;
   const int n = m.np * c->na;
   k_slice_amp_reduce<<<(n + 31) / 32, 512, 0, c->stream>>>(s->amp_part, m.amp, c->nk, n);
   ++c->launches;
@@ -1045,22 +1396,23 @@ int slice_mult_apply(ocn_ctx* c, int v) {
   k_slice_col_max<<<1, 512, 0, c->stream>>>(m.hamp, m.np, c->na, s->mxm);
   const int items = s->gm2.p.Ge * c->na * 4;
   k_slice_prep_b2<false><<<dim3((items + 255) / 256, 1), 256, 0, c->stream>>>(m.hamp, nullptr, m.np, c->na, s->gm2.p.Ge,
-                                                                      slice_merged(c->na) ? 1 : 0, s->mxm, s->bm, s->em);
+                                                                      slice_merged(c->na) ? 1 : 0, s->mxm, s->bm, s->em, s->mm, s->gm2.s8());
   c->launches += 2;
   OCN_CUDA(c, cudaGetLastError());
   double* part = c->d_accpart + (size_t)c->lr_xsplit * c->part_stride + (size_t)v * 2 * c->npsi;
-  for (int sp = 0; sp < c->nspn; ++sp)
-    if ((rc = slice_launch(c, s->gm2, s->gm2, s->bm, s->em, nullptr, part, sp, c->nspn))) return rc;
-  return OCN_OK;
+  return slice_contract(c, s->gm2, s->gm2, s->bm, s->mm, s->em, hamp, m.mpc, m.np * nbk, nbk, c->nb, nullptr, part);
 }
 
 // phi[k][x][t] of the nv vectors whose operand is in b1, t = v*Na + a.
-int slice_band_to_x(ocn_ctx* c, double2* phi, int nv) {
+int slice_band_to_x(ocn_ctx* c, const double* d_pr, const double* d_pi, size_t vstride, double2* phi, int nv) {
   SliceLR* s = c->slice;
   TimedScope ts(c, T_LR_GEMM1);
-  for (int sp = 0; sp < c->nspn; ++sp)
-    if (int rc = slice_launch(c, s->g1[nv - 1], s->g1[0], s->b1, s->e1, phi, nullptr, sp, c->nspn)) return rc;
-  return OCN_OK;
+  SliceColumns psi;
+  psi.pr = d_pr;
+  psi.pi = d_pi;
+  psi.vstride = vstride;
+  const size_t sx = (size_t)c->nk * c->nb;
+  return slice_contract(c, s->g1[nv - 1], s->g1[0], s->b1, s->m1, s->e1, psi, c->d_u, c->nx * sx, sx, c->nb, phi, nullptr);
 }
 
 // Exponents per (x, t) and maxima per (k, t) that fx_transform leaves with phi' in
@@ -1078,23 +1430,25 @@ int slice_x_to_band(ocn_ctx* c, const double2* phi, int nv, int v0, bool integer
   const int nae = c->na * nv;
   {
     TimedScope ts(c, T_LR_PREP);
-    const int items = g.p.Ge * nae * 4, merged = slice_merged(nae) ? 1 : 0;
+    const int items = g.p.Ge * nae * 4, merged = slice_merged(nae) ? 1 : 0, s8 = g.s8();
     const dim3 grid((items + 255) / 256, c->nk);
     if (integers) {
-      k_slice_prep_b2<true><<<grid, 256, 0, c->stream>>>(phi, s->ex2, c->nx, nae, g.p.Ge, merged, s->mx2, s->b2, s->e2);
+      k_slice_prep_b2<true><<<grid, 256, 0, c->stream>>>(phi, s->ex2, c->nx, nae, g.p.Ge, merged, s->mx2, s->b2, s->e2, s->m2, s8);
     } else {
       k_slice_col_max<<<c->nk, 512, 0, c->stream>>>(phi, c->nx, nae, s->mx2);
       ++c->launches;
-      k_slice_prep_b2<false><<<grid, 256, 0, c->stream>>>(phi, nullptr, c->nx, nae, g.p.Ge, merged, s->mx2, s->b2, s->e2);
+      k_slice_prep_b2<false><<<grid, 256, 0, c->stream>>>(phi, nullptr, c->nx, nae, g.p.Ge, merged, s->mx2, s->b2, s->e2, s->m2, s8);
     }
     ++c->launches;
     OCN_CUDA(c, cudaGetLastError());
   }
   TimedScope ts(c, T_LR_GEMM2);
-  for (int sp = 0; sp < c->nspn; ++sp)
-    if (int rc = slice_launch(c, g, s->g2[0], s->b2, s->e2, nullptr, c->d_accpart + (size_t)v0 * 2 * c->npsi, sp, c->nspn))
-      return rc;
-  return OCN_OK;
+  SliceColumns col;
+  col.f = phi;
+  col.ex = integers ? s->ex2 : nullptr;
+  const size_t sx = (size_t)c->nk * c->nb;
+  return slice_contract(c, g, s->g2[0], s->b2, s->m2, s->e2, col, c->d_u, c->nx * sx, sx, c->nb, nullptr,
+                        c->d_accpart + (size_t)v0 * 2 * c->npsi);
 }
 
 int slice_set_starve(ocn_ctx* c, int on) {
