@@ -10,6 +10,8 @@
 
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 namespace ocn {
 
 constexpr int FX_NAN = 0x40000000;  // block exponent of data that hold an Inf or NaN
@@ -188,5 +190,56 @@ __device__ __forceinline__ unsigned fx_or(const cfx& a) {
 }
 // Bits of the largest magnitude from the OR of the high words (an upper bound, 32 at least).
 __device__ __forceinline__ int fx_nbits(unsigned orw) { return 64 - __clz((int)orw); }
+
+// ---- passes of a block of transforms, four of them side by side (transform = lane mod 4)
+// f(integral_constant of the line length): NC, or n (1..8) when NC is 0
+template <int NC, class F>
+__device__ __forceinline__ void fx_len(int n, F f) {
+  if constexpr (NC > 0) {
+    f(std::integral_constant<int, NC>{});
+  } else {
+    switch (n) {
+      case 1: f(std::integral_constant<int, 1>{}); break;
+      case 2: f(std::integral_constant<int, 2>{}); break;
+      case 3: f(std::integral_constant<int, 3>{}); break;
+      case 4: f(std::integral_constant<int, 4>{}); break;
+      case 5: f(std::integral_constant<int, 5>{}); break;
+      case 6: f(std::integral_constant<int, 6>{}); break;
+      case 7: f(std::integral_constant<int, 7>{}); break;
+      case 8: f(std::integral_constant<int, 8>{}); break;
+    }
+  }
+}
+
+template <int N>
+__device__ __forceinline__ unsigned fx_or_line(const cfx (&v)[N]) {
+  unsigned m = 0;
+#pragma unroll
+  for (int j = 0; j < N; ++j) m |= fx_or(v[j]);
+  return m;
+}
+// the four transforms' words of a pass: OR over the lanes of each class (lane mod 4)
+__device__ __forceinline__ void fx_track(unsigned m, unsigned* word) {
+  for (int o = 4; o < 32; o <<= 1) m |= __shfl_xor_sync(0xffffffffu, m, o);
+  const int lane = threadIdx.x & 31;
+  if (lane < 4) atomicOr(&word[lane], m);
+}
+// right shift that leaves 58 bits
+__device__ __forceinline__ int fx_shift(unsigned orw) { return max(0, fx_nbits(orw) - FX_BITS); }
+
+template <int N>
+__device__ __forceinline__ void fx_load(cfx (&v)[N], const cfx* p, int st, int s) {
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    v[j] = p[j * st];
+    v[j].x >>= s;
+    v[j].y >>= s;
+  }
+}
+template <int N>
+__device__ __forceinline__ void fx_store(const cfx (&v)[N], cfx* p, int st) {
+#pragma unroll
+  for (int j = 0; j < N; ++j) p[j * st] = v[j];
+}
 
 }  // namespace ocn

@@ -52,55 +52,6 @@ struct FxParams {
   int n1, n2, n3;
 };
 
-template <int NC, class F>
-__device__ __forceinline__ void on_len(int n, F f) {
-  if constexpr (NC > 0) {
-    f(std::integral_constant<int, NC>{});
-  } else {
-    switch (n) {
-      case 1: f(std::integral_constant<int, 1>{}); break;
-      case 2: f(std::integral_constant<int, 2>{}); break;
-      case 3: f(std::integral_constant<int, 3>{}); break;
-      case 4: f(std::integral_constant<int, 4>{}); break;
-      case 5: f(std::integral_constant<int, 5>{}); break;
-      case 6: f(std::integral_constant<int, 6>{}); break;
-      case 7: f(std::integral_constant<int, 7>{}); break;
-      case 8: f(std::integral_constant<int, 8>{}); break;
-    }
-  }
-}
-
-template <int N>
-__device__ __forceinline__ unsigned or_line(const cfx (&v)[N]) {
-  unsigned m = 0;
-#pragma unroll
-  for (int j = 0; j < N; ++j) m |= fx_or(v[j]);
-  return m;
-}
-// the four transforms' words of a pass: OR over the lanes of each class (lane mod 4)
-__device__ __forceinline__ void track(unsigned m, unsigned* word) {
-  for (int o = 4; o < 32; o <<= 1) m |= __shfl_xor_sync(0xffffffffu, m, o);
-  const int lane = threadIdx.x & 31;
-  if (lane < 4) atomicOr(&word[lane], m);
-}
-// right shift that leaves 58 bits
-__device__ __forceinline__ int pass_shift(unsigned orw) { return max(0, fx_nbits(orw) - FX_BITS); }
-
-template <int N>
-__device__ __forceinline__ void load_shift(cfx (&v)[N], const cfx* p, int st, int s) {
-#pragma unroll
-  for (int j = 0; j < N; ++j) {
-    v[j] = p[j * st];
-    v[j].x >>= s;
-    v[j].y >>= s;
-  }
-}
-template <int N>
-__device__ __forceinline__ void store_line(const cfx (&v)[N], cfx* p, int st) {
-#pragma unroll
-  for (int j = 0; j < N; ++j) p[j * st] = v[j];
-}
-
 // N1, N2, N3: mesh extents known at compile time (0: from p).  INT: phi' stays integers
 // (re, im as 64-bit words in phi's place) for the digit operand of the next contraction.
 template <int N1, int N2, int N3, bool INT>
@@ -124,7 +75,7 @@ __global__ void __launch_bounds__(256, 3) k_fx_transform(const FxParams p) {
   const bool on1 = r < n23, on2 = r < n1 * n3, on3 = r < n1 * n2;
   int e0 = 0;
 
-  on_len<N1>(n1, [&](auto ic) {  // k1 backward, from HBM
+  fx_len<N1>(n1, [&](auto ic) {  // k1 backward, from HBM
     constexpr int N = decltype(ic)::value;
     double2 in[N];
     unsigned m = 0;
@@ -144,33 +95,33 @@ __global__ void __launch_bounds__(256, 3) k_fx_transform(const FxParams p) {
 #pragma unroll
       for (int j = 0; j < N; ++j) v[j] = {fx_from<FX_BITS>(in[j].x, e0), fx_from<FX_BITS>(in[j].y, e0)};
       fx_dft<N>(v);
-      store_line<N>(v, q1, n2 * P3);
-      m = or_line<N>(v);
+      fx_store<N>(v, q1, n2 * P3);
+      m = fx_or_line<N>(v);
     }
-    track(m, mx[1]);
+    fx_track(m, mx[1]);
   });
   __syncthreads();
-  on_len<N2>(n2, [&](auto ic) {  // k2 backward
+  fx_len<N2>(n2, [&](auto ic) {  // k2 backward
     constexpr int N = decltype(ic)::value;
     unsigned m = 0;
     if (on2) {
       cfx v[N];
-      load_shift<N>(v, q2, P3, pass_shift(mx[1][t]));
+      fx_load<N>(v, q2, P3, fx_shift(mx[1][t]));
       fx_dft<N>(v);
-      store_line<N>(v, q2, P3);
-      m = or_line<N>(v);
+      fx_store<N>(v, q2, P3);
+      m = fx_or_line<N>(v);
     }
-    track(m, mx[2]);
+    fx_track(m, mx[2]);
   });
   __syncthreads();
   int s3 = 0;
-  on_len<N3>(n3, [&](auto ic) {  // k3 backward, W / Nk, k3 forward (re and im exchanged from here on)
+  fx_len<N3>(n3, [&](auto ic) {  // k3 backward, W / Nk, k3 forward (re and im exchanged from here on)
     constexpr int N = decltype(ic)::value;
     cfx v[N];
     unsigned m = 0;
     if (on3) {
       const long long* w = p.W + (size_t)x * n1 * n23 + r * n3;
-      load_shift<N>(v, q3, 1, pass_shift(mx[2][t]));
+      fx_load<N>(v, q3, 1, fx_shift(mx[2][t]));
       fx_dft<N>(v);
 #pragma unroll
       for (int j = 0; j < N; ++j) {
@@ -178,9 +129,9 @@ __global__ void __launch_bounds__(256, 3) k_fx_transform(const FxParams p) {
         const int wh = (int)(wv >> 31), wl = (int)(wv & 0x7fffffff);
         v[j] = {fx_mul(v[j].y, wh, wl), fx_mul(v[j].x, wh, wl)};
       }
-      m = or_line<N>(v);
+      m = fx_or_line<N>(v);
     }
-    track(m, mx[3]);
+    fx_track(m, mx[3]);
     __syncthreads();
     s3 = fx_nbits(mx[3][t]) - FX_BITS;
     m = 0;
@@ -189,34 +140,34 @@ __global__ void __launch_bounds__(256, 3) k_fx_transform(const FxParams p) {
 #pragma unroll
       for (int j = 0; j < N; ++j) v[j] = {(long long)((unsigned long long)v[j].x << ls) >> rs, (long long)((unsigned long long)v[j].y << ls) >> rs};
       fx_dft<N>(v);
-      store_line<N>(v, q3, 1);
-      m = or_line<N>(v);
+      fx_store<N>(v, q3, 1);
+      m = fx_or_line<N>(v);
     }
-    track(m, mx[4]);
+    fx_track(m, mx[4]);
   });
   __syncthreads();
-  on_len<N2>(n2, [&](auto ic) {  // k2 forward
+  fx_len<N2>(n2, [&](auto ic) {  // k2 forward
     constexpr int N = decltype(ic)::value;
     unsigned m = 0;
     if (on2) {
       cfx v[N];
-      load_shift<N>(v, q2, P3, pass_shift(mx[4][t]));
+      fx_load<N>(v, q2, P3, fx_shift(mx[4][t]));
       fx_dft<N>(v);
-      store_line<N>(v, q2, P3);
-      m = or_line<N>(v);
+      fx_store<N>(v, q2, P3);
+      m = fx_or_line<N>(v);
     }
-    track(m, mx[5]);
+    fx_track(m, mx[5]);
   });
   __syncthreads();
-  on_len<N1>(n1, [&](auto ic) {  // k1 forward, to HBM
+  fx_len<N1>(n1, [&](auto ic) {  // k1 forward, to HBM
     constexpr int N = decltype(ic)::value;
     if (!on1) return;
     cfx v[N];
-    const int s5 = pass_shift(mx[5][t]), we = p.we[x];
-    load_shift<N>(v, q1, n2 * P3, s5);
+    const int s5 = fx_shift(mx[5][t]), we = p.we[x];
+    fx_load<N>(v, q1, n2 * P3, s5);
     fx_dft<N>(v);
     const bool bad = e0 == FX_NAN || we == FX_NAN;
-    const int e = e0 - FX_BITS + we + pass_shift(mx[1][t]) + pass_shift(mx[2][t]) + s3 + pass_shift(mx[4][t]) + s5;
+    const int e = e0 - FX_BITS + we + fx_shift(mx[1][t]) + fx_shift(mx[2][t]) + s3 + fx_shift(mx[4][t]) + s5;
     if (INT && r == 0) p.ex[(size_t)x * p.ld + tg] = bad ? FX_NAN : e;
 #pragma unroll
     for (int j = 0; j < N; ++j) {

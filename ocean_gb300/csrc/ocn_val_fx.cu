@@ -65,50 +65,6 @@ struct VfParams {
   int n1, n2, n3;
 };
 
-template <int NC, class F>
-__device__ __forceinline__ void vf_len(int n, F f) {
-  if constexpr (NC > 0) {
-    f(std::integral_constant<int, NC>{});
-  } else {
-    switch (n) {
-      case 1: f(std::integral_constant<int, 1>{}); break;
-      case 2: f(std::integral_constant<int, 2>{}); break;
-      case 3: f(std::integral_constant<int, 3>{}); break;
-      case 4: f(std::integral_constant<int, 4>{}); break;
-      case 5: f(std::integral_constant<int, 5>{}); break;
-      case 6: f(std::integral_constant<int, 6>{}); break;
-      case 7: f(std::integral_constant<int, 7>{}); break;
-      case 8: f(std::integral_constant<int, 8>{}); break;
-    }
-  }
-}
-template <int N>
-__device__ __forceinline__ unsigned vf_or(const cfx (&v)[N]) {
-  unsigned m = 0;
-#pragma unroll
-  for (int j = 0; j < N; ++j) m |= fx_or(v[j]);
-  return m;
-}
-__device__ __forceinline__ void vf_track(unsigned m, unsigned* word) {
-  for (int o = 4; o < 32; o <<= 1) m |= __shfl_xor_sync(0xffffffffu, m, o);
-  const int lane = threadIdx.x & 31;
-  if (lane < 4) atomicOr(&word[lane], m);
-}
-__device__ __forceinline__ int vf_right(unsigned orw) { return max(0, fx_nbits(orw) - FX_BITS); }
-template <int N>
-__device__ __forceinline__ void vf_load(cfx (&v)[N], const cfx* p, int st, int s) {
-#pragma unroll
-  for (int j = 0; j < N; ++j) {
-    v[j] = p[j * st];
-    v[j].x >>= s;
-    v[j].y >>= s;
-  }
-}
-template <int N>
-__device__ __forceinline__ void vf_store(const cfx (&v)[N], cfx* p, int st) {
-#pragma unroll
-  for (int j = 0; j < N; ++j) p[j * st] = v[j];
-}
 // by 2^-s, s of either sign: mostly to the right, so the left shift is a warp-uniform detour
 template <int N>
 __device__ __forceinline__ void vf_scale(cfx (&v)[N], int s) {
@@ -194,7 +150,7 @@ __global__ void __launch_bounds__(vf_cta(N1), vf_min_ctas(N1)) k_val_ladder_fx(c
       asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(p.L + ((size_t)yl * p.nx + x) * nk + k)
                    : "memory");
     }
-    vf_len<N1>(n1, [&](auto ic) {  // T on the k1 lines, forward along k1 (re and im exchanged)
+    fx_len<N1>(n1, [&](auto ic) {  // T on the k1 lines, forward along k1 (re and im exchanged)
       constexpr int N = decltype(ic)::value;
       cfx v[N];
       unsigned m = 0;
@@ -223,42 +179,42 @@ __global__ void __launch_bounds__(vf_cta(N1), vf_min_ctas(N1)) k_val_ladder_fx(c
           }
           v[j] = {hp - hn + ((mp - mn) >> VF_LOW), hr + (mr >> VF_LOW)};
         }
-        m = vf_or<N>(v);
+        m = fx_or_line<N>(v);
       }
-      vf_track(m, mx[0]);
+      fx_track(m, mx[0]);
       __syncthreads();
       m = 0;
       if (on1) {
-        vf_scale<N>(v, vf_right(mx[0][t]));  // (bits below T's last do not exist)
+        vf_scale<N>(v, fx_shift(mx[0][t]));  // (bits below T's last do not exist)
         fx_dft<N>(v);
-        vf_store<N>(v, q1, n2 * P3);
-        m = vf_or<N>(v);
+        fx_store<N>(v, q1, n2 * P3);
+        m = fx_or_line<N>(v);
       }
-      vf_track(m, mx[1]);
+      fx_track(m, mx[1]);
     });
     if (threadIdx.x < 32) mxs[par ^ 1][threadIdx.x >> 2][threadIdx.x & 3] = 0;  // the other set, last read a tile ago
     __syncthreads();
-    vf_len<N2>(n2, [&](auto ic) {
+    fx_len<N2>(n2, [&](auto ic) {
       constexpr int N = decltype(ic)::value;
       unsigned m = 0;
       if (on2) {
         cfx v[N];
-        vf_load<N>(v, q2, P3, vf_right(mx[1][t]));
+        fx_load<N>(v, q2, P3, fx_shift(mx[1][t]));
         fx_dft<N>(v);
-        vf_store<N>(v, q2, P3);
-        m = vf_or<N>(v);
+        fx_store<N>(v, q2, P3);
+        m = fx_or_line<N>(v);
       }
-      vf_track(m, mx[2]);
+      fx_track(m, mx[2]);
     });
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    vf_len<N3>(n3, [&](auto ic) {  // forward along k3, ladder / Nk, backward along k3
+    fx_len<N3>(n3, [&](auto ic) {  // forward along k3, ladder / Nk, backward along k3
       constexpr int N = decltype(ic)::value;
       cfx v[N];
       unsigned m = 0;
       if (on3) {
         const long long* w = Ls + 4 * r + t;
-        vf_load<N>(v, q3, 1, vf_right(mx[2][t]));
+        fx_load<N>(v, q3, 1, fx_shift(mx[2][t]));
         fx_dft<N>(v);
 #pragma unroll
         for (int j = 0; j < N; ++j) {
@@ -266,49 +222,49 @@ __global__ void __launch_bounds__(vf_cta(N1), vf_min_ctas(N1)) k_val_ladder_fx(c
           const int wh = (int)(wv >> 31), wl = (int)(wv & 0x7fffffff);
           v[j] = {fx_mul(v[j].y, wh, wl), fx_mul(v[j].x, wh, wl)};
         }
-        m = vf_or<N>(v);
+        m = fx_or_line<N>(v);
       }
-      vf_track(m, mx[3]);
+      fx_track(m, mx[3]);
       __syncthreads();
       m = 0;
       if (on3) {
         vf_scale<N>(v, fx_nbits(mx[3][t]) - FX_BITS);
         fx_dft<N>(v);
-        vf_store<N>(v, q3, 1);
-        m = vf_or<N>(v);
+        fx_store<N>(v, q3, 1);
+        m = fx_or_line<N>(v);
       }
-      vf_track(m, mx[4]);
+      fx_track(m, mx[4]);
     });
     __syncthreads();
-    vf_len<N2>(n2, [&](auto ic) {
+    fx_len<N2>(n2, [&](auto ic) {
       constexpr int N = decltype(ic)::value;
       unsigned m = 0;
       if (on2) {
         cfx v[N];
-        vf_load<N>(v, q2, P3, vf_right(mx[4][t]));
+        fx_load<N>(v, q2, P3, fx_shift(mx[4][t]));
         fx_dft<N>(v);
-        vf_store<N>(v, q2, P3);
-        m = vf_or<N>(v);
+        fx_store<N>(v, q2, P3);
+        m = fx_or_line<N>(v);
       }
-      vf_track(m, mx[5]);
+      fx_track(m, mx[5]);
     });
     __syncthreads();
     int etop;
-    vf_len<N1>(n1, [&](auto ic) {  // backward along k1, then one scale for the four y
+    fx_len<N1>(n1, [&](auto ic) {  // backward along k1, then one scale for the four y
       constexpr int N = decltype(ic)::value;
       cfx v[N];
       unsigned m = 0;
-      const int s5 = vf_right(mx[5][t]);
+      const int s5 = fx_shift(mx[5][t]);
       if (on1) {
-        vf_load<N>(v, q1, n2 * P3, s5);
+        fx_load<N>(v, q1, n2 * P3, s5);
         fx_dft<N>(v);
-        m = vf_or<N>(v);
+        m = fx_or_line<N>(v);
       }
-      vf_track(m, mx[6]);
+      fx_track(m, mx[6]);
       __syncthreads();
       // T' val = int 2^e (val int) 2^-57
-      const int e = eA + 2 * eV + eL - 2 * VF_FRAC + 2 * VF_LOW + vf_right(mx[0][t]) + vf_right(mx[1][t]) +
-                    vf_right(mx[2][t]) + (fx_nbits(mx[3][t]) - FX_BITS) + vf_right(mx[4][t]) + s5;
+      const int e = eA + 2 * eV + eL - 2 * VF_FRAC + 2 * VF_LOW + fx_shift(mx[0][t]) + fx_shift(mx[1][t]) +
+                    fx_shift(mx[2][t]) + (fx_nbits(mx[3][t]) - FX_BITS) + fx_shift(mx[4][t]) + s5;
       const bool fin = eA != FX_NAN && eV != FX_NAN && eL != FX_NAN;
       etop = ony && fin ? e + fx_nbits(mx[6][t]) : -(1 << 28);
       etop = max(etop, __shfl_xor_sync(0xffffffffu, etop, 1));
