@@ -371,13 +371,12 @@ bool fx_supported(const ocn_ctx* c);
 // phi[k][x][t] in place: binary64 (ex, mx null) or integers with exponents ex[x][t], maxima mx[k][t]
 int fx_transform(ocn_ctx* c, double2* phi, int nt, int* ex, int* mx);
 
-// ---- FP64 direct term of the valence action in 64-bit fixed point (ocn_val_fx.cu)
+// ---- FP64 direct term of the valence action, transforms in 64-bit fixed point (ocn_val_fx.cu)
 bool val_fx_supported(const int kmesh[3], int nv, size_t smem_optin);
 cudaError_t val_fx_plan(const int kmesh[3], int nv, size_t smem_optin, int* per_sm);
-void val_fx_states(const double2* val, int nv, int nk, int nx, void* V, int* eV, cudaStream_t s);
 void val_fx_ladder(double* lad, size_t rows, int nk, int* eL, int sm_count, cudaStream_t s);
-void val_fx_apply(const int kmesh[3], int nv, int nx, int yper, int ysplit, const double2* A, const void* V,
-                  const int* eV, const void* lad, const int* eL, double2* Bp, cudaStream_t s);
+void val_fx_apply(const int kmesh[3], int nv, int nx, int yper, int ysplit, const double2* A, const double2* V,
+                  const void* lad, const int* eL, double2* Bp, cudaStream_t s);
 
 // ---- FP64 contractions on the tensor cores (ocn_slice.cu)
 int slice_init(ocn_ctx* c);        // geometry and vector-side buffers

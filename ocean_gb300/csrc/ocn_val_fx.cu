@@ -1,28 +1,28 @@
-// ocn_val_fx.cu -- the FP64 direct term of the valence action in 64-bit block
-// fixed point (OCEAN_ladder.f90:155-1004; see ocn_valence.cu for the action):
+// ocn_val_fx.cu -- the FP64 direct term of the valence action (OCEAN_ladder.f90:155-1004;
+// see ocn_valence.cu for the action):
 //
 //   T(y,k)   = sum_v A(x,v,k) conj(val(y,v,k))
 //   T'(y,.)  = FFT_bwd[ ladder(.,x,y) o FFT_fwd[T(y,.)] ] / Nk
 //   B(x,v,k) += sum_y T'(y,k) val(y,v,k)
 //
-// for k-meshes of 1..8 points per axis and up to 8 valence bands.  On the FP64 pipe
-// (2 operations per clock and SM) the kernel is bound by it at any layout.  A, val, the ladder rows and each T have one
-// scale, so products are formed from two 28/29-bit halves with 32x32->64 integer
-// multiply-adds (high and middle partial sums; what is dropped is below 2^-58 of the
-// largest product) and the transforms on integers (ocn_fixed.cuh, as
-// ocn_fixfft.cu: shifted to 58 bits before every pass).  The sum over y is exact
-// within a tile of four y and added in binary64 across tiles.
+// for k-meshes of 1..8 points per axis and up to 8 valence bands, with the products in
+// binary64 and the transforms on 64-bit integers (block fixed point, ocn_fixed.cuh, as
+// ocn_fixfft.cu: shifted to 58 bits before every pass).  GB300 issues 2 FP64 operations per
+// clock and SM; a transform mixes the elements of a block, so its error is relative to the
+// block's largest element in any arithmetic and 58 bits hold more than binary64, while the
+// products are not: with the products on integers as well, A and val at 57 bits of the
+// largest element of a point, the sums lost accuracy wherever the two were graded
+// oppositely over the bands or T' and val over y.
 //
-// Measured per action, 4 bands: 6^3 k / 7^3 x 9.37 -> 1.27 ms, 8^3 k / 10^3 x 84.7 ->
-// 19.7 ms, 7x5x3 k / 210 x (3 bands, extents at run time) 1.96 -> 0.62 ms.  Bound by
-// integer issue and the latency of the val rows from L2 (1.6 instructions per clock;
-// 12 multiply-adds per complex product in T and again in B, about 700 instructions
-// per k-point and pair).
+// Measured per action, 4 bands: 6^3 k / 7^3 x 9.37 ms with everything on the FP64 pipe, 1.86 ms
+// now (1.27 with the products on integers); 8^3 k / 10^3 x 84.7, 32.0 (19.7); 7x5x3 k / 210 x
+// (3 bands, extents at run time) 1.96, 0.75 (0.62).  Bound by the FP64 pipe: the 32 multiply-adds
+// per k-point and pair take 1.39 of the 1.86 ms; the transforms' integers run beside them.
 //
 // One CTA per x-point and y-range.  A tile of four y is processed by 4 lanes per
 // line (t = lane mod 4 is the y): T is built on the k1 lines, transformed along
-// k1, k2, k3, multiplied, transformed back, brought to one scale over the tile, and
-// the B sums run with one thread per (k1 line, v), whose sums stay in registers.
+// k1, k2, k3, multiplied, transformed back, and the B sums run with one thread per
+// (k1 line, v).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -35,29 +35,12 @@ namespace ocn {
 
 namespace {
 
-constexpr int VF_FRAC = 57;  // A and val: |int| < 2^57 = 29-bit high and 28-bit low halves
-constexpr int VF_LOW = 28;
-constexpr int VF_HEAD = 2 * 8 * 4 * 4 + 64;  // shared words before A: two sets of pass maxima, block words
+constexpr int VF_HEAD = 2 * 8 * 4 * 4;  // shared words before A: two sets of pass maxima
 constexpr int VF_MAX_NV = 8;
-
-__device__ __forceinline__ int4 vf_split(long long x, long long y) {
-  constexpr long long mask = (1ll << VF_LOW) - 1;
-  return make_int4((int)(x >> VF_LOW), (int)(x & mask), (int)(y >> VF_LOW), (int)(y & mask));
-}
-__device__ __forceinline__ void mad(long long& s, int a, int b) { s += (long long)a * b; }
-
-// (h 2^28 + m) 2^e, |h|, |m| < 2^61: as many of the low bits as fit in 62 go along
-__device__ __forceinline__ double vf_value(long long h, long long m, int e) {
-  h += m >> VF_LOW;
-  const int ml = (int)(m & ((1ll << VF_LOW) - 1));
-  const int k = min(max(__clzll(h ^ (h >> 63)) - 2, 0), VF_LOW);
-  return fx_to_double((long long)((unsigned long long)h << k) + (ml >> (VF_LOW - k)), e + VF_LOW - k);
-}
 
 struct VfParams {
   const double2* A;     // [x][v][k]
-  const int4* V;        // [y][v][k] split halves (re high, low, im high, low)
-  const int* eV;        // [y]
+  const double2* V;     // [y][v][k]
   const long long* L;   // [y][x][k]: ladder / Nk = L 2^(eL - 62)
   const int* eL;        // [y][x]
   double2* Bp;          // [ys][k][v][x]
@@ -92,29 +75,17 @@ __global__ void __launch_bounds__(vf_cta(N1), vf_min_ctas(N1)) k_val_ladder_fx(c
   constexpr int NA = N1 ? N1 : 8;
   extern __shared__ __align__(16) unsigned char vfsm[];
   unsigned (*mxs)[8][4] = reinterpret_cast<unsigned (*)[8][4]>(vfsm);
-  unsigned* blk = reinterpret_cast<unsigned*>(vfsm + 256);
   const int n1 = N1 ? N1 : p.n1, n2 = N2 ? N2 : p.n2, n3 = N3 ? N3 : p.n3;
   const int n23 = n2 * n3, nk = n1 * n23, nv = NV ? NV : p.nv;
   const int P3 = n3 | 1, slab = (n1 * n2 * P3 + 7) / 8 * 8 + 2;
-  int4* As = reinterpret_cast<int4*>(vfsm + VF_HEAD);
+  double2* As = reinterpret_cast<double2*>(vfsm + VF_HEAD);
   cfx* buf = reinterpret_cast<cfx*>(As + nv * nk);
   long long* Ls = reinterpret_cast<long long*>(buf + 4 * slab);  // ladder of the tile, [j][k3 line][y]
   const int x = blockIdx.x, ybeg = blockIdx.y * p.yper, yend = min(p.nx, ybeg + p.yper);
   const int t = threadIdx.x & 3, r = threadIdx.x >> 2;
   for (int i = threadIdx.x; i < 64; i += blockDim.x) reinterpret_cast<unsigned*>(vfsm)[i] = 0;
-  if (threadIdx.x == 0) *blk = 0;
-  __syncthreads();
   const double2* Ax = p.A + (size_t)x * nv * nk;
-  {
-    unsigned m = 0;
-    for (int e = threadIdx.x; e < nv * nk; e += blockDim.x) m = max(m, max(fx_mag(Ax[e].x), fx_mag(Ax[e].y)));
-    m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0) atomicMax(blk, m);
-  }
-  __syncthreads();
-  const int eA = fx_exp(*blk);
-  for (int e = threadIdx.x; e < nv * nk; e += blockDim.x)
-    As[e] = vf_split(fx_from<VF_FRAC>(Ax[e].x, eA), fx_from<VF_FRAC>(Ax[e].y, eA));
+  for (int e = threadIdx.x; e < nv * nk; e += blockDim.x) As[e] = Ax[e];
 
   cfx* bt = buf + t * slab;
   cfx* q1 = bt + (r / n3) * P3 + r % n3;
@@ -133,7 +104,6 @@ __global__ void __launch_bounds__(vf_cta(N1), vf_min_ctas(N1)) k_val_ladder_fx(c
 #pragma unroll
       for (int j = 0; j < NA; ++j) acc[q][j] = make_double2(0.0, 0.0);
   }
-  bool bad = eA == FX_NAN;
   __syncthreads();
 
   int par = 0;
@@ -141,7 +111,8 @@ __global__ void __launch_bounds__(vf_cta(N1), vf_min_ctas(N1)) k_val_ladder_fx(c
     const int y = y0 + t;
     const bool ony = y < yend;
     const int yy = ony ? y : y0;  // padding lanes read a valid row and are left out
-    const int eV = p.eV[yy], eL = p.eL[(size_t)yy * p.nx + x];
+    const int eL = p.eL[(size_t)yy * p.nx + x];
+    int e0 = 0;  // |T| < 2^e0
     unsigned (*mx)[4] = mxs[par];
     // the tile's ladder rows travel while T is built and transformed
     for (int i = threadIdx.x; i < 4 * nk; i += blockDim.x) {
@@ -152,40 +123,36 @@ __global__ void __launch_bounds__(vf_cta(N1), vf_min_ctas(N1)) k_val_ladder_fx(c
     }
     fx_len<N1>(n1, [&](auto ic) {  // T on the k1 lines, forward along k1 (re and im exchanged)
       constexpr int N = decltype(ic)::value;
-      cfx v[N];
+      double2 T[N];
       unsigned m = 0;
       if (on1) {
-        const int4* Vy = p.V + (size_t)yy * nv * nk + r;
-        const int4* Ar = As + r;
+        const double2* Vy = p.V + (size_t)yy * nv * nk + r;
+        const double2* Ar = As + r;
 #pragma unroll
         for (int j = 0; j < N; ++j) {
-          long long hr = 0, mr = 0, hp = 0, mp = 0, hn = 0, mn = 0;  // re, im: positive and negative products
+          double re = 0.0, im = 0.0;
 #pragma unroll
           for (int vv = 0; vv < (NV ? NV : VF_MAX_NV); ++vv) {
             if (NV == 0 && vv >= nv) break;
-            const int4 b = __ldg(Vy + vv * nk + j * n23), a = Ar[vv * nk + j * n23];
-            mad(hr, a.x, b.x);
-            mad(hr, a.z, b.z);
-            mad(mr, a.x, b.y);
-            mad(mr, a.y, b.x);
-            mad(mr, a.z, b.w);
-            mad(mr, a.w, b.z);
-            mad(hp, a.z, b.x);
-            mad(hn, a.x, b.z);
-            mad(mp, a.z, b.y);
-            mad(mp, a.w, b.x);
-            mad(mn, a.x, b.w);
-            mad(mn, a.y, b.z);
+            const double2 b = __ldg(Vy + vv * nk + j * n23), a = Ar[vv * nk + j * n23];
+            re = __fma_rn(a.x, b.x, re);
+            im = __fma_rn(a.y, b.x, im);
+            re = __fma_rn(a.y, b.y, re);
+            im = __fma_rn(-a.x, b.y, im);
           }
-          v[j] = {hp - hn + ((mp - mn) >> VF_LOW), hr + (mr >> VF_LOW)};
+          T[j] = make_double2(re, im);
+          m = max(m, max(fx_mag(re), fx_mag(im)));
         }
-        m = fx_or_line<N>(v);
       }
-      fx_track(m, mx[0]);
+      for (int o = 4; o < 32; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+      if ((threadIdx.x & 31) < 4) atomicMax(&mx[0][threadIdx.x & 3], m);
       __syncthreads();
+      e0 = fx_exp(mx[0][t]);
       m = 0;
       if (on1) {
-        vf_scale<N>(v, fx_shift(mx[0][t]));  // (bits below T's last do not exist)
+        cfx v[N];
+#pragma unroll
+        for (int j = 0; j < N; ++j) v[j] = {fx_from<FX_BITS>(T[j].y, e0), fx_from<FX_BITS>(T[j].x, e0)};
         fx_dft<N>(v);
         fx_store<N>(v, q1, n2 * P3);
         m = fx_or_line<N>(v);
@@ -249,70 +216,49 @@ __global__ void __launch_bounds__(vf_cta(N1), vf_min_ctas(N1)) k_val_ladder_fx(c
       fx_track(m, mx[5]);
     });
     __syncthreads();
-    int etop;
-    fx_len<N1>(n1, [&](auto ic) {  // backward along k1, then one scale for the four y
+    fx_len<N1>(n1, [&](auto ic) {  // backward along k1, to binary64
       constexpr int N = decltype(ic)::value;
+      if (!on1) return;
       cfx v[N];
-      unsigned m = 0;
       const int s5 = fx_shift(mx[5][t]);
-      if (on1) {
-        fx_load<N>(v, q1, n2 * P3, s5);
-        fx_dft<N>(v);
-        m = fx_or_line<N>(v);
-      }
-      fx_track(m, mx[6]);
-      __syncthreads();
-      // T' val = int 2^e (val int) 2^-57
-      const int e = eA + 2 * eV + eL - 2 * VF_FRAC + 2 * VF_LOW + fx_shift(mx[0][t]) + fx_shift(mx[1][t]) +
-                    fx_shift(mx[2][t]) + (fx_nbits(mx[3][t]) - FX_BITS) + fx_shift(mx[4][t]) + s5;
-      const bool fin = eA != FX_NAN && eV != FX_NAN && eL != FX_NAN;
-      etop = ony && fin ? e + fx_nbits(mx[6][t]) : -(1 << 28);
-      etop = max(etop, __shfl_xor_sync(0xffffffffu, etop, 1));
-      etop = max(etop, __shfl_xor_sync(0xffffffffu, etop, 2));
-      if (__any_sync(0xffffffffu, ony && !fin)) bad = true;
-      if (on1) {
-        const bool use = ony && fin;
-        vf_scale<N>(v, use ? etop - VF_FRAC - e : 0);  // |int| < 2^57
+      fx_load<N>(v, q1, n2 * P3, s5);
+      fx_dft<N>(v);
+      const int e = e0 - FX_BITS + eL + fx_shift(mx[1][t]) + fx_shift(mx[2][t]) + (fx_nbits(mx[3][t]) - FX_BITS) +
+                    fx_shift(mx[4][t]) + s5;
+      const bool fin = e0 != FX_NAN && eL != FX_NAN;
 #pragma unroll
-        for (int j = 0; j < N; ++j)
-          *reinterpret_cast<int4*>(q1 + j * n2 * P3) = use ? vf_split(v[j].x, v[j].y) : make_int4(0, 0, 0, 0);
+      for (int j = 0; j < N; ++j) {
+        double2 z = make_double2(fx_to_double(v[j].x, e), fx_to_double(v[j].y, e));
+        if (!fin) z.x = z.y = __longlong_as_double(0x7ff8000000000000ll);
+        *reinterpret_cast<double2*>(q1 + j * n2 * P3) = z;
       }
     });
     __syncthreads();
-    // B(x, v, k) += sum_y T'(y, k) val(y, v, k), exact over the tile
+    // B(x, v, k) += sum_y T'(y, k) val(y, v, k)
     const int ny = min(4, yend - y0);
 #pragma unroll
     for (int q = 0; q < MAXC; ++q) {
       const int cb = threadIdx.x + q * blockDim.x;
       if (cb < npair) {
         const int vv = cb / n23, ln = cb - vv * n23;
-        const int4* Tl = reinterpret_cast<const int4*>(buf + (ln / n3) * P3 + ln % n3);
-        const int4* Vl = p.V + ((size_t)y0 * nv + vv) * nk + ln;
+        const double2* Tl = reinterpret_cast<const double2*>(buf + (ln / n3) * P3 + ln % n3);
+        const double2* Vl = p.V + ((size_t)y0 * nv + vv) * nk + ln;
 #pragma unroll
         for (int j = 0; j < NA; ++j) {
           if (N1 == 0 && j >= n1) continue;
-          long long hp = 0, mp = 0, hn = 0, mn = 0, hi = 0, mi = 0;
-#pragma unroll
-          for (int yl = 0; yl < 4; ++yl) {  // T' of padding y is zero; its val row is read in range
-            const int4 a = Tl[yl * slab + j * n2 * P3];
-            const int4 b = __ldg(Vl + (size_t)min(yl, ny - 1) * nv * nk + j * n23);
-            mad(hp, a.x, b.x);
-            mad(hn, a.z, b.z);
-            mad(mp, a.x, b.y);
-            mad(mp, a.y, b.x);
-            mad(mn, a.z, b.w);
-            mad(mn, a.w, b.z);
-            mad(hi, a.z, b.x);
-            mad(hi, a.x, b.z);
-            mad(mi, a.z, b.y);
-            mad(mi, a.w, b.x);
-            mad(mi, a.x, b.w);
-            mad(mi, a.y, b.z);
-          }
-          const int eb = etop - 2 * VF_FRAC + VF_LOW;
           double2& d = ACS ? accs[j * npair + cb] : acc[ACS ? 0 : q][ACS ? 0 : j];
-          d.x += vf_value(hp - hn, mp - mn, eb);
-          d.y += vf_value(hi, mi, eb);
+          double2 s = d;
+#pragma unroll
+          for (int yl = 0; yl < 4; ++yl) {
+            if (yl >= ny) break;
+            const double2 a = Tl[yl * slab + j * n2 * P3];
+            const double2 b = __ldg(Vl + (size_t)yl * nv * nk + j * n23);
+            s.x = __fma_rn(a.x, b.x, s.x);
+            s.y = __fma_rn(a.y, b.x, s.y);
+            s.x = __fma_rn(-a.y, b.y, s.x);
+            s.y = __fma_rn(a.x, b.y, s.y);
+          }
+          d = s;
         }
       }
     }
@@ -326,35 +272,11 @@ __global__ void __launch_bounds__(vf_cta(N1), vf_min_ctas(N1)) k_val_ladder_fx(c
 #pragma unroll
       for (int j = 0; j < NA; ++j) {
         if (N1 == 0 && j >= n1) continue;
-        double2 o = ACS ? accs[j * npair + cb] : acc[ACS ? 0 : q][ACS ? 0 : j];
-        if (bad) o.x = o.y = __longlong_as_double(0x7ff8000000000000ll);
+        const double2 o = ACS ? accs[j * npair + cb] : acc[ACS ? 0 : q][ACS ? 0 : j];
         p.Bp[(((size_t)blockIdx.y * nk + j * n23 + ln) * nv + vv) * p.nx + x] = o;
       }
     }
   }
-}
-
-// val [k][v][y] -> split halves [y][v][k] with one exponent per y (a CTA each)
-__global__ void __launch_bounds__(256) k_vf_states(const double2* __restrict__ val, int nv, int nk, int nx,
-                                                   int4* __restrict__ V, int* __restrict__ eV) {
-  __shared__ unsigned sm;
-  const int y = blockIdx.x;
-  if (threadIdx.x == 0) sm = 0;
-  __syncthreads();
-  unsigned m = 0;
-  for (int e = threadIdx.x; e < nv * nk; e += blockDim.x) {
-    const double2 z = val[((size_t)(e % nk) * nv + e / nk) * nx + y];
-    m = max(m, max(fx_mag(z.x), fx_mag(z.y)));
-  }
-  m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0) atomicMax(&sm, m);
-  __syncthreads();
-  const int ex = fx_exp(sm);
-  for (int e = threadIdx.x; e < nv * nk; e += blockDim.x) {
-    const double2 z = val[((size_t)(e % nk) * nv + e / nk) * nx + y];
-    V[(size_t)y * nv * nk + e] = vf_split(fx_from<VF_FRAC>(z.x, ex), fx_from<VF_FRAC>(z.y, ex));
-  }
-  if (threadIdx.x == 0) eV[y] = ex;
 }
 
 // ladder rows (y, x) in place: binary64 -> ladder / Nk as 62-bit integers (a warp each)
@@ -391,7 +313,8 @@ int vf_threads(const int n[3]) {
   const int lines = std::max({n[1] * n[2], n[0] * n[2], n[0] * n[1]});
   return (4 * lines + 31) / 32 * 32;
 }
-// four bands (one pair per thread) unrolled; other counts at run time
+// Four bands (one pair per thread) unrolled; other counts at run time: the FP64 pipe bounds
+// both (6^3 k / 7^3 x: 1.29, 1.61, 3.19 ms with 2, 3, 6 bands, 1.86 with 4).
 VfFn vf_select(const int n[3], int nv) {
   if (nv == 4) return vf_fn<4, 1>(n);
   return n[1] * n[2] * nv <= vf_threads(n) ? vf_fn<0, 1>(n) : vf_fn<0, 2>(n);
@@ -420,16 +343,12 @@ cudaError_t val_fx_plan(const int kmesh[3], int nv, size_t smem_optin, int* per_
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, f, vf_threads(kmesh), vf_smem(kmesh, nv));
 }
 
-void val_fx_states(const double2* val, int nv, int nk, int nx, void* V, int* eV, cudaStream_t s) {
-  k_vf_states<<<nx, 256, 0, s>>>(val, nv, nk, nx, static_cast<int4*>(V), eV);
-}
 void val_fx_ladder(double* lad, size_t rows, int nk, int* eL, int sm_count, cudaStream_t s) {
   k_vf_ladder<<<(unsigned)std::min<size_t>((rows + 7) / 8, (size_t)16 * sm_count), 256, 0, s>>>(lad, rows, nk, eL);
 }
-void val_fx_apply(const int kmesh[3], int nv, int nx, int yper, int ysplit, const double2* A, const void* V,
-                  const int* eV, const void* lad, const int* eL, double2* Bp, cudaStream_t s) {
-  const VfParams p = {A, static_cast<const int4*>(V), eV, static_cast<const long long*>(lad), eL, Bp, nv, nx, yper,
-                      kmesh[0], kmesh[1], kmesh[2]};
+void val_fx_apply(const int kmesh[3], int nv, int nx, int yper, int ysplit, const double2* A, const double2* V,
+                  const void* lad, const int* eL, double2* Bp, cudaStream_t s) {
+  const VfParams p = {A, V, static_cast<const long long*>(lad), eL, Bp, nv, nx, yper, kmesh[0], kmesh[1], kmesh[2]};
   vf_select(kmesh, nv)<<<dim3(nx, ysplit), vf_threads(kmesh), vf_smem(kmesh, nv), s>>>(p);
 }
 

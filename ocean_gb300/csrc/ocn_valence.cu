@@ -72,9 +72,8 @@ struct ocn_val_ctx {
   float2* d_val32 = nullptr;
   void* d_valT = nullptr;     // [y][v][k], double2 or float2 (cubic kernel in FP32: val_line_at)
   void* d_lad = nullptr;      // [y][x][k], double or float
-  bool fx = false;            // FP64 direct term in fixed point: d_valT holds split halves, d_lad integers
-  int* d_eV = nullptr;        // fx: exponents of val per (spin, y) and of the ladder per (y, x)
-  int* d_eL = nullptr;
+  bool fx = false;            // FP64 direct term with fixed-point transforms: d_lad holds integers
+  int* d_eL = nullptr;        // fx: exponents of the ladder per (y, x)
   double* d_bub = nullptr;    // [x]
   double* d_fxc = nullptr;    // [x] ALDA kernel; set: the f_xc term is on (OCEAN_fxc_act)
   bool have_fxc = false;
@@ -1065,8 +1064,8 @@ int apply_impl(ocn_val_ctx* c, const double* d_in, double* d_out, const int flag
         else tw = c->d_twk;
         if (c->fx) {
           if constexpr (sizeof(R) == 8)
-            ocn::val_fx_apply(c->dims.kmesh, c->nv, c->nx, c->yper, c->ysplit, A, valT_s(sv), c->d_eV + (size_t)sv * c->nx,
-                              c->d_lad, c->d_eL, Bp + b * bp_blk, c->stream);
+            ocn::val_fx_apply(c->dims.kmesh, c->nv, c->nx, c->yper, c->ysplit, A, valT_s(sv), c->d_lad, c->d_eL,
+                              Bp + b * bp_blk, c->stream);
         } else if (use_cube_kernel(c))
           ladder_cube_fn<R>(c)<<<dim3((c->nx + c->xper - 1) / c->xper, c->ysplit), VAL_THREADS, c->lad_smem,
                                  c->stream>>>(A, valT_s(sv), static_cast<const R*>(c->d_lad), Bp + b * bp_blk, c->nv,
@@ -1178,8 +1177,7 @@ int ocn_val_create(const ocn_val_dims* d, ocn_val_ctx** out) {
                    nxk * c->nv * c->ysplit * cs * c->vspin * c->vspin)) ||
       (rc = valloc(c, &c->d_vec, 8 * c->npsi)) || (rc = valloc(c, &c->d_red, 4 * (size_t)c->red_blocks)))
     return fail(rc);
-  if (c->fx && ((rc = valloc(c, &c->d_eV, (size_t)c->nx * c->nspn)) || (rc = valloc(c, &c->d_eL, (size_t)c->nx * c->nx))))
-    return fail(rc);
+  if (c->fx && (rc = valloc(c, &c->d_eL, (size_t)c->nx * c->nx))) return fail(rc);
   if (c->mixed && ((rc = valloc(c, &c->d_con32, nxk * c->nc * c->nspn)) ||
                    (rc = valloc(c, &c->d_val32, nxk * c->nv * c->nspn))))
     return fail(rc);
@@ -1218,7 +1216,7 @@ int ocn_val_destroy(ocn_val_ctx* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   void* bufs[] = {c->d_er, c->d_ei, c->d_allow, c->d_con, c->d_val, c->d_con32, c->d_val32, c->d_valT, c->d_lad, c->d_bub,
                   c->d_fxc, c->d_twk, c->d_twk32, c->d_twx, c->d_lp, c->d_s, c->d_A, c->d_Bp, c->d_vec, c->d_red,
-                  c->d_coef, c->d_eV, c->d_eL};
+                  c->d_coef, c->d_eL};
   for (void* p : bufs)
     if (p) cudaFree(p);
   if (c->stream) cudaStreamDestroy(c->stream);
@@ -1321,10 +1319,6 @@ static int set_states_impl(ocn_val_ctx* c, const double* conr, const double* con
     kv_to_float<<<g, 256, 0, c->stream>>>(reinterpret_cast<const double*>(c->d_val), 2 * nval,
                                           reinterpret_cast<float*>(c->d_val32));
   }
-  else if (c->fx)
-    for (int sp = 0; sp < c->nspn; ++sp)
-      ocn::val_fx_states(c->d_val + sp * nval1, c->nv, c->nk, c->nx, static_cast<double2*>(c->d_valT) + sp * nval1,
-                         c->d_eV + (size_t)sp * c->nx, c->stream);
   else
     for (int sp = 0; sp < c->nspn; ++sp)
       kv_transpose_val<double><<<g, 256, 0, c->stream>>>(c->d_val + sp * nval1, c->nv, c->nk, c->nx, 0,
