@@ -104,7 +104,7 @@ int apply_H_impl(ocn_ctx* c, const double* ir, const double* ii, double* orr, do
 
 // H on a block of nv vectors (vector v at in + 2*v*npsi): the Bloch functions are
 // read once for the block in mixed precision, once per fp64_nv vectors in FP64.
-// back_each (may be NULL): the backwards switch of each vector (H or H^dagger).
+// back_each (may be NULL, mixed precision only): the backwards switch of each vector (H or H^dagger).
 int apply_H_block_impl(ocn_ctx* c, int nv, const double* in, double* out, const int* hflag_in,
                        int backwards, const int* back_each) {
   const size_t n = c->npsi;
@@ -123,14 +123,7 @@ int apply_H_block_impl(ocn_ctx* c, int nv, const double* in, double* out, const 
       double* pout = out + 2 * v0 * n;
       c->acc_valid = false;
       if ((rc = terms_fp64(c, pin, pin + n, 2 * n, w, mult_on, lr_on))) return rc;
-      if (!back_each) {
-        if ((rc = combine(c, w, pin, pin + n, pout, pout + n, 2 * n, hflag, backwards))) return rc;
-        continue;
-      }
-      for (int v = 0; v < w; ++v)
-        if ((rc = combine(c, 1, pin + 2 * v * n, pin + 2 * v * n + n, pout + 2 * v * n, pout + 2 * v * n + n, 2 * n, hflag,
-                          back_each[v0 + v], v)))
-          return rc;
+      if ((rc = combine(c, w, pin, pin + n, pout, pout + n, 2 * n, hflag, backwards))) return rc;
     }
     return OCN_OK;
   }

@@ -123,18 +123,6 @@ __global__ void k_lr_fft_w_fp64(double2* __restrict__ phi, const double* __restr
   kmesh_convolve<double>(phi, W, nx, blockIdx.x, g, buf, tw);
 }
 
-template <int N, int NTC>
-__global__ void k_fft_cube_fp64(double2* __restrict__ phi, const double* __restrict__ W, int nx, int nt,
-                                const double2* __restrict__ twg) {
-  extern __shared__ double2 smem[];
-  double2* tw = smem;
-  double2* buf = smem + 3 * OCN_MAX_KDIM;
-  for (int i = threadIdx.x; i < 3 * OCN_MAX_KDIM; i += blockDim.x) tw[i] = twg[i];
-  __syncthreads();
-  kmesh_convolve_cube<double, N, NTC>(phi, W, nx, blockIdx.x, nt, nt, buf, tw);
-}
-typedef void (*CubeFnD)(double2*, const double*, int, int, const double2*);
-
 template <int N>
 __global__ void k_wgrad_cube_fp64(const double2* __restrict__ phx, const double2* __restrict__ phy, int nx,
                                   int nt, double* __restrict__ gW, double ca, double cb,
@@ -1013,17 +1001,11 @@ int kernels_init(ocn_ctx* c) {
   const size_t g1 = sizeof(double2) * ((size_t)c->nspn * G1_N * (G1_X + 1) + (size_t)c->na * G1_N);
   const size_t ma = sizeof(double2) * (size_t)c->na * 256;
   const bool cube = kmesh_cube_supported(c->dims.kmesh);
-  const size_t ff = cube ? kmesh_cube_smem<double>(c->dims.kmesh[0], c->na)
-                         : kmesh_smem(kmesh_geom<double>(c->dims.kmesh, c->na));
+  const size_t ff = cube ? 0 : kmesh_smem(kmesh_geom<double>(c->dims.kmesh, c->na));
   if (g1 > (size_t)optin || ma > (size_t)optin || ff > (size_t)optin)
     return set_err(c, OCN_ERR_ARG, "k-mesh or nalpha too large for the shared-memory kernels");
   if (int rc_ = allow_max_smem(c, k_lr_gemm1_fp64)) return rc_;
   if (int rc_ = allow_max_smem(c, k_lr_fft_w_fp64)) return rc_;
-  if (cube) {
-    CubeFnD f;
-    OCN_CUBE_DISPATCH(k_fft_cube_fp64, c->dims.kmesh[0], c->na, f);
-    if (int rc_ = allow_max_smem(c, f)) return rc_;
-  }
   if (int rc_ = allow_max_smem(c, k_mult_amp)) return rc_;
   return OCN_OK;
 }
@@ -1076,15 +1058,10 @@ int lr_apply_fp64(ocn_ctx* c, const double* d_pr, const double* d_pi, size_t vst
     if (fx_supported(c)) {
       TimedScope ts(c, T_LR_FFT);
       if (int rc = fx_transform(c, c->d_phi, na, nullptr, nullptr)) return rc;
-    } else {
+    } else {  // an axis beyond 8
       const KmeshGeom<double> g = kmesh_geom<double>(c->dims.kmesh, na);
       TimedScope ts(c, T_LR_FFT);
-      CubeFnD f = nullptr;
-      if (kmesh_cube_supported(c->dims.kmesh)) OCN_CUBE_DISPATCH(k_fft_cube_fp64, c->dims.kmesh[0], na, f);
-      if (f)
-        f<<<nx, 128, kmesh_cube_smem<double>(c->dims.kmesh[0], na), c->stream>>>(c->d_phi, c->d_W, nx, na, c->d_tw);
-      else
-        k_lr_fft_w_fp64<<<nx, 256, kmesh_smem(g), c->stream>>>(c->d_phi, c->d_W, nx, g, c->d_tw);
+      k_lr_fft_w_fp64<<<nx, 256, kmesh_smem(g), c->stream>>>(c->d_phi, c->d_W, nx, g, c->d_tw);
       ++c->launches;
       OCN_CUDA(c, cudaGetLastError());
     }

@@ -286,108 +286,6 @@ __device__ __forceinline__ void cube_pass(typename C2<R>::T* buf, int nt_rt, int
   }
 }
 
-// nt transforms of the x-point (alpha, or (vector, alpha) for a block of psi):
-// transform t of k-point k at phi[(k*nx + x)*ld + t], ld >= nt (a CTA may own a
-// slice of the transforms of its x-point).  Leaves Nk * phi'(k) of transform t
-// in buf[t*SLAB + (k/N)*(N+1) + k%N] (not yet divided by Nk); ends with a barrier.
-template <typename R, int N, int NTC>
-__device__ void kmesh_cube_transform(const typename C2<R>::T* __restrict__ phi, const R* __restrict__ W, int nx,
-                                     int x, int nt_rt, int ld, typename C2<R>::T* buf,
-                                     const typename C2<R>::T* __restrict__ tw) {
-  typedef typename C2<R>::T CT;
-  const int nt = NTC ? NTC : nt_rt;
-  constexpr int NK = N * N * N;
-  constexpr int P3 = N + 1;
-  constexpr int SLAB = cube_slab<CT>(N);
-  // t fastest across threads: a warp reads whole 32-byte sectors of phi, and the
-  // padded slab puts neighbouring transforms on different shared-memory banks.
-  // A compile-time count keeps a plain unrollable loop (several loads in
-  // flight); a runtime count advances (k, t) incrementally instead of dividing.
-  const int dt = blockDim.x % nt, dk = blockDim.x / nt;
-  if constexpr (NTC > 0) {
-    for (int e = threadIdx.x; e < NTC * NK; e += blockDim.x) {
-      const int k = e / NTC, t = e % NTC;
-      buf[t * SLAB + (k / N) * P3 + k % N] = phi[((size_t)k * nx + x) * ld + t];
-    }
-  } else {
-    int t = threadIdx.x % nt, k = threadIdx.x / nt;
-    while (k < NK) {
-      buf[t * SLAB + (k / N) * P3 + k % N] = phi[((size_t)k * nx + x) * ld + t];
-      t += dt;
-      k += dk;
-      if (t >= nt) {
-        t -= nt;
-        ++k;
-      }
-    }
-  }
-  __syncthreads();
-#pragma unroll
-  for (int ax = 0; ax < 3; ++ax) {
-    cube_pass<R, N, NTC>(buf, nt, ax, tw + ax * OCN_MAX_KDIM, (R)1);
-    __syncthreads();
-  }
-  for (int e = threadIdx.x; e < nt * NK; e += blockDim.x) {
-    const int a = e / NK, k = e % NK;
-    const R wv = W[(size_t)x * NK + k];
-    CT& v = buf[a * SLAB + (k / N) * P3 + k % N];
-    v.x *= wv;
-    v.y *= wv;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int ax = 0; ax < 3; ++ax) {
-    cube_pass<R, N, NTC>(buf, nt, ax, tw + ax * OCN_MAX_KDIM, (R)-1);
-    __syncthreads();
-  }
-}
-
-// The transformed planes of kmesh_cube_transform, divided by Nk, back into phi.
-template <typename R, int N, int NTC>
-__device__ void kmesh_cube_store(typename C2<R>::T* __restrict__ phi, int nx, int x, int nt_rt, int ld,
-                                 const typename C2<R>::T* buf) {
-  typedef typename C2<R>::T CT;
-  const int nt = NTC ? NTC : nt_rt;
-  constexpr int NK = N * N * N;
-  constexpr int P3 = N + 1;
-  constexpr int SLAB = cube_slab<CT>(N);
-  const int dt = blockDim.x % nt, dk = blockDim.x / nt;
-  const R norm = (R)1 / (R)NK;
-  if constexpr (NTC > 0) {
-    for (int e = threadIdx.x; e < NTC * NK; e += blockDim.x) {
-      const int k = e / NTC, t = e % NTC;
-      const CT v = buf[t * SLAB + (k / N) * P3 + k % N];
-      CT o;
-      o.x = v.x * norm;
-      o.y = v.y * norm;
-      phi[((size_t)k * nx + x) * ld + t] = o;
-    }
-  } else {
-    int t = threadIdx.x % nt, k = threadIdx.x / nt;
-    while (k < NK) {
-      const CT v = buf[t * SLAB + (k / N) * P3 + k % N];
-      CT o;
-      o.x = v.x * norm;
-      o.y = v.y * norm;
-      phi[((size_t)k * nx + x) * ld + t] = o;
-      t += dt;
-      k += dk;
-      if (t >= nt) {
-        t -= nt;
-        ++k;
-      }
-    }
-  }
-}
-
-template <typename R, int N, int NTC>
-__device__ void kmesh_convolve_cube(typename C2<R>::T* __restrict__ phi, const R* __restrict__ W, int nx,
-                                    int x, int nt_rt, int ld, typename C2<R>::T* buf,
-                                    const typename C2<R>::T* __restrict__ tw) {
-  kmesh_cube_transform<R, N, NTC>(phi, W, nx, x, nt_rt, ld, buf, tw);
-  kmesh_cube_store<R, N, NTC>(phi, nx, x, nt_rt, ld, buf);
-}
-
 // dL/dW of the long-range term for the x-point of this CTA, from the band-to-x
 // results of a solution pair (phx: x, phy: the adjoint y; layout [k][x][t]):
 // both are transformed back over the k-mesh (the F_b half of the convolution),
@@ -428,7 +326,7 @@ __device__ void kmesh_wgrad_cube(const typename C2<R>::T* __restrict__ phx, cons
   }
 }
 
-// dynamic shared memory of a kmesh_convolve_cube CTA: twiddles + padded planes
+// dynamic shared memory of a CTA with nt transforms of a cube: twiddles + padded planes
 template <typename R>
 inline size_t kmesh_cube_smem(int n, int nt) {
   typedef typename C2<R>::T CT;

@@ -946,8 +946,7 @@ __global__ void k_fft_b2(const float2* __restrict__ phi, const float* __restrict
 //   D  forward DFT along k2;
 //   E  per (k2, k3, group of 4): forward DFT along k1 in registers, / Nk, and the
 //      B2 columns of the 4 transforms for the N k-points of the line.
-// The same separable transform as kmesh_cube_transform (backward = +i), with the
-// W pass and the first / last passes fused.
+// A separable transform (backward = +i) with the W pass and the first / last passes fused.
 template <int N>
 __host__ __device__ constexpr size_t fft_b2_smem_elems(int nt) {
   return 3 * OCN_MAX_KDIM + (N * N * N + 1) / 2 + (size_t)nt * cube_slab<float2>(N);

@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(VAL_THREADS, (sizeof(R) == 4 && X == 1) ? 4 : 
   // line in the B sum (saves a shared-memory pass).  Smaller N leave threads of the B sum
   // idle and redo it in the others, FP64 is FP64-pipe bound: there it stays one shared
   // pass (us per H psi, redone / pass, 8^3 x, 4 bands: N = 8 984 / 997, 6 862 / 729,
-  // 5 575 / 534, 3 232 / 217; FP64 N = 8 104 / 85 ms at 10^3 x)
+  // 5 575 / 534, 3 232 / 217)
   constexpr bool FUSE_K3 = sizeof(R) == 4 && N == 8;
   constexpr bool LINES = sizeof(R) == 4;  // val in the order of val_line_at
   extern __shared__ __align__(16) unsigned char vsm[];
@@ -877,10 +877,13 @@ using LadderCubeFn = void (*)(const typename C2<R>::T*, const typename C2<R>::T*
 template <typename R, int N>
 LadderCubeFn<R> cube_fn2(const ocn_val_ctx* c) {
   const bool one = N * N * c->nv <= VAL_THREADS;
-  if (c->xper == 2) return one ? kv_ladder_cube<R, N, 1, 2> : kv_ladder_cube<R, N, 2, 2>;
+  if constexpr (sizeof(R) == 4) {
+    if (c->xper == 2) return one ? kv_ladder_cube<R, N, 1, 2> : kv_ladder_cube<R, N, 2, 2>;
+  }
   return one ? kv_ladder_cube<R, N, 1, 1> : kv_ladder_cube<R, N, 2, 1>;
 }
 
+// (FP64: more than 8 bands, or ocn_val_fx.cu has it; with N = 8 none are left)
 template <typename R>
 LadderCubeFn<R> ladder_cube_fn(const ocn_val_ctx* c) {
   switch (c->dims.kmesh[0]) {
@@ -889,7 +892,8 @@ LadderCubeFn<R> ladder_cube_fn(const ocn_val_ctx* c) {
     case 4: return cube_fn2<R, 4>(c);
     case 5: return cube_fn2<R, 5>(c);
     case 6: return cube_fn2<R, 6>(c);
-    case 8: return cube_fn2<R, 8>(c);
+    case 8:
+      if constexpr (sizeof(R) == 4) return cube_fn2<R, 8>(c);
   }
   return nullptr;
 }
@@ -960,7 +964,7 @@ int plan_ladder(ocn_val_ctx* c) {
   // cubic kernel: in FP32 two x-points per CTA and the largest y-tile that
   // leaves two CTAs per SM (measured on the 8^3 k-mesh, 10^3 x-mesh case: 5.9 ms
   // per H psi with one x-point and 56 KB, 5.2 ms with two and 56 KB, 5.0 ms with
-  // two and 110 KB); in FP64 two x-points spill registers (85 -> 104 ms), so one
+  // two and 110 KB); in FP64 two x-points spill registers, so one
   c->xper = (use_cube_kernel(c) && c->nx >= 2 && sizeof(R) == 4) ? 2 : 1;
   const size_t target = std::min<size_t>(c->smem_optin, 110 * 1024);
   // two x-points' A must fit with at least a one-y tile, else one x-point per CTA
