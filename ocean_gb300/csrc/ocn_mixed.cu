@@ -919,6 +919,32 @@ __device__ __forceinline__ void store_b2_rows(const Get& get, float norm, __nv_b
   }
 }
 
+// B2 columns of one k-point from the four transforms of a group of 4 lanes (this lane's: re, im).
+// Lane q writes word q = (split s, part) = (q / 2, q % 2) of the group's 4 alphas at o and, for
+// c = 1, 64 columns of rows on: for Na = 4 the 4 lanes write one 32-byte row segment.  Every lane
+// splits its own transform once, packs (re, im) of the high and of the low halves in a word each,
+// and gets the other three transforms' words of its split by a 4 x 4 exchange (3 shuffles); byte
+// permutes then pick re or im, and the sign of -re is a bit flip.  (Splitting all four transforms
+// in every lane took four times the conversions: 32 -> 27 us for the 6912 transforms of the 8^3 k
+// / 12^3 x case.)  Every lane of the warp takes part; those that are not on store nothing.
+__device__ __forceinline__ void store_b2_group(float re, float im, int s, int part, bool on, __nv_bfloat16* o, int ncol) {
+  const uint32_t sel0 = part ? 0x3276u : 0x5410u;  // c = 0: re (part 0) or im (part 1) of two transforms
+  const uint32_t sel1 = part ? 0x1054u : 0x7632u;  // c = 1: im or re
+  const uint32_t flip = part ? 0x80008000u : 0u;   //        -re
+  uint32_t hw, lw;
+  split_bf16x2(re, im, hw, lw);
+  const uint32_t keep = s ? lw : hw;                                   // transform q
+  const uint32_t recv = __shfl_xor_sync(0xffffffffu, s ? hw : lw, 2);  // q ^ 2
+  const uint32_t nk = __shfl_xor_sync(0xffffffffu, keep, 1);           // q ^ 1
+  const uint32_t nr = __shfl_xor_sync(0xffffffffu, recv, 1);           // q ^ 3
+  // this lane's transform order is (own pair, neighbour): sel0/sel1 put it in ascending order
+  const uint32_t x0 = s ? recv : keep, x1 = s ? nr : nk, y0 = s ? keep : recv, y1 = s ? nk : nr;
+  if (!on) return;
+  *reinterpret_cast<uint2*>(o) = make_uint2(__byte_perm(x0, x1, sel0), __byte_perm(y0, y1, sel0));
+  *reinterpret_cast<uint2*>(o + (size_t)64 * ncol) =
+      make_uint2(__byte_perm(x0, x1, sel1) ^ flip, __byte_perm(y0, y1, sel1) ^ flip);
+}
+
 // FP32 k-mesh transform of one x-point per CTA (ocn_kmesh_dft.cuh), B2 rows out: meshes
 // with an axis beyond 8
 __global__ void k_fft_b2(const float2* __restrict__ phi, const float* __restrict__ W, int nx,
@@ -1017,21 +1043,11 @@ __device__ __forceinline__ void fft_b2_cube_body(const float2* __restrict__ phi,
   // D: forward along k2
   cube_pass<float, N, NTC>(buf, nt, 1, tw + OCN_MAX_KDIM, -1.0f);
   __syncthreads();
-  // E: forward along k1 and the B2 columns.  Lane q of a group of 4 writes word q
-  // = (split s, part) = (q / 2, q % 2) of the group's 4 alphas: for Na = 4 the 4
-  // lanes write one 32-byte row segment.  Every lane splits its own transform once,
-  // packs (re, im) of the high and of the low halves in a word each, and gets the
-  // other three transforms' words of its split s by a 4 x 4 exchange (3 shuffles); byte
-  // permutes then pick re or im, and the sign of -re is a bit flip.  (Splitting all
-  // four transforms in every lane took four times the conversions: 32 -> 27 us for
-  // the 6912 transforms of the 8^3 k / 12^3 x case.)  Every lane of the warp takes
-  // part in the shuffles (tasks is a multiple of 4; idle lanes carry zeros).
+  // E: forward along k1 and the B2 columns (store_b2_group: tasks is a multiple of 4, idle
+  // lanes carry zeros)
   const float norm = 1.0f / (float)NK;
   const int row_x = ((x >> 6) << 7) + (x & 63);
   const int lane = threadIdx.x & 31, q = lane & 3, s = q >> 1, part = q & 1;
-  const uint32_t sel0 = part ? 0x3276u : 0x5410u;  // c = 0: re (part 0) or im (part 1) of two transforms
-  const uint32_t sel1 = part ? 0x1054u : 0x7632u;  // c = 1: im or re
-  const uint32_t flip = part ? 0x80008000u : 0u;   //        -re
   for (int base = 0; base < tasks; base += blockDim.x) {
     const int task = base + threadIdx.x;
     const bool on = task < tasks;
@@ -1049,21 +1065,8 @@ __device__ __forceinline__ void fft_b2_cube_body(const float2* __restrict__ phi,
     const int tg = t0 + (t & ~3), vv = tg / na, a0 = tg - vv * na;
     __nv_bfloat16* col = b2 + (size_t)vv * 4 * na + s * 2 * na + part * na + a0;
 #pragma unroll
-    for (int k1 = 0; k1 < N; ++k1) {
-      uint32_t hw, lw;
-      split_bf16x2(v[k1].x * norm, v[k1].y * norm, hw, lw);
-      const uint32_t keep = s ? lw : hw;                                              // transform q
-      const uint32_t recv = __shfl_xor_sync(0xffffffffu, s ? hw : lw, 2);             // q ^ 2
-      const uint32_t nk = __shfl_xor_sync(0xffffffffu, keep, 1);                      // q ^ 1
-      const uint32_t nr = __shfl_xor_sync(0xffffffffu, recv, 1);                      // q ^ 3
-      // this lane's transform order is (own pair, neighbour): sel0/sel1 put it in ascending order
-      const uint32_t x0 = s ? recv : keep, x1 = s ? nr : nk, y0 = s ? keep : recv, y1 = s ? nk : nr;
-      if (!on) continue;
-      __nv_bfloat16* o = col + ((size_t)(k1 * N2 + r) * k2ext + row_x) * ncol;
-      *reinterpret_cast<uint2*>(o) = make_uint2(__byte_perm(x0, x1, sel0), __byte_perm(y0, y1, sel0));
-      *reinterpret_cast<uint2*>(o + (size_t)64 * ncol) =
-          make_uint2(__byte_perm(x0, x1, sel1) ^ flip, __byte_perm(y0, y1, sel1) ^ flip);
-    }
+    for (int k1 = 0; k1 < N; ++k1)
+      store_b2_group(v[k1].x * norm, v[k1].y * norm, s, part, on, col + ((size_t)(k1 * N2 + r) * k2ext + row_x) * ncol, ncol);
   }
 }
 template <int N, int NTC>
@@ -1188,7 +1191,6 @@ __device__ __forceinline__ void mesh_out(const float2* buf, const MeshGeom& g, i
   const float norm = 1.0f / (float)g.nk;
   const int row_x = ((x >> 6) << 7) + (x & 63);
   const int lane = threadIdx.x & 31, q = lane & 3, s = q >> 1, part = q & 1;
-  const uint32_t sel0 = part ? 0x3276u : 0x5410u, sel1 = part ? 0x1054u : 0x7632u, flip = part ? 0x80008000u : 0u;
   const int tasks = g.n1 * g.n2 * nt;
   for (int base = 0; base < tasks; base += blockDim.x) {
     const int task = base + threadIdx.x;
@@ -1202,20 +1204,8 @@ __device__ __forceinline__ void mesh_out(const float2* buf, const MeshGeom& g, i
     const int tg = t & ~3, vv = tg / na, a0 = tg - vv * na;
     __nv_bfloat16* col = b2 + ((size_t)r * N * k2ext + row_x) * ncol + (size_t)vv * 4 * na + s * 2 * na + part * na + a0;
 #pragma unroll
-    for (int j = 0; j < N; ++j) {
-      uint32_t hw, lw;
-      split_bf16x2(v[j].x * norm, v[j].y * norm, hw, lw);
-      const uint32_t keep = s ? lw : hw;
-      const uint32_t recv = __shfl_xor_sync(0xffffffffu, s ? hw : lw, 2);
-      const uint32_t nk = __shfl_xor_sync(0xffffffffu, keep, 1);
-      const uint32_t nr = __shfl_xor_sync(0xffffffffu, recv, 1);
-      const uint32_t x0 = s ? recv : keep, x1 = s ? nr : nk, y0 = s ? keep : recv, y1 = s ? nk : nr;
-      if (!on) continue;
-      __nv_bfloat16* o = col + (size_t)j * k2ext * ncol;
-      *reinterpret_cast<uint2*>(o) = make_uint2(__byte_perm(x0, x1, sel0), __byte_perm(y0, y1, sel0));
-      *reinterpret_cast<uint2*>(o + (size_t)64 * ncol) =
-          make_uint2(__byte_perm(x0, x1, sel1) ^ flip, __byte_perm(y0, y1, sel1) ^ flip);
-    }
+    for (int j = 0; j < N; ++j)
+      store_b2_group(v[j].x * norm, v[j].y * norm, s, part, on, col + (size_t)j * k2ext * ncol, ncol);
   }
 }
 
