@@ -85,9 +85,6 @@ constexpr int slice_threads(int nae) { return nae == 4 ? 192 : 320; }
 constexpr int SL_MAX_STAGES = 6;
 constexpr size_t SL_SMEM = 222 * 1024;
 constexpr int SL_MAX_K = 2730;      // K per plane and accumulation: 2 * 2730 * 12 * 256 < 2^24
-// Most products of a sum: an epilogue that forms all sums of a tile in binary64 (3072 clocks
-// a product with 12 columns) stays below half of the pipeline's time limit.
-constexpr int SL_MAX_SUM = 1 << 18;
 static_assert(OCN_MAX_NB <= SL_MAX_K, "band -> x sums 2 Nb products (re n, im n) in one accumulation");
 constexpr unsigned long long SL_BIAS = 0x0842108421084210ull;  // sum of 16 * 32^i, i < 12
 
@@ -209,7 +206,7 @@ __device__ __forceinline__ double weigh(double x, double w) {
 // terms are all small against the product of the two maxima -- row and column graded
 // oppositely -- would be less accurate than in binary64.  The epilogue bounds sum |a||b| of
 // every sum from below by 8-bit magnitudes, and the sums that the bound does not clear are
-// formed in binary64 from u and the column instead.
+// formed in binary64 from u and the column after the CTA's tiles.
 //
 // The error of a digit sum of K complex products is sqrt(2) 2^-60.8 (2^eb |a|_2 + 2^ea |b|_2)
 // (the two in quadrature; rounding of the elements) and 2^-64.8 sqrt(2 K) 2^(ea + eb) (pairs
@@ -278,7 +275,7 @@ __device__ __forceinline__ bool check_part(const SliceParams& p, int k, int rg, 
 // Second pass: all of K and the norms.  The columns (bit t: h0 + t) of this lane's row (32 rg +
 // lane) that stay open.
 template <int NAE, int AH>
-__device__ __noinline__ unsigned check_whole(const SliceParams& p, int k, int rg, int h0) {
+__device__ __forceinline__ unsigned check_whole(const SliceParams& p, int k, int rg, int h0) {
   const int lane = threadIdx.x & 31, ngrp = (p.rows + 31) / 32;
   const uint4* A = p.A8 + ((size_t)(k + p.koff) * ngrp + rg) * 2 * p.S8 * 32 + lane;
   const uint2* B = check_column<NAE, AH>(p, k, h0);
@@ -286,7 +283,7 @@ __device__ __noinline__ unsigned check_whole(const SliceParams& p, int k, int rg
   for (int c0 = 0; c0 < p.S8; c0 += 512) {  // 512 steps of 32 products below 2^16 fit in 31 bits
     int d[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
     unsigned da[4] = {0, 0, 0, 0}, db = 0;
-#pragma unroll 4
+#pragma unroll 2
     for (int st = c0; st < min(p.S8, c0 + 512); ++st) {
       const uint4 a0 = __ldg(A + (size_t)st * 32), a1 = __ldg(A + (size_t)(p.S8 + st) * 32);
       const uint2 b = __ldg(B + (size_t)st * 4);
@@ -338,27 +335,26 @@ __device__ __noinline__ unsigned check_whole(const SliceParams& p, int k, int rg
   return bits;
 }
 
-// Columns h0 .. h0 + AH - 1 of the 32 rows of a warp in binary64, those in bits (bit j: h0 + j)
-// of this lane's row (clamped to the last) stored.  All columns at once, so that an element of
-// u is read for 4 AH products, and a column's element is fetched and converted by one lane:
-// bound by the FP64 pipe.  With every x -> band sum open, 512 k / 100 bands / 8^3 x: 2.3 ms for
-// that contraction (0.12 with none; the FP64-pipe kernel 1.75), the action 2.5 ms (pipe: 3.2).
+// Columns h0 .. h0 + AH - 1 of the 32 rows of a warp in binary64; those in bits (bit j: h0 + j)
+// of this lane's row are stored.  All columns at once, so that an element of u is read for
+// 4 AH products, and a column's element is fetched and converted by one lane: bound by the
+// FP64 pipe.  (Unrolled, the code beside the tile loop cost the 12-column contraction 8 %
+// when no sum was open.)  With every x -> band sum open, 512 k / 100 bands / 8^3 x: 2.3 ms
+// for that contraction (0.12 with none; the FP64-pipe kernel 1.75), the action 2.5 ms
+// (pipe: 3.2).
 template <int MODE, int NAE, int AH>
-__device__ __noinline__ void sum_binary64(const SliceParams& p, int k, int row, int h0, unsigned bits) {
-  constexpr int NI = 32 / AH;  // products in flight: a lane holds the column element of one (i, j)
+__device__ __forceinline__ void sum_binary64(const SliceParams& p, int k, int row, int h0, unsigned bits) {
+  constexpr int NI = 32 / AH;  // a lane holds the column element of one (i, j)
   const int lane = threadIdx.x & 31, li = lane / AH, lj = lane - li * AH, r = min(row, p.rows - 1);
   const int t = h0 + lj, v = t / p.na;
   const double2* u = p.u + (size_t)k * p.uk + (MODE == 1 ? (size_t)r * p.ux : (size_t)r);
-  double2 z[AH];
+  const size_t us = MODE == 1 ? 1 : p.ux;
+  double2 z[AH], next = u[0];
 #pragma unroll
   for (int j = 0; j < AH; ++j) z[j] = make_double2(0.0, 0.0);
+#pragma unroll 1
   for (int i0 = 0; i0 < p.K; i0 += NI) {
-    double2 a[NI], b = make_double2(0.0, 0.0);
-#pragma unroll
-    for (int q = 0; q < NI; ++q) {
-      const int i = min(i0 + q, p.K - 1);
-      a[q] = u[MODE == 1 ? (size_t)i : (size_t)i * p.ux];
-    }
+    double2 b = make_double2(0.0, 0.0);
     const int i = i0 + li;
     if (li < NI && i < p.K) {
       if (MODE == 1) {
@@ -373,18 +369,19 @@ __device__ __noinline__ void sum_binary64(const SliceParams& p, int k, int row, 
         }
       }
     }
-#pragma unroll
-    for (int q = 0; q < NI; ++q) {
-      if (i0 + q >= p.K) break;
+#pragma unroll 1
+    for (int q = 0; q < min(NI, p.K - i0); ++q) {
+      const double2 a = next;
+      next = u[(size_t)min(i0 + q + 1, p.K - 1) * us];
 #pragma unroll
       for (int j = 0; j < AH; ++j) {
         const double br = __shfl_sync(0xffffffffu, b.x, q * AH + j), bi = __shfl_sync(0xffffffffu, b.y, q * AH + j);
         if (MODE == 1) {
-          z[j].x += a[q].x * br - a[q].y * bi;
-          z[j].y += a[q].x * bi + a[q].y * br;
+          z[j].x += a.x * br - a.y * bi;
+          z[j].y += a.x * bi + a.y * br;
         } else {
-          z[j].x += a[q].x * br + a[q].y * bi;
-          z[j].y += a[q].x * bi - a[q].y * br;
+          z[j].x += a.x * br + a.y * bi;
+          z[j].y += a.x * bi - a.y * br;
         }
       }
     }
@@ -400,6 +397,34 @@ __device__ __noinline__ void sum_binary64(const SliceParams& p, int k, int row, 
                     (size_t)p.nb * ((size_t)k + (size_t)p.nk * (h0 + j - vj * p.na));
       out[0] = p.negate ? -z[j].x : z[j].x;
       out[p.npsi] = p.negate ? -z[j].y : z[j].y;
+    }
+  }
+}
+
+// The sums that the second pass leaves open in a warp's row group (quadrant q4) of the tiles
+// t0 .. t1 - 1 in left (bit min(t - t0, 63)): the whole sum goes to the first split, zero to the
+// others.  The thread that stored the digits' result overwrites it.
+template <int MODE, int NAE, int AH>
+__device__ __noinline__ void redo_sums(const SliceParams& p, int t0, int t1, unsigned long long left, int q4, int h0) {
+#pragma unroll 1
+  for (int t = t0; t < t1; ++t) {
+    if (!((left >> min(t - t0, 63)) & 1ull)) continue;
+    const SliceTile ti = slice_decode<MODE>(p, t);
+    const int rg = ti.mt * (SL_ROWS / 32) + q4, row = 32 * rg + (threadIdx.x & 31);
+    if (rg * 32 >= p.rows) continue;
+    const unsigned open = check_whole<NAE, AH>(p, ti.k, rg, h0);
+    if (!__any_sync(0xffffffffu, open != 0)) continue;
+    if (ti.sp == 0) {
+      sum_binary64<MODE, NAE, AH>(p, ti.k, row, h0, open);
+      continue;
+    }
+    for (int j = 0; j < AH; ++j) {
+      if (!((open >> j) & 1u)) continue;
+      const int v = (h0 + j) / p.na;
+      double* out = p.part + (size_t)ti.sp * p.part_stride + (size_t)v * 2 * p.npsi + (size_t)row +
+                    (size_t)p.nb * ((size_t)ti.k + (size_t)p.nk * (h0 + j - v * p.na));
+      out[0] = 0.0;
+      out[p.npsi] = 0.0;
     }
   }
 }
@@ -617,16 +642,16 @@ __global__ void __launch_bounds__(slice_threads(P == 1 ? C / 2 : C), 1) k_slice_
     const int q4 = warp & 3;  // tensor-memory lane quadrant of this warp
     const int row = q4 * 32 + lane, h0 = ((warp - 2) >> 2) * AH;
     uint32_t acc = 0, acc_phase = 0;
+    unsigned long long left = 0;  // tiles that the first pass of the check does not clear, see redo_sums
     for (int t = t0; t < t1; ++t) {
       const SliceTile ti = slice_decode<MODE>(p, t);
       __syncwarp();
-      const int rg = ti.mt * (SL_ROWS / 32) + q4;
-      unsigned open = 0;  // columns (from h0) of this row that the digits are not accurate enough for
-      if (!check_part<NAE, AH>(p, ti.k, rg, h0)) open = check_whole<NAE, AH>(p, ti.k, rg, h0);
+      if (!check_part<NAE, AH>(p, ti.k, ti.mt * (SL_ROWS / 32) + q4, h0)) left |= 1ull << min(t - t0, 63);
       // every lane the same way: the loop's warp-wide steps need all of them
       if (!__all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * acc, acc_phase, abort_flag, TC_WAIT_CYCLES))) {
         *abort_flag = 1;
         atomicOr(p.err, 4);
+        left = 0;
         break;
       }
       tc_fence_after();
@@ -666,10 +691,6 @@ __global__ void __launch_bounds__(slice_threads(P == 1 ? C / 2 : C), 1) k_slice_
           double vr = fx_to_double(hi[0][j], lo[0][j], es);
           double vi = fx_to_double(hi[1][j], lo[1][j], es);
           if (ea == FX_NAN || e == FX_NAN) vr = vi = __longlong_as_double(0x7ff8000000000000ll);
-          if ((open >> j) & 1u) {  // the whole sum goes to the first split, below
-            if (MODE == 1 || ti.sp == 0) continue;
-            vr = vi = 0.0;
-          }
           if (MODE == 1) {
             p.phi[((size_t)ti.k * p.rows + r) * NAE + a] = make_double2(vr, vi);
           } else {
@@ -681,8 +702,9 @@ __global__ void __launch_bounds__(slice_threads(P == 1 ? C / 2 : C), 1) k_slice_
           }
         }
       }
-      if (__any_sync(0xffffffffu, open != 0) && ti.sp == 0) sum_binary64<MODE, NAE, AH>(p, ti.k, r, h0, open);
     }
+    // sums that the digits do not hold as well as binary64 (after the loop, out of the pipeline's waits)
+    if (left) redo_sums<MODE, NAE, AH>(p, t0, t1, left, q4, h0);
   }
   __syncthreads();
   if (warp == 1) {
@@ -1236,7 +1258,8 @@ int slice_contract(ocn_ctx* c, const SliceGemm& g, const SliceGemm& a, const uin
   p.K = g.K;
   p.S8 = g.s8();
   const double rk = std::sqrt((double)g.K);
-  p.sample = std::min(p.S8, (int)std::ceil(6.0 * rk / 32.0));  // ungraded rows: ten times the least sum
+  // ungraded rows: ten times the least sum; at most what 31 bits hold
+  p.sample = std::min({p.S8, 512, (int)std::ceil(6.0 * rk / 32.0)});
   p.least = (int)std::ceil(std::sqrt(2.0 * SL_CHECK_M * 255.0 * 255.0 + SL_CHECK_K) * rk);
   p.ux = ux;
   p.uk = uk;
@@ -1309,7 +1332,7 @@ bool slice_ready(const ocn_ctx* c) { return c->slice && c->slice->ready; }
 int slice_set_bloch(ocn_ctx* c) {
   SliceLR* s = c->slice;
   if (!s) return OCN_OK;
-  if (!(c->digits & 1) || c->nx > SL_MAX_SUM || (!s->g1[0].A && !slice_alloc_a(c, &s->g1[0], &s->g2[0], c->nx))) {
+  if (!(c->digits & 1) || (!s->g1[0].A && !slice_alloc_a(c, &s->g1[0], &s->g2[0], c->nx))) {
     slice_drop_a(c);
     return OCN_OK;
   }
