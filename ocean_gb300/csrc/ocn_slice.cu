@@ -336,8 +336,8 @@ __device__ __forceinline__ unsigned check_whole(const SliceParams& p, int k, int
 }
 
 // Columns h0 .. h0 + AH - 1 of the 32 rows of a warp in binary64; those in bits (bit j: h0 + j)
-// of this lane's row are stored.  All columns at once, so that an element of u is read for
-// 4 AH products, and a column's element is fetched and converted by one lane: bound by the
+// of this lane's row are stored.  All open columns at once, so that an element of u is read for
+// up to 4 AH products, and a column's element is fetched and converted by one lane: bound by the
 // FP64 pipe.  (Unrolled, the code beside the tile loop cost the 12-column contraction 8 %
 // when no sum was open.)  With every x -> band sum open, 512 k / 100 bands / 8^3 x: 2.3 ms
 // for that contraction (0.12 with none; the FP64-pipe kernel 1.75), the action 2.5 ms
@@ -349,6 +349,7 @@ __device__ __forceinline__ void sum_binary64(const SliceParams& p, int k, int ro
   const int t = h0 + lj, v = t / p.na;
   const double2* u = p.u + (size_t)k * p.uk + (MODE == 1 ? (size_t)r * p.ux : (size_t)r);
   const size_t us = MODE == 1 ? 1 : p.ux;
+  const unsigned any = __reduce_or_sync(0xffffffffu, bits);  // columns that no row needs are left out
   double2 z[AH], next = u[0];
 #pragma unroll
   for (int j = 0; j < AH; ++j) z[j] = make_double2(0.0, 0.0);
@@ -375,6 +376,7 @@ __device__ __forceinline__ void sum_binary64(const SliceParams& p, int k, int ro
       next = u[(size_t)min(i0 + q + 1, p.K - 1) * us];
 #pragma unroll
       for (int j = 0; j < AH; ++j) {
+        if (!((any >> j) & 1u)) continue;
         const double br = __shfl_sync(0xffffffffu, b.x, q * AH + j), bi = __shfl_sync(0xffffffffu, b.y, q * AH + j);
         if (MODE == 1) {
           z[j].x += a.x * br - a.y * bi;
