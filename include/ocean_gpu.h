@@ -53,7 +53,7 @@ enum ocn_status {
 };
 
 enum ocn_precision {
-  OCN_PREC_FP64 = 0,   /* every product and sum in FP64 (reference numerics) */
+  OCN_PREC_FP64 = 0,   /* binary64 accuracy, element by element (see ocn_set_fp64_digits) */
   OCN_PREC_MIXED = 1   /* split-BF16 tcgen05 u2 contractions with FP32 accumulation,
                           FP32 k<->R FFT, FP64 vector/Lanczos/GMRES arithmetic */
 };
@@ -214,7 +214,8 @@ int ocn_apply_H_dev(ocn_ctx* ctx, const double* d_in_r, const double* d_in_i,
                     double* d_out_r, double* d_out_i, const int* hflag, int backwards);
 
 /* H applied to nv vectors at once (host buffers: nv consecutive (Nb,Nk,Na) planes
- * each).  Mixed precision reads the Bloch functions once for the whole block. */
+ * each).  Mixed precision reads the Bloch functions once for the whole block, FP64 once for
+ * every three 1s vectors (12 columns). */
 int ocn_apply_H_block(ocn_ctx* ctx, int nv, const double* in_r, const double* in_i,
                       double* out_r, double* out_i, const int* hflag, int backwards);
 
@@ -241,7 +242,7 @@ int ocn_haydock_dev(ocn_ctx* ctx, const double* d_psi0_r, const double* d_psi0_i
  * vectors.  Each chain is exactly OCEAN_haydock_Herm_do on its own psi0.
  * psi0_r/psi0_i: nv consecutive (Nb,Nk,Na) planes (host); real_a, imag_a,
  * real_b: nv consecutive arrays of niter+1; niter_done: nv entries (may be NULL).
- * nv <= dims.nvec; the FP64 path runs the chains one after another.  Returns
+ * nv <= dims.nvec; the FP64 path runs three 1s chains (one 2p chain) at a time.  Returns
  * OCN_ERR_NAN if any chain produced a NaN a_n (its niter_done entry stops there). */
 int ocn_haydock_block(ocn_ctx* ctx, int nv, const double* psi0_r, const double* psi0_i, int niter,
                       double* real_a, double* imag_a, double* real_b, int* niter_done);
@@ -607,7 +608,9 @@ int ocn_test_starve_tc(ocn_ctx* ctx, int on);
  * multiplet contractions (bit 1) run on digit operands on the tensor cores when these
  * fit (about three times the memory of the Bloch functions on top of it, at most a quarter
  * of the device memory that is free at ocn_lr_init and ocn_set_mult), else on the FP64 pipe,
- * an order of magnitude slower on large problems and different in the last bits.
+ * an order of magnitude slower on large problems and different in the last bits.  Either way
+ * a sum is as accurate as one of binary64 products: those that the digits would hold less
+ * well (a row small where its column is large) are formed in binary64.
  * ocn_fp64_digits tells which ones do (0 in mixed precision).  ocn_set_fp64_digits
  * declines them where a bit is 0 (default 3): a run is then the same whatever else
  * holds device memory; the operands are freed or built by the call. */
