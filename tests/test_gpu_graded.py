@@ -89,6 +89,34 @@ def test_long_range(lib_built, kmesh, nb, xmesh, core_l, nspn, nv, over, decades
             assert float(np.max(err / _bound(b[s], W, psi[v, mine]))) < 4.0 * U
 
 
+def test_more_open_tiles_than_a_cta_remembers(lib_built):
+    """82 row tiles per CTA, every one with open sums: the digits' path against the FP64 pipe's,
+    whose errors add up."""
+    capi.load(lib_built)
+    kmesh, nb, xmesh = (14, 14, 16), 2, (5, 8, 10)
+    w = WL.make("tiny", seed=1, nb=nb, kmesh=kmesh, xmesh=xmesh, core_l=0, with_mult=False)
+    rng = np.random.default_rng(14)
+    gn = np.array([1.0, 1e-5])
+    u = _gauss(rng, 1, w.nx, w.nk, nb) * gn
+    w.ur, w.ui = u.real.reshape(-1).copy(), u.imag.reshape(-1).copy()
+    w.er[:] = 0.0
+    psi = _gauss(rng, w.na, w.nk, nb) / gn
+    pr, pi = psi.real.reshape(-1).copy(), psi.imag.reshape(-1).copy()
+    W = rng.uniform(0.5, 1.0, (w.nx, w.nk))
+    ctx = capi.Context(w)
+    try:
+        ctx.set_W(W.reshape(-1))
+        b = [x.reshape(w.nx, w.nk, nb) for x in ctx.get_bloch()]
+        h = []
+        for mask in (1, 0):
+            ctx.set_fp64_digits(mask)
+            r, i = ctx.apply_H(pr, pi)
+            h.append((r + 1j * i).reshape(w.na, w.nk, nb))
+    finally:
+        ctx.close()
+    assert float(np.max(np.abs(h[0] - h[1]) / _bound(b[0] + 1j * b[1], W, psi))) < 8.0 * U
+
+
 @pytest.mark.parametrize("kmesh,nb,core_l,nspn,npl", [((2, 1, 2), 33, 0, 1, 20), ((1, 1, 1), 150, 1, 2, 7)])
 @pytest.mark.parametrize("decades", [0, 3, 6])
 def test_multiplet(lib_built, kmesh, nb, core_l, nspn, npl, decades):
