@@ -242,7 +242,7 @@ __device__ __forceinline__ const uint2* check_column(const SliceParams& p, int k
 // the largest error that any row and column of K elements can have, (sum)^2 >= K (2 * 42 *
 // 255^2 + 10100).  A partial sum bounds the whole from below; ungraded rows pass about ten
 // times over, so the magnitudes are read in part (512 k / 100 bands / 12^3 x: 57 and 17 of
-// 113 and 88 MB) while the tile's digits are still on their way.  As a kernel of its own
+// 113 MB each) while the tile's digits are still on their way.  As a kernel of its own
 // after the contraction the check took 18 and 10 us and a launch each.
 template <int NAE, int AH>
 __device__ __forceinline__ bool check_part(const SliceParams& p, int k, int rg, int h0) {
